@@ -4,6 +4,7 @@
 //   * im2col_bf16    : conv input (any strides: NCHW or channels_last) -> patch matrix
 //                      [N*Ho*Wo, ld] bf16, columns ordered (kh, kw, c) or (c, kh, kw).
 #include "host_utils.h"
+#include "row_walk.h"
 #include <cuda_bf16.h>
 
 namespace b200 {
@@ -17,20 +18,103 @@ __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return
 template <>
 __device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }
 
-template <typename T>
-__global__ void cast_pad_bf16_kernel(const T* __restrict__ src, long long lds, float scale,
-                                     __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
-                                     long long ldo, long long rows, int n) {
+// [rows, n] -> PARTS bf16 matrices of pitch ldo (a multiple of eight) whose sum carries the value: hi, hi + lo, or
+// hi + mid + lo.  Columns past n are zeros.  One thread writes eight columns (16 bytes per part) of a row and walks down
+// the rows (row_walk.h) with the loads of CAST_ROWS rows in flight; VEC: the source rows are 16-byte aligned.
+// The kernel does nothing but move bytes; one element per thread with a 64-bit division each ran at 2.6 TB/s
+// (12608 x 768 fp32 -> hi, lo: 29.4 us).
+constexpr int CAST_ROWS = 2;
+template <typename T, int PARTS, bool VEC>
+__global__ void __launch_bounds__(256)
+cast_parts_kernel(const T* __restrict__ src, long long lds, float scale, __nv_bfloat16* __restrict__ p0,
+                  __nv_bfloat16* __restrict__ p1, __nv_bfloat16* __restrict__ p2, long long ldo, long long rows, int n,
+                  int groups, int lanes) {
+  const int lane = threadIdx.x / groups;
+  const long long c0 = (static_cast<long long>(blockIdx.y) * groups + threadIdx.x % groups) * 8;
+  if (lane >= lanes || c0 >= ldo) return;
+  const long long step = static_cast<long long>(gridDim.x) * lanes;
+  for (long long r = static_cast<long long>(blockIdx.x) * lanes + lane; r < rows; r += CAST_ROWS * step) {
+    float v[CAST_ROWS][8];
+#pragma unroll
+    for (int u = 0; u < CAST_ROWS; ++u) {
+      const T* from = src + (r + u * step) * lds + c0;
+      const bool row_in = r + u * step < rows;
+      if (VEC && row_in && c0 + 8 <= n) {
+        uint4 raw[sizeof(T) / 2];
+#pragma unroll
+        for (int h = 0; h < static_cast<int>(sizeof(T) / 2); ++h) raw[h] = __ldg(reinterpret_cast<const uint4*>(from) + h);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[u][k] = to_f32<T>(reinterpret_cast<const T*>(raw)[k]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[u][k] = (row_in && c0 + k < n) ? to_f32<T>(from[k]) : 0.f;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < CAST_ROWS; ++u) {
+      if (r + u * step >= rows) break;
+      uint32_t w[PARTS][4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        float a = v[u][2 * k] * scale, b = v[u][2 * k + 1] * scale;
+#pragma unroll
+        for (int part = 0; part < PARTS; ++part) {
+          const __nv_bfloat16 ha = __float2bfloat16_rn(a), hb = __float2bfloat16_rn(b);
+          w[part][k] = static_cast<uint32_t>(__bfloat16_as_ushort(ha)) | (static_cast<uint32_t>(__bfloat16_as_ushort(hb)) << 16);
+          a -= __bfloat162float(ha);
+          b -= __bfloat162float(hb);
+        }
+      }
+      const long long at = (r + u * step) * ldo + c0;
+      *reinterpret_cast<uint4*>(p0 + at) = make_uint4(w[0][0], w[0][1], w[0][2], w[0][3]);
+      if (PARTS > 1) *reinterpret_cast<uint4*>(p1 + at) = make_uint4(w[PARTS > 1][0], w[PARTS > 1][1], w[PARTS > 1][2], w[PARTS > 1][3]);
+      if (PARTS > 2)
+        *reinterpret_cast<uint4*>(p2 + at) =
+            make_uint4(w[PARTS - 1][0], w[PARTS - 1][1], w[PARTS - 1][2], w[PARTS - 1][3]);
+    }
+  }
+}
+
+// The same for outputs whose rows are not 16-byte aligned: one element per thread.
+template <typename T, int PARTS>
+__global__ void cast_parts_scalar_kernel(const T* __restrict__ src, long long lds, float scale,
+                                         __nv_bfloat16* __restrict__ p0, __nv_bfloat16* __restrict__ p1,
+                                         __nv_bfloat16* __restrict__ p2, long long ldo, long long rows, int n) {
   const long long total = rows * ldo;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const long long r = i / ldo;
     const int c = static_cast<int>(i - r * ldo);
     float v = (c < n) ? to_f32<T>(src[r * lds + c]) * scale : 0.f;
-    __nv_bfloat16 h = __float2bfloat16_rn(v);
-    hi[i] = h;
-    if (lo != nullptr) lo[i] = __float2bfloat16_rn(v - __bfloat162float(h));
+    __nv_bfloat16* const parts[3] = {p0, p1, p2};
+#pragma unroll
+    for (int part = 0; part < PARTS; ++part) {
+      const __nv_bfloat16 h = __float2bfloat16_rn(v);
+      parts[part][i] = h;
+      v -= __bfloat162float(h);
+    }
   }
+}
+
+template <typename T, int PARTS>
+void launch_cast(const T* src, long long lds, float scale, __nv_bfloat16* p0, __nv_bfloat16* p1, __nv_bfloat16* p2,
+                 long long ldo, long long rows, int n, cudaStream_t stream) {
+  const uintptr_t outs = reinterpret_cast<uintptr_t>(p0) | (PARTS > 1 ? reinterpret_cast<uintptr_t>(p1) : 0) |
+                         (PARTS > 2 ? reinterpret_cast<uintptr_t>(p2) : 0);
+  if ((ldo & 7) != 0 || (outs & 15) != 0) {
+    const int blocks = static_cast<int>(std::min<long long>((rows * ldo + 255) / 256, 148 * 16));
+    cast_parts_scalar_kernel<T, PARTS><<<blocks, 256, 0, stream>>>(src, lds, scale, p0, p1, p2, ldo, rows, n);
+  } else {
+    const Walk w = walk_plan(static_cast<int>(ldo / 8));
+    const dim3 grid = walk_grid(w, rows, 6);
+    const bool vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && (lds * sizeof(T)) % 16 == 0;
+    if (vec)
+      cast_parts_kernel<T, PARTS, true><<<grid, 256, 0, stream>>>(src, lds, scale, p0, p1, p2, ldo, rows, n, w.groups, w.lanes);
+    else
+      cast_parts_kernel<T, PARTS, false><<<grid, 256, 0, stream>>>(src, lds, scale, p0, p1, p2, ldo, rows, n, w.groups, w.lanes);
+  }
+  B200_CUDA_CHECK(cudaGetLastError());
+  count_launch();
 }
 
 void cast_pad_bf16(at::Tensor src, at::Tensor hi, c10::optional<at::Tensor> lo, double scale) {
@@ -50,49 +134,29 @@ void cast_pad_bf16(at::Tensor src, at::Tensor hi, c10::optional<at::Tensor> lo, 
   const long long ldo = hi.size(1);
   const long long total = rows * ldo;
   if (total == 0) return;
-  const int threads = 256;
-  const int blocks = static_cast<int>(std::min<long long>((total + threads - 1) / threads, 148 * 16));
   auto stream = at::cuda::getCurrentCUDAStream().stream();
   auto* hi_p = reinterpret_cast<__nv_bfloat16*>(hi.data_ptr());
-  if (src.scalar_type() == at::kFloat) {
-    cast_pad_bf16_kernel<float><<<blocks, threads, 0, stream>>>(
-        src.data_ptr<float>(), src.stride(0), static_cast<float>(scale), hi_p, lo_p, ldo, rows, n);
-  } else if (src.scalar_type() == at::kBFloat16) {
-    cast_pad_bf16_kernel<__nv_bfloat16><<<blocks, threads, 0, stream>>>(
-        reinterpret_cast<const __nv_bfloat16*>(src.data_ptr()), src.stride(0),
-        static_cast<float>(scale), hi_p, lo_p, ldo, rows, n);
-  } else if (src.scalar_type() == at::kHalf) {
-    cast_pad_bf16_kernel<__half><<<blocks, threads, 0, stream>>>(
-        reinterpret_cast<const __half*>(src.data_ptr()), src.stride(0), static_cast<float>(scale),
-        hi_p, lo_p, ldo, rows, n);
-  } else {
+  const float s = static_cast<float>(scale);
+  auto run = [&](auto* from) {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(from)>>;
+    if (lo_p != nullptr)
+      launch_cast<T, 2>(from, src.stride(0), s, hi_p, lo_p, nullptr, ldo, rows, n, stream);
+    else
+      launch_cast<T, 1>(from, src.stride(0), s, hi_p, nullptr, nullptr, ldo, rows, n, stream);
+  };
+  if (src.scalar_type() == at::kFloat)
+    run(static_cast<const float*>(src.data_ptr<float>()));
+  else if (src.scalar_type() == at::kBFloat16)
+    run(reinterpret_cast<const __nv_bfloat16*>(src.data_ptr()));
+  else if (src.scalar_type() == at::kHalf)
+    run(reinterpret_cast<const __half*>(src.data_ptr()));
+  else
     TORCH_CHECK(false, "unsupported source dtype");
-  }
-  B200_CUDA_CHECK(cudaGetLastError());
-  count_launch();
 }
 
 // Three-way split of an fp32 matrix: v = hi + mid + lo with every part a bf16 number, which carries
 // the full 24-bit significand of v.  Six tensor-core products of such parts (hi*hi, hi*mid, mid*hi,
 // hi*lo, mid*mid, lo*hi) reproduce an fp32 product to ~2^-24.
-__global__ void cast_split3_kernel(const float* __restrict__ src, long long lds, __nv_bfloat16* __restrict__ hi,
-                                   __nv_bfloat16* __restrict__ mid, __nv_bfloat16* __restrict__ lo,
-                                   long long ldo, long long rows, int n) {
-  const long long total = rows * ldo;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long r = i / ldo;
-    const int c = static_cast<int>(i - r * ldo);
-    const float v = (c < n) ? src[r * lds + c] : 0.f;
-    const __nv_bfloat16 h = __float2bfloat16_rn(v);
-    const float r1 = v - __bfloat162float(h);
-    const __nv_bfloat16 m = __float2bfloat16_rn(r1);
-    hi[i] = h;
-    mid[i] = m;
-    lo[i] = __float2bfloat16_rn(r1 - __bfloat162float(m));
-  }
-}
-
 void cast_split3(at::Tensor src, at::Tensor hi, at::Tensor mid, at::Tensor lo) {
   TORCH_CHECK(src.is_cuda() && src.dim() == 2 && src.stride(1) == 1 && src.scalar_type() == at::kFloat,
               "src must be a 2-D fp32 CUDA tensor with unit column stride");
@@ -105,14 +169,9 @@ void cast_split3(at::Tensor src, at::Tensor hi, at::Tensor mid, at::Tensor lo) {
   const long long ldo = hi.size(1);
   if (rows == 0) return;
   auto stream = at::cuda::getCurrentCUDAStream().stream();
-  const long long total = rows * ldo;
-  const int blocks = static_cast<int>(std::min<long long>((total + 255) / 256, 148LL * 16));
-  cast_split3_kernel<<<blocks, 256, 0, stream>>>(
-      src.data_ptr<float>(), src.stride(0), reinterpret_cast<__nv_bfloat16*>(hi.data_ptr()),
-      reinterpret_cast<__nv_bfloat16*>(mid.data_ptr()), reinterpret_cast<__nv_bfloat16*>(lo.data_ptr()), ldo, rows,
-      static_cast<int>(src.size(1)));
-  B200_CUDA_CHECK(cudaGetLastError());
-  count_launch();
+  launch_cast<float, 3>(src.data_ptr<float>(), src.stride(0), 1.f, reinterpret_cast<__nv_bfloat16*>(hi.data_ptr()),
+                        reinterpret_cast<__nv_bfloat16*>(mid.data_ptr()), reinterpret_cast<__nv_bfloat16*>(lo.data_ptr()),
+                        ldo, rows, static_cast<int>(src.size(1)), stream);
 }
 
 // Grouped fp32 -> bf16 hi/lo staging: one launch converts many matrices.  Each table row holds
@@ -279,32 +338,149 @@ __global__ void im2col_generic_kernel(const T* __restrict__ x, __nv_bfloat16* __
   }
 }
 
-// Vector path: channels_last bf16 input, C % 8 == 0, (kh, kw, c) column order.  One thread moves
-// 8 channels (16 bytes) of one tap of one output pixel.
-__global__ void im2col_nhwc_vec8_kernel(const __nv_bfloat16* __restrict__ x,
-                                        __nv_bfloat16* __restrict__ out, Im2colParams p) {
-  const int c8n = p.C >> 3;
-  const int taps = p.KH * p.KW;
-  const long long rows = static_cast<long long>(p.N) * p.Ho * p.Wo;
-  const long long total = rows * taps * c8n;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int c8 = static_cast<int>(i % c8n);
-    const long long t = i / c8n;
-    const int tap = static_cast<int>(t % taps);
-    const long long r = t / taps;
-    const int kh = tap / p.KW, kw = tap - kh * p.KW;
-    const int wo = static_cast<int>(r % p.Wo);
-    const long long t2 = r / p.Wo;
-    const int ho = static_cast<int>(t2 % p.Ho);
-    const int n = static_cast<int>(t2 / p.Ho);
-    const int hi = ho * p.SH - p.PH + kh * p.DH;
-    const int wi = wo * p.SW - p.PW + kw * p.DW;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (hi >= 0 && hi < p.H && wi >= 0 && wi < p.W)
-      v = *reinterpret_cast<const uint4*>(x + n * p.sN + hi * p.sH + wi * p.sW + c8 * 8);
-    *reinterpret_cast<uint4*>(out + r * p.ldo + static_cast<long long>(tap) * p.C + c8 * 8) = v;
+// Output pixel -> (image, row, column), 32-bit (the host checks that the rows fit).
+__device__ __forceinline__ void im2col_pixel(const Im2colParams& p, unsigned r, int& n, int& ho, int& wo) {
+  const unsigned t = r / static_cast<unsigned>(p.Wo);
+  wo = static_cast<int>(r - t * p.Wo);
+  n = static_cast<int>(t / static_cast<unsigned>(p.Ho));
+  ho = static_cast<int>(t - static_cast<unsigned>(n) * p.Ho);
+}
+
+// Vector path: channels_last bf16 input, C % 8 == 0, (kh, kw, c) column order.  One thread owns 8 channels (16 bytes)
+// of one tap and walks down the output pixels (row_walk.h) with the loads of four in flight: the write of the patch
+// matrix bounds it (14 x 14 x 256 channels, 32 images, 3 x 3: 28.9 MB).
+__global__ void __launch_bounds__(256)
+im2col_nhwc_vec8_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ out, Im2colParams p,
+                        unsigned rows, int groups, int lanes) {
+  constexpr int U = 4;
+  const int c8n = p.C >> 3, lane = threadIdx.x / groups;
+  const int v = blockIdx.y * groups + threadIdx.x % groups;
+  if (lane >= lanes || v >= p.KH * p.KW * c8n) return;
+  const int tap = v / c8n, c8 = v - tap * c8n;
+  const int dh = (tap / p.KW) * p.DH - p.PH, dw = (tap % p.KW) * p.DW - p.PW;
+  const __nv_bfloat16* base = x + c8 * 8;
+  const unsigned step = gridDim.x * lanes;
+  for (unsigned long long r = static_cast<unsigned long long>(blockIdx.x) * lanes + lane; r < rows;
+       r += static_cast<unsigned long long>(U) * step) {
+    uint4 val[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      val[u] = make_uint4(0, 0, 0, 0);
+      const unsigned long long ru = r + static_cast<unsigned long long>(u) * step;
+      if (ru < rows) {
+        int n, ho, wo;
+        im2col_pixel(p, static_cast<unsigned>(ru), n, ho, wo);
+        const int hi = ho * p.SH + dh, wi = wo * p.SW + dw;
+        if (hi >= 0 && hi < p.H && wi >= 0 && wi < p.W)
+          val[u] = __ldg(reinterpret_cast<const uint4*>(base + n * p.sN + hi * p.sH + wi * p.sW));
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const unsigned long long ru = r + static_cast<unsigned long long>(u) * step;
+      if (ru < rows) *reinterpret_cast<uint4*>(out + ru * p.ldo + static_cast<long long>(v) * 8) = val[u];
+    }
   }
+}
+
+// Tile path (any dtype and strides): a CTA stages the input rows that one output row and `cc` channels need in shared
+// memory, then every thread assembles eight consecutive columns of a patch from there (a table in shared memory maps
+// column -> staged element) and writes 16 bytes per part.  Input is read once per filter row and coalesced along W (or
+// along C for channels-innermost strides); what remains is the write of the patch matrix.  The element-wise kernel
+// spent 497 us on 128 x 64 x 32 x 32 fp32, 3 x 3 (302 MB of patches) in index divisions, 2-byte stores and strided reads.
+// grid: (N * Ho, channel chunks).  c_major columns of a chunk are contiguous; (kh, kw, c) order needs all channels.
+template <typename T, bool LO>
+__global__ void __launch_bounds__(256)
+im2col_tile_kernel(const T* __restrict__ x, __nv_bfloat16* __restrict__ out, __nv_bfloat16* __restrict__ out_lo,
+                   Im2colParams p, int cc, int wp) {
+  extern __shared__ float4 im2col_smem[];
+  float* tile = reinterpret_cast<float*>(im2col_smem);   // [cc][KH][wp], then a zero, then the column table
+  const int taps = p.KH * p.KW, c_begin = blockIdx.y * cc, nc = min(cc, p.C - c_begin);
+  const int elems = cc * p.KH * wp, cols = nc * taps;
+  const bool last = c_begin + nc == p.C;
+  const long long col0 = static_cast<long long>(c_begin) * taps;
+  const int width = last ? static_cast<int>(p.ldo - col0) : cols;   // with the zero padding of the row pitch
+  unsigned short* table = reinterpret_cast<unsigned short*>(tile + (elems + 4) / 4 * 4);
+  const int n = blockIdx.x / p.Ho, ho = blockIdx.x - n * p.Ho;
+  for (int col = threadIdx.x; col < width; col += 256) {
+    int at = elems;   // the zero element: padding columns
+    if (col < cols) {
+      const int c = p.c_major ? col / taps : col % p.C, t = p.c_major ? col - c * taps : col / p.C;
+      at = (c * p.KH + t / p.KW) * wp + (t % p.KW) * p.DW;
+    }
+    table[col] = static_cast<unsigned short>(at);
+  }
+  // the zero and what an output pixel past a padding column may address behind it
+  for (int e = elems + threadIdx.x; e < (elems + 4) / 4 * 4; e += 256) tile[e] = 0.f;
+  const T* base = x + n * p.sN + c_begin * p.sC;
+  const int h0 = ho * p.SH - p.PH, live = nc * p.KH * wp;
+  for (int e = threadIdx.x; e < live; e += 256) {
+    int c, kh, w;
+    if (p.sC == 1) {
+      c = e % nc;
+      const int t = e / nc;
+      w = t % wp;
+      kh = t / wp;
+    } else {
+      w = e % wp;
+      const int t = e / wp;
+      kh = t % p.KH;
+      c = t / p.KH;
+    }
+    const int hi = h0 + kh * p.DH, wi = w - p.PW;
+    tile[(c * p.KH + kh) * wp + w] =
+        (hi >= 0 && hi < p.H && wi >= 0 && wi < p.W) ? to_f32<T>(base[c * p.sC + hi * p.sH + wi * p.sW]) : 0.f;
+  }
+  __syncthreads();
+  const int vecs = width / 8, total = vecs * p.Wo;
+  __nv_bfloat16* const row0 = out + static_cast<long long>(blockIdx.x) * p.Wo * p.ldo + col0;
+  __nv_bfloat16* const lo0 = LO ? out_lo + static_cast<long long>(blockIdx.x) * p.Wo * p.ldo + col0 : nullptr;
+  for (int e = threadIdx.x; e < total; e += 256) {
+    const int wo = e / vecs, v = e - wo * vecs, shift = wo * p.SW;
+    const uint4 raw = *reinterpret_cast<const uint4*>(table + v * 8);
+    const uint32_t pairs[4] = {raw.x, raw.y, raw.z, raw.w};
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i0 = pairs[k] & 0xffffu, i1 = pairs[k] >> 16;
+      const float a = tile[i0 == elems ? elems : i0 + shift], b = tile[i1 == elems ? elems : i1 + shift];
+      const __nv_bfloat16 ha = __float2bfloat16_rn(a), hb = __float2bfloat16_rn(b);
+      hi[k] = static_cast<uint32_t>(__bfloat16_as_ushort(ha)) | (static_cast<uint32_t>(__bfloat16_as_ushort(hb)) << 16);
+      if (LO)
+        lo[k] = static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(a - __bfloat162float(ha)))) |
+                (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(b - __bfloat162float(hb)))) << 16);
+    }
+    const long long at = static_cast<long long>(wo) * p.ldo + v * 8;
+    *reinterpret_cast<uint4*>(row0 + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    if (LO) *reinterpret_cast<uint4*>(lo0 + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  }
+}
+
+// Channels per CTA of the tile path, 0 if it does not apply: the staged rows and the column table fit `IM2COL_SMEM`,
+// every element has a 16-bit index, and each chunk starts on a multiple of eight columns.
+constexpr int IM2COL_SMEM = 44 * 1024;
+struct Im2colTile {
+  int cc, wp, smem;
+};
+Im2colTile im2col_tile_plan(const Im2colParams& p) {
+  const long long taps = static_cast<long long>(p.KH) * p.KW;
+  const long long wp = (static_cast<long long>(p.Wo - 1) * p.SW + static_cast<long long>(p.KW - 1) * p.DW + 1) | 1;
+  auto smem = [&](long long cc) {
+    return ((cc * p.KH * wp + 4) / 4 * 4) * 4 + (cc * taps + 8) * 2 + (p.ldo - static_cast<long long>(p.C) * taps) * 2;
+  };
+  auto fits = [&](long long cc) { return smem(cc) <= IM2COL_SMEM && cc * p.KH * wp < 65535; };
+  if (p.ldo % 8 != 0 || static_cast<long long>(p.N) * p.Ho >= (1ll << 31)) return {0, 0, 0};
+  long long cc = p.C;
+  if (!fits(cc)) {
+    if (!p.c_major) return {0, 0, 0};
+    cc = p.C / 8 * 8;
+    while (cc > 0 && !fits(cc)) cc -= 8;
+    if (cc <= 0) return {0, 0, 0};
+    const long long chunks = (p.C + cc - 1) / cc;             // equal chunks
+    cc = ((p.C + chunks - 1) / chunks + 7) / 8 * 8;
+  }
+  if ((p.C + cc - 1) / cc > 65535) return {0, 0, 0};
+  return {static_cast<int>(cc), static_cast<int>(wp), static_cast<int>(smem(cc))};
 }
 
 // x: 4-D conv input [N, C, H, W] (logical), any memory format.  out: [N*Ho*Wo, ld] bf16, contiguous.
@@ -336,30 +512,38 @@ void im2col_bf16(at::Tensor x, at::Tensor out, c10::optional<at::Tensor> out_lo,
                     out_lo->scalar_type() == at::kBFloat16, "out_lo must match out");
     lo_p = reinterpret_cast<__nv_bfloat16*>(out_lo->data_ptr());
   }
-  const int threads = 256;
   // with a single filter tap the (c, kh, kw) and (kh, kw, c) column orders are the same
   const bool vec = lo_p == nullptr && (!c_major || p.KH * p.KW == 1) && x.scalar_type() == at::kBFloat16 && p.sC == 1 && (p.C % 8) == 0 &&
                    p.ldo == static_cast<long long>(p.C) * p.KH * p.KW && (p.sW % 8) == 0 &&
-                   (p.sH % 8) == 0 && (p.sN % 8) == 0 &&
-                   (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0;
+                   (p.sH % 8) == 0 && (p.sN % 8) == 0 && rows < (1ll << 32) &&
+                   ((reinterpret_cast<uintptr_t>(x.data_ptr()) | reinterpret_cast<uintptr_t>(out_p)) & 15) == 0;
+  const bool aligned = ((reinterpret_cast<uintptr_t>(out_p) | reinterpret_cast<uintptr_t>(lo_p)) & 15) == 0;
+  const Im2colTile tile = (vec || !aligned) ? Im2colTile{0, 0, 0} : im2col_tile_plan(p);
+  auto run = [&](auto* from) {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(from)>>;
+    if (tile.cc > 0) {
+      const dim3 grid(static_cast<unsigned>(static_cast<long long>(p.N) * p.Ho), (p.C + tile.cc - 1) / tile.cc);
+      if (lo_p != nullptr)
+        im2col_tile_kernel<T, true><<<grid, 256, tile.smem, stream>>>(from, out_p, lo_p, p, tile.cc, tile.wp);
+      else
+        im2col_tile_kernel<T, false><<<grid, 256, tile.smem, stream>>>(from, out_p, nullptr, p, tile.cc, tile.wp);
+    } else {
+      const int blocks = static_cast<int>(std::min<long long>((rows * p.ldo + 255) / 256, 148 * 32));
+      im2col_generic_kernel<T><<<blocks, 256, 0, stream>>>(from, out_p, lo_p, p);
+    }
+  };
   if (vec) {
-    const long long total = rows * p.KH * p.KW * (p.C >> 3);
-    const int blocks = static_cast<int>(std::min<long long>((total + threads - 1) / threads, 148 * 32));
-    im2col_nhwc_vec8_kernel<<<blocks, threads, 0, stream>>>(
-        reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), out_p, p);
+    const Walk w = walk_plan(p.KH * p.KW * (p.C >> 3));
+    im2col_nhwc_vec8_kernel<<<walk_grid(w, (rows + 3) / 4, 8), 256, 0, stream>>>(
+        reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), out_p, p, static_cast<unsigned>(rows), w.groups, w.lanes);
+  } else if (x.scalar_type() == at::kFloat) {
+    run(static_cast<const float*>(x.data_ptr<float>()));
+  } else if (x.scalar_type() == at::kBFloat16) {
+    run(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()));
+  } else if (x.scalar_type() == at::kHalf) {
+    run(reinterpret_cast<const __half*>(x.data_ptr()));
   } else {
-    const long long total = rows * p.ldo;
-    const int blocks = static_cast<int>(std::min<long long>((total + threads - 1) / threads, 148 * 32));
-    if (x.scalar_type() == at::kFloat)
-      im2col_generic_kernel<float><<<blocks, threads, 0, stream>>>(x.data_ptr<float>(), out_p, lo_p, p);
-    else if (x.scalar_type() == at::kBFloat16)
-      im2col_generic_kernel<__nv_bfloat16><<<blocks, threads, 0, stream>>>(
-          reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), out_p, lo_p, p);
-    else if (x.scalar_type() == at::kHalf)
-      im2col_generic_kernel<__half><<<blocks, threads, 0, stream>>>(
-          reinterpret_cast<const __half*>(x.data_ptr()), out_p, lo_p, p);
-    else
-      TORCH_CHECK(false, "unsupported input dtype");
+    TORCH_CHECK(false, "unsupported input dtype");
   }
   B200_CUDA_CHECK(cudaGetLastError());
   count_launch();
