@@ -90,9 +90,9 @@ void g2_launch_reduce_list(const GemmProblem2* d_probs, const GemmWork2* d_work,
   GemmProblem2 dummy;
   std::memset(&dummy, 0, sizeof(dummy));
   if (wide)
-    splitk_reduce2_kernel<256><<<dim3(n_work, 32, 1), 256, 0, stream>>>(dummy, d_probs, d_work, nullptr, 0);
+    splitk_reduce2_kernel<256><<<dim3(n_work, g2_reduce_patches<256>(), 1), 256, 0, stream>>>(dummy, d_probs, d_work, nullptr, 0);
   else
-    splitk_reduce2_kernel<128><<<dim3(n_work, 16, 1), 256, 0, stream>>>(dummy, d_probs, d_work, nullptr, 0);
+    splitk_reduce2_kernel<128><<<dim3(n_work, g2_reduce_patches<128>(), 1), 256, 0, stream>>>(dummy, d_probs, d_work, nullptr, 0);
   B200_CUDA_CHECK(cudaGetLastError());
   count_launch();
 }
@@ -246,9 +246,9 @@ void gemm_launch_single(const GemmProblem2& P, int dev, cudaStream_t stream) {
     g2_run_plain(P, nullptr, nullptr, n_work, n_sms, stream);
   if (needs_ws(P)) {
     if (wide)
-      splitk_reduce2_kernel<256><<<dim3(P.ntiles, 32, 1), 256, 0, stream>>>(P, nullptr, nullptr, nullptr, 0);
+      splitk_reduce2_kernel<256><<<dim3(P.ntiles, g2_reduce_patches<256>(), 1), 256, 0, stream>>>(P, nullptr, nullptr, nullptr, 0);
     else
-      splitk_reduce2_kernel<128><<<dim3(P.ntiles, 16, 1), 256, 0, stream>>>(P, nullptr, nullptr, nullptr, 0);
+      splitk_reduce2_kernel<128><<<dim3(P.ntiles, g2_reduce_patches<128>(), 1), 256, 0, stream>>>(P, nullptr, nullptr, nullptr, 0);
     B200_CUDA_CHECK(cudaGetLastError());
     count_launch();
   }
@@ -355,7 +355,7 @@ static void batch_flush(cudaStream_t stream) {
     const GemmProblem2* dp = reinterpret_cast<const GemmProblem2*>(d);
     g2_run_plain(dummy, dp, nullptr, items, n_sms, stream, reinterpret_cast<const int*>(d + probs_bytes), n);
     if (rtiles > 0) {
-      splitk_reduce2_kernel<128><<<dim3(rtiles, 16, 1), 256, 0, stream>>>(
+      splitk_reduce2_kernel<128><<<dim3(rtiles, g2_reduce_patches<128>(), 1), 256, 0, stream>>>(
           dummy, dp, nullptr, reinterpret_cast<const int*>(d + probs_bytes + prefix_bytes), n);
       B200_CUDA_CHECK(cudaGetLastError());
       count_launch();

@@ -828,14 +828,21 @@ umma_gemm2_kernel(const __grid_constant__ GemmProblem2 single, const GemmProblem
   }
 }
 
-// Sums split-K partials and applies the epilogue.  One block handles a 32x32 patch of one tile:
-// reads and direct stores are 128-byte coalesced, the mirrored store goes through shared memory.
-// grid: (work items, 4 * BN / 32).
+// Sums split-K partials and applies the epilogue.  One block handles a 32 x 64 patch of one tile; a thread owns four
+// consecutive columns of two rows, so the partials of four splits are eight 16-byte loads in flight (the kernel reads
+// nsplit times what it writes and does nothing else; with 4-byte loads of one split at a time it ran at 1.3 TB/s).  The
+// mirrored store goes through shared memory.  Partials are added in split order.
+// grid: (work items, 4 * BN / 64).
+constexpr int G2_RED_ROWS = 32, G2_RED_COLS = 64;
+template <int BN>
+constexpr int g2_reduce_patches() {
+  return (G2_BM / G2_RED_ROWS) * (BN / G2_RED_COLS);
+}
 template <int BN>
 __global__ void __launch_bounds__(256)
 splitk_reduce2_kernel(const __grid_constant__ GemmProblem2 single, const GemmProblem2* __restrict__ probs,
                       const GemmWork2* __restrict__ work, const int* __restrict__ tile_prefix, int n_probs) {
-  __shared__ float tile[32][33];
+  __shared__ float tile[G2_RED_ROWS][G2_RED_COLS + 1];
   GemmWork2 w;
   const GemmProblem2* Pp;
   if (work != nullptr) {
@@ -859,97 +866,147 @@ splitk_reduce2_kernel(const __grid_constant__ GemmProblem2 single, const GemmPro
   }
   const G2Epi P = g2_epi(*Pp);
   const bool sym = (P.flags & G2F_SYM) != 0;
-  constexpr int PC = BN / 32;  // patches per tile row
+  constexpr int PC = BN / G2_RED_COLS;  // patches per tile row
   const int sub_r = blockIdx.y / PC, sub_c = blockIdx.y % PC;
+  const int row0 = w.c_row + sub_r * G2_RED_ROWS, col0 = w.c_col + sub_c * G2_RED_COLS;
   const int tm = w.c_row / G2_BM;
-  const int cb = (w.c_col + sub_c * 32) / G2_BM;  // 128-wide column block of this patch
+  const int cb = col0 / G2_BM;  // 128-wide column block of this patch
   if (sym && cb > tm) return;
   const bool diag_tile = sym && cb == tm;
-  if (diag_tile && (w.c_col + sub_c * 32) > (w.c_row + sub_r * 32)) return;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  if (diag_tile && col0 > row0 + G2_RED_ROWS - 1) return;
   // patches that lie completely outside the matrix (edge tiles of small problems) have no work
-  if (w.c_row + sub_r * 32 >= P.M || w.c_col + sub_c * 32 >= P.N) return;
-  const float* base = P.ws + static_cast<size_t>(w.tile_id) * P.nsplit * (G2_BM * BN);
-  const int gc = w.c_col + sub_c * 32 + tx;
-  // sum the partials in split order; the loads of the four rows of a thread and of four splits are
-  // issued together (16 independent loads in flight per thread)
-  float accs[4] = {0.f, 0.f, 0.f, 0.f};
-  {
-    const float* p0 = base + static_cast<size_t>(sub_r * 32 + ty) * BN + sub_c * 32 + tx;
-    int s = 0;
-    for (; s + 4 <= P.nsplit; s += 4) {
-      float v[4][4];
+  if (row0 >= P.M || col0 >= P.N) return;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  constexpr size_t SPLIT = static_cast<size_t>(G2_BM) * BN;   // floats of one split's partial tile
+  const float* p0 = P.ws + static_cast<size_t>(w.tile_id) * P.nsplit * SPLIT +
+                    static_cast<size_t>(sub_r * G2_RED_ROWS + ty) * BN + sub_c * G2_RED_COLS + tx * 4;
+  const int gc = col0 + tx * 4;
+  const bool full = gc + 4 <= P.N;
+  const bool vec_in = full && g2_vec_ok(P.Cin, P.ldc), vec_out = full && g2_vec_ok(P.C, P.ldc);
+  float cin[2][4];
+  if (P.beta != 0.f) {   // issued ahead of the partials
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 2; ++i) {
+      const int gr = row0 + ty + 16 * i;
+      const float* c = P.Cin + static_cast<size_t>(gr) * P.ldc + gc;
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          v[i][u] = __ldcg(p0 + static_cast<size_t>(8 * i) * BN + static_cast<size_t>(s + u) * (G2_BM * BN));
+      for (int j = 0; j < 4; ++j) cin[i][j] = 0.f;
+      if (gr < P.M) {
+        if (vec_in) {
+          const float4 v = *reinterpret_cast<const float4*>(c);
+          cin[i][0] = v.x;
+          cin[i][1] = v.y;
+          cin[i][2] = v.z;
+          cin[i][3] = v.w;
+        } else {
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int u = 0; u < 4; ++u) accs[i] += v[i][u];
+          for (int j = 0; j < 4; ++j)
+            if (gc + j < P.N) cin[i][j] = c[j];
+        }
+      }
     }
-    for (; s < P.nsplit; ++s)
+  }
+  float acc[2][4] = {};
+  for (int s = 0; s < P.nsplit; s += 4) {
+    float4 v[2][4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        accs[i] += __ldcg(p0 + static_cast<size_t>(8 * i) * BN + static_cast<size_t>(s) * (G2_BM * BN));
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        v[i][u] = s + u < P.nsplit
+                      ? __ldcg(reinterpret_cast<const float4*>(p0 + static_cast<size_t>(16 * i) * BN + static_cast<size_t>(s + u) * SPLIT))
+                      : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (s + u < P.nsplit) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          acc[i][0] += v[i][u].x;
+          acc[i][1] += v[i][u].y;
+          acc[i][2] += v[i][u].z;
+          acc[i][3] += v[i][u].w;
+        }
+      }
   }
   const bool mirror_bf16 = sym && !(P.flags & G2F_LOWER);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int lr = ty + 8 * i;
-    const int gr = w.c_row + sub_r * 32 + lr;
-    float val = P.alpha * accs[i];
-    const bool inb = gr < P.M && gc < P.N;
-    if (inb && P.beta != 0.f) val += P.beta * P.Cin[static_cast<size_t>(gr) * P.ldc + gc];
-    tile[lr][tx] = val;
-    const bool keep = inb && !(diag_tile && gc > gr);
-    if (keep) {
-      if (P.C != nullptr) P.C[static_cast<size_t>(gr) * P.ldc + gc] = val;
-      for (int e = 0; e < P.n_extra; ++e) {
-        float* dst = P.full->C_extra[e] + static_cast<size_t>(gr) * P.ldc + gc;
-        if (P.flags & G2F_MCAST)
-          g2_multimem_st_f32(dst, val);
-        else
-          *dst = val;
+  for (int i = 0; i < 2; ++i) {
+    const int lr = ty + 16 * i, gr = row0 + lr;
+    float val[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      val[j] = P.alpha * acc[i][j];
+      if (P.beta != 0.f) val[j] += P.beta * cin[i][j];
+      tile[lr][tx * 4 + j] = val[j];
+    }
+    if (gr >= P.M) continue;
+    // entries above the diagonal are not this patch's to write
+    const int keep = diag_tile ? min(4, gr - gc + 1) : 4;
+    if (P.C != nullptr) {
+      float* c = P.C + static_cast<size_t>(gr) * P.ldc + gc;
+      if (vec_out && keep == 4) {
+        *reinterpret_cast<float4*>(c) = make_float4(val[0], val[1], val[2], val[3]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (j < keep && gc + j < P.N) c[j] = val[j];
       }
-      if (P.out_hi != nullptr) {
-        const size_t o = static_cast<size_t>(gr) * P.ld_out + gc;
-        const size_t om = static_cast<size_t>(gc) * P.ld_out + gr;
-        const bool mir = mirror_bf16 && gc != gr;
-        const __nv_bfloat16 h = __float2bfloat16_rn(val);
-        P.out_hi[o] = h;
-        if (mir) P.out_hi[om] = h;
-        if (P.out_lo != nullptr) {
-          const float r1 = val - __bfloat162float(h);
-          if (P.out_mid != nullptr) {
-            const __nv_bfloat16 m = __float2bfloat16_rn(r1);
-            const __nv_bfloat16 l = __float2bfloat16_rn(r1 - __bfloat162float(m));
-            P.out_mid[o] = m;
-            P.out_lo[o] = l;
-            if (mir) {
-              P.out_mid[om] = m;
-              P.out_lo[om] = l;
-            }
-          } else {
-            const __nv_bfloat16 l = __float2bfloat16_rn(r1);
-            P.out_lo[o] = l;
-            if (mir) P.out_lo[om] = l;
-          }
+    }
+    for (int e = 0; e < P.n_extra; ++e) {
+      float* dst = P.full->C_extra[e] + static_cast<size_t>(gr) * P.ldc + gc;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j < keep && gc + j < P.N) {
+          if (P.flags & G2F_MCAST)
+            g2_multimem_st_f32(dst + j, val[j]);
+          else
+            dst[j] = val[j];
+        }
+    }
+    if (P.out_hi != nullptr) {
+      unsigned short part[3][4];   // hi, mid, lo (hi, lo in a two-way split)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const __nv_bfloat16 h = __float2bfloat16_rn(val[j]);
+        const float r1 = val[j] - __bfloat162float(h);
+        const __nv_bfloat16 m = __float2bfloat16_rn(r1);
+        part[0][j] = __bfloat16_as_ushort(h);
+        part[1][j] = __bfloat16_as_ushort(m);
+        part[2][j] = __bfloat16_as_ushort(__float2bfloat16_rn(r1 - __bfloat162float(m)));
+      }
+      __nv_bfloat16* const outs[3] = {P.out_hi, P.out_mid != nullptr ? P.out_mid : P.out_lo,
+                                      P.out_mid != nullptr ? P.out_lo : nullptr};
+      const size_t o = static_cast<size_t>(gr) * P.ld_out + gc;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        if (outs[q] == nullptr) continue;
+        if (full && keep == 4 && (P.ld_out & 3) == 0 && (reinterpret_cast<uintptr_t>(outs[q]) & 7) == 0) {
+          *reinterpret_cast<uint2*>(outs[q] + o) =
+              make_uint2(part[q][0] | (static_cast<uint32_t>(part[q][1]) << 16), part[q][2] | (static_cast<uint32_t>(part[q][3]) << 16));
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (j < keep && gc + j < P.N) outs[q][o + j] = __ushort_as_bfloat16(part[q][j]);
+        }
+        if (mirror_bf16) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (j < keep && gc + j < P.N && gc + j != gr)
+              outs[q][static_cast<size_t>(gc + j) * P.ld_out + gr] = __ushort_as_bfloat16(part[q][j]);
         }
       }
     }
   }
   if (!sym || P.C == nullptr || (P.flags & G2F_LOWER)) return;
   __syncthreads();
-  // mirrored store: element (r, c) of the patch goes to C[c][r]
+  // mirrored store: element (r, c) of the patch goes to C[c][r]; a warp writes 32 consecutive columns of one row
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int lc = ty + 8 * i;                       // patch column -> destination row
-    const int dst_r = w.c_col + sub_c * 32 + lc;     // global column index of the source
-    const int dst_c = w.c_row + sub_r * 32 + tx;     // global row index of the source
+  for (int i = 0; i < G2_RED_COLS / 8; ++i) {
+    const int lc = warp + 8 * i;            // patch column -> destination row
+    const int dst_r = col0 + lc, dst_c = row0 + lane;
     if (dst_r < P.N && dst_c < P.M && dst_r < dst_c)
-      P.C[static_cast<size_t>(dst_r) * P.ldc + dst_c] = tile[tx][lc];
+      P.C[static_cast<size_t>(dst_r) * P.ldc + dst_c] = tile[lane][lc];
   }
 }
 
