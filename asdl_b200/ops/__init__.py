@@ -328,9 +328,11 @@ def kron_apply(left: torch.Tensor, mid: torch.Tensor, right: torch.Tensor) -> to
     m, n = mid.shape
     x3 = _use_x3(torch.float32) if (left.dtype == torch.float32 or mid.dtype == torch.float32) \
         else _use_x3(mid.dtype)
-    l_hi, l_lo = _stage_bf16(left, x3)
+    # a symmetric matrix that is stored column by column (a torch.cholesky_inverse result) is read through its
+    # row-major transpose, which is the same matrix, instead of being copied
+    l_hi, l_lo = _stage_bf16(left.t() if left.stride(1) != 1 and left.stride(0) == 1 else left, x3)
     g_hi, g_lo = _stage_bf16(mid, x3)
-    r_hi, r_lo = _stage_bf16(right, x3)
+    r_hi, r_lo = _stage_bf16(right.t() if right.stride(1) != 1 and right.stride(0) == 1 else right, x3)
     ld = _round_up(max(n, 8), 8)
     t_hi = torch.empty(m, ld, device=mid.device, dtype=torch.bfloat16)
     t_lo = torch.empty_like(t_hi) if x3 else None
