@@ -1,0 +1,88 @@
+"""Staging, reduction, normalisation and factorisation kernels at the sizes where their tiles, vectors and lanes end."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from asdl_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = 'cuda'
+
+
+@pytest.fixture(scope='module')
+def ext():
+    e = ops.extension()
+    yield e
+    ops.check_status()
+
+
+def _gen(seed):
+    g = torch.Generator(device=DEV)
+    g.manual_seed(seed)
+    return g
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize('rows,n,ld,offset', [(1, 1, 8, 0), (3, 7, 8, 0), (37, 64, 64, 0), (130, 65, 72, 0), (2, 2057, 2064, 0),
+                                              (1300, 24, 24, 0), (9, 40, 40, 1), (5, 9, 12, 0)])
+def test_cast_parts(ext, dtype, rows, n, ld, offset):
+    x = torch.randn(rows, n + offset, device=DEV, generator=_gen(0)).to(dtype)[:, offset:]
+    hi = torch.full((rows, ld), float('nan'), device=DEV, dtype=torch.bfloat16)
+    lo = torch.full_like(hi, float('nan'))
+    ext.cast_pad_bf16(x, hi, lo, 1.0)
+    want = F.pad(x.float(), (0, ld - n))
+    assert torch.equal(hi, want.to(torch.bfloat16))
+    assert torch.equal(lo, (want - hi.float()).to(torch.bfloat16))
+    one = torch.empty_like(hi)
+    ext.cast_pad_bf16(x, one, None, 0.5)
+    assert torch.equal(one, (want * 0.5).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize('cfg', [  # n, c, h, w, kernel, stride, padding, dilation
+    (2, 8, 9, 7, 3, 1, 1, 1), (1, 3, 12, 11, 7, 2, 3, 1), (2, 24, 8, 8, 3, 2, 1, 1), (1, 5, 13, 13, 3, 1, 2, 2),
+    (1, 300, 9, 9, 5, 1, 2, 1), (3, 16, 5, 5, 1, 2, 0, 1), (1, 1, 3, 40, 3, 1, 1, 1)])
+@pytest.mark.parametrize('layout', ['nchw', 'nhwc', 'sliced'])
+def test_im2col_layouts(ext, cfg, dtype, layout):
+    n, c, h, w, k, s, p, d = cfg
+    x = torch.randn(n, c, h, w + 1, device=DEV, generator=_gen(1)).to(dtype)
+    x = x[..., 1:] if layout == 'sliced' else x[..., :w].contiguous()
+    if layout == 'nhwc':
+        x = x.contiguous(memory_format=torch.channels_last)
+    cols = F.unfold(x.float(), k, padding=p, stride=s, dilation=d)                 # n x (c kh kw) x pixels
+    ld = (c * k * k + 7) // 8 * 8
+    for c_major in (True, False):
+        want = cols if c_major else cols.view(n, c, k * k, -1).transpose(1, 2).reshape(n, c * k * k, -1)
+        want = F.pad(want.transpose(1, 2).reshape(-1, c * k * k), (0, ld - c * k * k))
+        for with_lo in (False, True):
+            out = torch.full((want.shape[0], ld), float('nan'), device=DEV, dtype=torch.bfloat16)
+            lo = torch.full_like(out, float('nan')) if with_lo else None
+            ext.im2col_bf16(x, out, lo, [k, k], [s, s], [p, p], [d, d], c_major)
+            assert torch.equal(out, want.to(torch.bfloat16))
+            if with_lo:
+                assert torch.equal(lo, (want - out.float()).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize('rows,n', [(700, 33), (3000, 130), (2048, 257), (5000, 64)])
+@pytest.mark.parametrize('nsplit', [2, 5, 9])
+@pytest.mark.parametrize('beta', [0.0, 0.9])
+def test_split_k_reduction(ext, rows, n, nsplit, beta):
+    x = torch.randn(rows, (n + 7) // 8 * 8, device=DEV, generator=_gen(2)).to(torch.bfloat16)[:, :n]
+    old = torch.randn(n, n, device=DEV, generator=_gen(3))
+    old = old + old.T
+    c = old.clone() if beta else torch.full((n, n), float('nan'), device=DEV)
+    ext.umma_gemm([x], [x], False, False, c, 0.25, beta, True, None, None, nsplit)
+    want = 0.25 * (x.double().T @ x.double()) + beta * old.double()
+    # exact products; every one of the `rows` additions loses at most 2^-22 of the running sum (truncating accumulator)
+    bound = rows * 2.0 ** -22 * 0.25 * (x.double().abs().T @ x.double().abs()) + 2.0 ** -22 * beta * old.double().abs()
+    assert ((c.double() - want).abs() <= bound).all()
+    assert torch.equal(c, c.T)
+
+
+def test_kron_apply_reads_either_order_of_a_symmetric_factor():
+    left, right = (torch.randn(n, n, device=DEV, generator=_gen(4 + n)) for n in (72, 130))
+    left, right = left + left.T, right + right.T
+    mid = torch.randn(72, 130, device=DEV, generator=_gen(4))
+    row = ops.kron_apply(left, mid, right)
+    col = ops.kron_apply(left.T.contiguous().T, mid, right.T.contiguous().T)
+    assert torch.equal(row, col)
