@@ -86,3 +86,29 @@ def test_kron_apply_reads_either_order_of_a_symmetric_factor():
     row = ops.kron_apply(left, mid, right)
     col = ops.kron_apply(left.T.contiguous().T, mid, right.T.contiguous().T)
     assert torch.equal(row, col)
+
+
+@pytest.mark.parametrize('n', [1, 31, 32, 33, 64, 65, 96, 97, 127, 128, 129, 160, 225, 257])
+def test_inverse_at_the_edges_of_the_diagonal_stages(n):
+    x = torch.randn(2 * n, n, device=DEV, generator=_gen(19))
+    a = x.T @ x / (2 * n)
+    before = a.clone()
+    got = ops.spd_inverse(a, 1e-2)
+    d = a.double()
+    d.diagonal().add_(1e-2)
+    want = torch.linalg.inv(d)
+    # n * 2^-24 times the condition number bounds the error of a Cholesky inverse, relative to the largest entry
+    cond = torch.linalg.cond(d).item()
+    assert (got.double() - want).abs().max() <= 4 * max(n, 8) * 2.0 ** -24 * cond * want.abs().max()
+    assert torch.equal(a, before)
+    ops.check_status()
+
+
+@pytest.mark.parametrize('n,at', [(40, 35), (128, 0), (128, 100), (200, 150)])
+def test_a_negative_pivot_in_any_stage_is_reported(n, at):
+    a = torch.eye(n, device=DEV)
+    a[at, at] = -1.0
+    got = ops.spd_inverse(a, 0.0)
+    with pytest.raises(RuntimeError, match='not positive definite'):
+        ops.check_status()
+    assert torch.isfinite(got).all()
