@@ -23,6 +23,8 @@ namespace {
 
 constexpr int LN_WARPS = 8;
 constexpr int LN_THREADS = LN_WARPS * 32;
+// CTAs of the backward kernel that an SM holds: 40 registers per vector slot leave room for two up to VPL = 2
+constexpr int ln_bwd_ctas(int vpl) { return vpl <= 2 ? 2 : 1; }
 
 __device__ __forceinline__ void ln_unpack8(const uint4& raw, float (&out)[8]) {
   const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
@@ -126,8 +128,10 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ gam
   }
 }
 
+// The next row of x and dy is loaded while the current one is reduced: a warp has only a few rows, and each waited for its
+// loads.  Rows are kept as the loaded bf16 vectors (half the registers of their fp32 values), unpacked once per use.
 template <int VPL, int SPLIT>
-__global__ void __launch_bounds__(LN_THREADS)
+__global__ void __launch_bounds__(LN_THREADS, ln_bwd_ctas(VPL))
 ln_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
               const float* __restrict__ gamma, const float* __restrict__ mean, const float* __restrict__ rstd,
               __nv_bfloat16* __restrict__ dx, float* __restrict__ part, long long rows) {
@@ -138,6 +142,21 @@ ln_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
   int slot = 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int group = warp / SPLIT, col0 = (warp % SPLIT) * 256 * VPL;
+  const long long step = static_cast<long long>(gridDim.x) * GROUPS;
+  long long r = static_cast<long long>(blockIdx.x) * GROUPS + group;
+  uint4 rx[VPL], rg[VPL];
+  float mu = 0.f, rs = 0.f;
+  auto load_row = [&](long long row, uint4 (&ax)[VPL], uint4 (&ag)[VPL], float& m, float& s) {
+    const long long at = row * D + col0 + lane * 8;
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) {
+      ax[v] = __ldg(reinterpret_cast<const uint4*>(x + at + v * 256));
+      ag[v] = __ldg(reinterpret_cast<const uint4*>(dy + at + v * 256));
+    }
+    m = __ldg(mean + row);
+    s = __ldg(rstd + row);
+  };
+  if (r < rows) load_row(r, rx, rg, mu, rs);
   float g[VPL][8], dg[VPL][8], db[VPL][8];
 #pragma unroll
   for (int v = 0; v < VPL; ++v) {
@@ -145,34 +164,45 @@ ln_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
 #pragma unroll
     for (int i = 0; i < 8; ++i) dg[v][i] = db[v][i] = 0.f;
   }
-  for (long long r = static_cast<long long>(blockIdx.x) * GROUPS + group; r < rows;
-       r += static_cast<long long>(gridDim.x) * GROUPS) {
-    const float mu = mean[r], rs = rstd[r];
-    float xh[VPL][8], gy[VPL][8];
+  for (; r < rows; r += step) {
+    uint4 nx[VPL], ng[VPL];
+    float nmu = 0.f, nrs = 0.f;
+    const bool more = r + step < rows;
+    if (more) load_row(r + step, nx, ng, nmu, nrs);
     float c1 = 0.f, c2 = 0.f;
 #pragma unroll
     for (int v = 0; v < VPL; ++v) {
       float xv[8], dv[8];
-      ln_unpack8(__ldg(reinterpret_cast<const uint4*>(x + r * D + col0 + (v * 32 + lane) * 8)), xv);
-      ln_unpack8(__ldg(reinterpret_cast<const uint4*>(dy + r * D + col0 + (v * 32 + lane) * 8)), dv);
+      ln_unpack8(rx[v], xv);
+      ln_unpack8(rg[v], dv);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        xh[v][i] = (xv[i] - mu) * rs;
-        dg[v][i] = fmaf(dv[i], xh[v][i], dg[v][i]);
+        const float xh = (xv[i] - mu) * rs, gy = dv[i] * g[v][i];
+        dg[v][i] = fmaf(dv[i], xh, dg[v][i]);
         db[v][i] += dv[i];
-        gy[v][i] = dv[i] * g[v][i];
-        c1 = fmaf(gy[v][i], xh[v][i], c1);
-        c2 += gy[v][i];
+        c1 = fmaf(gy, xh, c1);
+        c2 += gy;
       }
     }
     c1 = ln_group_sum<SPLIT>(c1, scratch, slot, warp) * (1.f / D);
     c2 = ln_group_sum<SPLIT>(c2, scratch, slot, warp) * (1.f / D);
 #pragma unroll
     for (int v = 0; v < VPL; ++v) {
-      float out[8];
+      float xv[8], dv[8], out[8];
+      ln_unpack8(rx[v], xv);
+      ln_unpack8(rg[v], dv);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) out[i] = rs * (gy[v][i] - c2 - xh[v][i] * c1);
+      for (int i = 0; i < 8; ++i) out[i] = rs * (dv[i] * g[v][i] - c2 - (xv[i] - mu) * rs * c1);
       *reinterpret_cast<uint4*>(dx + r * D + col0 + (v * 32 + lane) * 8) = ln_pack8(out);
+    }
+    if (more) {
+#pragma unroll
+      for (int v = 0; v < VPL; ++v) {
+        rx[v] = nx[v];
+        rg[v] = ng[v];
+      }
+      mu = nmu;
+      rs = nrs;
     }
   }
   // combine the warps of the CTA that hold the same columns, one vector slot at a time
@@ -196,22 +226,32 @@ ln_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
   }
 }
 
-// dgamma[j] = sum over CTAs of part[c][0][j], dbeta[j] likewise (coalesced over j).
-__global__ void ln_bwd_finalize(const float* __restrict__ part, float* __restrict__ dgamma,
-                                float* __restrict__ dbeta, int ctas, int d) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= d) return;
-  float sg = 0.f, sb = 0.f;
-  for (int c = 0; c < ctas; ++c) {
-    sg += part[(static_cast<size_t>(c) * 2) * d + j];
-    sb += part[(static_cast<size_t>(c) * 2 + 1) * d + j];
-  }
-  dgamma[j] = sg;
-  dbeta[j] = sb;
+// dgamma[j] = sum over CTAs of part[c][0][j], dbeta[j] likewise.  A CTA takes 32 of the 2 d sums (one 128-byte line per
+// part) with FIN_LANES parts in flight at a time: one thread per sum walked all parts alone, a chain of as many loads as
+// there are CTAs on eight SMs.
+constexpr int FIN_LANES = 16;
+__global__ void __launch_bounds__(32 * FIN_LANES)
+ln_bwd_finalize(const float* __restrict__ part, float* __restrict__ dgamma, float* __restrict__ dbeta, int ctas, int d) {
+  __shared__ float red[FIN_LANES][32];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, j = blockIdx.x * 32 + tx;   // d is a multiple of 32
+  const float* from = part + j;
+  float s = 0.f;
+#pragma unroll 4
+  for (int c = ty; c < ctas; c += FIN_LANES) s += from[static_cast<size_t>(c) * 2 * d];
+  red[ty][tx] = s;
+  __syncthreads();
+  if (ty != 0) return;
+  s = 0.f;
+#pragma unroll
+  for (int k = 0; k < FIN_LANES; ++k) s += red[k][tx];
+  if (j < d)
+    dgamma[j] = s;
+  else
+    dbeta[j - d] = s;
 }
 
-int ln_grid(long long rows, int groups) {
-  return static_cast<int>(std::max<long long>(1, std::min<long long>((rows + groups - 1) / groups, 148LL * 2)));
+int ln_grid(long long rows, int groups, int per_sm) {
+  return static_cast<int>(std::max<long long>(1, std::min<long long>((rows + groups - 1) / groups, 148LL * per_sm)));
 }
 
 void ln_check(const at::Tensor& x, const at::Tensor& gamma, int& vpl, long long& rows) {
@@ -254,6 +294,7 @@ void launch_bwd(int grid, cudaStream_t stream, const __nv_bfloat16* x, const __n
   }
 
 // warps of a CTA that work on different rows at a time
+int ln_vpl_of_warp(int vpl) { return vpl <= 4 ? vpl : (vpl % 3 == 0 ? 3 : 4); }
 int ln_groups(int vpl) { return vpl <= 4 ? LN_WARPS : (vpl <= 8 ? LN_WARPS / 2 : LN_WARPS / 4); }
 
 }  // namespace
@@ -277,7 +318,7 @@ std::vector<at::Tensor> ln_forward(at::Tensor x, at::Tensor weight, at::Tensor b
   auto y = at::empty_like(x);
   auto mean = at::empty({rows}, weight.options()), rstd = at::empty({rows}, weight.options());
   if (rows == 0) return {y, mean, rstd};
-  const int grid = ln_grid(rows, ln_groups(vpl));
+  const int grid = ln_grid(rows, ln_groups(vpl), 2);
   const auto* xp = reinterpret_cast<const __nv_bfloat16*>(x.data_ptr());
   auto* yp = reinterpret_cast<__nv_bfloat16*>(y.data_ptr());
   LN_DISPATCH(vpl, launch_fwd, grid, stream, xp, weight.data_ptr<float>(), bias.data_ptr<float>(), yp,
@@ -303,16 +344,16 @@ std::vector<at::Tensor> ln_backward(at::Tensor x, at::Tensor dy, at::Tensor weig
   auto stream = at::cuda::getCurrentCUDAStream(dev).stream();
   const long long d = x.size(-1);
   auto dx = at::empty_like(x);
-  auto dweight = at::zeros({d}, weight.options()), dbias = at::zeros({d}, weight.options());
-  if (rows == 0) return {dx, dweight, dbias};
-  const int grid = ln_grid(rows, ln_groups(vpl));
+  if (rows == 0) return {dx, at::zeros({d}, weight.options()), at::zeros({d}, weight.options())};
+  auto dweight = at::empty({d}, weight.options()), dbias = at::empty({d}, weight.options());
+  const int grid = ln_grid(rows, ln_groups(vpl), ln_bwd_ctas(ln_vpl_of_warp(vpl)));
   auto part = at::empty({grid, 2, d}, weight.options());
   const auto* xp = reinterpret_cast<const __nv_bfloat16*>(x.data_ptr());
   const auto* gp = reinterpret_cast<const __nv_bfloat16*>(dy.data_ptr());
   auto* dxp = reinterpret_cast<__nv_bfloat16*>(dx.data_ptr());
   LN_DISPATCH(vpl, launch_bwd, grid, stream, xp, gp, weight.data_ptr<float>(), mean.data_ptr<float>(),
               rstd.data_ptr<float>(), dxp, part.data_ptr<float>(), rows);
-  ln_bwd_finalize<<<static_cast<int>((d + 127) / 128), 128, 0, stream>>>(
+  ln_bwd_finalize<<<static_cast<int>(2 * d / 32), 32 * FIN_LANES, 0, stream>>>(
       part.data_ptr<float>(), dweight.data_ptr<float>(), dbias.data_ptr<float>(), grid, static_cast<int>(d));
   B200_CUDA_CHECK(cudaGetLastError());
   count_launch(2);

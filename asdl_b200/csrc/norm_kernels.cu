@@ -70,7 +70,8 @@ bn_stats_partial(const T* __restrict__ y, const T* __restrict__ g, const float* 
       bias[i] = b[c0 + i];
     }
     const size_t base = static_cast<size_t>(n) * hw * channels + c0;
-    for (int p = hw_begin + lane; p < hw_end; p += BN_LANES) {
+#pragma unroll 4
+    for (int p = hw_begin + lane; p < hw_end; p += BN_LANES) {   // the loads of four positions in flight
       float yv[VEC], gv[VEC];
       VecLoad<T, VEC>::load(y + base + static_cast<size_t>(p) * channels, yv);
       VecLoad<T, VEC>::load(g + base + static_cast<size_t>(p) * channels, gv);
@@ -125,7 +126,8 @@ bn_stats_partial_xhat(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* 
       is[i] = invstd[c0 + i];
     }
     const size_t base = static_cast<size_t>(n) * hw * channels + c0;
-    for (int p = hw_begin + lane; p < hw_end; p += BN_LANES) {
+#pragma unroll 4
+    for (int p = hw_begin + lane; p < hw_end; p += BN_LANES) {   // the loads of four positions in flight
       float xv[VEC], gv[VEC];
       VecLoad<__nv_bfloat16, 8>::load(x + base + static_cast<size_t>(p) * channels, xv);
       VecLoad<__nv_bfloat16, 8>::load(dy + base + static_cast<size_t>(p) * channels, gv);

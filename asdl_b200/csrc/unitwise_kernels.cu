@@ -31,7 +31,72 @@ __device__ __forceinline__ float to_f<float>(float v) { return v; }
 template <>
 __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 
-// grid: (column chunks of 256, row chunks); thread = one column, walks its chunk of rows
+// Partial sums part[chunk][3][d] over a chunk of rows.  A CTA covers 8 vector columns (VEC elements, 16 bytes each: 128
+// bytes of a row) with 32 row lanes, four rows of both tensors in flight per thread.  With one 2-byte column per thread
+// and a serial walk, 8192 x 1024 bf16 was bound by the latency of single loads.
+constexpr int LS_GROUPS = 8, LS_LANES = 32, LS_ROWS = 4;
+template <typename T>
+__global__ void __launch_bounds__(LS_GROUPS * LS_LANES)
+ln_stats_partial_vec(const T* __restrict__ y, const T* __restrict__ g, const float* __restrict__ weight,
+                     const float* __restrict__ bias, float* __restrict__ part, long long rows, int d,
+                     long long rows_per_chunk) {
+  constexpr int VEC = 16 / sizeof(T);
+  __shared__ float red[LS_GROUPS * LS_LANES / 32][3][LS_GROUPS * VEC];
+  const int group = threadIdx.x % LS_GROUPS, lane = threadIdx.x / LS_GROUPS, warp = threadIdx.x >> 5;
+  const int c0 = (blockIdx.x * LS_GROUPS + group) * VEC;
+  const long long r0 = blockIdx.y * rows_per_chunk, r1 = min(rows, r0 + rows_per_chunk);
+  float acc[3][VEC];
+#pragma unroll
+  for (int k = 0; k < VEC; ++k) acc[0][k] = acc[1][k] = acc[2][k] = 0.f;
+  if (c0 < d) {   // d is a multiple of VEC
+    float b[VEC], iw[VEC];
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) {
+      b[k] = bias[c0 + k];
+      iw[k] = 1.f / weight[c0 + k];
+    }
+    for (long long r = r0 + lane; r < r1; r += LS_ROWS * LS_LANES) {
+      uint4 ry[LS_ROWS], rg[LS_ROWS];
+#pragma unroll
+      for (int u = 0; u < LS_ROWS; ++u)
+        if (r + u * LS_LANES < r1) {
+          ry[u] = __ldg(reinterpret_cast<const uint4*>(y + (r + u * LS_LANES) * d + c0));
+          rg[u] = __ldg(reinterpret_cast<const uint4*>(g + (r + u * LS_LANES) * d + c0));
+        }
+#pragma unroll
+      for (int u = 0; u < LS_ROWS; ++u) {
+        if (r + u * LS_LANES >= r1) break;
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) {
+          const float gv = to_f(reinterpret_cast<const T*>(&rg[u])[k]);
+          const float gw = (to_f(reinterpret_cast<const T*>(&ry[u])[k]) - b[k]) * iw[k] * gv;
+          acc[0][k] = fmaf(gw, gw, acc[0][k]);
+          acc[1][k] = fmaf(gw, gv, acc[1][k]);
+          acc[2][k] = fmaf(gv, gv, acc[2][k]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < 3; ++m)
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) {   // the four row lanes of a warp, then the warps through shared memory
+      float v = acc[m][k];
+      v += __shfl_xor_sync(0xffffffffu, v, 8);
+      v += __shfl_xor_sync(0xffffffffu, v, 16);
+      if ((threadIdx.x & 31) < LS_GROUPS) red[warp][m][group * VEC + k] = v;
+    }
+  __syncthreads();
+  for (int e = threadIdx.x; e < 3 * LS_GROUPS * VEC; e += LS_GROUPS * LS_LANES) {
+    const int m = e / (LS_GROUPS * VEC), k = e - m * (LS_GROUPS * VEC), c = blockIdx.x * LS_GROUPS * VEC + k;
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < LS_GROUPS * LS_LANES / 32; ++w) s += red[w][m][k];
+    if (c < d) part[(static_cast<size_t>(blockIdx.y) * 3 + m) * d + c] = s;
+  }
+}
+
+// The same for rows that are not 16-byte aligned.  grid: (column chunks of 256, row chunks); thread = one column.
 template <typename T>
 __global__ void __launch_bounds__(256) ln_stats_partial(const T* __restrict__ y, const T* __restrict__ g,
                                                         const float* __restrict__ weight,
@@ -43,6 +108,7 @@ __global__ void __launch_bounds__(256) ln_stats_partial(const T* __restrict__ y,
   const long long r1 = (r0 + rows_per_chunk < rows) ? r0 + rows_per_chunk : rows;
   const float b = bias[c], iw = 1.f / weight[c];
   float ww = 0.f, wb = 0.f, bb = 0.f;
+#pragma unroll 4
   for (long long r = r0; r < r1; ++r) {
     const float gv = to_f(g[r * d + c]);
     const float gw = (to_f(y[r * d + c]) - b) * iw * gv;
@@ -50,22 +116,37 @@ __global__ void __launch_bounds__(256) ln_stats_partial(const T* __restrict__ y,
     wb = fmaf(gw, gv, wb);
     bb = fmaf(gv, gv, bb);
   }
-  float* p = part + (static_cast<size_t>(blockIdx.y) * d + c) * 3;
+  float* p = part + static_cast<size_t>(blockIdx.y) * 3 * d + c;
   p[0] = ww;
-  p[1] = wb;
-  p[2] = bb;
+  p[d] = wb;
+  p[2 * static_cast<size_t>(d)] = bb;
 }
 
-__global__ void ln_stats_finalize(const float* __restrict__ part, float* __restrict__ stats, int d, int chunks,
-                                  float alpha, float beta) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d) return;
-  double ww = 0.0, wb = 0.0, bb = 0.0;   // chunks are summed in a fixed order: deterministic
-  for (int k = 0; k < chunks; ++k) {
-    const float* p = part + (static_cast<size_t>(k) * d + c) * 3;
-    ww += p[0];
-    wb += p[1];
-    bb += p[2];
+// 32 features per CTA, eight chunks at a time; chunks are summed in double precision in a fixed order: deterministic.
+__global__ void __launch_bounds__(256) ln_stats_finalize(const float* __restrict__ part, float* __restrict__ stats, int d,
+                                                         int chunks, float alpha, float beta) {
+  __shared__ double red[8][3][32];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, c = blockIdx.x * 32 + tx;
+  double ww = 0.0, wb = 0.0, bb = 0.0;
+  if (c < d) {
+#pragma unroll 4
+    for (int k = ty; k < chunks; k += 8) {
+      const float* p = part + static_cast<size_t>(k) * 3 * d + c;
+      ww += p[0];
+      wb += p[d];
+      bb += p[2 * static_cast<size_t>(d)];
+    }
+  }
+  red[ty][0][tx] = ww;
+  red[ty][1][tx] = wb;
+  red[ty][2][tx] = bb;
+  __syncthreads();
+  if (ty != 0 || c >= d) return;
+#pragma unroll
+  for (int k = 1; k < 8; ++k) {
+    ww += red[k][0][tx];
+    wb += red[k][1][tx];
+    bb += red[k][2][tx];
   }
   float* s = stats + 4 * static_cast<size_t>(c);
   const float o0 = beta != 0.f ? beta * s[0] : 0.f, o1 = beta != 0.f ? beta * s[1] : 0.f;
@@ -234,22 +315,31 @@ void ln_unitwise_stats(at::Tensor y, at::Tensor g, at::Tensor weight, at::Tensor
   const int dev = y.get_device();
   c10::cuda::CUDAGuard guard(dev);
   auto stream = at::cuda::getCurrentCUDAStream(dev).stream();
-  const int col_chunks = (d + 255) / 256;
-  int chunks = std::max(1, (4 * sms(dev)) / col_chunks);
-  chunks = static_cast<int>(std::min<long long>(chunks, (rows + 15) / 16));
+  const bool vec = (d * y.element_size()) % 16 == 0 &&
+                   ((reinterpret_cast<uintptr_t>(y.data_ptr()) | reinterpret_cast<uintptr_t>(g.data_ptr())) & 15) == 0;
+  // about four CTAs per SM; at least 16 rows per thread column, or one row per lane of the vector kernel
+  const int width = vec ? LS_GROUPS * (bf16 ? 8 : 4) : 256, least = vec ? LS_LANES : 16;
+  const int col_chunks = (d + width - 1) / width;
+  long long chunks = std::max<long long>(1, std::min<long long>((4 * sms(dev)) / col_chunks, (rows + least - 1) / least));
   const long long per = (rows + chunks - 1) / chunks;
-  chunks = static_cast<int>((rows + per - 1) / per);
-  auto part = at::empty({chunks, d, 3}, stats.options());
-  dim3 grid(col_chunks, chunks);
+  chunks = (rows + per - 1) / per;
+  auto part = at::empty({chunks, 3, d}, stats.options());
+  const dim3 grid(col_chunks, static_cast<unsigned>(chunks));
+  const float *wp = weight.data_ptr<float>(), *bp = bias.data_ptr<float>();
+  float* pp = part.data_ptr<float>();
+  auto run = [&](auto* yp, auto* gp) {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(yp)>>;
+    if (vec)
+      ln_stats_partial_vec<T><<<grid, LS_GROUPS * LS_LANES, 0, stream>>>(yp, gp, wp, bp, pp, rows, d, per);
+    else
+      ln_stats_partial<T><<<grid, 256, 0, stream>>>(yp, gp, wp, bp, pp, rows, d, per);
+  };
   if (bf16)
-    ln_stats_partial<__nv_bfloat16><<<grid, 256, 0, stream>>>(
-        reinterpret_cast<const __nv_bfloat16*>(y.data_ptr()), reinterpret_cast<const __nv_bfloat16*>(g.data_ptr()),
-        weight.data_ptr<float>(), bias.data_ptr<float>(), part.data_ptr<float>(), rows, d, per);
+    run(reinterpret_cast<const __nv_bfloat16*>(y.data_ptr()), reinterpret_cast<const __nv_bfloat16*>(g.data_ptr()));
   else
-    ln_stats_partial<float><<<grid, 256, 0, stream>>>(y.data_ptr<float>(), g.data_ptr<float>(), weight.data_ptr<float>(),
-                                                      bias.data_ptr<float>(), part.data_ptr<float>(), rows, d, per);
-  ln_stats_finalize<<<(d + 255) / 256, 256, 0, stream>>>(part.data_ptr<float>(), stats.data_ptr<float>(), d, chunks,
-                                                         static_cast<float>(alpha), static_cast<float>(beta));
+    run(static_cast<const float*>(y.data_ptr<float>()), static_cast<const float*>(g.data_ptr<float>()));
+  ln_stats_finalize<<<(d + 31) / 32, 256, 0, stream>>>(pp, stats.data_ptr<float>(), d, static_cast<int>(chunks),
+                                                       static_cast<float>(alpha), static_cast<float>(beta));
   B200_CUDA_CHECK(cudaGetLastError());
   count_launch(2);
 }

@@ -112,3 +112,36 @@ def test_a_negative_pivot_in_any_stage_is_reported(n, at):
     with pytest.raises(RuntimeError, match='not positive definite'):
         ops.check_status()
     assert torch.isfinite(got).all()
+
+
+@pytest.mark.parametrize('d', [256, 512, 768, 1024, 1536, 2048, 4096])
+@pytest.mark.parametrize('rows', [1, 7, 148 * 8 + 1, 148 * 16 + 5])
+def test_layer_norm_backward_rows(rows, d):
+    x = torch.randn(rows, d, device=DEV, generator=_gen(10)).to(torch.bfloat16).requires_grad_(True)
+    dy = torch.randn(rows, d, device=DEV, generator=_gen(11)).to(torch.bfloat16)
+    weight = (1 + 0.1 * torch.randn(d, device=DEV, generator=_gen(12))).requires_grad_(True)
+    bias = torch.randn(d, device=DEV, generator=_gen(13)).requires_grad_(True)
+    got = torch.autograd.grad(ops.layer_norm(x, weight, bias), [x, weight, bias], dy)
+    leaves = [t.detach().double().requires_grad_(True) for t in (x, weight, bias)]
+    want = torch.autograd.grad(F.layer_norm(leaves[0], (d,), leaves[1], leaves[2]), leaves, dy.double())
+    assert ((got[0].double() - want[0]).abs() <= 2.0 ** -8 * want[0].abs() + 1e-4).all()   # bf16 result, fp32 row sums
+    for a, b in zip(got[1:], want[1:]):   # fp32 sums of `rows` terms of size ~ 1: at most rows * 2^-24 of sqrt(rows) * few
+        assert (a.double() - b).abs().max() <= 1e-5 * max(1.0, rows ** 0.5) + 1e-5
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize('rows,d', [(1, 8), (31, 64), (33, 72), (700, 12), (3001, 1024), (257, 1001), (5000, 256)])
+def test_layer_norm_curvature_chunks(dtype, rows, d):
+    y = torch.randn(rows, d, device=DEV, generator=_gen(14)).to(dtype)
+    g = torch.randn(rows, d, device=DEV, generator=_gen(15)).to(dtype)
+    weight = 1 + 0.1 * torch.randn(d, device=DEV, generator=_gen(16))
+    bias = 0.1 * torch.randn(d, device=DEV, generator=_gen(17))
+    gw, gb = (y.double() - bias.double()) / weight.double() * g.double(), g.double()
+    want = torch.stack([torch.stack([(gw * gw).sum(0), (gw * gb).sum(0)], 1),
+                        torch.stack([(gw * gb).sum(0), (gb * gb).sum(0)], 1)], 1)
+    size = torch.stack([torch.stack([(gw * gw).sum(0), (gw * gb).abs().sum(0)], 1),
+                        torch.stack([(gw * gb).abs().sum(0), (gb * gb).sum(0)], 1)], 1)
+    old = torch.randn(d, 2, 2, device=DEV, generator=_gen(18))
+    got = ops.layernorm_unitwise_stats(y, g, weight, bias, out=old.clone(), alpha=0.5, beta=0.25)
+    # a few fp32 roundings per term and a sum of at most 64 per lane before double precision takes over
+    assert ((got.double() - (0.25 * old.double() + 0.5 * want)).abs() <= 64 * 2.0 ** -24 * size + 1e-6).all()
