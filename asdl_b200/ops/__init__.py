@@ -552,10 +552,13 @@ class _BatchNormTrain(torch.autograd.Function):
         ctx.mask_from_x = ctx.relu and not ctx.has_residual and BN_RELU_MASK_FROM_X
         ctx.save_for_backward(x, weight, mean, invstd, *([bias] if ctx.mask_from_x else ([y] if relu else [])))
         ctx.mark_non_differentiable(mean, invstd)
+        ctx.set_materialize_grads(False)   # no zero tensors for the statistics on every backward pass
         return y, mean, invstd
 
     @staticmethod
     def backward(ctx, dy, _dmean, _dinvstd):
+        if dy is None:
+            return (None,) * 10
         x, weight, mean, invstd, *rest = ctx.saved_tensors
         if not dy.is_contiguous(memory_format=torch.channels_last):
             dy = dy.contiguous(memory_format=torch.channels_last)

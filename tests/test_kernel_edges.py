@@ -145,3 +145,25 @@ def test_layer_norm_curvature_chunks(dtype, rows, d):
     got = ops.layernorm_unitwise_stats(y, g, weight, bias, out=old.clone(), alpha=0.5, beta=0.25)
     # a few fp32 roundings per term and a sum of at most 64 per lane before double precision takes over
     assert ((got.double() - (0.25 * old.double() + 0.5 * want)).abs() <= 64 * 2.0 ** -24 * size + 1e-6).all()
+
+
+@pytest.mark.parametrize('relu,residual', [(False, False), (True, False), (False, True), (True, True)])
+@pytest.mark.parametrize('n,c,h,w', [(2, 8, 1, 1), (3, 16, 5, 7), (1, 2056, 3, 3), (5, 264, 11, 9), (16, 64, 40, 40)])
+def test_batch_norm_row_walk(n, c, h, w, relu, residual):
+    def act(seed):
+        return torch.randn(n, c, h, w, device=DEV, generator=_gen(seed)).to(torch.bfloat16).contiguous(
+            memory_format=torch.channels_last)
+    x, dy, res = act(5).requires_grad_(True), act(6), act(7).requires_grad_(True) if residual else None
+    weight = (1 + 0.1 * torch.randn(c, device=DEV, generator=_gen(8))).requires_grad_(True)
+    bias = (0.1 * torch.randn(c, device=DEV, generator=_gen(9))).requires_grad_(True)
+    y = ops.batch_norm_train(x, weight, bias, None, None, residual=res, relu=relu)
+    grads = torch.autograd.grad(y, [x, weight, bias] + ([res] if residual else []), dy)
+    xd, wd, bd = (t.detach().double().requires_grad_(True) for t in (x, weight, bias))
+    rd = res.detach().double().requires_grad_(True) if residual else None
+    pre = F.batch_norm(xd, None, None, wd, bd, training=True)
+    pre = pre + rd if residual else pre
+    yd = pre * (y > 0) if relu else pre        # the mask of the stored output: a value may round to zero
+    want = torch.autograd.grad(yd, [xd, wd, bd] + ([rd] if residual else []), dy.double())
+    # bf16 results: 2^-8 of the value; of the largest value where terms cancel (y near 0, dx of two rows)
+    for got, ref in zip((y,) + grads, (yd,) + want):
+        assert ((got.double() - ref).abs() <= 2.0 ** -8 * (ref.abs() + ref.abs().max()) + 1e-5).all()
