@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const TcMat* mats, cons
 //            share S.  A warp takes four rows of each row block, a lane one column of each column block.
 // Every entry sees the same roundings in the same order as a column-by-column elimination, and gives the same bits.  That
 // elimination, with a barrier per column and the block in the registers of a 16 x 16 thread grid, took longer, and the
-// panel steps of all matrices wait for this kernel: six matrices up to 784 x 784 749 -> 596 us, the 107 factors of
+// panel steps of all matrices wait for this kernel: six matrices up to 784 x 784 749 -> 589 us, the 107 factors of
 // ResNet-50 8.61 -> 8.05 ms.
 //
 // The code is kept small (one body for all stages, eight columns of a substitution unrolled, the registers shifted by eight
@@ -114,21 +114,26 @@ __device__ __forceinline__ void diag_shift(float (&v)[32]) {
   for (int c = 0; c < 32; ++c) v[c] = c < 24 ? v[c + 8 < 32 ? c + 8 : 31] : 0.f;
 }
 
-// column 8 * j8 + J of the block's factor, by one warp (lane = row)
-template <int J>
-__device__ __forceinline__ void diag_factor_step(float (&a)[32], float& next, float* Lk, float* inv, int j8, int lane, bool& bad) {
-  const int j = j8 + J;
-  float d = __shfl_sync(0xffffffffu, next, j);
+// 1 / sqrt(pivot) of column j; a pivot that is not positive is reported and replaced by 1
+__device__ __forceinline__ float diag_pivot(float mine, int j, bool& bad) {
+  float d = __shfl_sync(0xffffffffu, mine, j & 31);
   if (!(d > 0.f)) {
-    bad = true;
+    bad |= j < 32;   // j = 32: there is no such column, and its result is not used
     d = 1.f;
   }
-  float iv = rsqrtf(d);
-  iv = iv * fmaf(-0.5f * d, iv * iv, 1.5f);   // one Newton step: full fp32 accuracy
+  const float iv = rsqrtf(d);
+  return iv * fmaf(-0.5f * d, iv * iv, 1.5f);   // one Newton step: full fp32 accuracy
+}
+
+// column j8 + J of the block's factor, by one warp (lane = row).  `iv`: 1 / sqrt of its pivot on entry, of the next pivot on
+// return; that one is formed ahead of the elimination, which fills the latency of the chain.
+template <int J>
+__device__ __forceinline__ void diag_factor_step(float (&a)[32], float& iv, float* Lk, float* inv, int j8, int lane, bool& bad) {
+  const int j = j8 + J;
   const float l = a[J] * iv;
-  next = fmaf(-l, l, a[J + 1]);
   Lk[j * DG_LP + lane] = l;   // rows above j: not used
   if (lane == 0) inv[j] = iv;
+  iv = diag_pivot(fmaf(-l, l, a[J + 1]), j + 1, bad);
   __syncwarp();
   diag_eliminate<J>(a, l, Lk + j * DG_LP + j8);
 }
@@ -170,17 +175,17 @@ __global__ void __launch_bounds__(256, 1) tc_diag_kernel(const TcMat* mats, int 
       float a[32];
 #pragma unroll
       for (int c = 0; c < 32; ++c) a[c] = S[(kb + lane) * DG_SP + kb + c];   // c > lane: not used
-      float next = a[0];
+      float iv = diag_pivot(a[0], 0, bad);
 #pragma unroll 1
       for (int j8 = 0; j8 < 32; j8 += 8) {
-        diag_factor_step<0>(a, next, Lk, inv, j8, lane, bad);
-        diag_factor_step<1>(a, next, Lk, inv, j8, lane, bad);
-        diag_factor_step<2>(a, next, Lk, inv, j8, lane, bad);
-        diag_factor_step<3>(a, next, Lk, inv, j8, lane, bad);
-        diag_factor_step<4>(a, next, Lk, inv, j8, lane, bad);
-        diag_factor_step<5>(a, next, Lk, inv, j8, lane, bad);
-        diag_factor_step<6>(a, next, Lk, inv, j8, lane, bad);
-        diag_factor_step<7>(a, next, Lk, inv, j8, lane, bad);
+        diag_factor_step<0>(a, iv, Lk, inv, j8, lane, bad);
+        diag_factor_step<1>(a, iv, Lk, inv, j8, lane, bad);
+        diag_factor_step<2>(a, iv, Lk, inv, j8, lane, bad);
+        diag_factor_step<3>(a, iv, Lk, inv, j8, lane, bad);
+        diag_factor_step<4>(a, iv, Lk, inv, j8, lane, bad);
+        diag_factor_step<5>(a, iv, Lk, inv, j8, lane, bad);
+        diag_factor_step<6>(a, iv, Lk, inv, j8, lane, bad);
+        diag_factor_step<7>(a, iv, Lk, inv, j8, lane, bad);
         diag_shift(a);
       }
     }
