@@ -385,102 +385,124 @@ im2col_nhwc_vec8_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __re
 
 // Tile path (any dtype and strides): a CTA stages the input rows that one output row and `cc` channels need in shared
 // memory, then every thread assembles eight consecutive columns of a patch from there (a table in shared memory maps
-// column -> staged element) and writes 16 bytes per part.  Input is read once per filter row and coalesced along W (or
-// along C for channels-innermost strides); what remains is the write of the patch matrix.  The element-wise kernel
-// spent 497 us on 128 x 64 x 32 x 32 fp32, 3 x 3 (302 MB of patches) in index divisions, 2-byte stores and strided reads.
-// grid: (N * Ho, channel chunks).  c_major columns of a chunk are contiguous; (kh, kw, c) order needs all channels.
+// column -> byte offset of the staged element) and writes 16 bytes per part.  Input is read once per filter row and
+// coalesced along W (or along C for channels-innermost strides) with IM2COL_LOADS loads in flight per thread; padding is
+// zeroed shared memory and the columns of the row pitch point at a zero row, so the assembly has no conditions.  What
+// remains is the write of the patch matrix.  grid: (N * Ho, channel chunks).  c_major columns of a chunk are contiguous;
+// (kh, kw, c) order needs all channels.
+constexpr int IM2COL_LOADS = 8;
 template <typename T, bool LO>
 __global__ void __launch_bounds__(256)
 im2col_tile_kernel(const T* __restrict__ x, __nv_bfloat16* __restrict__ out, __nv_bfloat16* __restrict__ out_lo,
-                   Im2colParams p, int cc, int wp) {
+                   Im2colParams p, int cc, int wp, int fast_lanes) {
   extern __shared__ float4 im2col_smem[];
-  float* tile = reinterpret_cast<float*>(im2col_smem);   // [cc][KH][wp], then a zero, then the column table
+  float* tile = reinterpret_cast<float*>(im2col_smem);   // [cc][KH][wp], a zero row [wp], then the column table
   const int taps = p.KH * p.KW, c_begin = blockIdx.y * cc, nc = min(cc, p.C - c_begin);
-  const int elems = cc * p.KH * wp, cols = nc * taps;
+  const int elems = cc * p.KH * wp, cols = nc * taps, floats = (elems + wp + 3) / 4 * 4;
   const bool last = c_begin + nc == p.C;
   const long long col0 = static_cast<long long>(c_begin) * taps;
   const int width = last ? static_cast<int>(p.ldo - col0) : cols;   // with the zero padding of the row pitch
-  unsigned short* table = reinterpret_cast<unsigned short*>(tile + (elems + 4) / 4 * 4);
+  unsigned short* table = reinterpret_cast<unsigned short*>(tile + floats);
   const int n = blockIdx.x / p.Ho, ho = blockIdx.x - n * p.Ho;
+  for (int e = threadIdx.x; e < floats / 4; e += 256) im2col_smem[e] = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int col = threadIdx.x; col < width; col += 256) {
-    int at = elems;   // the zero element: padding columns
+    int at = elems;   // the zero row: padding columns
     if (col < cols) {
       const int c = p.c_major ? col / taps : col % p.C, t = p.c_major ? col - c * taps : col / p.C;
       at = (c * p.KH + t / p.KW) * wp + (t % p.KW) * p.DW;
     }
-    table[col] = static_cast<unsigned short>(at);
-  }
-  // the zero and what an output pixel past a padding column may address behind it
-  for (int e = elems + threadIdx.x; e < (elems + 4) / 4 * 4; e += 256) tile[e] = 0.f;
-  const T* base = x + n * p.sN + c_begin * p.sC;
-  const int h0 = ho * p.SH - p.PH, live = nc * p.KH * wp;
-  for (int e = threadIdx.x; e < live; e += 256) {
-    int c, kh, w;
-    if (p.sC == 1) {
-      c = e % nc;
-      const int t = e / nc;
-      w = t % wp;
-      kh = t / wp;
-    } else {
-      w = e % wp;
-      const int t = e / wp;
-      kh = t % p.KH;
-      c = t / p.KH;
-    }
-    const int hi = h0 + kh * p.DH, wi = w - p.PW;
-    tile[(c * p.KH + kh) * wp + w] =
-        (hi >= 0 && hi < p.H && wi >= 0 && wi < p.W) ? to_f32<T>(base[c * p.sC + hi * p.sH + wi * p.sW]) : 0.f;
+    table[col] = static_cast<unsigned short>(at * 4);
   }
   __syncthreads();
-  const int vecs = width / 8, total = vecs * p.Wo;
+  // `fast_lanes` consecutive threads read consecutive elements of the dimension with the smaller stride (W, or C for
+  // channels-innermost strides) of one row (c, kh), or (w, kh)
+  const T* base = x + n * p.sN + c_begin * p.sC;
+  const int h0 = ho * p.SH - p.PH, w_end = min(p.W, wp - p.PW);   // input columns that some output pixel reads
+  const bool along_c = p.sC == 1;
+  const int fast = along_c ? nc : w_end, slow = (along_c ? w_end : nc) * p.KH;
+  const int f0 = threadIdx.x % fast_lanes, rows = 256 / fast_lanes;
+  for (int f = f0; f < fast; f += fast_lanes) {
+    for (int t0 = threadIdx.x / fast_lanes; t0 < slow; t0 += IM2COL_LOADS * rows) {
+      T v[IM2COL_LOADS];
+      int to[IM2COL_LOADS];
+#pragma unroll
+      for (int u = 0; u < IM2COL_LOADS; ++u) {
+        const int t = t0 + u * rows, s = t / p.KH, kh = t - s * p.KH, hi = h0 + kh * p.DH;
+        const int c = along_c ? f : s, w = along_c ? s : f;
+        to[u] = -1;
+        if (t < slow && hi >= 0 && hi < p.H) {
+          to[u] = (c * p.KH + kh) * wp + w + p.PW;
+          v[u] = __ldg(base + c * p.sC + hi * p.sH + w * p.sW);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < IM2COL_LOADS; ++u)
+        if (to[u] >= 0) tile[to[u]] = to_f32<T>(v[u]);
+    }
+  }
+  __syncthreads();
+  const int vecs = width / 8;
   __nv_bfloat16* const row0 = out + static_cast<long long>(blockIdx.x) * p.Wo * p.ldo + col0;
   __nv_bfloat16* const lo0 = LO ? out_lo + static_cast<long long>(blockIdx.x) * p.Wo * p.ldo + col0 : nullptr;
-  for (int e = threadIdx.x; e < total; e += 256) {
-    const int wo = e / vecs, v = e - wo * vecs, shift = wo * p.SW;
+  const int step_wo = 256 / vecs, step_v = 256 - step_wo * vecs;
+  int wo = threadIdx.x / vecs, v = threadIdx.x - wo * vecs;
+  while (wo < p.Wo) {
     const uint4 raw = *reinterpret_cast<const uint4*>(table + v * 8);
     const uint32_t pairs[4] = {raw.x, raw.y, raw.z, raw.w};
+    const char* from = reinterpret_cast<const char*>(tile + wo * p.SW);
     uint32_t hi[4], lo[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const int i0 = pairs[k] & 0xffffu, i1 = pairs[k] >> 16;
-      const float a = tile[i0 == elems ? elems : i0 + shift], b = tile[i1 == elems ? elems : i1 + shift];
-      const __nv_bfloat16 ha = __float2bfloat16_rn(a), hb = __float2bfloat16_rn(b);
-      hi[k] = static_cast<uint32_t>(__bfloat16_as_ushort(ha)) | (static_cast<uint32_t>(__bfloat16_as_ushort(hb)) << 16);
-      if (LO)
-        lo[k] = static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(a - __bfloat162float(ha)))) |
-                (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(b - __bfloat162float(hb)))) << 16);
+      const float a = *reinterpret_cast<const float*>(from + (pairs[k] & 0xffffu));
+      const float b = *reinterpret_cast<const float*>(from + (pairs[k] >> 16));
+      const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+      hi[k] = *reinterpret_cast<const uint32_t*>(&h);
+      if (LO) {
+        const __nv_bfloat162 l = __floats2bfloat162_rn(a - __low2float(h), b - __high2float(h));
+        lo[k] = *reinterpret_cast<const uint32_t*>(&l);
+      }
     }
     const long long at = static_cast<long long>(wo) * p.ldo + v * 8;
     *reinterpret_cast<uint4*>(row0 + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
     if (LO) *reinterpret_cast<uint4*>(lo0 + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    wo += step_wo;
+    v += step_v;
+    if (v >= vecs) {
+      v -= vecs;
+      ++wo;
+    }
   }
 }
 
-// Channels per CTA of the tile path, 0 if it does not apply: the staged rows and the column table fit `IM2COL_SMEM`,
-// every element has a 16-bit index, and each chunk starts on a multiple of eight columns.
+// Channels per CTA of the tile path, 0 if it does not apply: the staged rows and the column table fit `IM2COL_SMEM` (so a
+// byte offset has 16 bits), and each chunk starts on a multiple of eight columns.
 constexpr int IM2COL_SMEM = 44 * 1024;
 struct Im2colTile {
-  int cc, wp, smem;
+  int cc, wp, smem, fast_lanes;
 };
 Im2colTile im2col_tile_plan(const Im2colParams& p) {
+  const Im2colTile none{0, 0, 0, 0};
   const long long taps = static_cast<long long>(p.KH) * p.KW;
   const long long wp = (static_cast<long long>(p.Wo - 1) * p.SW + static_cast<long long>(p.KW - 1) * p.DW + 1) | 1;
   auto smem = [&](long long cc) {
-    return ((cc * p.KH * wp + 4) / 4 * 4) * 4 + (cc * taps + 8) * 2 + (p.ldo - static_cast<long long>(p.C) * taps) * 2;
+    return ((cc * p.KH * wp + wp + 3) / 4 * 4) * 4 + (cc * taps + 8) * 2 + (p.ldo - static_cast<long long>(p.C) * taps) * 2;
   };
-  auto fits = [&](long long cc) { return smem(cc) <= IM2COL_SMEM && cc * p.KH * wp < 65535; };
-  if (p.ldo % 8 != 0 || static_cast<long long>(p.N) * p.Ho >= (1ll << 31)) return {0, 0, 0};
+  auto fits = [&](long long cc) { return smem(cc) <= IM2COL_SMEM; };
+  if (p.ldo % 8 != 0 || static_cast<long long>(p.N) * p.Ho >= (1ll << 31)) return none;
   long long cc = p.C;
   if (!fits(cc)) {
-    if (!p.c_major) return {0, 0, 0};
+    if (!p.c_major) return none;
     cc = p.C / 8 * 8;
     while (cc > 0 && !fits(cc)) cc -= 8;
-    if (cc <= 0) return {0, 0, 0};
+    if (cc <= 0) return none;
     const long long chunks = (p.C + cc - 1) / cc;             // equal chunks
     cc = ((p.C + chunks - 1) / chunks + 7) / 8 * 8;
   }
-  if ((p.C + cc - 1) / cc > 65535) return {0, 0, 0};
-  return {static_cast<int>(cc), static_cast<int>(wp), static_cast<int>(smem(cc))};
+  if ((p.C + cc - 1) / cc > 65535) return none;
+  const long long fast = p.sC == 1 ? std::min<long long>(cc, p.C) : std::min<long long>(p.W, wp);
+  int lanes = 4;
+  while (lanes < fast && lanes < 32) lanes *= 2;
+  return {static_cast<int>(cc), static_cast<int>(wp), static_cast<int>(smem(cc)), lanes};
 }
 
 // x: 4-D conv input [N, C, H, W] (logical), any memory format.  out: [N*Ho*Wo, ld] bf16, contiguous.
@@ -518,15 +540,15 @@ void im2col_bf16(at::Tensor x, at::Tensor out, c10::optional<at::Tensor> out_lo,
                    (p.sH % 8) == 0 && (p.sN % 8) == 0 && rows < (1ll << 32) &&
                    ((reinterpret_cast<uintptr_t>(x.data_ptr()) | reinterpret_cast<uintptr_t>(out_p)) & 15) == 0;
   const bool aligned = ((reinterpret_cast<uintptr_t>(out_p) | reinterpret_cast<uintptr_t>(lo_p)) & 15) == 0;
-  const Im2colTile tile = (vec || !aligned) ? Im2colTile{0, 0, 0} : im2col_tile_plan(p);
+  const Im2colTile tile = (vec || !aligned) ? Im2colTile{0, 0, 0, 0} : im2col_tile_plan(p);
   auto run = [&](auto* from) {
     using T = std::remove_const_t<std::remove_pointer_t<decltype(from)>>;
     if (tile.cc > 0) {
       const dim3 grid(static_cast<unsigned>(static_cast<long long>(p.N) * p.Ho), (p.C + tile.cc - 1) / tile.cc);
       if (lo_p != nullptr)
-        im2col_tile_kernel<T, true><<<grid, 256, tile.smem, stream>>>(from, out_p, lo_p, p, tile.cc, tile.wp);
+        im2col_tile_kernel<T, true><<<grid, 256, tile.smem, stream>>>(from, out_p, lo_p, p, tile.cc, tile.wp, tile.fast_lanes);
       else
-        im2col_tile_kernel<T, false><<<grid, 256, tile.smem, stream>>>(from, out_p, nullptr, p, tile.cc, tile.wp);
+        im2col_tile_kernel<T, false><<<grid, 256, tile.smem, stream>>>(from, out_p, nullptr, p, tile.cc, tile.wp, tile.fast_lanes);
     } else {
       const int blocks = static_cast<int>(std::min<long long>((rows * p.ldo + 255) / 256, 148 * 32));
       im2col_generic_kernel<T><<<blocks, 256, 0, stream>>>(from, out_p, lo_p, p);
