@@ -23,7 +23,6 @@ namespace {
 constexpr int GROUPS = 8;    // channel groups of 8 channels per CTA -> 64 channels
 constexpr int LANES = 32;    // row lanes per CTA
 constexpr int THREADS = GROUPS * LANES;
-constexpr int SUMS_CTAS = 4, BWD_SUMS_CTAS = 3;   // resident on an SM: 64 and 80 registers per thread
 constexpr int UNROLL = 8;    // independent 16-byte loads in flight per thread (forward sums)
 
 __device__ __forceinline__ void unpack8(const uint4& raw, float (&out)[8]) {
@@ -70,7 +69,7 @@ __device__ __forceinline__ void cta_reduce_store(float (&first)[8], float (&seco
   }
 }
 
-__global__ void __launch_bounds__(THREADS, SUMS_CTAS)
+__global__ void __launch_bounds__(THREADS)
 bn_sums(const __nv_bfloat16* __restrict__ x, float* __restrict__ part, long long rows, int channels,
         long long rows_per_split) {
   const int group = threadIdx.x % GROUPS;
@@ -236,7 +235,7 @@ bn_dx(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
 }
 
 template <int MASK>
-__global__ void __launch_bounds__(THREADS, BWD_SUMS_CTAS)
+__global__ void __launch_bounds__(THREADS)
 bn_bwd_sums(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
             const __nv_bfloat16* __restrict__ y, const float* __restrict__ mean,
             const float* __restrict__ invstd, const float* __restrict__ weight, const float* __restrict__ bias,
@@ -363,9 +362,7 @@ struct Shape {
   long long rows_per_split;
 };
 
-// `per_sm`: CTAs of the sums kernel that an SM holds; the splits fill one wave of them.  A second, part-filled wave cost as
-// much as the first (784 CTAs for 592 or 444 places at 32 x 56 x 56 x 256).
-Shape plan(const at::Tensor& x, int per_sm) {
+Shape plan(const at::Tensor& x) {
   TORCH_CHECK(x.is_cuda() && x.dim() == 4 && x.scalar_type() == at::kBFloat16 &&
                   x.is_contiguous(at::MemoryFormat::ChannelsLast),
               "expected a 4-d channels_last bf16 CUDA tensor");
@@ -375,8 +372,8 @@ Shape plan(const at::Tensor& x, int per_sm) {
   TORCH_CHECK(s.channels % 8 == 0 && s.rows > 0, "the channel count must be a multiple of 8");
   TORCH_CHECK((reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0, "16-byte alignment required");
   s.chunks = (s.channels + GROUPS * 8 - 1) / (GROUPS * 8);
-  long long want = 148LL * per_sm / s.chunks;
-  long long most = (s.rows + UNROLL * LANES - 1) / (UNROLL * LANES);   // one unrolled trip each
+  long long want = (148 * 8 + s.chunks - 1) / s.chunks;                   // ~8 CTAs per SM in total
+  long long most = (s.rows + 2 * UNROLL * LANES - 1) / (2 * UNROLL * LANES);  // >= 2 unrolled trips each
   long long splits = std::max<long long>(1, std::min(want, most));
   s.rows_per_split = (s.rows + splits - 1) / splits;
   s.splits = static_cast<int>((s.rows + s.rows_per_split - 1) / s.rows_per_split);
@@ -408,7 +405,7 @@ std::vector<at::Tensor> bn_forward_train(at::Tensor x, at::Tensor weight, at::Te
                                          c10::optional<at::Tensor> running_var,
                                          c10::optional<at::Tensor> num_batches_tracked, double momentum,
                                          double eps, c10::optional<at::Tensor> residual, bool relu) {
-  const Shape s = plan(x, SUMS_CTAS);
+  const Shape s = plan(x);
   check_vec(weight, s.channels, "weight");
   check_vec(bias, s.channels, "bias");
   float *rm = nullptr, *rv = nullptr;
@@ -469,7 +466,7 @@ std::vector<at::Tensor> bn_forward_train(at::Tensor x, at::Tensor weight, at::Te
 std::vector<at::Tensor> bn_backward_train(at::Tensor x, at::Tensor dy, at::Tensor weight, at::Tensor mean,
                                           at::Tensor invstd, c10::optional<at::Tensor> y, bool want_dres,
                                           c10::optional<at::Tensor> bias_for_mask) {
-  const Shape s = plan(x, BWD_SUMS_CTAS);
+  const Shape s = plan(x);
   check_like(dy, x, "dy");
   check_vec(weight, s.channels, "weight");
   check_vec(mean, s.channels, "mean");
