@@ -62,6 +62,7 @@ void symm_reduce_slots(at::Tensor local, at::Tensor table, int64_t world, int64_
 void chol_inverse(std::vector<at::Tensor> mats, std::vector<at::Tensor> outs, at::Tensor damping);
 void chol_inverse_tc(std::vector<at::Tensor> mats, std::vector<at::Tensor> outs, at::Tensor damping);
 void chol_inverse_tc_clear_cache();
+std::pair<int64_t, int64_t> chol_inverse_tc_cache_info();
 std::vector<at::Tensor> jacobi_eigh(at::Tensor mats, bool want_vectors);
 void ln_unitwise_stats(at::Tensor y, at::Tensor g, at::Tensor weight, at::Tensor bias, at::Tensor stats, double alpha,
                        double beta);
@@ -129,6 +130,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("chol_inverse", &b200::chol_inverse, "grouped damped SPD inverse (fp32, CUDA cores)");
   m.def("chol_inverse_tc", &b200::chol_inverse_tc, "grouped damped SPD inverse (fp32-accurate, tensor cores)");
   m.def("chol_inverse_tc_clear_cache", &b200::chol_inverse_tc_clear_cache);
+  m.def("chol_inverse_tc_cache_info", &b200::chol_inverse_tc_cache_info, "(entries, entries that captured graphs keep)");
   m.def("jacobi_eigh", &b200::jacobi_eigh, "batched symmetric eigendecomposition, n <= 128 (parallel cyclic Jacobi)");
   m.def("ln_unitwise_stats", &b200::ln_unitwise_stats);
   m.def("unitwise_inverse_mt", &b200::unitwise_inverse_mt);

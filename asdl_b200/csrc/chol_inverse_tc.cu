@@ -21,15 +21,15 @@
 // All matrices of a call advance through the same launches ("grouped"): a launch's work list
 // holds the tiles of every matrix that has work at that step.  Problem tables, work lists and the
 // bf16 split buffers depend only on the addresses and sizes of the matrices; they are built once
-// and cached, so a repeated call (the K-FAC state) issues no host-to-device copy and can be
-// captured in a CUDA graph.  Inputs are not modified; a non-positive pivot sets the status word to
+// and cached (prepared_cache.h), so a repeated call (the K-FAC state) issues no host-to-device copy
+// and can be captured in a CUDA graph, which then keeps them.  Inputs are not modified; a non-positive pivot sets the status word to
 // ERR_NOT_SPD and the factorisation continues with pivot 1.
 //
 // Stands in for asdl/utils.py:91-96 (torch.linalg.cholesky + cholesky_inverse).
 #include <cstring>
-#include <list>
 
 #include "gemm2_host.h"
+#include "prepared_cache.h"
 
 namespace b200 {
 
@@ -283,11 +283,11 @@ struct Prepared {
   std::vector<Launch> launches;
   int count = 0;
   int prepare_blocks = 1;   // row groups of the prepare kernel: the largest matrix has 8 rows per block
+  GraphPins pins;
 };
 
 std::mutex g_cache_mutex;
-std::list<Prepared> g_cache;
-constexpr size_t kCacheEntries = 4;
+PreparedCache<Prepared, 4> g_cache;   // four sets of matrices beside those that graphs refer to
 
 int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 
@@ -346,7 +346,8 @@ void chol_inverse_tc(std::vector<at::Tensor> mats, std::vector<at::Tensor> outs,
                   damping.numel() == count, "damping must be a CUDA fp32 vector with one entry per matrix");
   const int dev = mats[0].get_device();
   c10::cuda::CUDAGuard guard(dev);
-  auto stream = at::cuda::getCurrentCUDAStream(dev).stream();
+  const auto current = at::cuda::getCurrentCUDAStream(dev);
+  const cudaStream_t stream = current.stream();
   std::vector<const void*> key;
   key.reserve(4 * count + 1);
   key.push_back(reinterpret_cast<const void*>(static_cast<intptr_t>(dev)));
@@ -366,9 +367,7 @@ void chol_inverse_tc(std::vector<at::Tensor> mats, std::vector<at::Tensor> outs,
   }
 
   std::lock_guard<std::mutex> lock(g_cache_mutex);
-  Prepared* prep = nullptr;
-  for (auto& p : g_cache)
-    if (p.key == key) prep = &p;
+  Prepared* prep = g_cache.find(key);
   if (prep == nullptr) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     B200_CUDA_CHECK(cudaStreamIsCapturing(stream, &cap));
@@ -501,10 +500,9 @@ void chol_inverse_tc(std::vector<at::Tensor> mats, std::vector<at::Tensor> outs,
     P.d_work = upload(work.data(), work.size() * sizeof(GemmWork2));
     TORCH_CHECK((reinterpret_cast<uintptr_t>(P.d_probs.data_ptr()) & 63) == 0, "problem table is not 64-byte aligned");
     B200_CUDA_CHECK(cudaStreamSynchronize(stream));  // the pinned staging buffers are released after this
-    if (g_cache.size() >= kCacheEntries) g_cache.pop_front();
-    g_cache.push_back(std::move(P));
-    prep = &g_cache.back();
+    prep = g_cache.insert(std::move(P));
   }
+  prep->pins.use(current, {prep->splits, prep->d_mats, prep->d_probs, prep->d_work});
 
   const TcMat* dm = reinterpret_cast<const TcMat*>(prep->d_mats.data_ptr());
   const GemmProblem2* dp = reinterpret_cast<const GemmProblem2*>(prep->d_probs.data_ptr());
@@ -524,10 +522,16 @@ void chol_inverse_tc(std::vector<at::Tensor> mats, std::vector<at::Tensor> outs,
   B200_CUDA_CHECK(cudaGetLastError());
 }
 
-// Drops the cached tables and split buffers of the tensor-core inverse.
+// Drops the cached tables and split buffers of the tensor-core inverse that no captured graph refers to.
 void chol_inverse_tc_clear_cache() {
   std::lock_guard<std::mutex> lock(g_cache_mutex);
-  g_cache.clear();
+  g_cache.drop_idle();
+}
+
+// (entries, entries that captured graphs refer to)
+std::pair<int64_t, int64_t> chol_inverse_tc_cache_info() {
+  std::lock_guard<std::mutex> lock(g_cache_mutex);
+  return {static_cast<int64_t>(g_cache.size()), static_cast<int64_t>(g_cache.pinned())};
 }
 
 }  // namespace b200
