@@ -13,6 +13,7 @@
 #include <cstring>
 
 #include "host_utils.h"
+#include "prepared_cache.h"
 #include "sm100_ptx.cuh"
 
 namespace b200 {
@@ -326,6 +327,25 @@ __global__ void __launch_bounds__(256) lauum_kernel(const CholMat* mats) {
 }
 
 // ---- host ------------------------------------------------------------------------------------
+// The descriptor table and the sort permutation depend only on the addresses and sizes of the matrices.  Callers with
+// persistent buffers (the K-FAC state) repeat the same call, so both are cached on the device (prepared_cache.h): a
+// repeated call issues no host-to-device copy and can be captured in a CUDA graph, which then keeps them (the scratch
+// buffers come from the graph's memory pool).
+struct CholPrepared {
+  std::vector<const void*> key;
+  at::Tensor desc_static;   // CholMat table without the per-call scratch pointers
+  at::Tensor perm;
+  GraphPins pins;
+};
+static std::mutex g_chol_cache_mutex;
+static PreparedCache<CholPrepared, 16> g_chol_cache;
+
+// (entries, entries that captured graphs refer to)
+std::pair<int64_t, int64_t> chol_inverse_cache_info() {
+  std::lock_guard<std::mutex> lock(g_chol_cache_mutex);
+  return {static_cast<int64_t>(g_chol_cache.size()), static_cast<int64_t>(g_chol_cache.pinned())};
+}
+
 void chol_inverse(std::vector<at::Tensor> mats, std::vector<at::Tensor> outs, at::Tensor damping) {
   const int count = static_cast<int>(mats.size());
   TORCH_CHECK(count > 0 && outs.size() == mats.size(), "mats and outs must have the same length");
@@ -333,7 +353,8 @@ void chol_inverse(std::vector<at::Tensor> mats, std::vector<at::Tensor> outs, at
                   damping.numel() == count, "damping must be a CUDA fp32 vector with one entry per matrix");
   const int dev = mats[0].get_device();
   c10::cuda::CUDAGuard guard(dev);
-  auto stream = at::cuda::getCurrentCUDAStream(dev).stream();
+  const auto current = at::cuda::getCurrentCUDAStream(dev);
+  const cudaStream_t stream = current.stream();
 
   // process the matrices in order of decreasing size so that "still active at block k" is a prefix
   std::vector<int> order(count);
@@ -378,17 +399,6 @@ void chol_inverse(std::vector<at::Tensor> mats, std::vector<at::Tensor> outs, at
     d_off += static_cast<size_t>(M.nb) * CB * CB;
     nb_max = std::max(nb_max, M.nb);
   }
-  // The descriptor table and the sort permutation depend only on the addresses and sizes of the
-  // matrices.  Callers with persistent buffers (the K-FAC state) repeat the same call, so both are
-  // cached on the device: a repeated call issues no host-to-device copy and can be captured in a
-  // CUDA graph (the scratch buffers then come from the graph's memory pool).
-  struct Prepared {
-    std::vector<const void*> key;
-    at::Tensor desc_static;   // CholMat table without the per-call scratch pointers
-    at::Tensor perm;
-  };
-  static std::mutex cache_mutex;
-  static std::vector<Prepared> cache;
   std::vector<const void*> key;
   key.reserve(2 * count + 1);
   key.push_back(reinterpret_cast<const void*>(static_cast<intptr_t>(dev)));
@@ -400,13 +410,9 @@ void chol_inverse(std::vector<at::Tensor> mats, std::vector<at::Tensor> outs, at
   }
   at::Tensor desc, perm_t;
   {
-    std::lock_guard<std::mutex> lock(cache_mutex);
-    for (auto& p : cache)
-      if (p.key == key) {
-        desc = p.desc_static;
-        perm_t = p.perm;
-      }
-    if (!desc.defined()) {
+    std::lock_guard<std::mutex> lock(g_chol_cache_mutex);
+    CholPrepared* prep = g_chol_cache.find(key);
+    if (prep == nullptr) {
       // X / D are stored as offsets (in floats) from the scratch bases; the prepare kernel turns them
       // into pointers for this call
       std::vector<CholMat> rel = host;
@@ -417,11 +423,15 @@ void chol_inverse(std::vector<at::Tensor> mats, std::vector<at::Tensor> outs, at
       at::Tensor staged = at::empty({static_cast<int64_t>(count * sizeof(CholMat))},
                                     at::TensorOptions().dtype(at::kByte).pinned_memory(true));
       std::memcpy(staged.data_ptr(), rel.data(), count * sizeof(CholMat));
-      desc = staged.to(at::Device(at::kCUDA, dev));
-      perm_t = at::tensor(perm, at::TensorOptions().dtype(at::kLong)).to(damping.device());
-      if (cache.size() >= 16) cache.erase(cache.begin());
-      cache.push_back({key, desc, perm_t});
+      CholPrepared fresh;
+      fresh.key = key;
+      fresh.desc_static = staged.to(at::Device(at::kCUDA, dev));
+      fresh.perm = at::tensor(perm, at::TensorOptions().dtype(at::kLong)).to(damping.device());
+      prep = g_chol_cache.insert(std::move(fresh));
     }
+    desc = prep->desc_static;
+    perm_t = prep->perm;
+    prep->pins.use(current, {desc, perm_t});
   }
   // per-call table: the cached one with the scratch bases of this call added
   at::Tensor desc_call = at::empty_like(desc);

@@ -27,7 +27,8 @@ def _check(mats, outs, damping):
         assert (o.double() - want).abs().max() <= bound
 
 
-@pytest.mark.parametrize('backend,info,capacity', [('tensor_core', 'chol_inverse_tc_cache_info', 4)])
+@pytest.mark.parametrize('backend,info,capacity', [('tensor_core', 'chol_inverse_tc_cache_info', 4),
+                                                    ('cuda_core', 'chol_inverse_cache_info', 16)])
 def test_a_captured_inverse_keeps_its_tables(monkeypatch, backend, info, capacity):
     monkeypatch.setattr(ops, 'CHOLESKY_BACKEND', backend)
     info = getattr(ops.extension(), info)
@@ -65,7 +66,7 @@ def test_a_captured_inverse_keeps_its_tables(monkeypatch, backend, info, capacit
     assert info()[0] - info()[1] <= capacity
 
 
-@pytest.mark.parametrize('backend', ['tensor_core'])
+@pytest.mark.parametrize('backend', ['tensor_core', 'cuda_core'])
 def test_tables_evicted_while_another_stream_uses_them(monkeypatch, backend):
     monkeypatch.setattr(ops, 'CHOLESKY_BACKEND', backend)
     mats = [_spd(n, 60 + n) for n in (260, 500, 64)]
