@@ -88,6 +88,18 @@ def test_kron_apply_reads_either_order_of_a_symmetric_factor():
     assert torch.equal(row, col)
 
 
+@pytest.mark.parametrize('dtype', [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize('m,n', [(1, 1), (8, 24), (72, 130), (257, 129), (129, 640)])
+def test_kron_apply_gives_the_same_bits_for_either_order_of_storage(m, n, dtype):
+    # not symmetric, so that a factor read as its transpose shows: inverses are symmetric up to their last bits only
+    left, right = (torch.randn(k, k, device=DEV, generator=_gen(4 + k)).to(dtype) for k in (m, n))
+    mid = torch.randn(m, n, device=DEV, generator=_gen(4)).to(dtype)
+    row = ops.kron_apply(left, mid, right)
+    for a in (left, left.T.contiguous().T):
+        for b in (right, right.T.contiguous().T):
+            assert torch.equal(ops.kron_apply(a, mid, b), row)
+
+
 @pytest.mark.parametrize('n', [1, 31, 32, 33, 64, 65, 96, 97, 127, 128, 129, 160, 225, 257])
 def test_inverse_at_the_edges_of_the_diagonal_stages(n):
     x = torch.randn(2 * n, n, device=DEV, generator=_gen(19))
