@@ -168,6 +168,7 @@ void cast_split3(at::Tensor src, at::Tensor hi, at::Tensor mid, at::Tensor lo) {
   const long long rows = src.size(0);
   const long long ldo = hi.size(1);
   if (rows == 0) return;
+  TORCH_CHECK(ldo > 0, "the outputs have no columns");
   auto stream = at::cuda::getCurrentCUDAStream().stream();
   launch_cast<float, 3>(src.data_ptr<float>(), src.stride(0), 1.f, reinterpret_cast<__nv_bfloat16*>(hi.data_ptr()),
                         reinterpret_cast<__nv_bfloat16*>(mid.data_ptr()), reinterpret_cast<__nv_bfloat16*>(lo.data_ptr()),
@@ -525,6 +526,7 @@ void im2col_bf16(at::Tensor x, at::Tensor out, c10::optional<at::Tensor> out_lo,
   TORCH_CHECK(out.size(0) == rows && p.ldo >= static_cast<long long>(p.C) * p.KH * p.KW,
               "out has the wrong shape");
   if (rows == 0) return;
+  TORCH_CHECK(p.ldo > 0, "the patch matrix has no columns");
   c10::cuda::CUDAGuard guard(x.get_device());
   auto stream = at::cuda::getCurrentCUDAStream().stream();
   auto* out_p = reinterpret_cast<__nv_bfloat16*>(out.data_ptr());

@@ -38,6 +38,15 @@ def test_cast_parts(ext, dtype, rows, n, ld, offset):
     assert torch.equal(one, (want * 0.5).to(torch.bfloat16))
 
 
+def test_outputs_without_columns_are_refused(ext):
+    parts = [torch.empty(3, 0, device=DEV, dtype=torch.bfloat16) for _ in range(3)]
+    with pytest.raises(RuntimeError, match='no columns'):
+        ext.cast_split3(torch.empty(3, 0, device=DEV), *parts)
+    x = torch.empty(1, 0, 4, 4, device=DEV, dtype=torch.bfloat16).as_strided((1, 0, 4, 4), (0, 1, 0, 0))
+    with pytest.raises(RuntimeError, match='no columns'):
+        ext.im2col_bf16(x, torch.empty(16, 0, device=DEV, dtype=torch.bfloat16), None, [1, 1], [1, 1], [0, 0], [1, 1], False)
+
+
 @pytest.mark.parametrize('dtype', [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize('cfg', [  # n, c, h, w, kernel, stride, padding, dilation
     (2, 8, 9, 7, 3, 1, 1, 1), (1, 3, 12, 11, 7, 2, 3, 1), (2, 24, 8, 8, 3, 2, 1, 1), (1, 5, 13, 13, 3, 1, 2, 2),
