@@ -173,7 +173,7 @@ bn_apply(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ 
          long long rows, int channels, int groups, int lanes) {
   constexpr int APPLY_ROWS = RES ? APPLY_ROWS_RES : APPLY_ROWS_PLAIN;
   const int lane = threadIdx.x / groups;
-  const int c0 = (blockIdx.y * groups + threadIdx.x % groups) * 8;
+  const int c0 = ((blockIdx.z * gridDim.y + blockIdx.y) * groups + threadIdx.x % groups) * 8;
   if (lane >= lanes || c0 >= channels) return;
   float a[8], b[8];
   load8(scale + c0, a);
@@ -227,7 +227,7 @@ bn_dx(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
       const float* __restrict__ k_const, __nv_bfloat16* __restrict__ dx, __nv_bfloat16* __restrict__ dres,
       long long rows, int channels, int groups, int lanes) {
   const int lane = threadIdx.x / groups;
-  const int c0 = (blockIdx.y * groups + threadIdx.x % groups) * 8;
+  const int c0 = ((blockIdx.z * gridDim.y + blockIdx.y) * groups + threadIdx.x % groups) * 8;
   if (lane >= lanes || c0 >= channels) return;
   float a[8], b[8], c[8], sc[8], sh[8];
   load8(k_dy + c0, a);
@@ -479,7 +479,7 @@ std::vector<at::Tensor> bn_forward_train(at::Tensor x, at::Tensor weight, at::Te
       invstd.data_ptr<float>(), coef.data_ptr<float>(), tracked, s.channels, s.splits, s.rows,
       static_cast<float>(momentum), static_cast<float>(eps));
   const Walk w = walk_plan(s.channels / 8);
-  const dim3 grid = walk_grid(w, (s.rows + 1) / 2, 4);   // at least two rows a thread
+  const dim3 grid = walk_grid_layers(w, (s.rows + 1) / 2, 4);   // at least two rows a thread
   const float* scale = coef.data_ptr<float>();
   const float* shift = scale + s.channels;
   if (rp != nullptr && relu)
@@ -550,7 +550,7 @@ std::vector<at::Tensor> bn_backward_train(at::Tensor x, at::Tensor dy, at::Tenso
       part.data_ptr<float>(), wp, bp, mp, ip, dweight.data_ptr<float>(), dbias.data_ptr<float>(), coef.data_ptr<float>(),
       s.channels, s.splits, s.rows);
   const Walk w = walk_plan(s.channels / 8);
-  const dim3 grid = walk_grid(w, (s.rows + 1) / 2, 3);
+  const dim3 grid = walk_grid_layers(w, (s.rows + 1) / 2, 3);
   const float* k = coef.data_ptr<float>();
   const float *sc = k, *sh = k + s.channels;
   const float *k_dy = k + 2 * s.channels, *k_x = k + 3 * s.channels, *k_c = k + 4 * s.channels;

@@ -75,7 +75,7 @@ cast_parts_kernel(const T* __restrict__ src, long long lds, float scale, __nv_bf
   }
 }
 
-// The same for outputs whose rows are not 16-byte aligned: one element per thread.
+// The same for outputs whose rows are not 16-byte aligned, and for rows that walk_grid does not take: one element per thread.
 template <typename T, int PARTS>
 __global__ void cast_parts_scalar_kernel(const T* __restrict__ src, long long lds, float scale,
                                          __nv_bfloat16* __restrict__ p0, __nv_bfloat16* __restrict__ p1,
@@ -101,11 +101,13 @@ void launch_cast(const T* src, long long lds, float scale, __nv_bfloat16* p0, __
                  long long ldo, long long rows, int n, cudaStream_t stream) {
   const uintptr_t outs = reinterpret_cast<uintptr_t>(p0) | (PARTS > 1 ? reinterpret_cast<uintptr_t>(p1) : 0) |
                          (PARTS > 2 ? reinterpret_cast<uintptr_t>(p2) : 0);
-  if ((ldo & 7) != 0 || (outs & 15) != 0) {
+  // rows of more than 134 million columns have more CTAs across than a grid takes on y
+  const bool vec_out = (ldo & 7) == 0 && (outs & 15) == 0;
+  const Walk w = vec_out ? walk_plan(static_cast<int>(ldo / 8)) : Walk{};
+  if (!vec_out || w.chunks > MAX_WALK_CHUNKS) {
     const int blocks = static_cast<int>(std::min<long long>((rows * ldo + 255) / 256, 148 * 16));
     cast_parts_scalar_kernel<T, PARTS><<<blocks, 256, 0, stream>>>(src, lds, scale, p0, p1, p2, ldo, rows, n);
   } else {
-    const Walk w = walk_plan(static_cast<int>(ldo / 8));
     const dim3 grid = walk_grid(w, rows, 6);
     const bool vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && (lds * sizeof(T)) % 16 == 0;
     if (vec)
@@ -540,7 +542,8 @@ void im2col_bf16(at::Tensor x, at::Tensor out, c10::optional<at::Tensor> out_lo,
   const bool vec = lo_p == nullptr && (!c_major || p.KH * p.KW == 1) && x.scalar_type() == at::kBFloat16 && p.sC == 1 && (p.C % 8) == 0 &&
                    p.ldo == static_cast<long long>(p.C) * p.KH * p.KW && (p.sW % 8) == 0 &&
                    (p.sH % 8) == 0 && (p.sN % 8) == 0 && rows < (1ll << 32) &&
-                   ((reinterpret_cast<uintptr_t>(x.data_ptr()) | reinterpret_cast<uintptr_t>(out_p)) & 15) == 0;
+                   ((reinterpret_cast<uintptr_t>(x.data_ptr()) | reinterpret_cast<uintptr_t>(out_p)) & 15) == 0 &&
+                   p.ldo <= MAX_WALK_CHUNKS * 1024ll;   // below, a CTA covers half its vectors or more
   const bool aligned = ((reinterpret_cast<uintptr_t>(out_p) | reinterpret_cast<uintptr_t>(lo_p)) & 15) == 0;
   const Im2colTile tile = (vec || !aligned) ? Im2colTile{0, 0, 0, 0} : im2col_tile_plan(p);
   auto run = [&](auto* from) {

@@ -28,11 +28,22 @@ inline Walk walk_plan(int vecs) {
   return best;
 }
 
-// One wave of CTAs (`per_sm` resident on each SM), fewer where a thread would have no row.
+// One wave of CTAs (`per_sm` resident on each SM), fewer where a thread would have no row.  The CTAs across a row are on y,
+// at most MAX_WALK_CHUNKS of them.  On x they cost 25 % where the loads are scalar (16 x 1000003 fp32 -> hi, lo: 25.0 and
+// 31.3 us): neighbouring CTAs then share a row instead of a column.
+constexpr int MAX_WALK_CHUNKS = 65535;
 inline dim3 walk_grid(const Walk& w, long long rows, int per_sm) {
   const long long most = (rows + w.lanes - 1) / w.lanes;
   const long long wave = std::max<long long>(1, (148LL * per_sm + w.chunks - 1) / w.chunks);
   return dim3(static_cast<unsigned>(std::min(most, wave)), static_cast<unsigned>(w.chunks));
+}
+
+// The same for any number of them: the CTA across a row is blockIdx.z * gridDim.y + blockIdx.y, the last ones may have no work.
+inline dim3 walk_grid_layers(const Walk& w, long long rows, int per_sm) {
+  dim3 grid = walk_grid(w, rows, per_sm);
+  grid.z = (grid.y + MAX_WALK_CHUNKS - 1) / MAX_WALK_CHUNKS;
+  grid.y = (grid.y + grid.z - 1) / grid.z;
+  return grid;
 }
 
 }  // namespace b200

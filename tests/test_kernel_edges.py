@@ -38,6 +38,29 @@ def test_cast_parts(ext, dtype, rows, n, ld, offset):
     assert torch.equal(one, (want * 0.5).to(torch.bfloat16))
 
 
+@pytest.mark.parametrize('rows', [1, 3])
+def test_cast_of_more_columns_than_a_grid_has_blocks_on_y(ext, rows):
+    n = 65535 * 2048 + 11
+    x = torch.randn(rows, n, device=DEV, generator=_gen(20))
+    hi, lo = (torch.full((rows, (n + 7) // 8 * 8), float('nan'), device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    ext.cast_pad_bf16(x, hi, lo, 1.0)
+    assert torch.equal(hi[:, :n], x.to(torch.bfloat16)) and not hi[:, n:].any()
+    assert torch.equal(lo[:, :n], (x - hi[:, :n].float()).to(torch.bfloat16)) and not lo[:, n:].any()
+
+
+def test_batch_norm_of_more_channels_than_a_grid_has_blocks_on_y():
+    c = 65535 * 2048 + 8
+    x = torch.randn(2, c, 1, 1, device=DEV, generator=_gen(21), dtype=torch.bfloat16)
+    x = x.contiguous(memory_format=torch.channels_last).requires_grad_(True)
+    weight, bias = torch.full((c,), 0.5, device=DEV), torch.full((c,), 0.25, device=DEV)
+    y = ops.batch_norm_train(x, weight, bias)
+    dx, = torch.autograd.grad(y, x, torch.ones_like(y))
+    d = (x[0] - x[1]).detach().float().flatten() / 2
+    want = 0.25 + 0.5 * d * torch.rsqrt(d * d + 1e-5)
+    assert (y[0].flatten() - want).abs().max() <= 2.0 ** -8     # one bf16 rounding of values below 1
+    assert dx.abs().max() <= 1e-3                               # a constant gradient has no component along x or 1
+
+
 def test_outputs_without_columns_are_refused(ext):
     parts = [torch.empty(3, 0, device=DEV, dtype=torch.bfloat16) for _ in range(3)]
     with pytest.raises(RuntimeError, match='no columns'):
