@@ -38,6 +38,17 @@ def test_cast_parts(ext, dtype, rows, n, ld, offset):
     assert torch.equal(one, (want * 0.5).to(torch.bfloat16))
 
 
+@pytest.mark.parametrize('scale', [float('inf'), float('nan'), -1.0])
+@pytest.mark.parametrize('dtype', [torch.float32, torch.bfloat16])
+def test_cast_pads_with_zeros_whatever_the_scale(ext, dtype, scale):
+    x = torch.ones(5, 11, device=DEV, dtype=dtype)
+    hi, lo = (torch.full((5, 24), float('nan'), device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    ext.cast_pad_bf16(x, hi, lo, scale)
+    assert torch.equal(hi[:, :11], torch.full((5, 11), scale, device=DEV).to(torch.bfloat16)) or scale != scale
+    for part in (hi, lo):
+        assert not part[:, 11:].view(torch.int16).any()
+
+
 @pytest.mark.parametrize('rows', [1, 3])
 def test_cast_of_more_columns_than_a_grid_has_blocks_on_y(ext, rows):
     n = 65535 * 2048 + 11
