@@ -558,9 +558,9 @@ class _BatchNormTrain(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy, _dmean, _dinvstd):
-        if dy is None:
-            return (None,) * 10
         x, weight, mean, invstd, *rest = ctx.saved_tensors
+        if dy is None:   # an undefined gradient of y counts as zeros
+            dy = torch.zeros_like(x)
         if not dy.is_contiguous(memory_format=torch.channels_last):
             dy = dy.contiguous(memory_format=torch.channels_last)
         y = rest[0] if (ctx.relu and not ctx.mask_from_x) else None

@@ -222,3 +222,27 @@ def test_batch_norm_row_walk(n, c, h, w, relu, residual):
     # bf16 results: 2^-8 of the value; of the largest value where terms cancel (y near 0, dx of two rows)
     for got, ref in zip((y,) + grads, (yd,) + want):
         assert ((got.double() - ref).abs() <= 2.0 ** -8 * (ref.abs() + ref.abs().max()) + 1e-5).all()
+
+
+class _Cut(torch.autograd.Function):
+    """Identity whose backward gives no gradient."""
+
+    @staticmethod
+    def forward(ctx, x):
+        return x.view_as(x)
+
+    @staticmethod
+    def backward(ctx, dy):
+        return None
+
+
+@pytest.mark.parametrize('relu', [False, True])
+def test_batch_norm_counts_an_undefined_gradient_as_zeros(relu):
+    def act(seed):
+        x = torch.randn(2, 16, 3, 3, device=DEV, generator=_gen(seed)).to(torch.bfloat16)
+        return x.contiguous(memory_format=torch.channels_last).requires_grad_(True)
+    x, res = act(22), act(23)
+    weight, bias = (torch.ones(16, device=DEV, requires_grad=True) for _ in range(2))
+    _Cut.apply(ops.batch_norm_train(x, weight, bias, residual=res, relu=relu)).sum().backward()
+    for leaf in (x, res, weight, bias):
+        assert leaf.grad is not None and not leaf.grad.any()
