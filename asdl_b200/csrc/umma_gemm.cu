@@ -1,6 +1,8 @@
 // Host launcher for the persistent tcgen05 TN-GEMM / SYRK kernel (see umma_gemm2.cuh).
 #include "gemm2_host.h"
 
+#include <c10/cuda/CUDACachingAllocator.h>
+
 #include <algorithm>
 #include <unordered_map>
 
@@ -10,11 +12,12 @@ namespace {
 
 // Split-K partials of single launches go through one scratch buffer per device, used as a ring.
 // Launches on one stream reuse it in order; a launch on another stream first waits for the
-// stream that used the ring last, so two streams never overlap on it.
+// stream that used the ring last, so two streams never overlap on it.  A launch under capture does not
+// use it: its partials come from the graph's memory pool, which nothing outside of the graph writes
+// and which lives as long as the graph (the ring is replaced by a larger one when a product needs it).
 struct Ring {
   size_t off = 0;
-  cudaStream_t last = nullptr;
-  bool used = false;
+  c10::optional<c10::cuda::CUDAStream> last;
   cudaEvent_t ev = nullptr;
 };
 Ring g_scratch_ring[16];
@@ -206,28 +209,42 @@ void gemm_fill_problem(GemmProblem2& P, const std::vector<at::Tensor>& a_segs,
 static bool needs_ws(const GemmProblem2& P) { return P.nsplit > 1 && !(P.flags & G2F_ATOMIC); }
 static int tile_width(const GemmProblem2& P) { return (P.flags & (G2F_WIDE | G2F_PAIR)) ? 256 : 128; }
 
-void gemm_attach_scratch(GemmProblem2& P, int dev, cudaStream_t stream) {
+// Replaces the ring of a device by a larger one; the old one is not reused before its last user has passed.
+static void grow_ring(int dev, size_t nfloats) {
   DeviceState& st = device_state(dev);
-  P.status = st.status.data_ptr<int>();
-  const int slot = dev & 15;
-  if (needs_ws(P)) {
-    const size_t need = static_cast<size_t>(P.ntiles) * P.nsplit * G2_BM * tile_width(P);
-    const size_t cap_min = need * 4;
-    float* base = ensure_scratch(dev, cap_min);
-    const size_t cap = static_cast<size_t>(device_state(dev).scratch.numel());
-    Ring& sr = g_scratch_ring[slot];
-    if (sr.used && sr.last != stream && !stream_is_capturing(stream) && !stream_is_capturing(sr.last)) {
-      // another stream used the ring last: order this launch after that stream's work
-      if (sr.ev == nullptr) B200_CUDA_CHECK(cudaEventCreateWithFlags(&sr.ev, cudaEventDisableTiming));
-      B200_CUDA_CHECK(cudaEventRecord(sr.ev, sr.last));
-      B200_CUDA_CHECK(cudaStreamWaitEvent(stream, sr.ev, 0));
-    }
-    sr.last = stream;
-    sr.used = true;
-    if (sr.off + need > cap) sr.off = 0;
-    P.ws = base + sr.off;
-    sr.off += need;
+  const size_t now = st.scratch.defined() ? static_cast<size_t>(st.scratch.numel()) : 0;
+  if (now >= nfloats) return;
+  Ring& sr = g_scratch_ring[dev & 15];
+  if (now > 0 && sr.last.has_value())   // its earlier users were ordered before that stream's work
+    c10::cuda::CUDACachingAllocator::recordStream(st.scratch.storage().data_ptr(), *sr.last);
+  ensure_scratch(dev, nfloats);
+  sr.off = 0;
+}
+
+// Gives a split-K product the memory of its partials; the result keeps it until the launches are enqueued.
+at::Tensor gemm_attach_scratch(GemmProblem2& P, int dev, const c10::cuda::CUDAStream& stream) {
+  P.status = device_state(dev).status.data_ptr<int>();
+  if (!needs_ws(P)) return {};
+  const size_t need = static_cast<size_t>(P.ntiles) * P.nsplit * G2_BM * tile_width(P);
+  if (stream_is_capturing(stream.stream())) {
+    at::Tensor own = at::empty({static_cast<int64_t>(need)}, at::TensorOptions().dtype(at::kFloat).device(at::kCUDA, dev));
+    P.ws = own.data_ptr<float>();
+    return own;
   }
+  grow_ring(dev, need * 4);
+  const at::Tensor& ring = device_state(dev).scratch;
+  Ring& sr = g_scratch_ring[dev & 15];
+  if (sr.last.has_value() && *sr.last != stream && !stream_is_capturing(sr.last->stream())) {
+    // another stream used the ring last: order this launch after that stream's work
+    if (sr.ev == nullptr) B200_CUDA_CHECK(cudaEventCreateWithFlags(&sr.ev, cudaEventDisableTiming));
+    B200_CUDA_CHECK(cudaEventRecord(sr.ev, sr.last->stream()));
+    B200_CUDA_CHECK(cudaStreamWaitEvent(stream.stream(), sr.ev, 0));
+  }
+  sr.last = stream;
+  if (sr.off + need > static_cast<size_t>(ring.numel())) sr.off = 0;
+  P.ws = ring.data_ptr<float>() + sr.off;
+  sr.off += need;
+  return ring;
 }
 
 void gemm_launch_single(const GemmProblem2& P, int dev, cudaStream_t stream) {
@@ -430,9 +447,9 @@ void umma_gemm(std::vector<at::Tensor> a_segs, std::vector<at::Tensor> b_segs, b
   GemmProblem2 P;
   gemm_fill_problem(P, a_segs, b_segs, a_kmajor, b_kmajor, C, alpha, beta, sym, out_hi, out_mid, out_lo,
                     nsplit, split3, g2_sm_count(dev), false, x3wide);
-  auto stream = at::cuda::getCurrentCUDAStream(dev).stream();
+  const auto stream = at::cuda::getCurrentCUDAStream(dev);
   if (out_hi.has_value() || !batch_append(P, dev, nsplit, stream, a_segs, b_segs, C)) {
-    gemm_attach_scratch(P, dev, stream);
+    const at::Tensor partials = gemm_attach_scratch(P, dev, stream);
     gemm_launch_single(P, dev, stream);
   }
 }
@@ -541,9 +558,9 @@ void umma_syrk_conv(at::Tensor x, c10::optional<at::Tensor> C_opt, int64_t kh, i
     nsplit = std::min(std::min(nsplit, kb_total / 8), 32);
   }
   P.nsplit = std::max(1, std::min(nsplit, kb_total));
-  auto stream = at::cuda::getCurrentCUDAStream(dev).stream();
+  const auto stream = at::cuda::getCurrentCUDAStream(dev);
   if (!batch_append(P, dev, nsplit_req, stream, {x}, {}, C_opt)) {
-    gemm_attach_scratch(P, dev, stream);
+    const at::Tensor partials = gemm_attach_scratch(P, dev, stream);
     gemm_launch_single(P, dev, stream);
   }
 }
@@ -583,9 +600,9 @@ void umma_gemm_to_ptr(std::vector<at::Tensor> a_segs, std::vector<at::Tensor> b_
     TORCH_CHECK(!sym && atomic == 0, "multicast destinations take the plain result of a non-symmetric product");
     P.flags |= G2F_MCAST;
   }
-  auto stream = at::cuda::getCurrentCUDAStream(dev).stream();
+  const auto stream = at::cuda::getCurrentCUDAStream(dev);
   if (!batch_append(P, dev, nsplit, stream, a_segs, b_segs, c10::nullopt)) {
-    gemm_attach_scratch(P, dev, stream);
+    const at::Tensor partials = gemm_attach_scratch(P, dev, stream);
     gemm_launch_single(P, dev, stream);
   }
 }
@@ -777,7 +794,7 @@ int64_t launch_count() { return static_cast<int64_t>(launch_counter().load()); }
 
 void reserve_scratch(int64_t dev, int64_t nfloats) {
   c10::cuda::CUDAGuard guard(static_cast<int>(dev));
-  ensure_scratch(static_cast<int>(dev), static_cast<size_t>(nfloats));
+  grow_ring(static_cast<int>(dev), static_cast<size_t>(nfloats));
 }
 
 }  // namespace b200

@@ -1,4 +1,6 @@
-"""Device tables of the grouped inverses outlive the CUDA graphs and the streams that use them."""
+"""What captured CUDA graphs and other streams read stays in place: tables of the grouped inverses, split-K partials."""
+import subprocess
+import sys
 import time
 
 import pytest
@@ -84,3 +86,26 @@ def test_tables_evicted_while_another_stream_uses_them(monkeypatch, backend):
     torch.cuda.current_stream().wait_stream(side)
     _check(mats, outs, 1e-2)
     ops.check_status()
+
+
+_REPLAY_AFTER_GROWTH = """
+import torch
+from asdl_b200 import ops
+x = torch.randn(4096, 200, device='cuda', generator=torch.Generator(device='cuda').manual_seed(0)).to(torch.bfloat16)
+want = ops.gram(x)                                     # creates the ring of split-K partials
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    out = ops.gram(x)
+ops.extension().reserve_scratch(0, 64 << 20)           # a larger one takes its place
+fillers = [torch.ones(4 << 20, device='cuda') for _ in range(4)]   # ... and others get the memory of the first
+out.zero_()
+graph.replay()
+torch.cuda.synchronize()
+assert torch.equal(out, want)
+assert all(bool((f == 1).all()) for f in fillers), 'the replay wrote to memory that is not its own'
+"""
+
+
+def test_a_replay_leaves_the_former_ring_of_partials_alone():
+    done = subprocess.run([sys.executable, '-c', _REPLAY_AFTER_GROWTH], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
