@@ -429,24 +429,32 @@ im2col_tile_kernel(const T* __restrict__ x, __nv_bfloat16* __restrict__ out, __n
   const bool along_c = p.sC == 1;
   const int fast = along_c ? nc : w_end, slow = (along_c ? w_end : nc) * p.KH;
   const int f0 = threadIdx.x % fast_lanes, rows = 256 / fast_lanes;
-  for (int f = f0; f < fast; f += fast_lanes) {
-    for (int t0 = threadIdx.x / fast_lanes; t0 < slow; t0 += IM2COL_LOADS * rows) {
-      T v[IM2COL_LOADS];
-      int to[IM2COL_LOADS];
+  // FULL: all slots of the round have work.  The slots of other rounds are skipped by a branch: where the slow dimension is
+  // short, most are empty, and their divisions bounded the kernel; in full rounds the branch keeps loads from overlapping.
+  auto round = [&](auto full, int f, int t0) {
+    constexpr bool FULL = decltype(full)::value;
+    T v[IM2COL_LOADS];
+    int to[IM2COL_LOADS];
 #pragma unroll
-      for (int u = 0; u < IM2COL_LOADS; ++u) {
-        const int t = t0 + u * rows, s = t / p.KH, kh = t - s * p.KH, hi = h0 + kh * p.DH;
-        const int c = along_c ? f : s, w = along_c ? s : f;
-        to[u] = -1;
-        if (t < slow && hi >= 0 && hi < p.H) {
-          to[u] = (c * p.KH + kh) * wp + w + p.PW;
-          v[u] = __ldg(base + c * p.sC + hi * p.sH + w * p.sW);
-        }
+    for (int u = 0; u < IM2COL_LOADS; ++u) {
+      const int t = t0 + u * rows;
+      to[u] = -1;
+      if (!FULL && t >= slow) continue;
+      const int s = t / p.KH, kh = t - s * p.KH, hi = h0 + kh * p.DH;
+      const int c = along_c ? f : s, w = along_c ? s : f;
+      if (hi >= 0 && hi < p.H) {
+        to[u] = (c * p.KH + kh) * wp + w + p.PW;
+        v[u] = __ldg(base + c * p.sC + hi * p.sH + w * p.sW);
       }
-#pragma unroll
-      for (int u = 0; u < IM2COL_LOADS; ++u)
-        if (to[u] >= 0) tile[to[u]] = to_f32<T>(v[u]);
     }
+#pragma unroll
+    for (int u = 0; u < IM2COL_LOADS; ++u)
+      if (to[u] >= 0) tile[to[u]] = to_f32<T>(v[u]);
+  };
+  for (int f = f0; f < fast; f += fast_lanes) {
+    int t0 = threadIdx.x / fast_lanes;
+    for (; t0 + (IM2COL_LOADS - 1) * rows < slow; t0 += IM2COL_LOADS * rows) round(std::true_type{}, f, t0);
+    if (t0 < slow) round(std::false_type{}, f, t0);
   }
   __syncthreads();
   const int vecs = width / 8;
@@ -483,11 +491,34 @@ im2col_tile_kernel(const T* __restrict__ x, __nv_bfloat16* __restrict__ out, __n
 }
 
 // Channels per CTA of the tile path, 0 if it does not apply: the staged rows and the column table fit `IM2COL_SMEM` (so a
-// byte offset has 16 bits), and each chunk starts on a multiple of eight columns.
+// byte offset has 16 bits), each chunk starts on a multiple of eight columns, and it is expected to take less time than the
+// element-wise kernel.
 constexpr int IM2COL_SMEM = 44 * 1024;
 struct Im2colTile {
   int cc, wp, smem, fast_lanes;
 };
+
+// Expected times in us, fitted to 480 shapes of 30 thousand to 58 million patch elements (5 % and 13 % off on average; the
+// rule they give picks a kernel within 0.2 % of the better one on average).  The element-wise kernel is bound by its index
+// divisions per element.  A CTA of the tile kernel goes through rounds of loads, the divisions of its column table and the
+// assembly: one such chain where every SM has at most one CTA, the sum of their issue times where it has several.  Below
+// 100 thousand elements, for images of one output pixel and for 1 x 1 filters over few pixels and many channels the former is
+// faster (32 x 64 x 8 x 8 under an 8 x 8 filter: 3.6 and 7.6 us; 32 x 1024 x 14 x 14 channels_last fp32 under a strided
+// 1 x 1 filter: 17 and 25 us).
+inline float im2col_generic_us(const Im2colParams& p) {
+  return 2.5f + 7.7e-6f * static_cast<float>(p.N) * p.Ho * p.Wo * p.ldo;
+}
+inline float im2col_tile_us(const Im2colParams& p, const Im2colTile& t) {
+  auto up = [](long long a, long long b) { return static_cast<float>((a + b - 1) / b); };
+  const long long w_end = std::min(p.W, t.wp), fast = p.sC == 1 ? t.cc : w_end, slow = (p.sC == 1 ? w_end : t.cc) * p.KH;
+  const long long lane_rows = 256 / t.fast_lanes, cols = static_cast<long long>(t.cc) * p.KH * p.KW;
+  const float rounds = up(fast, t.fast_lanes) * up(slow, lane_rows * IM2COL_LOADS);
+  const float loads = up(fast, t.fast_lanes) * up(slow, lane_rows), table = up(cols, 256), pieces = up(cols * p.Wo, 8 * 256);
+  const float ctas = static_cast<float>(p.N) * p.Ho * up(p.C, t.cc);
+  return std::max(2.05f + 0.35f * rounds + 0.12f * loads + 0.18f * table + 0.15f * pieces,
+                  2.f + ctas / 148 * (0.165f * rounds + 0.084f * loads + 0.173f * table + 0.081f * pieces));
+}
+
 Im2colTile im2col_tile_plan(const Im2colParams& p) {
   const Im2colTile none{0, 0, 0, 0};
   const long long taps = static_cast<long long>(p.KH) * p.KW;
@@ -496,7 +527,7 @@ Im2colTile im2col_tile_plan(const Im2colParams& p) {
     return ((cc * p.KH * wp + wp + 3) / 4 * 4) * 4 + (cc * taps + 8) * 2 + (p.ldo - static_cast<long long>(p.C) * taps) * 2;
   };
   auto fits = [&](long long cc) { return smem(cc) <= IM2COL_SMEM; };
-  if (p.ldo % 8 != 0 || static_cast<long long>(p.N) * p.Ho >= (1ll << 31)) return none;
+  if (p.ldo % 8 != 0 || p.PH < 0 || p.PW < 0 || static_cast<long long>(p.N) * p.Ho >= (1ll << 31)) return none;
   long long cc = p.C;
   if (!fits(cc)) {
     if (!p.c_major) return none;
@@ -510,7 +541,8 @@ Im2colTile im2col_tile_plan(const Im2colParams& p) {
   const long long fast = p.sC == 1 ? std::min<long long>(cc, p.C) : std::min<long long>(p.W, wp);
   int lanes = 4;
   while (lanes < fast && lanes < 32) lanes *= 2;
-  return {static_cast<int>(cc), static_cast<int>(wp), static_cast<int>(smem(cc)), lanes};
+  const Im2colTile tile{static_cast<int>(cc), static_cast<int>(wp), static_cast<int>(smem(cc)), lanes};
+  return im2col_tile_us(p, tile) < im2col_generic_us(p) ? tile : none;
 }
 
 // x: 4-D conv input [N, C, H, W] (logical), any memory format.  out: [N*Ho*Wo, ld] bf16, contiguous.
@@ -566,7 +598,10 @@ void im2col_bf16(at::Tensor x, at::Tensor out, c10::optional<at::Tensor> out_lo,
   };
   if (vec) {
     const Walk w = walk_plan(p.KH * p.KW * (p.C >> 3));
-    im2col_nhwc_vec8_kernel<<<walk_grid(w, (rows + 3) / 4, 8), 256, 0, stream>>>(
+    // four pixels per thread; where that leaves SMs without a CTA, one (32 x 32 x 8 x 8, 3 x 3: 2.9 -> 2.4 us)
+    dim3 grid = walk_grid(w, (rows + 3) / 4, 8);
+    if (grid.x * grid.y < 148) grid = walk_grid(w, rows, 8);
+    im2col_nhwc_vec8_kernel<<<grid, 256, 0, stream>>>(
         reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), out_p, p, static_cast<unsigned>(rows), w.groups, w.lanes);
   } else if (x.scalar_type() == at::kFloat) {
     run(static_cast<const float*>(x.data_ptr<float>()));

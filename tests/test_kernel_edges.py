@@ -106,6 +106,15 @@ def test_im2col_layouts(ext, cfg, dtype, layout):
                 assert torch.equal(lo, (want - out.float()).to(torch.bfloat16))
 
 
+@pytest.mark.parametrize('dtype', [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize('cfg', [  # rows of pixels enough for the tile kernel: full and part-filled rounds of loads, both chunkings
+    (24, 16, 9, 40, 3, 1, 1, 1), (160, 6, 14, 14, 5, 1, 0, 1), (32, 300, 9, 9, 3, 1, 1, 1), (256, 64, 8, 8, 8, 1, 0, 1),
+    (16, 24, 30, 31, 2, 2, 0, 1), (40, 33, 12, 12, 3, 1, 2, 2), (512, 1, 28, 28, 5, 1, 0, 1)])
+@pytest.mark.parametrize('layout', ['nchw', 'nhwc', 'sliced'])
+def test_im2col_tiles(ext, cfg, dtype, layout):
+    test_im2col_layouts(ext, cfg, dtype, layout)
+
+
 @pytest.mark.parametrize('rows,n', [(700, 33), (3000, 130), (2048, 257), (5000, 64)])
 @pytest.mark.parametrize('nsplit', [2, 5, 9])
 @pytest.mark.parametrize('beta', [0.0, 0.9])
