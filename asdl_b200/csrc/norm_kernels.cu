@@ -46,6 +46,11 @@ struct VecLoad<float, 4> {
 constexpr int BN_GROUPS = 8;    // channel groups (of VEC channels) per CTA
 constexpr int BN_LANES = 32;    // hw lanes per CTA
 constexpr int BN_THREADS = BN_GROUPS * BN_LANES;
+// Positions of a split from which the masked kernel, with three tensors to load, keeps those of two positions in flight: five
+// per lane.  32 x 256 x 56 x 56: 40.8 -> 32.6 us, 32 x 64 x 56 x 56 (165 positions): 18.4 -> 17.6; below, the registers cost more
+// CTAs per SM than the loads gain (32 x 1024 x 14 x 14, 98 positions: 14.0 -> 15.9).  Without a mask two positions change
+// nothing; four gain 4 % from 600 positions on and lose up to 60 % below (32 x 1024 x 14 x 14: 12.5 -> 20.0).
+constexpr int BN_PAIR_HW = 160;
 
 template <typename T, int VEC>
 __global__ void __launch_bounds__(BN_THREADS)
@@ -70,8 +75,7 @@ bn_stats_partial(const T* __restrict__ y, const T* __restrict__ g, const float* 
       bias[i] = b[c0 + i];
     }
     const size_t base = static_cast<size_t>(n) * hw * channels + c0;
-#pragma unroll 4
-    for (int p = hw_begin + lane; p < hw_end; p += BN_LANES) {   // the loads of four positions in flight
+    for (int p = hw_begin + lane; p < hw_end; p += BN_LANES) {
       float yv[VEC], gv[VEC];
       VecLoad<T, VEC>::load(y + base + static_cast<size_t>(p) * channels, yv);
       VecLoad<T, VEC>::load(g + base + static_cast<size_t>(p) * channels, gv);
@@ -100,8 +104,8 @@ bn_stats_partial(const T* __restrict__ y, const T* __restrict__ g, const float* 
 
 // Same partial sums for a layer whose output has passed through a fused activation / residual
 // add: the normalised input comes from the layer input and the batch statistics, and the output
-// gradient is masked by the activation (g = dy where y > 0).
-template <bool RELU>
+// gradient is masked by the activation (g = dy where y > 0).  PAIRS: the loads of two positions in flight (BN_PAIR_HW).
+template <bool RELU, bool PAIRS>
 __global__ void __launch_bounds__(BN_THREADS)
 bn_stats_partial_xhat(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
                       const __nv_bfloat16* __restrict__ y, const float* __restrict__ mean,
@@ -126,8 +130,7 @@ bn_stats_partial_xhat(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* 
       is[i] = invstd[c0 + i];
     }
     const size_t base = static_cast<size_t>(n) * hw * channels + c0;
-#pragma unroll 4
-    for (int p = hw_begin + lane; p < hw_end; p += BN_LANES) {   // the loads of four positions in flight
+    auto add = [&](int p) {
       float xv[VEC], gv[VEC];
       VecLoad<__nv_bfloat16, 8>::load(x + base + static_cast<size_t>(p) * channels, xv);
       VecLoad<__nv_bfloat16, 8>::load(dy + base + static_cast<size_t>(p) * channels, gv);
@@ -142,6 +145,12 @@ bn_stats_partial_xhat(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* 
         acc_w[i] = fmaf((xv[i] - mu[i]) * is[i], gv[i], acc_w[i]);
         acc_b[i] += gv[i];
       }
+    };
+    if (PAIRS) {
+#pragma unroll 2
+      for (int p = hw_begin + lane; p < hw_end; p += BN_LANES) add(p);
+    } else {
+      for (int p = hw_begin + lane; p < hw_end; p += BN_LANES) add(p);
     }
   }
 #pragma unroll
@@ -274,14 +283,17 @@ void bn_unitwise_stats_xhat(at::Tensor x, at::Tensor dy, c10::optional<at::Tenso
   dim3 grid(chunks, n, splits);
   const auto* xp = reinterpret_cast<const __nv_bfloat16*>(x.data_ptr());
   const auto* gp = reinterpret_cast<const __nv_bfloat16*>(dy.data_ptr());
-  if (y.has_value())
-    bn_stats_partial_xhat<true><<<grid, BN_THREADS, 0, stream>>>(
-        xp, gp, reinterpret_cast<const __nv_bfloat16*>(y->data_ptr()), mean.data_ptr<float>(),
-        invstd.data_ptr<float>(), part.data_ptr<float>(), n, c, hw, hw_per_split);
+  const auto* yp = y.has_value() ? reinterpret_cast<const __nv_bfloat16*>(y->data_ptr()) : nullptr;
+  auto run = [&](auto kernel) {
+    kernel<<<grid, BN_THREADS, 0, stream>>>(xp, gp, yp, mean.data_ptr<float>(), invstd.data_ptr<float>(),
+                                            part.data_ptr<float>(), n, c, hw, hw_per_split);
+  };
+  if (yp == nullptr)
+    run(bn_stats_partial_xhat<false, false>);
+  else if (hw_per_split < BN_PAIR_HW)
+    run(bn_stats_partial_xhat<true, false>);
   else
-    bn_stats_partial_xhat<false><<<grid, BN_THREADS, 0, stream>>>(
-        xp, gp, nullptr, mean.data_ptr<float>(), invstd.data_ptr<float>(), part.data_ptr<float>(), n, c, hw,
-        hw_per_split);
+    run(bn_stats_partial_xhat<true, true>);
   bn_stats_finalize<<<(c + 7) / 8, 256, 0, stream>>>(part.data_ptr<float>(), stats.data_ptr<float>(), n, c,
                                                      splits, static_cast<float>(alpha), static_cast<float>(beta));
   B200_CUDA_CHECK(cudaGetLastError());

@@ -255,3 +255,26 @@ def test_batch_norm_counts_an_undefined_gradient_as_zeros(relu):
     _Cut.apply(ops.batch_norm_train(x, weight, bias, residual=res, relu=relu)).sum().backward()
     for leaf in (x, res, weight, bias):
         assert leaf.grad is not None and not leaf.grad.any()
+
+
+@pytest.mark.parametrize('masked', [False, True])
+@pytest.mark.parametrize('n,c,h,w', [(600, 8, 1, 31), (600, 8, 3, 53), (600, 8, 10, 16), (600, 8, 7, 23), (600, 8, 18, 18), (3, 72, 29, 31)])
+def test_batch_norm_curvature_positions(n, c, h, w, masked):
+    def act(seed):
+        return torch.randn(n, c, h, w, device=DEV, generator=_gen(seed)).to(torch.bfloat16).contiguous(
+            memory_format=torch.channels_last)
+    x, dy, y = act(24), act(25), act(26) if masked else None
+    mean, invstd = (0.1 * torch.randn(c, device=DEV, generator=_gen(27)), 0.5 + torch.rand(c, device=DEV, generator=_gen(28)))
+    old = torch.randn(c, 2, 2, device=DEV, generator=_gen(29))
+    got = ops.batchnorm_unitwise_stats_from_input(x, dy, y, mean, invstd, old.clone(), alpha=0.5, beta=0.25)
+    g = dy.double() * (y > 0) if masked else dy.double()
+    terms = (x.double() - mean.double().view(1, -1, 1, 1)) * invstd.double().view(1, -1, 1, 1) * g
+    sums = [terms.sum((2, 3)), g.sum((2, 3))]                                     # per sample and channel
+    sizes = [terms.abs().sum((2, 3)), g.abs().sum((2, 3))]
+    pairs = [(0, 0), (0, 1), (1, 0), (1, 1)]
+    want = torch.stack([(sums[a] * sums[b]).sum(0) for a, b in pairs], 1).view(c, 2, 2)
+    size = torch.stack([(sizes[a] * sizes[b]).sum(0) for a, b in pairs], 1).view(c, 2, 2)
+    # both factors of a product lose at most 2^-24 of their absolute sum per addition: h w / 32 per lane, 32 lanes, the splits;
+    # the samples add another 2^-24 each (n / 32 per lane of a warp, then five steps)
+    steps = 2 * (h * w / 32 + 32 + 8) + n / 32 + 8
+    assert ((got.double() - (0.25 * old.double() + 0.5 * want)).abs() <= steps * 2.0 ** -24 * size + 1e-6).all()
