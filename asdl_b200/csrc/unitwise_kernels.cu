@@ -96,7 +96,7 @@ ln_stats_partial_vec(const T* __restrict__ y, const T* __restrict__ g, const flo
   }
 }
 
-// The same for rows that are not 16-byte aligned.  grid: (column chunks of 256, row chunks); thread = one column.
+// The same for few rows and for rows that are not 16-byte aligned.  grid: (column chunks of 256, row chunks); thread = one column.
 template <typename T>
 __global__ void __launch_bounds__(256) ln_stats_partial(const T* __restrict__ y, const T* __restrict__ g,
                                                         const float* __restrict__ weight,
@@ -122,28 +122,33 @@ __global__ void __launch_bounds__(256) ln_stats_partial(const T* __restrict__ y,
   p[2 * static_cast<size_t>(d)] = bb;
 }
 
-// 32 features per CTA, eight chunks at a time; chunks are summed in double precision in a fixed order: deterministic.
+// COLS features per CTA, 256 / COLS chunks at a time; chunks are summed in double precision in a fixed order: deterministic.
+// 32 features where there are chunks to share out, else 256 (1 x 50304, one chunk: 9.1 and 3.7 us with the sums).
+template <int COLS>
 __global__ void __launch_bounds__(256) ln_stats_finalize(const float* __restrict__ part, float* __restrict__ stats, int d,
                                                          int chunks, float alpha, float beta) {
-  __shared__ double red[8][3][32];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, c = blockIdx.x * 32 + tx;
+  constexpr int LANES = 256 / COLS;
+  __shared__ double red[LANES > 1 ? LANES : 1][3][LANES > 1 ? COLS : 1];
+  const int tx = threadIdx.x % COLS, ty = threadIdx.x / COLS, c = blockIdx.x * COLS + tx;
   double ww = 0.0, wb = 0.0, bb = 0.0;
   if (c < d) {
 #pragma unroll 4
-    for (int k = ty; k < chunks; k += 8) {
+    for (int k = ty; k < chunks; k += LANES) {
       const float* p = part + static_cast<size_t>(k) * 3 * d + c;
       ww += p[0];
       wb += p[d];
       bb += p[2 * static_cast<size_t>(d)];
     }
   }
-  red[ty][0][tx] = ww;
-  red[ty][1][tx] = wb;
-  red[ty][2][tx] = bb;
-  __syncthreads();
+  if (LANES > 1) {
+    red[ty][0][tx] = ww;
+    red[ty][1][tx] = wb;
+    red[ty][2][tx] = bb;
+    __syncthreads();
+  }
   if (ty != 0 || c >= d) return;
 #pragma unroll
-  for (int k = 1; k < 8; ++k) {
+  for (int k = 1; k < LANES; ++k) {
     ww += red[k][0][tx];
     wb += red[k][1][tx];
     bb += red[k][2][tx];
@@ -315,7 +320,12 @@ void ln_unitwise_stats(at::Tensor y, at::Tensor g, at::Tensor weight, at::Tensor
   const int dev = y.get_device();
   c10::cuda::CUDAGuard guard(dev);
   auto stream = at::cuda::getCurrentCUDAStream(dev).stream();
-  const bool vec = (d * y.element_size()) % 16 == 0 &&
+  // The vector kernel needs rows to fill its 32 lanes with four loads each: below a thousand the one with a thread per column
+  // is faster (bf16, 64 x 512: 4.6 and 4.2 us, 500 x 1024: 5.7 and 4.9, 500 x 4096: 8.3 and 5.9), unless bytes bound both
+  // (700 x 16384: 18.6 and 20.6; 8192 x 1024: 15.9 and 18.5).  In fp32 its vectors are four columns and its CTAs twice as many,
+  // and it is 5 % faster from 16 rows on, until the row chunks of the other fill the SMs.
+  const bool many = rows >= 1000 || rows * d > 10'000'000, some = !bf16 && rows >= 16 && rows < 400 && d < 2048;
+  const bool vec = (many || some) && (d * y.element_size()) % 16 == 0 &&
                    ((reinterpret_cast<uintptr_t>(y.data_ptr()) | reinterpret_cast<uintptr_t>(g.data_ptr())) & 15) == 0;
   // about four CTAs per SM; at least 16 rows per thread column, or one row per lane of the vector kernel
   const int width = vec ? LS_GROUPS * (bf16 ? 8 : 4) : 256, least = vec ? LS_LANES : 16;
@@ -338,8 +348,11 @@ void ln_unitwise_stats(at::Tensor y, at::Tensor g, at::Tensor weight, at::Tensor
     run(reinterpret_cast<const __nv_bfloat16*>(y.data_ptr()), reinterpret_cast<const __nv_bfloat16*>(g.data_ptr()));
   else
     run(static_cast<const float*>(y.data_ptr<float>()), static_cast<const float*>(g.data_ptr<float>()));
-  ln_stats_finalize<<<(d + 31) / 32, 256, 0, stream>>>(pp, stats.data_ptr<float>(), d, static_cast<int>(chunks),
-                                                       static_cast<float>(alpha), static_cast<float>(beta));
+  const float a = static_cast<float>(alpha), b = static_cast<float>(beta);
+  if (chunks < 4)
+    ln_stats_finalize<256><<<(d + 255) / 256, 256, 0, stream>>>(pp, stats.data_ptr<float>(), d, static_cast<int>(chunks), a, b);
+  else
+    ln_stats_finalize<32><<<(d + 31) / 32, 256, 0, stream>>>(pp, stats.data_ptr<float>(), d, static_cast<int>(chunks), a, b);
   B200_CUDA_CHECK(cudaGetLastError());
   count_launch(2);
 }

@@ -211,6 +211,12 @@ def test_layer_norm_curvature_chunks(dtype, rows, d):
     assert ((got.double() - (0.25 * old.double() + 0.5 * want)).abs() <= 64 * 2.0 ** -24 * size + 1e-6).all()
 
 
+@pytest.mark.parametrize('dtype', [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize('rows,d', [(1, 16384), (112, 64), (113, 64), (999, 512), (1000, 512), (1031, 72), (513, 16384)])
+def test_layer_norm_curvature_rows(dtype, rows, d):
+    test_layer_norm_curvature_chunks(dtype, rows, d)
+
+
 @pytest.mark.parametrize('relu,residual', [(False, False), (True, False), (False, True), (True, True)])
 @pytest.mark.parametrize('n,c,h,w', [(2, 8, 1, 1), (3, 16, 5, 7), (1, 2056, 3, 3), (5, 264, 11, 9), (16, 64, 40, 40)])
 def test_batch_norm_row_walk(n, c, h, w, relu, residual):
