@@ -87,17 +87,28 @@ void g2_launch_list(const GemmProblem2* d_probs, const GemmWork2* d_work, int n_
     g2_run_plain(dummy, d_probs, d_work, n_work, n_sms, stream);
 }
 
+// Reduction of `tiles` tiles that are BN wide; the tiles come from `single`, a work list or a batch (splitk_reduce2_kernel).
+template <int BN>
+static void launch_reduce(int tiles, const GemmProblem2& single, const GemmProblem2* probs, const GemmWork2* work,
+                          const int* prefix, int n_probs, cudaStream_t stream) {
+  // 50000 x 64 bf16, one tile of 32 splits: 21.6 -> 18.6 us with the product; 4096 x 512, ten tiles of 8: 13.4 -> 14.9
+  if (tiles * g2_reduce_patches<BN, 16>() <= 148)
+    splitk_reduce2_kernel<BN, 16><<<dim3(tiles, g2_reduce_patches<BN, 16>()), 256, 0, stream>>>(single, probs, work, prefix, n_probs);
+  else
+    splitk_reduce2_kernel<BN, 32><<<dim3(tiles, g2_reduce_patches<BN, 32>()), 256, 0, stream>>>(single, probs, work, prefix, n_probs);
+  B200_CUDA_CHECK(cudaGetLastError());
+  count_launch();
+}
+
 void g2_launch_reduce_list(const GemmProblem2* d_probs, const GemmWork2* d_work, int n_work, bool wide,
                            cudaStream_t stream) {
   if (n_work <= 0) return;
   GemmProblem2 dummy;
   std::memset(&dummy, 0, sizeof(dummy));
   if (wide)
-    splitk_reduce2_kernel<256><<<dim3(n_work, g2_reduce_patches<256>(), 1), 256, 0, stream>>>(dummy, d_probs, d_work, nullptr, 0);
+    launch_reduce<256>(n_work, dummy, d_probs, d_work, nullptr, 0, stream);
   else
-    splitk_reduce2_kernel<128><<<dim3(n_work, g2_reduce_patches<128>(), 1), 256, 0, stream>>>(dummy, d_probs, d_work, nullptr, 0);
-  B200_CUDA_CHECK(cudaGetLastError());
-  count_launch();
+    launch_reduce<128>(n_work, dummy, d_probs, d_work, nullptr, 0, stream);
 }
 
 // Fills the scalar fields of a problem and encodes its tensor maps.
@@ -263,11 +274,9 @@ void gemm_launch_single(const GemmProblem2& P, int dev, cudaStream_t stream) {
     g2_run_plain(P, nullptr, nullptr, n_work, n_sms, stream);
   if (needs_ws(P)) {
     if (wide)
-      splitk_reduce2_kernel<256><<<dim3(P.ntiles, g2_reduce_patches<256>(), 1), 256, 0, stream>>>(P, nullptr, nullptr, nullptr, 0);
+      launch_reduce<256>(P.ntiles, P, nullptr, nullptr, nullptr, 0, stream);
     else
-      splitk_reduce2_kernel<128><<<dim3(P.ntiles, g2_reduce_patches<128>(), 1), 256, 0, stream>>>(P, nullptr, nullptr, nullptr, 0);
-    B200_CUDA_CHECK(cudaGetLastError());
-    count_launch();
+      launch_reduce<128>(P.ntiles, P, nullptr, nullptr, nullptr, 0, stream);
   }
 }
 
@@ -371,12 +380,8 @@ static void batch_flush(cudaStream_t stream) {
     std::memset(&dummy, 0, sizeof(dummy));
     const GemmProblem2* dp = reinterpret_cast<const GemmProblem2*>(d);
     g2_run_plain(dummy, dp, nullptr, items, n_sms, stream, reinterpret_cast<const int*>(d + probs_bytes), n);
-    if (rtiles > 0) {
-      splitk_reduce2_kernel<128><<<dim3(rtiles, g2_reduce_patches<128>(), 1), 256, 0, stream>>>(
-          dummy, dp, nullptr, reinterpret_cast<const int*>(d + probs_bytes + prefix_bytes), n);
-      B200_CUDA_CHECK(cudaGetLastError());
-      count_launch();
-    }
+    if (rtiles > 0)
+      launch_reduce<128>(rtiles, dummy, dp, nullptr, reinterpret_cast<const int*>(d + probs_bytes + prefix_bytes), n, stream);
   }
   B.problems.clear();
   B.nsplit_req.clear();

@@ -828,21 +828,23 @@ umma_gemm2_kernel(const __grid_constant__ GemmProblem2 single, const GemmProblem
   }
 }
 
-// Sums split-K partials and applies the epilogue.  One block handles a 32 x 64 patch of one tile; a thread owns four
-// consecutive columns of two rows, so the partials of four splits are eight 16-byte loads in flight (the kernel reads
-// nsplit times what it writes and does nothing else; with 4-byte loads of one split at a time it ran at 1.3 TB/s).  The
-// mirrored store goes through shared memory.  Partials are added in split order.
-// grid: (work items, 4 * BN / 64).
-constexpr int G2_RED_ROWS = 32, G2_RED_COLS = 64;
-template <int BN>
+// Sums split-K partials and applies the epilogue.  One block handles a ROWS x 64 patch of one tile; a thread owns four
+// consecutive columns of ROWS / 16 rows, and eight 16-byte loads of partials are in flight (the kernel reads nsplit times what
+// it writes and does nothing else; with 4-byte loads of one split at a time it ran at 1.3 TB/s).  The mirrored store goes
+// through shared memory.  Partials are added in split order.  Patches have 32 rows, or 16 where those still leave SMs without a
+// block: what one SM can load bounds it then.
+// grid: (work items, 128 / ROWS * BN / 64).
+constexpr int G2_RED_COLS = 64;
+template <int BN, int ROWS>
 constexpr int g2_reduce_patches() {
-  return (G2_BM / G2_RED_ROWS) * (BN / G2_RED_COLS);
+  return (G2_BM / ROWS) * (BN / G2_RED_COLS);
 }
-template <int BN>
+template <int BN, int ROWS>
 __global__ void __launch_bounds__(256)
 splitk_reduce2_kernel(const __grid_constant__ GemmProblem2 single, const GemmProblem2* __restrict__ probs,
                       const GemmWork2* __restrict__ work, const int* __restrict__ tile_prefix, int n_probs) {
-  __shared__ float tile[G2_RED_ROWS][G2_RED_COLS + 1];
+  constexpr int R = ROWS / 16, SPLITS = 8 / R;   // rows of a thread, splits in flight
+  __shared__ float tile[ROWS][G2_RED_COLS + 1];
   GemmWork2 w;
   const GemmProblem2* Pp;
   if (work != nullptr) {
@@ -868,25 +870,25 @@ splitk_reduce2_kernel(const __grid_constant__ GemmProblem2 single, const GemmPro
   const bool sym = (P.flags & G2F_SYM) != 0;
   constexpr int PC = BN / G2_RED_COLS;  // patches per tile row
   const int sub_r = blockIdx.y / PC, sub_c = blockIdx.y % PC;
-  const int row0 = w.c_row + sub_r * G2_RED_ROWS, col0 = w.c_col + sub_c * G2_RED_COLS;
+  const int row0 = w.c_row + sub_r * ROWS, col0 = w.c_col + sub_c * G2_RED_COLS;
   const int tm = w.c_row / G2_BM;
   const int cb = col0 / G2_BM;  // 128-wide column block of this patch
   if (sym && cb > tm) return;
   const bool diag_tile = sym && cb == tm;
-  if (diag_tile && col0 > row0 + G2_RED_ROWS - 1) return;
+  if (diag_tile && col0 > row0 + ROWS - 1) return;
   // patches that lie completely outside the matrix (edge tiles of small problems) have no work
   if (row0 >= P.M || col0 >= P.N) return;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   constexpr size_t SPLIT = static_cast<size_t>(G2_BM) * BN;   // floats of one split's partial tile
   const float* p0 = P.ws + static_cast<size_t>(w.tile_id) * P.nsplit * SPLIT +
-                    static_cast<size_t>(sub_r * G2_RED_ROWS + ty) * BN + sub_c * G2_RED_COLS + tx * 4;
+                    static_cast<size_t>(sub_r * ROWS + ty) * BN + sub_c * G2_RED_COLS + tx * 4;
   const int gc = col0 + tx * 4;
   const bool full = gc + 4 <= P.N;
   const bool vec_in = full && g2_vec_ok(P.Cin, P.ldc), vec_out = full && g2_vec_ok(P.C, P.ldc);
-  float cin[2][4];
+  float cin[R][4];
   if (P.beta != 0.f) {   // issued ahead of the partials
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < R; ++i) {
       const int gr = row0 + ty + 16 * i;
       const float* c = P.Cin + static_cast<size_t>(gr) * P.ldc + gc;
 #pragma unroll
@@ -906,31 +908,35 @@ splitk_reduce2_kernel(const __grid_constant__ GemmProblem2 single, const GemmPro
       }
     }
   }
-  float acc[2][4] = {};
-  for (int s = 0; s < P.nsplit; s += 4) {
-    float4 v[2][4];
+  float acc[R][4] = {};
+  auto add_round = [&](auto all, int s) {   // all: every split of the round exists
+    float4 v[R][SPLITS];
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < SPLITS; ++u)
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
-        v[i][u] = s + u < P.nsplit
+      for (int i = 0; i < R; ++i)
+        v[i][u] = all || s + u < P.nsplit
                       ? __ldcg(reinterpret_cast<const float4*>(p0 + static_cast<size_t>(16 * i) * BN + static_cast<size_t>(s + u) * SPLIT))
                       : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (s + u < P.nsplit) {
+    for (int u = 0; u < SPLITS; ++u)
+      if (all || s + u < P.nsplit) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < R; ++i) {
           acc[i][0] += v[i][u].x;
           acc[i][1] += v[i][u].y;
           acc[i][2] += v[i][u].z;
           acc[i][3] += v[i][u].w;
         }
       }
-  }
+  };
+  int s = 0;
+  if constexpr (ROWS == 16)   // many splits: 1 us of 19 less; with few splits per tile it costs as much
+    for (; s + SPLITS <= P.nsplit; s += SPLITS) add_round(std::true_type{}, s);
+  for (; s < P.nsplit; s += SPLITS) add_round(std::false_type{}, s);
   const bool mirror_bf16 = sym && !(P.flags & G2F_LOWER);
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
+  for (int i = 0; i < R; ++i) {
     const int lr = ty + 16 * i, gr = row0 + lr;
     float val[4];
 #pragma unroll
@@ -999,14 +1005,13 @@ splitk_reduce2_kernel(const __grid_constant__ GemmProblem2 single, const GemmPro
   }
   if (!sym || P.C == nullptr || (P.flags & G2F_LOWER)) return;
   __syncthreads();
-  // mirrored store: element (r, c) of the patch goes to C[c][r]; a warp writes 32 consecutive columns of one row
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // mirrored store: element (r, c) of the patch goes to C[c][r]; neighbouring threads write neighbouring columns
 #pragma unroll
-  for (int i = 0; i < G2_RED_COLS / 8; ++i) {
-    const int lc = warp + 8 * i;            // patch column -> destination row
-    const int dst_r = col0 + lc, dst_c = row0 + lane;
+  for (int i = 0; i < ROWS * G2_RED_COLS / 256; ++i) {
+    const int e = threadIdx.x + 256 * i, lr = e % ROWS, lc = e / ROWS;   // patch column -> destination row
+    const int dst_r = col0 + lc, dst_c = row0 + lr;
     if (dst_r < P.N && dst_c < P.M && dst_r < dst_c)
-      P.C[static_cast<size_t>(dst_r) * P.ldc + dst_c] = tile[lane][lc];
+      P.C[static_cast<size_t>(dst_r) * P.ldc + dst_c] = tile[lr][lc];
   }
 }
 

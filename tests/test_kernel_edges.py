@@ -131,6 +131,12 @@ def test_split_k_reduction(ext, rows, n, nsplit, beta):
     assert torch.equal(c, c.T)
 
 
+@pytest.mark.parametrize('rows,n', [(20000, 40), (9000, 200), (4000, 400), (4000, 513)])   # 16- and 32-row patches
+@pytest.mark.parametrize('nsplit', [0, 3, 8, 17, 32])
+def test_split_k_reduction_patches(ext, rows, n, nsplit):
+    test_split_k_reduction(ext, rows, n, nsplit, 0.9)
+
+
 def test_kron_apply_reads_either_order_of_a_symmetric_factor():
     left, right = (torch.randn(n, n, device=DEV, generator=_gen(4 + n)) for n in (72, 130))
     left, right = left + left.T, right + right.T
