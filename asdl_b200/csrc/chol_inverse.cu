@@ -338,7 +338,7 @@ struct CholPrepared {
   GraphPins pins;
 };
 static std::mutex g_chol_cache_mutex;
-static PreparedCache<CholPrepared, 16> g_chol_cache;
+static PreparedCache<CholPrepared, 16>& g_chol_cache = *new PreparedCache<CholPrepared, 16>;   // never destroyed
 
 // (entries, entries that captured graphs refer to)
 std::pair<int64_t, int64_t> chol_inverse_cache_info() {

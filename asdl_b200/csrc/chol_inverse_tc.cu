@@ -287,7 +287,8 @@ struct Prepared {
 };
 
 std::mutex g_cache_mutex;
-PreparedCache<Prepared, 4> g_cache;   // four sets of matrices beside those that graphs refer to
+// four sets of matrices beside those that graphs refer to; never destroyed (see PreparedCache)
+PreparedCache<Prepared, 4>& g_cache = *new PreparedCache<Prepared, 4>;
 
 int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 

@@ -64,6 +64,8 @@ class GraphPins {
 
 // Entry needs `key` (comparable) and `pins` (GraphPins).  The caller holds its own lock around every call and for as long
 // as it uses the returned entry.
+// A process-wide cache is to be allocated and never deleted: when static objects are destroyed, the CUDA context may be gone,
+// and freeing memory that several streams have used records events there.
 template <typename Entry, size_t Capacity>
 class PreparedCache {
  public:

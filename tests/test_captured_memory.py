@@ -109,3 +109,23 @@ assert all(bool((f == 1).all()) for f in fillers), 'the replay wrote to memory t
 def test_a_replay_leaves_the_former_ring_of_partials_alone():
     done = subprocess.run([sys.executable, '-c', _REPLAY_AFTER_GROWTH], capture_output=True, text=True, timeout=300)
     assert done.returncode == 0, done.stderr[-2000:]
+
+
+_EXIT_AFTER_SIDE_STREAM = """
+import torch
+from asdl_b200 import ops
+for backend in ('tensor_core', 'cuda_core'):
+    ops.CHOLESKY_BACKEND = backend
+    a, out = torch.eye(200, device='cuda'), torch.empty(200, 200, device='cuda')
+    ops.spd_inverse_grouped([a], [out], 1e-2)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        ops.spd_inverse_grouped([a], [out], 1e-2)
+torch.cuda.synchronize()
+"""
+
+
+def test_a_process_that_used_two_streams_ends_cleanly():
+    done = subprocess.run([sys.executable, '-c', _EXIT_AFTER_SIDE_STREAM], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
