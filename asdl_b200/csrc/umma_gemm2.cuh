@@ -958,16 +958,25 @@ splitk_reduce2_kernel(const __grid_constant__ GemmProblem2 single, const GemmPro
           if (j < keep && gc + j < P.N) c[j] = val[j];
       }
     }
-    for (int e = 0; e < P.n_extra; ++e) {
-      float* dst = P.full->C_extra[e] + static_cast<size_t>(gr) * P.ldc + gc;
+    for (int e = 0; e < P.n_extra; ++e) {   // copies on peers: 16-byte stores over NVLink where the rows allow it
+      float* extra = P.full->C_extra[e];
+      float* dst = extra + static_cast<size_t>(gr) * P.ldc + gc;
+      const bool mcast = (P.flags & G2F_MCAST) != 0;
+      if (full && keep == 4 && g2_vec_ok(extra, P.ldc)) {
+        if (mcast)
+          g2_multimem_st_v4(dst, val[0], val[1], val[2], val[3]);
+        else
+          *reinterpret_cast<float4*>(dst) = make_float4(val[0], val[1], val[2], val[3]);
+      } else {
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (j < keep && gc + j < P.N) {
-          if (P.flags & G2F_MCAST)
-            g2_multimem_st_f32(dst + j, val[j]);
-          else
-            dst[j] = val[j];
-        }
+        for (int j = 0; j < 4; ++j)
+          if (j < keep && gc + j < P.N) {
+            if (mcast)
+              g2_multimem_st_f32(dst + j, val[j]);
+            else
+              dst[j] = val[j];
+          }
+      }
     }
     if (P.out_hi != nullptr) {
       unsigned short part[3][4];   // hi, mid, lo (hi, lo in a two-way split)

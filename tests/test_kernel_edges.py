@@ -137,6 +137,23 @@ def test_split_k_reduction_patches(ext, rows, n, nsplit):
     test_split_k_reduction(ext, rows, n, nsplit, 0.9)
 
 
+@pytest.mark.parametrize('m,n,ldc', [(70, 72, 72), (40, 65, 68), (130, 63, 63), (300, 258, 260)])
+@pytest.mark.parametrize('nsplit', [1, 3, 17])
+def test_split_k_reduction_replicates_its_result(ext, m, n, ldc, nsplit):
+    k = 64 * 20
+    a, b = (torch.randn(k, (c + 7) // 8 * 8, device=DEV, generator=_gen(30 + c)).to(torch.bfloat16)[:, :c] for c in (m, n))
+    outs = [torch.full((m + 1, ldc), 7.0, device=DEV) for _ in range(3)]
+    ext.umma_gemm_to_ptr([a], [b], False, False, outs[0].data_ptr(), ldc, 2.0, False, 0, [t.data_ptr() for t in outs[1:]],
+                         nsplit, False)
+    want = 2.0 * (a.double().T @ b.double())
+    # every one of the k additions loses at most 2^-22 of the running sum (truncating accumulator)
+    bound = k * 2.0 ** -22 * 2.0 * (a.double().abs().T @ b.double().abs())
+    assert ((outs[0][:m, :n].double() - want).abs() <= bound).all()
+    for t in outs:
+        assert torch.equal(t[:m, :n], outs[0][:m, :n])
+        assert (t[m:] == 7).all() and (t[:, n:] == 7).all()      # nothing outside of the matrix is written
+
+
 def test_kron_apply_reads_either_order_of_a_symmetric_factor():
     left, right = (torch.randn(n, n, device=DEV, generator=_gen(4 + n)) for n in (72, 130))
     left, right = left + left.T, right + right.T
