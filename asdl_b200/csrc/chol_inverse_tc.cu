@@ -11,7 +11,7 @@
 // epilogue.  Only the 128 x 128 diagonal blocks are factored and inverted on the CUDA cores (one
 // CTA each, 32 columns at a time).
 //
-//   potrf, step k:  diag(k):   T_k = L_kk^-1, L_kk = chol(A_kk)                  (CUDA cores)
+//   potrf, step k:  diag(k):   T_k = L_kk^-1, L_kk = chol(A_kk) (not stored)     (CUDA cores)
 //                   panel(k):  L_ik = A_ik T_k^T                  for i > k      (GEMM, K = 128)
 //                   trail(k):  A_ij -= L_ik L_jk^T                for k < j <= i (GEMM, K = 128)
 //   trtri, level l: blocks of s = 2^l panels are merged pairwise:
@@ -83,10 +83,10 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const TcMat* mats, cons
 //   update   S[i][c] -= sum_j P[j][i] P[j][c] for the rows i >= be: the trailing block right of be, the right-hand side of
 //            the inverse left of it.  Finished columns of the factor are dead (only the inverse leaves the kernel), so both
 //            share S.  A warp takes four rows of each row block, a lane one column of each column block.
-// Every entry sees the same roundings in the same order as a column-by-column elimination, and gives the same bits.  That
-// elimination, with a barrier per column and the block in the registers of a 16 x 16 thread grid, took longer, and the
-// panel steps of all matrices wait for this kernel: six matrices up to 784 x 784 749 -> 589 us, the 107 factors of
-// ResNet-50 8.61 -> 8.05 ms.
+// Every entry sees the same roundings in the same order as a column-by-column elimination, and gives the same bits.  The panel
+// steps of all matrices wait for this kernel: with that elimination, a barrier per column and the block in the registers of
+// a 16 x 16 thread grid, six matrices up to 784 x 784 took 749 us and the 107 factors of ResNet-50 8.61 ms; now 589 us and
+// 8.05 ms, of which 46 us are a step of this kernel.  The chain of pivots in one warp bounds it.
 //
 // The code is kept small (one body for all stages, eight columns of a substitution unrolled, the registers shifted by eight
 // between them): with every stage unrolled the kernel was bound by instruction fetch (653 us and 8.71 ms).

@@ -114,6 +114,7 @@ def test_a_replay_leaves_the_former_ring_of_partials_alone():
 _EXIT_AFTER_SIDE_STREAM = """
 import torch
 from asdl_b200 import ops
+ops.extension()                       # loaded before CUDA starts, so its static objects outlive CUDA's
 for backend in ('tensor_core', 'cuda_core'):
     ops.CHOLESKY_BACKEND = backend
     a, out = torch.eye(200, device='cuda'), torch.empty(200, 200, device='cuda')
