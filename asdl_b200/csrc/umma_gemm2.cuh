@@ -1016,8 +1016,8 @@ splitk_reduce2_kernel(const __grid_constant__ GemmProblem2 single, const GemmPro
   __syncthreads();
   // mirrored store: element (r, c) of the patch goes to C[c][r]; neighbouring threads write neighbouring columns
 #pragma unroll
-  for (int i = 0; i < ROWS * G2_RED_COLS / 256; ++i) {
-    const int e = threadIdx.x + 256 * i, lr = e % ROWS, lc = e / ROWS;   // patch column -> destination row
+  for (int i = 0; i < G2_RED_COLS / (256 / ROWS); ++i) {
+    const int lr = threadIdx.x & (ROWS - 1), lc = (threadIdx.x / ROWS) + (256 / ROWS) * i;   // patch column -> destination row
     const int dst_r = col0 + lc, dst_c = row0 + lr;
     if (dst_r < P.N && dst_c < P.M && dst_r < dst_c)
       P.C[static_cast<size_t>(dst_r) * P.ldc + dst_c] = tile[lr][lc];
