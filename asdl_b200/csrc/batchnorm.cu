@@ -481,7 +481,7 @@ std::vector<at::Tensor> bn_forward_train(at::Tensor x, at::Tensor weight, at::Te
       invstd.data_ptr<float>(), coef.data_ptr<float>(), tracked, s.channels, s.splits, s.rows,
       static_cast<float>(momentum), static_cast<float>(eps));
   const Walk w = walk_plan(s.channels / 8);
-  const dim3 grid = walk_grid_layers(w, (s.rows + 1) / 2, 4);   // at least two rows a thread
+  const dim3 grid = walk_grid_layers(w, s.rows, 4);
   const float* scale = coef.data_ptr<float>();
   const float* shift = scale + s.channels;
   if (rp != nullptr && relu)
@@ -552,7 +552,7 @@ std::vector<at::Tensor> bn_backward_train(at::Tensor x, at::Tensor dy, at::Tenso
       part.data_ptr<float>(), wp, bp, mp, ip, dweight.data_ptr<float>(), dbias.data_ptr<float>(), coef.data_ptr<float>(),
       s.channels, s.splits, s.rows);
   const Walk w = walk_plan(s.channels / 8);
-  const dim3 grid = walk_grid_layers(w, (s.rows + 1) / 2, 3);
+  const dim3 grid = walk_grid_layers(w, s.rows, 3);
   const float* k = coef.data_ptr<float>();
   const float *sc = k, *sh = k + s.channels;
   const float *k_dy = k + 2 * s.channels, *k_x = k + 3 * s.channels, *k_c = k + 4 * s.channels;
