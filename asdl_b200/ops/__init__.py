@@ -353,10 +353,10 @@ def kron_apply(left: torch.Tensor, mid: torch.Tensor, right: torch.Tensor) -> to
 #: stride-1 convolutions on channels_last bf16 inputs with a multiple of 64 channels: gather the patch tiles
 #: inside the SYRK (4-D TMA boxes) instead of writing the patch matrix to memory first
 IMPLICIT_IM2COL = os.environ.get('ASDL_B200_IMPLICIT_IM2COL', '1') != '0'
-#: ... when the patch matrix would take at least this many MiB.  Measured on single layers (32 images): at 56 x 56 x 64
-#: channels (110 MiB of patches) the implicit SYRK takes the time of im2col + SYRK (0.128 vs 0.124 ms); on the small
-#: maps of deep layers (14 x 14 x 256: 28 MiB) the 4-D boxes of 2 x 2 pixels x 16 images load at half the rate of the
-#: 2-D boxes of an explicit matrix (0.144 vs 0.077 ms), so those keep the explicit path.
+#: ... when the patch matrix would take at least this many MiB, for the memory: the matrix is never written.  In time the
+#: explicit path is ahead on every layer measured (32 images): at 56 x 56 x 64 channels (110 MiB of patches) 0.099 ms for
+#: im2col + SYRK and 0.128 for the implicit SYRK; on the small maps of deep layers (14 x 14 x 256: 28 MiB) the 4-D boxes of
+#: 2 x 2 pixels x 16 images load at half the rate of the 2-D boxes of an explicit matrix (0.065 and 0.146 ms).
 IMPLICIT_IM2COL_MIN_MB = float(os.environ.get('ASDL_B200_IMPLICIT_IM2COL_MIN_MB', '64'))
 
 
