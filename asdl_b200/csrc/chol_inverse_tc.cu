@@ -1,29 +1,36 @@
 // Grouped fp32-accurate inverse of damped symmetric positive-definite matrices on the tensor cores:
 //     out_m = (A_m + damping_m * I)^-1        for m = 0 .. count-1, sizes n_m arbitrary.
 //
-// Blocked right-looking Cholesky with 128-wide panels, triangular inverse by recursive doubling,
-// then X^T X.  Every O(n^3) product runs on the persistent tcgen05 GEMM (umma_gemm2.cuh) from
-// three-way bf16 splits of the fp32 values (v = hi + mid + lo carries the whole significand; the
-// kernel's "split3" flavour issues the six significant part products small-magnitude-first and
-// sums the contraction in fp32 registers, one 64-wide K block per TMEM chunk), and every
-// subtraction between products happens in fp32 on the CUDA cores: the trailing update of a
-// right-looking factorisation is a K = 128 product subtracted from the fp32 matrix in the GEMM
-// epilogue.  Only the 128 x 128 diagonal blocks are factored and inverted on the CUDA cores (one
-// CTA each, 32 columns at a time).
+// Cholesky factor L, X = L^-1 row by row beside it, then X^T X, in 128 x 128 tiles.  A tile is one task:
 //
-//   potrf, step k:  diag(k):   T_k = L_kk^-1, L_kk = chol(A_kk) (not stored)     (CUDA cores)
-//                   panel(k):  L_ik = A_ik T_k^T                  for i > k      (GEMM, K = 128)
-//                   trail(k):  A_ij -= L_ik L_jk^T                for k < j <= i (GEMM, K = 128)
-//   trtri, level l: blocks of s = 2^l panels are merged pairwise:
-//                   W   = L_21 X_11,   X_21 = -X_22 W                            (two GEMM launches)
-//   lauum:          out = X^T X  (lower tiles, mirrored)                         (one GEMM launch)
+//   DIAG(j)      S = A_jj - sum_{k<j} L_jk L_jk^T;   T_j = chol(S)^-1 on the CUDA cores (L_jj itself is not stored)
+//   FACTOR(i,j)  S = A_ij - sum_{k<j} L_ik L_jk^T;   L_ij = S T_j^T                       for i > j
+//   INV(i,j)     W = sum_{j<=k<i} L_ik X_kj;         X_ij = -T_i W                        for i > j  (X_jj = T_j)
+//   OUT(i,j)     out_ij = sum_{r>=i} X_ri^T X_rj, mirrored                                for i >= j
 //
-// All matrices of a call advance through the same launches ("grouped"): a launch's work list
-// holds the tiles of every matrix that has work at that step.  Problem tables, work lists and the
-// bf16 split buffers depend only on the addresses and sizes of the matrices; they are built once
-// and cached (prepared_cache.h), so a repeated call (the K-FAC state) issues no host-to-device copy
-// and can be captured in a CUDA graph, which then keeps them.  Inputs are not modified; a non-positive pivot sets the status word to
-// ERR_NOT_SPD and the factorisation continues with pivot 1.
+// ONE persistent launch runs the tasks of all matrices.  CTAs claim them in the order of a list in which a task stands behind
+// everything it needs, and a task waits for its operands K block by K block: per block row of a matrix there are two progress
+// words, the number of finished tiles of that row of L and of that column of X.  Since the first unfinished task of the list
+// never waits for a later one, any number of resident CTAs makes progress.  The sums run ahead of the chain
+// DIAG -> FACTOR -> DIAG: only their last K blocks remain when a diagonal block is done.
+//
+// Sums are formed by the tensor cores from three-way bf16 splits of the fp32 values (v = hi + mid + lo carries the whole
+// significand; six significant part products, small magnitudes first, as in the split3 flavour of umma_gemm2.cuh): every
+// 64-wide K block goes to a fresh TMEM accumulator that the eight epilogue warps read back and add to a running fp32 sum in
+// registers; A enters at the end (a sum that starts from -A has roundings of A's size in every step: 5 % more error in the
+// inverse).  The second product of FACTOR and INV takes that sum from the same CTA: the epilogue writes its three parts into
+// the operand half of a ring stage whose other half TMA fills with T.
+//
+// What bounds it: the chain of diagonal blocks (DIAG, one FACTOR tile, the last K panel of the next DIAG), and beside it the
+// operand traffic of the ring, 96 KiB per K block of 1536 tensor cycles.  The former version ran the same arithmetic
+// right-looking in 28 (six factors up to 784) to 121 (the 107 factors of ResNet-50) dependent launches: every K = 128 update
+// read and wrote the fp32 matrix, each lane a row of its own, and every launch drained before the next began.
+// Six factors 784, 4 x 512, 10: 594 -> 304 us; ResNet-50's 107 factors: 8.06 -> 3.80 ms.
+//
+// Tables, task lists and the bf16 split buffers depend only on the addresses and sizes of the matrices; they are built once
+// and cached (prepared_cache.h), so a repeated call (the K-FAC state) issues no host-to-device copy and can be captured in a
+// CUDA graph, which then keeps them.  Inputs are not modified; a non-positive pivot sets the status word to ERR_NOT_SPD and the
+// factorisation continues with pivot 1.
 //
 // Stands in for asdl/utils.py:91-96 (torch.linalg.cholesky + cholesky_inverse).
 #include <cstring>
@@ -35,67 +42,64 @@ namespace b200 {
 
 namespace {
 
-constexpr int TB = 128;  // panel width
+constexpr int TB = 128;  // tile
+
+enum : int { TASK_DIAG = 0, TASK_FACTOR = 1, TASK_INV = 2, TASK_OUT = 3, TASK_END = 4 };
+
+// L and X are kept as the images that the products want in shared memory.  Tile (i, j), j <= i, has index i (i + 1) / 2 + j and
+// consists of two halves of 64 columns; a half is three parts (hi, mid, lo) of 128 rows of 128 bytes, the 16-byte pieces of a row
+// exchanged as the 128-byte swizzle does it.  A half of a part is a K block of a K-major operand (16 KiB, one copy); its rows
+// [64 b, 64 b + 64) are 64 columns of K block b of an MN-major operand (8 KiB).  Rows and columns past the matrix are stored too.
+constexpr int PART_BYTES = 128 * 128, TILE_BYTES = 6 * PART_BYTES;
 
 struct TcMat {
-  const float* A;         // input n x n (ld = lda)
-  float* L;               // n x n fp32 work matrix (the output buffer)
-  __nv_bfloat16* Ls[3];   // splits of L (strictly-lower blocks) / of the current panel column
-  __nv_bfloat16* Xs[3];   // splits of X = L^-1 (lower triangular)
-  int n, nb, lda, ldp, orig, pad;
+  const float* A;          // input n x n (pitch lda)
+  float* out;              // n x n
+  uint8_t* L;              // tiles of L; those of the diagonal are not used
+  uint8_t* X;              // tiles of X
+  int* row_l;              // finished tiles of block row i of L
+  int* col_x;              // block column j of X is finished down to (not including) this block row
+  int n, nb, lda, orig;
 };
 
-__device__ __forceinline__ void split3_store(__nv_bfloat16* const* parts, size_t idx, float v) {
-  const __nv_bfloat16 h = __float2bfloat16_rn(v);
-  const float r1 = v - __bfloat162float(h);
-  const __nv_bfloat16 m = __float2bfloat16_rn(r1);
-  const __nv_bfloat16 l = __float2bfloat16_rn(r1 - __bfloat162float(m));
-  parts[0][idx] = h;
-  parts[1][idx] = m;
-  parts[2][idx] = l;
+__device__ __forceinline__ uint8_t* tile_at(uint8_t* base, int i, int j) {
+  return base + (static_cast<size_t>(i) * (i + 1) / 2 + j) * TILE_BYTES;
 }
 
-// ---- phase 0: L = A + damping * I, splits of block column 0 -----------------------------------
-// grid: (row groups, matrices); a warp walks along one row
-__global__ void __launch_bounds__(256) tc_prepare_kernel(const TcMat* mats, const float* damping) {
-  const TcMat M = mats[blockIdx.y];
-  const float d = damping[M.orig];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int r = blockIdx.x * 8 + warp; r < M.n; r += gridDim.x * 8) {
-    const float* src = M.A + static_cast<size_t>(r) * M.lda;
-    float* dst = M.L + static_cast<size_t>(r) * M.n;
-    for (int c = lane; c < M.n; c += 32) {
-      float v = src[c];
-      if (r == c) v += d;
-      dst[c] = v;
-      if (c < TB && r >= TB) split3_store(M.Ls, static_cast<size_t>(r) * M.ldp + c, v);
-    }
-  }
+struct Task {
+  int mat, kind, i, j;
+};
+
+// K blocks of a task's sum
+__host__ __device__ inline int task_blocks(int kind, int i, int j, int n) {
+  if (kind == TASK_OUT) return (n - i * TB + G2_BK - 1) / G2_BK;
+  return kind == TASK_INV ? 2 * (i - j) : 2 * j;
 }
 
-// ---- diagonal block k: Cholesky factor and its inverse ----------------------------------------
-// Four stages of 32 columns on one CTA.  Stage q, columns [kb, be):
-//   factor   warp 0, one row of the 32 x 32 block per lane, in registers.  The next pivot is the lane's own product, so the
-//            chain from pivot to pivot is a shuffle, a reciprocal square root and three roundings, without a barrier;
-//   panel    one thread per row below (forward substitution with the block) and one per column of the inverse's rows
-//            [kb, be): 128 threads in all, the same substitution on different inputs.  P[j][c] = T[kb + j][c] for c < be and
-//            L[c][kb + j] for c >= be;
+// ---- diagonal block: Cholesky factor and its inverse ----------------------------------------
+// Four stages of 32 columns on the eight epilogue warps of a CTA.  Stage q, columns [kb, be):
+//   factor   one warp, a row of the 32 x 32 block per lane, in registers.  From a pivot to the next the chain is a product, a
+//            shuffle and a reciprocal square root; a column is applied to the columns behind the next one a step later, in the
+//            latency of that chain;
+//   panel    four warps, one thread per row below (forward substitution with the block) and one per column of the inverse's
+//            rows [kb, be), eight columns behind the factor.  P[j][c] = T[kb + j][c] for c < be and L[c][kb + j] for c >= be;
 //   update   S[i][c] -= sum_j P[j][i] P[j][c] for the rows i >= be: the trailing block right of be, the right-hand side of
 //            the inverse left of it.  Finished columns of the factor are dead (only the inverse leaves the kernel), so both
-//            share S.  A warp takes four rows of each row block, a lane one column of each column block.
-// Every entry sees the same roundings in the same order as a column-by-column elimination, and gives the same bits.  The panel
-// steps of all matrices wait for this kernel: with that elimination, a barrier per column and the block in the registers of
-// a 16 x 16 thread grid, six matrices up to 784 x 784 took 749 us and the 107 factors of ResNet-50 8.61 ms; now 589 us and
-// 8.05 ms, of which 46 us are a step of this kernel.  The chain of pivots in one warp bounds it.
-//
-// The code is kept small (one body for all stages, eight columns of a substitution unrolled, the registers shifted by eight
-// between them): with every stage unrolled the kernel was bound by instruction fetch (653 us and 8.71 ms).
+//            share S.  A warp takes four rows of each row block, a lane one column of each column block up to the diagonal;
+//   store    of the rows [kb, be) of T from P, by the other warps while the next stage is factored.
+// Every entry sees the same roundings in the same order as a column-by-column elimination, and gives the same bits.  The chain
+// of pivots bounds it, and the code is kept small (eight columns unrolled, registers shifted by eight between them) since
+// instructions are fetched once per block.  The same stages one after the other, each column applied at once, took 65 000
+// clocks, 23 000 of them to factor; now 49 000.
 constexpr int DG_SP = TB + 1;   // pitch of S: lanes on consecutive rows of a column, or on consecutive columns
 constexpr int DG_PP = TB + 4;   // pitches of P and of the factored block: 16-byte reads
-constexpr int DG_LP = 60;       // the entries from 32 on are zeros: what shifted registers past the block are updated with
-constexpr int DG_SMEM = (TB * DG_SP + 32 * DG_PP + 32 * DG_LP + 32) * 4;
+constexpr int DG_LP = 64;       // the entries from 32 on are zeros: what shifted registers past the block are updated with
+constexpr int DG_SMEM = (TB * DG_SP + 2 * 32 * DG_PP + 32 * DG_LP + 32) * 4;
 
-// v[c] -= x * o[c] for the columns c > j of the 32 in registers
+// Barrier of the eight epilogue warps.
+__device__ __forceinline__ void epi_sync() { named_bar_sync(1, 256); }
+
+// v[c] -= x * o[c] for the columns c > J of the 32 in registers
 template <int J>
 __device__ __forceinline__ void diag_eliminate(float (&v)[32], float x, const float* o) {
 #pragma unroll
@@ -114,9 +118,8 @@ __device__ __forceinline__ void diag_shift(float (&v)[32]) {
   for (int c = 0; c < 32; ++c) v[c] = c < 24 ? v[c + 8 < 32 ? c + 8 : 31] : 0.f;
 }
 
-// 1 / sqrt(pivot) of column j; a pivot that is not positive is reported and replaced by 1
-__device__ __forceinline__ float diag_pivot(float mine, int j, bool& bad) {
-  float d = __shfl_sync(0xffffffffu, mine, j & 31);
+// 1 / sqrt(pivot d) of column j; a pivot that is not positive is reported and replaced by 1
+__device__ __forceinline__ float diag_pivot(float d, int j, bool& bad) {
   if (!(d > 0.f)) {
     bad |= j < 32;   // j = 32: there is no such column, and its result is not used
     d = 1.f;
@@ -125,164 +128,701 @@ __device__ __forceinline__ float diag_pivot(float mine, int j, bool& bad) {
   return iv * fmaf(-0.5f * d, iv * iv, 1.5f);   // one Newton step: full fp32 accuracy
 }
 
-// column j8 + J of the block's factor, by one warp (lane = row).  `iv`: 1 / sqrt of its pivot on entry, of the next pivot on
-// return; that one is formed ahead of the elimination, which fills the latency of the chain.
+// Column j8 + J of the block's factor, by one warp (lane = row).  `iv`: 1 / sqrt of its pivot on entry, of the next pivot on
+// return.  On entry the column before (this lane's entry `last`, the rows' entries `o`) is still to be applied to the columns
+// from J + 1 on; on return this one to those from J + 2 on.
 template <int J>
-__device__ __forceinline__ void diag_factor_step(float (&a)[32], float& iv, float* Lk, float* inv, int j8, int lane, bool& bad) {
+__device__ __forceinline__ void diag_factor_step(float (&a)[32], float (&o)[32], float& last, float& iv, float* Lk, float* inv,
+                                                 int j8, int lane, bool& bad) {
   const int j = j8 + J;
   const float l = a[J] * iv;
   Lk[j * DG_LP + lane] = l;   // rows above j: not used
   if (lane == 0) inv[j] = iv;
-  iv = diag_pivot(fmaf(-l, l, a[J + 1]), j + 1, bad);
+  a[J + 1] = fmaf(-last, o[J + 1], a[J + 1]);
+  const float d = __shfl_sync(0xffffffffu, fmaf(-l, l, a[J + 1]), (j + 1) & 31);
+  const float next = __shfl_sync(0xffffffffu, l, (j + 1) & 31);
+#pragma unroll
+  for (int c = J + 2; c < 32; ++c) a[c] = fmaf(-last, o[c], a[c]);
   __syncwarp();
-  diag_eliminate<J>(a, l, Lk + j * DG_LP + j8);
+  constexpr int SHIFT = J == 7 ? 8 : 0;   // the registers are shifted after the eighth column
+#pragma unroll
+  for (int c4 = 0; c4 < 32; c4 += 4) {
+    if (c4 + 3 + SHIFT < J + 2) continue;
+    const float4 q = *reinterpret_cast<const float4*>(Lk + j * DG_LP + j8 + SHIFT + c4);
+    o[c4] = q.x;
+    o[c4 + 1] = q.y;
+    o[c4 + 2] = q.z;
+    o[c4 + 3] = q.w;
+  }
+  iv = diag_pivot(d, j + 1, bad);
+  a[J + 1] = fmaf(-l, next, a[J + 1]);
+  last = l;
 }
 
 template <int J>
-__device__ __forceinline__ void diag_panel_step(float (&v)[32], const float* Lk, const float* inv, float* P, int j8, int c) {
-  const float x = v[J] * inv[j8 + J];
-  P[(j8 + J) * DG_PP + c] = x;
-  diag_eliminate<J>(v, x, Lk + (j8 + J) * DG_LP + j8);
+__device__ __forceinline__ void diag_panel_step(float (&v)[32], const float* Lk, const float* inv, int j8) {
+  v[J] *= inv[j8 + J];
+  diag_eliminate<J>(v, v[J], Lk + (j8 + J) * DG_LP + j8);
 }
 
-__global__ void __launch_bounds__(256, 1) tc_diag_kernel(const TcMat* mats, int k, int* status) {
-  const TcMat M = mats[blockIdx.x];
-  if (k >= M.nb) return;
-  extern __shared__ float4 dg_smem[];
-  float* S = reinterpret_cast<float*>(dg_smem);
-  float* P = S + TB * DG_SP;            // TB * DG_SP is a multiple of four
-  float* Lk = P + 32 * DG_PP;
-  float* inv = Lk + 32 * DG_LP;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r0 = k * TB;
-#pragma unroll 4
-  for (int r = warp; r < TB; r += 8) {
-    const float* src = M.L + static_cast<size_t>(r0 + r) * M.n + r0;
+// Rows and columns behind stage KQ, whose columns are [32 KQ, 32 KQ + 32).
+template <int KQ>
+__device__ __forceinline__ void diag_update(float* S, const float* P, int warp, int lane) {
+  constexpr int NB = 3 - KQ;   // row blocks
+  float acc[NB][4][4];
+  float* const rows = S + (32 * (KQ + 1) + 4 * warp) * DG_SP + lane;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int c = lane + 32 * q;
-      // identity padding keeps the block factorisable
-      S[r * DG_SP + c] = (r0 + r < M.n && r0 + c < M.n) ? (c <= r ? src[c] : 0.f) : (r == c ? 1.f : 0.f);
+  for (int b = 0; b < NB; ++b)
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int q = 0; q <= KQ + 1 + b; ++q) acc[b][r][q] = q == KQ ? 0.f : rows[(32 * b + r) * DG_SP + 32 * q];
+#pragma unroll 2
+  for (int j = 0; j < 32; ++j) {
+    float pc[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) pc[q] = P[j * DG_PP + lane + 32 * q];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const float4 raw = *reinterpret_cast<const float4*>(P + j * DG_PP + 32 * (KQ + 1 + b) + 4 * warp);
+      const float pr[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+      for (int q = 0; q <= KQ + 1 + b; ++q)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) acc[b][r][q] = fmaf(-pr[r], pc[q], acc[b][r][q]);
     }
   }
-  for (int e = tid; e < 32 * DG_LP; e += 256) Lk[e] = 0.f;
-  __syncthreads();
+#pragma unroll
+  for (int b = 0; b < NB; ++b)
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int q = 0; q <= KQ + 1 + b; ++q) rows[(32 * b + r) * DG_SP + 32 * q] = acc[b][r][q];
+}
+
+// Factors the block that S (in shared memory, zeros above the diagonal, identity past the matrix) holds and stores its
+// inverse T as the tile `image`.  `live`: rows of the matrix in the block (the others are padding).  `tid`: thread among the 256 of the epilogue warps.
+__device__ __noinline__ void diag_block(uint8_t* image, int live, float* S, int tid, int* status) {
+  float* const P0 = S + TB * DG_SP;            // TB * DG_SP is a multiple of four
+  float* const Lk = P0 + 2 * 32 * DG_PP;
+  float* const inv = Lk + 32 * DG_LP;
+  const int lane = tid & 31, warp = tid >> 5;
+  // warp 0 factors; the panel is on four warps of the other schedulers
+  const int panel = warp == 5 ? 3 : (warp >= 1 && warp <= 3 ? warp - 1 : -1);
+  const int c = 32 * panel + lane;             // row or column of a panel thread
   bool bad = false;
-  const int live = min(TB, M.n - r0);   // rows of the matrix in this block (the others are padding)
+  auto store_row = [&](int r, int col, const uint32_t (&w)[3][2]) {   // columns col .. col + 3, col a multiple of four
+    uint8_t* at = image + (col >> 6) * (3 * PART_BYTES) + r * 128 + ((((col & 63) >> 3) ^ (r & 7)) << 4) + (col & 4) * 2;
+#pragma unroll
+    for (int part = 0; part < 3; ++part) *reinterpret_cast<uint2*>(at + part * PART_BYTES) = make_uint2(w[part][0], w[part][1]);
+  };
+  // rows [kb, kb + 32) of the inverse are final: split and stored, zeros right of the diagonal
+  auto store = [&](int kb, int first, int threads) {
+    const float* P = P0 + (kb >> 5 & 1) * 32 * DG_PP;
+#pragma unroll 1
+    for (int e = first; e < 32 * (TB / 4); e += threads) {
+      const int j = e >> 5, col = (e & 31) * 4;
+      const float4 raw = *reinterpret_cast<const float4*>(P + j * DG_PP + col);
+      const float t[4] = {raw.x, raw.y, raw.z, raw.w};
+      uint32_t w[3][2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float x0 = col + 2 * h <= kb + j ? t[2 * h] : 0.f, x1 = col + 2 * h + 1 <= kb + j ? t[2 * h + 1] : 0.f;
+#pragma unroll
+        for (int part = 0; part < 3; ++part) {
+          const __nv_bfloat16 b0 = __float2bfloat16_rn(x0), b1 = __float2bfloat16_rn(x1);
+          w[part][h] = static_cast<uint32_t>(__bfloat16_as_ushort(b0)) | (static_cast<uint32_t>(__bfloat16_as_ushort(b1)) << 16);
+          x0 -= __bfloat162float(b0);
+          x1 -= __bfloat162float(b1);
+        }
+      }
+      store_row(kb + j, col, w);
+    }
+  };
+  for (int e = tid; e < 32 * DG_LP; e += 256) Lk[e] = 0.f;
 #pragma unroll 1
   for (int kb = 0; kb < live; kb += 32) {
-    const int be = kb + 32;
+    epi_sync();
+    float* const P = P0 + (kb >> 5 & 1) * 32 * DG_PP;
     if (warp == 0) {
-      float a[32];
+      float a[32], o[32], last = 0.f;
 #pragma unroll
-      for (int c = 0; c < 32; ++c) a[c] = S[(kb + lane) * DG_SP + kb + c];   // c > lane: not used
-      float iv = diag_pivot(a[0], 0, bad);
+      for (int i = 0; i < 32; ++i) {
+        a[i] = S[(kb + lane) * DG_SP + kb + i];   // i > lane: not used
+        o[i] = 0.f;
+      }
+      float iv = diag_pivot(__shfl_sync(0xffffffffu, a[0], 0), 0, bad);
 #pragma unroll 1
       for (int j8 = 0; j8 < 32; j8 += 8) {
-        diag_factor_step<0>(a, iv, Lk, inv, j8, lane, bad);
-        diag_factor_step<1>(a, iv, Lk, inv, j8, lane, bad);
-        diag_factor_step<2>(a, iv, Lk, inv, j8, lane, bad);
-        diag_factor_step<3>(a, iv, Lk, inv, j8, lane, bad);
-        diag_factor_step<4>(a, iv, Lk, inv, j8, lane, bad);
-        diag_factor_step<5>(a, iv, Lk, inv, j8, lane, bad);
-        diag_factor_step<6>(a, iv, Lk, inv, j8, lane, bad);
-        diag_factor_step<7>(a, iv, Lk, inv, j8, lane, bad);
+        diag_factor_step<0>(a, o, last, iv, Lk, inv, j8, lane, bad);
+        diag_factor_step<1>(a, o, last, iv, Lk, inv, j8, lane, bad);
+        diag_factor_step<2>(a, o, last, iv, Lk, inv, j8, lane, bad);
+        diag_factor_step<3>(a, o, last, iv, Lk, inv, j8, lane, bad);
+        diag_factor_step<4>(a, o, last, iv, Lk, inv, j8, lane, bad);
+        diag_factor_step<5>(a, o, last, iv, Lk, inv, j8, lane, bad);
+        diag_factor_step<6>(a, o, last, iv, Lk, inv, j8, lane, bad);
+        diag_factor_step<7>(a, o, last, iv, Lk, inv, j8, lane, bad);
         diag_shift(a);
+        asm volatile("barrier.cta.arrive %0, 160;" ::"r"(2 + (j8 >> 3)) : "memory");
       }
-    }
-    __syncthreads();
-    if (tid < TB) {
-      float v[32];
-      const float* from = tid >= be ? S + tid * DG_SP + kb : S + kb * DG_SP + tid;
-      const int pitch = tid >= be ? 1 : DG_SP;
+    } else {
+      if (kb > 0) store(kb - 32, tid - 32, 224);
+      if (panel >= 0) {
+        float v[32];
+        const float* from = c >= kb + 32 ? S + c * DG_SP + kb : S + kb * DG_SP + c;
+        const int pitch = c >= kb + 32 ? 1 : DG_SP;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = from[j * pitch];
-      if (warp == kb / 32) {   // the block's own columns of the inverse start from the identity
+        for (int j = 0; j < 32; ++j) v[j] = from[j * pitch];
+        if (panel == kb / 32) {   // the block's own columns of the inverse start from the identity
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = lane == j ? 1.f : 0.f;
-      }
-#pragma unroll 1
-      for (int j8 = 0; j8 < 32; j8 += 8) {
-        diag_panel_step<0>(v, Lk, inv, P, j8, tid);
-        diag_panel_step<1>(v, Lk, inv, P, j8, tid);
-        diag_panel_step<2>(v, Lk, inv, P, j8, tid);
-        diag_panel_step<3>(v, Lk, inv, P, j8, tid);
-        diag_panel_step<4>(v, Lk, inv, P, j8, tid);
-        diag_panel_step<5>(v, Lk, inv, P, j8, tid);
-        diag_panel_step<6>(v, Lk, inv, P, j8, tid);
-        diag_panel_step<7>(v, Lk, inv, P, j8, tid);
-        diag_shift(v);
-      }
-    }
-    __syncthreads();
-    // rows [kb, be) of the inverse are final: split and stored, zeros right of the diagonal (the pitch of Xs is a multiple
-    // of 64)
-#pragma unroll 1
-    for (int e = tid; e < 32 * (TB / 4); e += 256) {
-      const int j = e >> 5, c = (e & 31) * 4, row = r0 + kb + j, col = r0 + c;
-      if (row < M.n && col < M.ldp) {
-        const float4 raw = *reinterpret_cast<const float4*>(P + j * DG_PP + c);
-        const float t[4] = {raw.x, raw.y, raw.z, raw.w};
-        uint32_t w[3][2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          float x0 = c + 2 * h <= kb + j ? t[2 * h] : 0.f, x1 = c + 2 * h + 1 <= kb + j ? t[2 * h + 1] : 0.f;
-#pragma unroll
-          for (int part = 0; part < 3; ++part) {
-            const __nv_bfloat16 b0 = __float2bfloat16_rn(x0), b1 = __float2bfloat16_rn(x1);
-            w[part][h] = static_cast<uint32_t>(__bfloat16_as_ushort(b0)) | (static_cast<uint32_t>(__bfloat16_as_ushort(b1)) << 16);
-            x0 -= __bfloat162float(b0);
-            x1 -= __bfloat162float(b1);
-          }
+          for (int j = 0; j < 32; ++j) v[j] = lane == j ? 1.f : 0.f;
         }
-        const size_t at = static_cast<size_t>(row) * M.ldp + col;
-#pragma unroll
-        for (int part = 0; part < 3; ++part) *reinterpret_cast<uint2*>(M.Xs[part] + at) = make_uint2(w[part][0], w[part][1]);
-      }
-    }
 #pragma unroll 1
-    for (int rb = be; rb < live; rb += 32) {   // row blocks below; blocks right of the diagonal are computed and never read
-      float acc[4][4];
-      float* const row0 = S + (rb + 4 * warp) * DG_SP + lane;
+        for (int j8 = 0; j8 < 32; j8 += 8) {
+          named_bar_sync(2 + (j8 >> 3), 160);
+          diag_panel_step<0>(v, Lk, inv, j8);
+          diag_panel_step<1>(v, Lk, inv, j8);
+          diag_panel_step<2>(v, Lk, inv, j8);
+          diag_panel_step<3>(v, Lk, inv, j8);
+          diag_panel_step<4>(v, Lk, inv, j8);
+          diag_panel_step<5>(v, Lk, inv, j8);
+          diag_panel_step<6>(v, Lk, inv, j8);
+          diag_panel_step<7>(v, Lk, inv, j8);
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) acc[r][q] = 32 * q == kb ? 0.f : row0[r * DG_SP + 32 * q];
-#pragma unroll 8
-      for (int j = 0; j < 32; ++j) {
-        const float4 raw = *reinterpret_cast<const float4*>(P + j * DG_PP + rb + 4 * warp);
-        const float pr[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float pc = P[j * DG_PP + lane + 32 * q];
-#pragma unroll
-          for (int r = 0; r < 4; ++r) acc[r][q] = fmaf(-pr[r], pc, acc[r][q]);
+          for (int j = 0; j < 8; ++j) P[(j8 + j) * DG_PP + c] = v[j];
+          diag_shift(v);
         }
       }
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) row0[r * DG_SP + 32 * q] = acc[r][q];
     }
-    __syncthreads();
+    epi_sync();
+    if (kb == 0)
+      diag_update<0>(S, P, warp, lane);
+    else if (kb == 32)
+      diag_update<1>(S, P, warp, lane);
+    else if (kb == 64)
+      diag_update<2>(S, P, warp, lane);
   }
+  const int stages = (live + 31) / 32;
+  store(32 * stages - 32, tid, 256);
+  constexpr uint32_t none[3][2] = {};
+#pragma unroll 1
+  for (int e = tid + stages * 32 * 32; e < TB * 32; e += 256) store_row(e >> 5, (e & 31) * 4, none);   // rows of padding
   if (bad && tid == 0) set_error(status, ERR_NOT_SPD);
 }
 
-struct Launch {
-  int kind;   // 0: diagonal blocks of step `arg`, 1: GEMM work list
-  int arg;    // step k (kind 0) / offset into the work list (kind 1)
-  int count;  // CTAs (kind 0) / work items (kind 1)
-};
+// ---- the task kernel ------------------------------------------------------------------------------
+// The ring holds two K blocks of six operand parts (roles), and every role of a block has a slot and an `empty` barrier of its
+// own: a part is loaded again as soon as the last product that reads it is done, not when the block is.  Products are issued in
+// the order (mid,mid) (lo,hi) (hi,lo) (mid,hi) (hi,mid) (hi,hi): small magnitudes first, and every role has at least a block's
+// time between its release and its next use.
+constexpr int TC_STAGES = 2, TC_ITEMS = 4, TC_EPI_WARPS = 8;
+constexpr int TC_STAGE_BYTES = 6 * PART_BYTES;
+enum : int { ROLE_A_HI = 0, ROLE_A_MID, ROLE_A_LO, ROLE_B_HI, ROLE_B_MID, ROLE_B_LO, ROLES };   // slots of a K block, in order
+constexpr int TC_THREADS = 64 + 32 * TC_EPI_WARPS;
+constexpr int TC_STAGING = 4096;                    // per epilogue warp
+constexpr int TC_SMEM = 1024 /*alignment*/ + TC_STAGES * TC_STAGE_BYTES + TC_EPI_WARPS * TC_STAGING + 512 /*barriers, tasks*/;
+static_assert(DG_SMEM <= TC_STAGES * TC_STAGE_BYTES && TC_SMEM <= 232448, "shared memory of the task kernel");
+
+__device__ __forceinline__ int ld_acquire(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release(int* p, int v) {
+  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+// Orders this thread's generic accesses (global and shared) with the async proxy's (TMA, MMA operands).
+__device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
+// Waits until a progress word has reached `want`; `seen` remembers what was read.  Bounded in time; ends early when another
+// CTA gave up.
+__device__ __forceinline__ bool wait_progress(const int* word, int want, int& seen, const int* abort) {
+  if (seen >= want) return true;
+  seen = ld_acquire(word);
+  if (seen < want) {
+    const uint64_t t0 = globaltimer_ns();
+    uint32_t spins = 0;
+    while ((seen = ld_acquire(word)) < want)
+      if ((++spins & 63) == 0 && (ld_acquire(abort) != 0 || globaltimer_ns() - t0 > B200_WAIT_NS)) return false;
+  }
+  proxy_fence();
+  return true;
+}
+
+// Copy of `bytes` (a multiple of 16, both sides 16-byte aligned) from global to shared memory, counted on `bar`.
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
+// Warp-collective store of 32 lanes x 32 consecutive fp32 columns to tensor memory.
+__device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
+      "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]),
+      "r"(r[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// True on all 256 threads when `bad` is set on any of them.
+__device__ __forceinline__ bool epi_any(bool bad) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.or.pred q, 1, 256, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"(static_cast<uint32_t>(bad))
+      : "memory");
+  return r != 0;
+}
+
+// A warp's 32 x 32 patch of fp32 values in its staging memory: rows of 128 bytes, the 16-byte pieces of a row exchanged.
+__device__ __forceinline__ void stage_patch(const float* v, uint8_t* stg, int lane) {
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+    *reinterpret_cast<float4*>(stg + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+  __syncwarp();
+}
+// Three-way split of a staged patch, columns [32 h, 32 h + 32) of an image whose first row is at `base` (global or shared memory).
+// A lane splits eight values at a time.  The loop is not unrolled: code that runs once per tile is bound by instruction fetch
+// (unrolled over 64 values of a row per thread it took 5 us to split and store a tile).
+__device__ __noinline__ void split_patch(const uint8_t* stg, uint8_t* base, int h, int lane) {
+#pragma unroll 1
+  for (int i = 0; i < 4; ++i) {
+    const int r = i * 8 + (lane >> 2), g = lane & 3;
+    const float4 lo = *reinterpret_cast<const float4*>(stg + r * 128 + (((2 * g) ^ (r & 7)) << 4));
+    const float4 hi = *reinterpret_cast<const float4*>(stg + r * 128 + (((2 * g + 1) ^ (r & 7)) << 4));
+    float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    uint8_t* at = base + r * 128 + (((4 * h + g) ^ (r & 7)) << 4);
+#pragma unroll
+    for (int part = 0; part < 3; ++part) {
+      uint32_t w[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const __nv_bfloat16 b0 = __float2bfloat16_rn(v[2 * k]), b1 = __float2bfloat16_rn(v[2 * k + 1]);
+        w[k] = static_cast<uint32_t>(__bfloat16_as_ushort(b0)) | (static_cast<uint32_t>(__bfloat16_as_ushort(b1)) << 16);
+        v[2 * k] -= __bfloat162float(b0);
+        v[2 * k + 1] -= __bfloat162float(b1);
+      }
+      *reinterpret_cast<uint4*>(at + part * PART_BYTES) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+}
+// Stores a staged patch (element (r, c) at r * 32 + (c ^ r)) to out[row0 ..][col0 ..] and its mirror image.
+__device__ __noinline__ void store_patch(const float* stg, float* out, int n, int row0, int col0, bool diag, int lane) {
+  const int gc = col0 + lane, gr = row0 + lane;
+#pragma unroll 8
+  for (int r = 0; r < 32; ++r)
+    if (row0 + r < n && gc < n && (!diag || gc <= row0 + r)) out[static_cast<size_t>(row0 + r) * n + gc] = stg[r * 32 + (lane ^ r)];
+#pragma unroll 8
+  for (int c = 0; c < 32; ++c)
+    if (gr < n && col0 + c < n && (!diag || col0 + c < gr)) out[static_cast<size_t>(col0 + c) * n + gr] = stg[lane * 32 + (c ^ lane)];
+}
+
+__global__ void __launch_bounds__(TC_THREADS, 1)
+tc_tasks_kernel(const TcMat* __restrict__ mats, const Task* __restrict__ tasks, int n_tasks, const float* __restrict__ damping,
+                int* ctrl, int* status) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint8_t* staging = smem + TC_STAGES * TC_STAGE_BYTES;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(staging + TC_EPI_WARPS * TC_STAGING);
+  uint64_t* empty_bar = full_bar + TC_STAGES * 3;   // full: (mid, mid), (A lo, B hi), (A hi, B lo) of a block; empty: its roles
+  uint64_t* acc_full = empty_bar + TC_STAGES * ROLES;
+  uint64_t* acc_empty = acc_full + 2;
+  uint64_t* item_full = acc_empty + 2;
+  uint64_t* item_empty = item_full + TC_ITEMS;
+  uint64_t* operand_bar = item_empty + TC_ITEMS;   // the epilogue's half of a stage of a second product is written
+  uint64_t* diag_bar = operand_bar + 2;            // the epilogue has left the ring after a diagonal block
+  Task* items = reinterpret_cast<Task*>(diag_bar + 2);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(items + TC_ITEMS);
+  int* const next_task = ctrl;
+  int* const abort = ctrl + 1;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int b = 0; b < TC_STAGES * 3; ++b) mbar_init(&full_bar[b], 2);
+    for (int b = 0; b < TC_STAGES * ROLES; ++b) mbar_init(&empty_bar[b], 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], TC_EPI_WARPS);
+      mbar_init(&operand_bar[b], 4);   // the four warps that hold this K block of the operand
+    }
+    for (int b = 0; b < TC_ITEMS; ++b) {
+      mbar_init(&item_full[b], 1);
+      mbar_init(&item_empty[b], 1 + TC_EPI_WARPS);
+    }
+    mbar_init(diag_bar, 1);
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 512);   // two accumulators and a tile of A
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  auto give_up = [&](int code) {
+    set_error(status, code);
+    atomicExch(abort, 1);
+  };
+
+  if (warp == 0) {
+    // ---- claims tasks, waits for their operands, loads them
+    if (lane == 0) {
+      uint32_t it = 0, diags = 0;
+      bool ok = true;
+      for (uint32_t tk = 0; ok; ++tk) {
+        const int idx = atomicAdd(next_task, 1);
+        Task t;
+        if (idx < n_tasks)
+          t = tasks[idx];
+        else
+          t = {0, TASK_END, 0, 0};
+        const uint32_t slot = tk % TC_ITEMS;
+        if (!mbar_wait(&item_empty[slot], ((tk / TC_ITEMS) & 1) ^ 1)) {
+          give_up(ERR_WAIT_EMPTY);
+          break;
+        }
+        items[slot] = t;
+        mbar_arrive(&item_full[slot]);
+        if (t.kind == TASK_END) break;
+        const TcMat& M = mats[t.mat];
+        const int i0 = t.i * TB, j0 = t.j * TB;
+        const bool two = t.kind == TASK_FACTOR || t.kind == TASK_INV;   // a second product follows
+        const bool shared_ab = t.kind == TASK_DIAG || (t.kind == TASK_OUT && t.i == t.j);
+        const int k0 = t.kind == TASK_INV ? j0 : (t.kind == TASK_OUT ? i0 : 0);
+        // progress of the two operands: L by rows, X by columns
+        const int* wa = t.kind == TASK_OUT ? M.col_x + t.i : M.row_l + t.i;
+        const int* wb = t.kind == TASK_INV || t.kind == TASK_OUT ? M.col_x + t.j : M.row_l + t.j;
+        int seen_a = -1, seen_b = -1;
+        const int nkb = task_blocks(t.kind, t.i, t.j, M.n), total = nkb + (two ? 2 : 0);
+        uint8_t* const la = t.kind == TASK_OUT ? M.X : M.L;                              // operands of the sum
+        uint8_t* const lb = t.kind == TASK_INV || t.kind == TASK_OUT ? M.X : M.L;
+        const bool a_k = t.kind != TASK_OUT, b_k = t.kind == TASK_FACTOR;
+        for (int kb = 0; kb < total && ok; ++kb, ++it) {
+          const uint32_t s = it % TC_STAGES, parity = ((it / TC_STAGES) & 1) ^ 1;
+          const uint8_t *src_a = nullptr, *src_b = nullptr;   // null: nothing to load (shared, or written by the epilogue)
+          bool major_a = a_k, major_b = b_k;
+          if (kb < nkb) {
+            const int k = k0 + kb * G2_BK, panel = k / TB, hb = (k / G2_BK) & 1;   // hb: half of the panel
+            if (!wait_progress(wa, panel + 1, seen_a, abort) || (!shared_ab && !wait_progress(wb, panel + 1, seen_b, abort))) {
+              give_up(ERR_WAIT_FULL);
+              ok = false;
+              break;
+            }
+            src_a = a_k ? tile_at(la, t.i, panel) + hb * 3 * PART_BYTES : tile_at(la, panel, t.i) + hb * (PART_BYTES / 2);
+            if (!shared_ab)
+              src_b = b_k ? tile_at(lb, t.j, panel) + hb * 3 * PART_BYTES : tile_at(lb, panel, t.j) + hb * (PART_BYTES / 2);
+          } else {   // T, the other operand of the second product
+            const int d = t.kind == TASK_FACTOR ? t.j : t.i;
+            int seen = -1;
+            if (!wait_progress(M.col_x + d, d + 1, seen, abort)) {
+              give_up(ERR_WAIT_FULL);
+              ok = false;
+              break;
+            }
+            (t.kind == TASK_FACTOR ? src_b : src_a) = tile_at(M.X, d, d) + (kb - nkb) * 3 * PART_BYTES;
+            major_a = major_b = true;
+          }
+          // roles in the order in which the block before the last releases them
+          constexpr int ORDER[ROLES] = {ROLE_A_LO, ROLE_B_LO, ROLE_A_MID, ROLE_B_MID, ROLE_B_HI, ROLE_A_HI};
+          constexpr int GROUP[ROLES] = {2, 0, 1, 1, 0, 2};   // full barrier of a role
+#pragma unroll
+          for (int o = 0; o < ROLES; ++o) {
+            const int role = ORDER[o], part = role % 3;
+            if (ok && !mbar_wait(&empty_bar[s * ROLES + role], parity)) {
+              give_up(ERR_WAIT_EMPTY);
+              ok = false;
+            }
+            if (!ok) break;
+            const uint8_t* src = role < 3 ? src_a : src_b;
+            const bool k_major = role < 3 ? major_a : major_b;
+            uint64_t* const bar = &full_bar[s * 3 + GROUP[role]];
+            uint8_t* const dst = smem + s * TC_STAGE_BYTES + role * PART_BYTES;
+            if (src == nullptr) {
+              mbar_arrive(bar);
+              continue;
+            }
+            mbar_expect_tx(bar, PART_BYTES);
+            if (k_major) {
+              bulk_load(dst, src + part * PART_BYTES, PART_BYTES, bar);
+            } else {   // 64 rows of both halves
+              bulk_load(dst, src + part * PART_BYTES, PART_BYTES / 2, bar);
+              bulk_load(dst + PART_BYTES / 2, src + (3 + part) * PART_BYTES, PART_BYTES / 2, bar);
+            }
+          }
+        }
+        if (ok && t.kind == TASK_DIAG) {   // the diagonal block is factored in the ring's memory
+          if (!mbar_wait(diag_bar, diags & 1)) {
+            give_up(ERR_WAIT_EMPTY);
+            ok = false;
+          }
+          ++diags;
+        }
+      }
+      if (!ok) {   // copies that are still in flight get a bounded chance to land before teardown
+        for (uint32_t jt = it < 2 ? 0 : it - 2; jt <= it; ++jt)   // the last one may not have been loaded in full
+          for (int g = 0; g < 3; ++g) mbar_wait(&full_bar[jt % TC_STAGES * 3 + g], (jt / TC_STAGES) & 1);
+      }
+    }
+  } else if (warp == 1) {
+    // ---- issues the products.  The whole warp runs the loop and one lane issues, so that addresses stay in uniform registers;
+    // descriptors are a base and constants.  A loop of one lane that builds every descriptor needs 2206 clocks for the 24
+    // products of a K block, this one 1587; the tensor core needs 1536.
+    const bool lead = elect_one();
+    uint32_t it = 0, seconds = 0;
+    bool ok = true;
+    for (uint32_t tk = 0; ok; ++tk) {
+      const uint32_t slot = tk % TC_ITEMS;
+      if (!mbar_wait(&item_full[slot], (tk / TC_ITEMS) & 1)) {
+        give_up(ERR_WAIT_FULL);
+        break;
+      }
+      const Task t = items[slot];
+      __syncwarp();
+      if (lead) mbar_arrive(&item_empty[slot]);
+      if (t.kind == TASK_END) break;
+      const bool two = t.kind == TASK_FACTOR || t.kind == TASK_INV;
+      const bool shared_ab = t.kind == TASK_DIAG || (t.kind == TASK_OUT && t.i == t.j);
+      const bool a_k = t.kind != TASK_OUT;                                // K-major operands
+      const bool b_k = t.kind == TASK_DIAG || t.kind == TASK_FACTOR;      // ... in both products: L and T, X and W are alike
+      const uint32_t idesc = make_idesc_bf16(TB, TB, !a_k, !b_k);
+      // 16 elements of K: 32 bytes of a K-major row, 16 rows of 128 bytes of an MN-major operand
+      const uint32_t step_a = a_k ? 2 : 128, step_b = b_k ? 2 : 128;
+      const uint64_t desc_a = make_smem_desc_sw128(smem_u32(smem), a_k ? 16 : G2_BK * 128, 1024);
+      const uint64_t desc_b = make_smem_desc_sw128(smem_u32(smem) + (shared_ab ? 0 : 3 * PART_BYTES), b_k ? 16 : G2_BK * 128, 1024);
+      const int nkb = task_blocks(t.kind, t.i, t.j, mats[t.mat].n), total = nkb + (two ? 2 : 0);
+      for (int kb = 0; kb < total; ++kb, ++it) {
+        const uint32_t ab = it & 1, s = it % TC_STAGES;
+        ok = mbar_wait(&acc_empty[ab], ((it >> 1) & 1) ^ 1) && (kb < nkb || mbar_wait(&operand_bar[kb - nkb], seconds & 1));
+        const uint32_t tacc = tmem_base + ab * TB;
+        constexpr int PART_A[6] = {1, 2, 0, 1, 0, 0};   // (mid,mid) (lo,hi) (hi,lo) (mid,hi) (hi,mid) (hi,hi)
+        constexpr int PART_B[6] = {1, 0, 2, 0, 1, 0};
+        constexpr int RELEASE[6] = {-1, ROLE_A_LO, ROLE_B_LO, ROLE_A_MID, ROLE_B_MID, ROLE_A_HI};   // done with after the product
+#pragma unroll
+        for (int pr = 0; pr < 6; ++pr) {
+          if (pr < 3) {
+            ok = ok && mbar_wait(&full_bar[s * 3 + pr], (it / TC_STAGES) & 1);
+            // where A is both operands, (lo,hi) reads what (hi,lo) waits for
+            if (pr == 1 && shared_ab) ok = ok && mbar_wait(&full_bar[s * 3 + 2], (it / TC_STAGES) & 1);
+            if (!ok) break;
+            tc_fence_after_sync();
+          }
+          const uint64_t da = desc_a + ((s * TC_STAGE_BYTES + PART_A[pr] * PART_BYTES) >> 4);
+          const uint64_t db = desc_b + ((s * TC_STAGE_BYTES + PART_B[pr] * PART_BYTES) >> 4);
+#pragma unroll
+          for (int k = 0; k < G2_BK / 16; ++k)
+            if (lead) umma_bf16(tacc, da + k * step_a, db + k * step_b, idesc, (pr | k) ? 1u : 0u);
+          if (RELEASE[pr] >= 0 && !shared_ab && lead) umma_commit(&empty_bar[s * ROLES + RELEASE[pr]]);
+        }
+        if (!ok) {
+          give_up(ERR_WAIT_FULL);
+          break;
+        }
+        if (lead) {
+          if (shared_ab)   // the parts of A are both operands: all roles are free at the end
+            for (int role = 0; role < ROLES; ++role) umma_commit(&empty_bar[s * ROLES + role]);
+          else
+            umma_commit(&empty_bar[s * ROLES + ROLE_B_HI]);
+          umma_commit(&acc_full[ab]);
+        }
+        __syncwarp();
+      }
+      if (two) ++seconds;
+    }
+  } else {
+    // ---- epilogue: sums, splits, diagonal blocks, stores
+    const int tid = threadIdx.x - 64, ew = warp - 2;
+    const int q = warp & 3, half = ew >> 2;      // TMEM lanes [32 q, 32 q + 32), columns [64 half, 64 half + 64) of a tile
+    const int row = q * 32 + lane;               // this thread's row of a tile
+    uint8_t* const stg = staging + ew * TC_STAGING;
+    float* const stgf = reinterpret_cast<float*>(stg);
+    const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + half * 64;
+    uint32_t it = 0;
+    bool ok = true;
+    // A wait that runs out (`ok` false) only stops further waits: all warps pass the barriers of the task and leave together.
+    for (uint32_t tk = 0;; ++tk) {
+      const uint32_t slot = tk % TC_ITEMS;
+      if (ok && !mbar_wait(&item_full[slot], (tk / TC_ITEMS) & 1)) {
+        ok = false;
+        give_up(ERR_WAIT_FULL);
+      }
+      if (epi_any(!ok)) break;
+      const Task t = items[slot];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&item_empty[slot]);
+      if (t.kind == TASK_END) break;
+      const TcMat& M = mats[t.mat];
+      const int n = M.n, i0 = t.i * TB, j0 = t.j * TB;
+      const int row0 = i0 + q * 32, col0 = j0 + half * 64;   // of this warp's 32 x 64 patch
+      const int nkb = task_blocks(t.kind, t.i, t.j, n);
+      float run[64];
+      if (t.kind == TASK_DIAG || t.kind == TASK_FACTOR) {
+        // A + damping I waits in tensor memory: rows are read along the lanes and turned in shared memory, 32 loads in flight
+        const float* A = M.A;
+        const float d = damping[M.orig];
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+          const int gc = col0 + 32 * h + lane;
+          float v[32];
+#pragma unroll
+          for (int r = 0; r < 32; ++r)
+            v[r] = row0 + r < n && gc < n ? __ldg(A + static_cast<size_t>(row0 + r) * M.lda + gc) : 0.f;
+          __syncwarp();
+#pragma unroll
+          for (int r = 0; r < 32; ++r) stgf[r * 32 + (lane ^ r)] = row0 + r == gc ? v[r] + d : v[r];
+          __syncwarp();
+          uint32_t w[32];
+#pragma unroll
+          for (int c = 0; c < 32; ++c) w[c] = __float_as_uint(stgf[lane * 32 + (c ^ lane)]);
+          tmem_st_32x32(taddr + 2 * TB + 32 * h, w);
+        }
+        tmem_st_wait();
+      }
+#pragma unroll
+      for (int c = 0; c < 64; ++c) run[c] = 0.f;
+      auto add_blocks = [&](int count) {
+        for (int kb = 0; kb < count; ++kb, ++it) {
+          const uint32_t ab = it & 1;
+          if (ok && !mbar_wait(&acc_full[ab], (it >> 1) & 1)) {
+            ok = false;
+            give_up(ERR_WAIT_ACC);
+          }
+          __syncwarp();
+          tc_fence_after_sync();
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t w[32];
+            tmem_ld_32x32(taddr + ab * TB + 32 * h, w);
+            tmem_ld_wait();
+            if (h == 1) {
+              tc_fence_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&acc_empty[ab]);
+            }
+#pragma unroll
+            for (int c = 0; c < 32; ++c) run[32 * h + c] += __uint_as_float(w[c]);
+          }
+        }
+      };
+      add_blocks(nkb);
+      if (t.kind == TASK_DIAG || t.kind == TASK_FACTOR) {   // S = A - sum
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t w[32];
+          tmem_ld_32x32(taddr + 2 * TB + 32 * h, w);
+          tmem_ld_wait();
+#pragma unroll
+          for (int c = 0; c < 32; ++c) run[32 * h + c] = __uint_as_float(w[c]) - run[32 * h + c];
+        }
+      }
+
+      if (t.kind == TASK_DIAG) {
+        // every product that read the ring is done (its accumulator was read) and the producer waits
+        float* S = reinterpret_cast<float*>(smem);
+        const int live = min(TB, n - i0);
+#pragma unroll
+        for (int c = 0; c < 64; ++c) S[row * DG_SP + half * 64 + c] = half * 64 + c <= row ? run[c] : 0.f;
+        if (row >= live) {   // identity padding keeps the block factorisable
+#pragma unroll 1
+          for (int c = half * 64; c < half * 64 + 64; ++c) S[row * DG_SP + c] = row == c ? 1.f : 0.f;
+        }
+        diag_block(tile_at(M.X, t.j, t.j), live, S, tid, status);
+        proxy_fence();
+        epi_sync();
+        if (tid == 0) {
+          st_release(M.col_x + t.j, t.j + 1);
+          mbar_arrive(diag_bar);
+        }
+        continue;
+      }
+      if (t.kind == TASK_OUT) {
+        // lower tiles; diagonal tiles keep their lower triangle; both are mirrored, so the result is exactly symmetric
+        const bool diag = t.i == t.j;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          __syncwarp();
+#pragma unroll
+          for (int c = 0; c < 32; ++c) stgf[lane * 32 + (c ^ lane)] = run[32 * h + c];
+          __syncwarp();
+          store_patch(stgf, M.out, n, row0, col0 + 32 * h, diag, lane);
+        }
+        continue;
+      }
+
+      // second product: the sum is the operand.  FACTOR: S (A operand, K-major), this warp's columns are K block `half`;
+      // INV: W (B operand, MN-major), this warp's rows are in K block q / 2.
+      const int kb2 = t.kind == TASK_FACTOR ? half : q >> 1;
+      const uint32_t it2 = it + kb2, s2 = it2 % TC_STAGES;
+      for (int part = 0; part < 3; ++part)
+        if (ok && !mbar_wait(&empty_bar[s2 * ROLES + (t.kind == TASK_FACTOR ? ROLE_A_HI : ROLE_B_HI) + part], ((it2 / TC_STAGES) & 1) ^ 1)) {
+          ok = false;
+          give_up(ERR_WAIT_EMPTY);
+        }
+      __syncwarp();
+      uint8_t* const stage = smem + s2 * TC_STAGE_BYTES;
+      uint8_t* const operand = t.kind == TASK_FACTOR ? stage + q * 32 * 128
+                                                     : stage + 3 * PART_BYTES + half * (G2_BK * 128) + (q & 1) * 32 * 128;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        stage_patch(run + 32 * h, stg, lane);
+        split_patch(stg, operand, h, lane);
+      }
+      proxy_fence();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&operand_bar[kb2]);
+#pragma unroll
+      for (int c = 0; c < 64; ++c) run[c] = 0.f;
+      add_blocks(2);
+      if (t.kind == TASK_INV) {
+#pragma unroll
+        for (int c = 0; c < 64; ++c) run[c] = -run[c];
+      }
+      // parts of the result: this warp's 32 rows of a half are 4 KiB in a row
+      uint8_t* const image = tile_at(t.kind == TASK_FACTOR ? M.L : M.X, t.i, t.j) + half * (3 * PART_BYTES) + q * 32 * 128;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        stage_patch(run + 32 * h, stg, lane);
+        split_patch(stg, image, h, lane);
+      }
+      proxy_fence();
+      epi_sync();   // the release of one thread covers what the others stored before the barrier
+      if (tid == 0) {
+        if (t.kind == TASK_FACTOR)
+          st_release(M.row_l + t.i, t.j + 1);
+        else
+          st_release(M.col_x + t.j, t.i + 1);
+      }
+    }
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 1) {
+    __syncwarp();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
 
 struct Prepared {
   std::vector<const void*> key;
-  at::Tensor splits;     // bf16 storage of all split buffers
-  at::Tensor d_mats;     // TcMat table (sorted by decreasing size)
-  at::Tensor d_probs;    // GemmProblem2 table
-  at::Tensor d_work;     // all work lists, back to back
-  std::vector<Launch> launches;
-  int count = 0;
-  int prepare_blocks = 1;   // row groups of the prepare kernel: the largest matrix has 8 rows per block
+  at::Tensor splits;     // tiles of L and X of all matrices
+  at::Tensor d_mats;     // TcMat table
+  at::Tensor d_tasks;    // Task list
+  at::Tensor d_ctrl;     // claim counter, abort word, progress words: zeroed by every call
+  int n_tasks = 0;
   GraphPins pins;
 };
 
@@ -290,52 +830,63 @@ std::mutex g_cache_mutex;
 // four sets of matrices beside those that graphs refer to; never destroyed (see PreparedCache)
 PreparedCache<Prepared, 4>& g_cache = *new PreparedCache<Prepared, 4>;
 
-int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
-
-// problem indices inside a matrix's group of five
-enum { PB_PANEL = 0, PB_TRAIL = 1, PB_W = 2, PB_X21 = 3, PB_LAUUM = 4, PB_COUNT = 5 };
-
-void fill_problem(GemmProblem2& P, __nv_bfloat16* const* a_parts, bool a_k, __nv_bfloat16* const* b_parts, bool b_k,
-                  int n, int ldp, float* C, int ldc, float alpha, float beta, int flags,
-                  __nv_bfloat16* const* out_parts, int* status) {
-  std::memset(&P, 0, sizeof(P));
-  for (int s = 0; s < 3; ++s) {  // (hi, mid, lo) parts; the kernel forms the six part products itself
-    g2_encode_operand(&P.tmA[s], a_parts[s], n, n, ldp, a_k, G2_BM);
-    g2_encode_operand(&P.tmB[s], b_parts[s], n, n, ldp, b_k, 128);
+// The task list of matrices of `sizes` for `ctas` CTAs.  Any order in which a task follows what it needs is correct; this one
+// is made for speed.  Time is cut into slots of one step of a chain (DIAG, FACTOR of the next row, last panel of the next
+// DIAG).  In a slot every matrix may take one step, and the longest remaining chains always do; shorter ones join while the
+// slot has room, and OUT tiles, which nothing waits for, fill the rest.
+std::vector<Task> make_tasks(const std::vector<int>& sizes, int ctas) {
+  constexpr int STEP_US = 35, BLOCK_US = 1, TILE_US = 5, DIAG_US = 28;
+  const int count = static_cast<int>(sizes.size());
+  std::vector<int> nb(count), step(count, 0), order(count), out_i(count, 0), out_j(count, 0);
+  for (int m = 0; m < count; ++m) {
+    nb[m] = (sizes[m] + TB - 1) / TB;
+    order[m] = m;
   }
-  P.nseg = 3;
-  P.M = P.N = P.K = n;
-  P.C = C;
-  P.Cin = C;
-  P.ldc = ldc;
-  P.alpha = alpha;
-  P.beta = beta;
-  P.flags = flags | G2F_SPLIT3 | (a_k ? G2F_A_KMAJOR : 0) | (b_k ? G2F_B_KMAJOR : 0);
-  P.nsplit = 1;
-  P.tiles_m = P.tiles_n = (n + TB - 1) / TB;
-  P.ntiles = 0;
-  P.status = status;
-  if (out_parts != nullptr) {
-    P.out_hi = out_parts[0];
-    P.out_mid = out_parts[1];
-    P.out_lo = out_parts[2];
-    P.ld_out = ldp;
+  std::vector<Task> tasks;
+  for (int m = 0; m < count; ++m) tasks.push_back({m, TASK_DIAG, 0, 0});
+  std::stable_sort(tasks.begin(), tasks.end(), [&](const Task& a, const Task& b) { return nb[a.mat] > nb[b.mat]; });
+  int left = count;
+  const long long room = static_cast<long long>(ctas) * STEP_US;
+  std::vector<int> taken;
+  while (left > 0) {
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return nb[a] - step[a] > nb[b] - step[b]; });
+    const int longest = nb[order[0]] - step[order[0]];
+    long long used = 0;
+    taken.clear();
+    for (int m : order) {
+      if (step[m] >= nb[m]) continue;
+      const int j = step[m];
+      const long long work = DIAG_US + 2 * BLOCK_US * j + static_cast<long long>(nb[m] - j - 1) * (2 * BLOCK_US * j + TILE_US) +
+                             static_cast<long long>(j) * (TILE_US + BLOCK_US * (j + 1));
+      if (nb[m] - j != longest && used + work > room) continue;
+      used += work;
+      taken.push_back(m);
+    }
+    for (int m : taken) {
+      const int j = step[m];
+      for (int i = j + 1; i < nb[m]; ++i) {
+        tasks.push_back({m, TASK_FACTOR, i, j});
+        if (i == j + 1) tasks.push_back({m, TASK_DIAG, i, i});
+      }
+    }
+    for (int m : taken)
+      for (int c = 0; c < step[m]; ++c) tasks.push_back({m, TASK_INV, step[m], c});
+    for (int m : taken) ++step[m];
+    for (int m : order) {   // OUT tiles of matrices whose chain has ended
+      if (step[m] < nb[m] || out_i[m] >= nb[m]) continue;
+      while (out_i[m] < nb[m] && (used < room || longest <= 1)) {
+        tasks.push_back({m, TASK_OUT, out_i[m], out_j[m]});
+        used += 2 * BLOCK_US * (nb[m] - out_i[m]) + TILE_US;
+        if (++out_j[m] > out_i[m]) {
+          ++out_i[m];
+          out_j[m] = 0;
+        }
+      }
+    }
+    left = 0;
+    for (int m = 0; m < count; ++m) left += out_i[m] < nb[m];
   }
-}
-
-GemmWork2 item(int problem, int a_mn, int b_mn, int a_k0, int b_k0, int nkb, int c_row, int c_col, int wflags) {
-  GemmWork2 w;
-  std::memset(&w, 0, sizeof(w));
-  w.problem = problem;
-  w.a_mn = a_mn;
-  w.b_mn = b_mn;
-  w.a_k0 = a_k0;
-  w.b_k0 = b_k0;
-  w.nkb = nkb;
-  w.c_row = c_row;
-  w.c_col = c_col;
-  w.wflags = wflags;
-  return w;
+  return tasks;
 }
 
 }  // namespace
@@ -376,119 +927,39 @@ void chol_inverse_tc(std::vector<at::Tensor> mats, std::vector<at::Tensor> outs,
                 "tables and cannot run inside a CUDA graph capture; call it once before capturing");
     Prepared P;
     P.key = key;
-    P.count = count;
-    std::vector<int> order(count);
-    for (int i = 0; i < count; ++i) order[i] = i;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return mats[a].size(0) > mats[b].size(0); });
-    // split storage: per matrix Ls, Xs, Ws with three parts each
-    int64_t total = 0;
+    int64_t total = 0, words = 2;
     std::vector<int64_t> base(count);
-    for (int s = 0; s < count; ++s) {
-      const int64_t n = mats[order[s]].size(0), ldp = round_up(n, 64);
-      base[s] = total;
-      total += 9 * round_up(n * ldp, 64);
+    std::vector<int> sizes(count);
+    for (int i = 0; i < count; ++i) {
+      const int64_t nb = (mats[i].size(0) + TB - 1) / TB;
+      sizes[i] = static_cast<int>(mats[i].size(0));
+      base[i] = total;
+      total += 2 * (nb * (nb + 1) / 2) * TILE_BYTES;
+      words += 2 * nb;
     }
-    P.splits = at::zeros({total}, at::TensorOptions().dtype(at::kBFloat16).device(at::kCUDA, dev));
-    __nv_bfloat16* sp = reinterpret_cast<__nv_bfloat16*>(P.splits.data_ptr());
-    int* status = device_state(dev).status.data_ptr<int>();
-
+    P.splits = at::empty({total}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, dev));
+    P.d_ctrl = at::empty({words}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, dev));
+    uint8_t* sp = P.splits.data_ptr<uint8_t>();
+    TORCH_CHECK((reinterpret_cast<uintptr_t>(sp) & 15) == 0, "split buffers are not 16-byte aligned");
+    int* progress = P.d_ctrl.data_ptr<int>() + 2;
     std::vector<TcMat> host(count);
-    std::vector<GemmProblem2> probs(static_cast<size_t>(count) * PB_COUNT);
-    int nb_max = 0;
-    for (int s = 0; s < count; ++s) {
-      const int i = order[s];
-      TcMat& M = host[s];
+    for (int i = 0; i < count; ++i) {
+      TcMat& M = host[i];
       std::memset(&M, 0, sizeof(M));
       M.A = mats[i].data_ptr<float>();
       M.lda = static_cast<int>(mats[i].stride(0));
-      M.L = outs[i].data_ptr<float>();
-      M.n = static_cast<int>(mats[i].size(0));
+      M.out = outs[i].data_ptr<float>();
+      M.n = sizes[i];
       M.nb = (M.n + TB - 1) / TB;
-      M.ldp = static_cast<int>(round_up(M.n, 64));
       M.orig = i;
-      const int64_t part = round_up(static_cast<int64_t>(M.n) * M.ldp, 64);
-      __nv_bfloat16* Ws[3];
-      for (int p = 0; p < 3; ++p) {
-        M.Ls[p] = sp + base[s] + (0 + p) * part;
-        M.Xs[p] = sp + base[s] + (3 + p) * part;
-        Ws[p] = sp + base[s] + (6 + p) * part;
-      }
-      nb_max = std::max(nb_max, M.nb);
-      P.prepare_blocks = std::max(P.prepare_blocks, std::min((M.n + 7) / 8, 1024));
-      GemmProblem2* pb = &probs[static_cast<size_t>(s) * PB_COUNT];
-      // L_ik = A_ik T_k^T : both operands K-major, result to L (fp32) and Ls (splits), in place
-      fill_problem(pb[PB_PANEL], M.Ls, true, M.Xs, true, M.n, M.ldp, M.L, M.n, 1.f, 0.f, 0, M.Ls, status);
-      // A_ij -= L_ik L_jk^T : lower tiles of the fp32 matrix; splits written for the next panel column only
-      fill_problem(pb[PB_TRAIL], M.Ls, true, M.Ls, true, M.n, M.ldp, M.L, M.n, -1.f, 1.f,
-                   G2F_SYM | G2F_LOWER, M.Ls, status);
-      // W = L_21 X_11 and X_21 = -X_22 W : bf16 splits only
-      fill_problem(pb[PB_W], M.Ls, true, M.Xs, false, M.n, M.ldp, nullptr, M.n, 1.f, 0.f, 0, Ws, status);
-      fill_problem(pb[PB_X21], M.Xs, true, Ws, false, M.n, M.ldp, nullptr, M.n, -1.f, 0.f, 0, M.Xs, status);
-      // out = X^T X : both operands MN-major, lower tiles mirrored
-      fill_problem(pb[PB_LAUUM], M.Xs, false, M.Xs, false, M.n, M.ldp, M.L, M.n, 1.f, 0.f,
-                   G2F_SYM, nullptr, status);
+      M.row_l = progress;
+      M.col_x = progress + M.nb;
+      progress += 2 * M.nb;
+      M.L = sp + base[i];
+      M.X = M.L + static_cast<size_t>(M.nb) * (M.nb + 1) / 2 * TILE_BYTES;
     }
-    std::vector<GemmWork2> work;
-    auto push_list = [&](const std::vector<GemmWork2>& items) {
-      if (items.empty()) return;
-      P.launches.push_back({1, static_cast<int>(work.size()), static_cast<int>(items.size())});
-      work.insert(work.end(), items.begin(), items.end());
-    };
-    auto active = [&](int k) {  // matrices (a prefix of the sorted order) with more than k panels
-      int c = 0;
-      while (c < count && host[c].nb > k) ++c;
-      return c;
-    };
-    // ---- potrf
-    for (int k = 0; k < nb_max; ++k) {
-      P.launches.push_back({0, k, active(k)});
-      std::vector<GemmWork2> panel, trail;
-      for (int s = 0; s < count && host[s].nb > k + 1; ++s) {
-        const int nb = host[s].nb, pbase = s * PB_COUNT;
-        for (int i = k + 1; i < nb; ++i)
-          panel.push_back(item(pbase + PB_PANEL, i * TB, k * TB, k * TB, k * TB, 2, i * TB, k * TB, 0));
-        // tiles of the next panel column first: the next diagonal block and panel depend on them
-        for (int j = k + 1; j < nb; ++j)
-          for (int i = j; i < nb; ++i)
-            trail.push_back(item(pbase + PB_TRAIL, i * TB, j * TB, k * TB, k * TB, 2, i * TB, j * TB,
-                                 (j == k + 1 && i > j) ? 0 : G2W_NO_SPLIT_OUT));
-      }
-      push_list(panel);
-      push_list(trail);
-    }
-    // ---- trtri by recursive doubling
-    for (int s_blk = 1; s_blk < nb_max; s_blk *= 2) {
-      std::vector<GemmWork2> wl, xl;
-      for (int s = 0; s < count && host[s].nb > s_blk; ++s) {
-        const int nb = host[s].nb, pbase = s * PB_COUNT;
-        for (int f0 = 0; f0 + s_blk < nb; f0 += 2 * s_blk) {
-          const int e = f0 + s_blk;                       // first = [f0, e), second = [e, s1)
-          const int s1 = std::min(e + s_blk, nb);
-          for (int r = e; r < s1; ++r)
-            for (int c = f0; c < e; ++c) {
-              wl.push_back(item(pbase + PB_W, r * TB, c * TB, c * TB, c * TB, 2 * (e - c), r * TB, c * TB, 0));
-              xl.push_back(item(pbase + PB_X21, r * TB, c * TB, e * TB, e * TB, 2 * (r - e + 1), r * TB, c * TB, 0));
-            }
-        }
-      }
-      auto by_cost = [](const GemmWork2& a, const GemmWork2& b) { return a.nkb > b.nkb; };
-      std::stable_sort(wl.begin(), wl.end(), by_cost);
-      std::stable_sort(xl.begin(), xl.end(), by_cost);
-      push_list(wl);
-      push_list(xl);
-    }
-    // ---- lauum
-    {
-      std::vector<GemmWork2> ll;
-      for (int s = 0; s < count; ++s) {
-        const int nb = host[s].nb, pbase = s * PB_COUNT;
-        for (int i = 0; i < nb; ++i)
-          for (int j = 0; j <= i; ++j)
-            ll.push_back(item(pbase + PB_LAUUM, i * TB, j * TB, i * TB, i * TB, 2 * (nb - i), i * TB, j * TB, 0));
-      }
-      std::stable_sort(ll.begin(), ll.end(), [](const GemmWork2& a, const GemmWork2& b) { return a.nkb > b.nkb; });
-      push_list(ll);
-    }
+    const std::vector<Task> tasks = make_tasks(sizes, g2_sm_count(dev));
+    P.n_tasks = static_cast<int>(tasks.size());
     auto upload = [&](const void* src, size_t bytes) {
       at::Tensor hostt = at::empty({static_cast<int64_t>(bytes)}, at::TensorOptions().dtype(at::kByte).pinned_memory(true));
       std::memcpy(hostt.data_ptr(), src, bytes);
@@ -496,31 +967,20 @@ void chol_inverse_tc(std::vector<at::Tensor> mats, std::vector<at::Tensor> outs,
       return d;
     };
     P.d_mats = upload(host.data(), host.size() * sizeof(TcMat));
-    P.d_probs = upload(probs.data(), probs.size() * sizeof(GemmProblem2));
-    if (work.empty()) work.push_back(item(0, 0, 0, 0, 0, 0, 0, 0, 0));
-    P.d_work = upload(work.data(), work.size() * sizeof(GemmWork2));
-    TORCH_CHECK((reinterpret_cast<uintptr_t>(P.d_probs.data_ptr()) & 63) == 0, "problem table is not 64-byte aligned");
+    P.d_tasks = upload(tasks.data(), tasks.size() * sizeof(Task));
     B200_CUDA_CHECK(cudaStreamSynchronize(stream));  // the pinned staging buffers are released after this
     prep = g_cache.insert(std::move(P));
   }
-  prep->pins.use(current, {prep->splits, prep->d_mats, prep->d_probs, prep->d_work});
+  prep->pins.use(current, {prep->splits, prep->d_mats, prep->d_tasks, prep->d_ctrl});
 
-  const TcMat* dm = reinterpret_cast<const TcMat*>(prep->d_mats.data_ptr());
-  const GemmProblem2* dp = reinterpret_cast<const GemmProblem2*>(prep->d_probs.data_ptr());
-  const GemmWork2* dw = reinterpret_cast<const GemmWork2*>(prep->d_work.data_ptr());
-  int* status = device_state(dev).status.data_ptr<int>();
-  tc_prepare_kernel<<<dim3(prep->prepare_blocks, count), 256, 0, stream>>>(dm, damping.data_ptr<float>());
-  count_launch();
-  B200_CUDA_CHECK(cudaFuncSetAttribute(tc_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
-  for (const Launch& l : prep->launches) {
-    if (l.kind == 0) {
-      tc_diag_kernel<<<l.count, 256, DG_SMEM, stream>>>(dm, l.arg, status);
-      count_launch();
-    } else {
-      g2_launch_list(dp, dw + l.arg, l.count, G2_SPLIT3, dev, stream);
-    }
-  }
+  int* ctrl = prep->d_ctrl.data_ptr<int>();
+  B200_CUDA_CHECK(cudaMemsetAsync(ctrl, 0, prep->d_ctrl.numel() * sizeof(int), stream));
+  B200_CUDA_CHECK(cudaFuncSetAttribute(tc_tasks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM));
+  tc_tasks_kernel<<<std::min(prep->n_tasks, g2_sm_count(dev)), TC_THREADS, TC_SMEM, stream>>>(
+      reinterpret_cast<const TcMat*>(prep->d_mats.data_ptr()), reinterpret_cast<const Task*>(prep->d_tasks.data_ptr()),
+      prep->n_tasks, damping.data_ptr<float>(), ctrl, device_state(dev).status.data_ptr<int>());
   B200_CUDA_CHECK(cudaGetLastError());
+  count_launch();
 }
 
 // Drops the cached tables and split buffers of the tensor-core inverse that no captured graph refers to.

@@ -191,6 +191,29 @@ def test_inverse_at_the_edges_of_the_diagonal_stages(n):
     ops.check_status()
 
 
+@pytest.mark.parametrize('sizes', [(1, 128, 129, 256, 384, 385), (640, 8, 513, 64, 257, 191, 1), (1153, 1024), (130,) * 90 + (400,) * 40])
+def test_grouped_inverse_of_mixed_sizes(sizes):
+    """Tiles at and past the edges, chains of several lengths side by side, more tasks than CTAs; inputs with a row pitch."""
+    mats, damp = [], torch.rand(len(sizes), device=DEV, generator=_gen(6)) * 1e-2 + 1e-2
+    for i, n in enumerate(sizes):
+        x = torch.randn(2 * n, n, device=DEV, generator=_gen(30 + i))
+        wide = torch.full((n, n + 1 + i % 3), float('nan'), device=DEV)
+        wide[:, :n] = x.T @ x / (2 * n)
+        mats.append(wide[:, :n])
+    outs = [torch.full((n, n), float('nan'), device=DEV) for n in sizes]
+    for _ in range(3):
+        ops.spd_inverse_grouped(mats, outs, damp)
+    ops.check_status()
+    for m, o, d, n in zip(mats, outs, damp, sizes):
+        want = m.double()
+        want.diagonal().add_(d.double())
+        cond = torch.linalg.cond(want).item()
+        want = torch.linalg.inv(want)
+        # n * 2^-24 times the condition number bounds the error of a Cholesky inverse, relative to the largest entry
+        assert (o.double() - want).abs().max() <= 4 * max(n, 8) * 2.0 ** -24 * cond * want.abs().max()
+        assert torch.equal(o, o.T)
+
+
 @pytest.mark.parametrize('n,at', [(40, 35), (128, 0), (128, 100), (200, 150)])
 def test_a_negative_pivot_in_any_stage_is_reported(n, at):
     a = torch.eye(n, device=DEV)
