@@ -25,7 +25,7 @@
 // operand traffic of the ring, 96 KiB per K block of 1536 tensor cycles.  The former version ran the same arithmetic
 // right-looking in 28 (six factors up to 784) to 121 (the 107 factors of ResNet-50) dependent launches: every K = 128 update
 // read and wrote the fp32 matrix, each lane a row of its own, and every launch drained before the next began.
-// Six factors 784, 4 x 512, 10: 594 -> 304 us; ResNet-50's 107 factors: 8.06 -> 3.80 ms.
+// Six factors 784, 4 x 512, 10: 600 -> 263 us; ResNet-50's 107 factors: 8.08 -> 3.63 ms.
 //
 // Tables, task lists and the bf16 split buffers depend only on the addresses and sizes of the matrices; they are built once
 // and cached (prepared_cache.h), so a repeated call (the K-FAC state) issues no host-to-device copy and can be captured in a
@@ -78,19 +78,19 @@ __host__ __device__ inline int task_blocks(int kind, int i, int j, int n) {
 
 // ---- diagonal block: Cholesky factor and its inverse ----------------------------------------
 // Four stages of 32 columns on the eight epilogue warps of a CTA.  Stage q, columns [kb, be):
-//   factor   one warp, a row of the 32 x 32 block per lane, in registers.  From a pivot to the next the chain is a product, a
-//            shuffle and a reciprocal square root; a column is applied to the columns behind the next one a step later, in the
-//            latency of that chain;
+//   factor   one warp, a row of the 32 x 32 block per lane, in registers.  Eight columns at a time: inside of the eight a column
+//            is passed on by shuffles, so the chain from pivot to pivot is a product, a shuffle and a reciprocal square root;
+//            then the eight are applied to the columns behind them;
 //   panel    four warps, one thread per row below (forward substitution with the block) and one per column of the inverse's
 //            rows [kb, be), eight columns behind the factor.  P[j][c] = T[kb + j][c] for c < be and L[c][kb + j] for c >= be;
 //   update   S[i][c] -= sum_j P[j][i] P[j][c] for the rows i >= be: the trailing block right of be, the right-hand side of
 //            the inverse left of it.  Finished columns of the factor are dead (only the inverse leaves the kernel), so both
 //            share S.  A warp takes four rows of each row block, a lane one column of each column block up to the diagonal;
 //   store    of the rows [kb, be) of T from P, by the other warps while the next stage is factored.
-// Every entry sees the same roundings in the same order as a column-by-column elimination, and gives the same bits.  The chain
-// of pivots bounds it, and the code is kept small (eight columns unrolled, registers shifted by eight between them) since
-// instructions are fetched once per block.  The same stages one after the other, each column applied at once, took 65 000
-// clocks, 23 000 of them to factor; now 49 000.
+// Every entry sees the same roundings in the same order as a column-by-column elimination, and gives the same bits.  Two things
+// bound it: the chain of pivots (80 clocks each), and the number of instructions that a single warp per scheduler issues:
+// products are taken in pairs (fma.f32x2), and loops over groups of eight columns are not unrolled.  With each column applied at
+// once to all behind it, in single products, the block took 49 000 clocks, 27 800 of them to factor; now 44 000.
 constexpr int DG_SP = TB + 1;   // pitch of S: lanes on consecutive rows of a column, or on consecutive columns
 constexpr int DG_PP = TB + 4;   // pitches of P and of the factored block: 16-byte reads
 constexpr int DG_LP = 64;       // the entries from 32 on are zeros: what shifted registers past the block are updated with
@@ -99,105 +99,103 @@ constexpr int DG_SMEM = (TB * DG_SP + 2 * 32 * DG_PP + 32 * DG_LP + 32) * 4;
 // Barrier of the eight epilogue warps.
 __device__ __forceinline__ void epi_sync() { named_bar_sync(1, 256); }
 
-// v[c] -= x * o[c] for the columns c > J of the 32 in registers
-template <int J>
-__device__ __forceinline__ void diag_eliminate(float (&v)[32], float x, const float* o) {
-#pragma unroll
-  for (int c4 = 0; c4 < 32; c4 += 4) {
-    if (c4 + 3 <= J) continue;
-    const float4 q = *reinterpret_cast<const float4*>(o + c4);
-    if (c4 > J) v[c4] = fmaf(-x, q.x, v[c4]);
-    if (c4 + 1 > J) v[c4 + 1] = fmaf(-x, q.y, v[c4 + 1]);
-    if (c4 + 2 > J) v[c4 + 2] = fmaf(-x, q.z, v[c4 + 2]);
-    v[c4 + 3] = fmaf(-x, q.w, v[c4 + 3]);
-  }
+// Two fp32 values in one register pair; fma2: a * b + c of both, each rounded as fmaf does.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
 }
 
-__device__ __forceinline__ void diag_shift(float (&v)[32]) {
-#pragma unroll
-  for (int c = 0; c < 32; ++c) v[c] = c < 24 ? v[c + 8 < 32 ? c + 8 : 31] : 0.f;
-}
-
-// 1 / sqrt(pivot d) of column j; a pivot that is not positive is reported and replaced by 1
-__device__ __forceinline__ float diag_pivot(float d, int j, bool& bad) {
-  if (!(d > 0.f)) {
-    bad |= j < 32;   // j = 32: there is no such column, and its result is not used
-    d = 1.f;
+// 1 / sqrt(pivot d); a pivot that is not positive is reported and replaced by 1.  The usual case has no branch in the chain:
+// rsqrt.approx.ftz is exact enough for the Newton step that follows, and subnormal pivots go another way.
+__device__ __forceinline__ float diag_pivot(float d, bool& bad) {
+  float iv;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(iv) : "f"(d));
+  if (!(d >= 1.17549435e-38f)) {
+    if (!(d > 0.f)) {
+      bad = true;
+      d = 1.f;
+    }
+    iv = rsqrtf(d);
   }
-  const float iv = rsqrtf(d);
   return iv * fmaf(-0.5f * d, iv * iv, 1.5f);   // one Newton step: full fp32 accuracy
 }
 
-// Column j8 + J of the block's factor, by one warp (lane = row).  `iv`: 1 / sqrt of its pivot on entry, of the next pivot on
-// return.  On entry the column before (this lane's entry `last`, the rows' entries `o`) is still to be applied to the columns
-// from J + 1 on; on return this one to those from J + 2 on.
-template <int J>
-__device__ __forceinline__ void diag_factor_step(float (&a)[32], float (&o)[32], float& last, float& iv, float* Lk, float* inv,
-                                                 int j8, int lane, bool& bad) {
-  const int j = j8 + J;
-  const float l = a[J] * iv;
-  Lk[j * DG_LP + lane] = l;   // rows above j: not used
-  if (lane == 0) inv[j] = iv;
-  a[J + 1] = fmaf(-last, o[J + 1], a[J + 1]);
-  const float d = __shfl_sync(0xffffffffu, fmaf(-l, l, a[J + 1]), (j + 1) & 31);
-  const float next = __shfl_sync(0xffffffffu, l, (j + 1) & 31);
+// A row of 32 columns, of which the first eight are scalars and the others pairs.
+struct DiagRow {
+  float g[8];
+  f32x2 v[12];
+  // the next eight columns become the first ones
+  __device__ __forceinline__ void shift() {
 #pragma unroll
-  for (int c = J + 2; c < 32; ++c) a[c] = fmaf(-last, o[c], a[c]);
-  __syncwarp();
-  constexpr int SHIFT = J == 7 ? 8 : 0;   // the registers are shifted after the eighth column
+    for (int i = 0; i < 4; ++i) unpack2(v[i], g[2 * i], g[2 * i + 1]);
 #pragma unroll
-  for (int c4 = 0; c4 < 32; c4 += 4) {
-    if (c4 + 3 + SHIFT < J + 2) continue;
-    const float4 q = *reinterpret_cast<const float4*>(Lk + j * DG_LP + j8 + SHIFT + c4);
-    o[c4] = q.x;
-    o[c4 + 1] = q.y;
-    o[c4 + 2] = q.z;
-    o[c4 + 3] = q.w;
+    for (int i = 0; i < 12; ++i) v[i] = i < 8 ? v[i + 4 < 12 ? i + 4 : 11] : 0ull;
   }
-  iv = diag_pivot(d, j + 1, bad);
-  a[J + 1] = fmaf(-l, next, a[J + 1]);
-  last = l;
-}
-
-template <int J>
-__device__ __forceinline__ void diag_panel_step(float (&v)[32], const float* Lk, const float* inv, int j8) {
-  v[J] *= inv[j8 + J];
-  diag_eliminate<J>(v, v[J], Lk + (j8 + J) * DG_LP + j8);
-}
+  // columns from the ninth on -= x[j] * o[j * DG_LP + 8 ...] for the eight finished columns j, in their order
+  __device__ __forceinline__ void apply(const float (&x)[8], const float* o) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const f32x2 m = pack2(-x[j], -x[j]);
+#pragma unroll
+      for (int i = 0; i < 12; i += 2) {
+        const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(o + j * DG_LP + 8 + 2 * i);
+        v[i] = fma2(m, q.x, v[i]);
+        v[i + 1] = fma2(m, q.y, v[i + 1]);
+      }
+    }
+  }
+};
 
 // Rows and columns behind stage KQ, whose columns are [32 KQ, 32 KQ + 32).
 template <int KQ>
 __device__ __forceinline__ void diag_update(float* S, const float* P, int warp, int lane) {
   constexpr int NB = 3 - KQ;   // row blocks
-  float acc[NB][4][4];
+  f32x2 acc[NB][2][4];         // pairs of rows
   float* const rows = S + (32 * (KQ + 1) + 4 * warp) * DG_SP + lane;
 #pragma unroll
   for (int b = 0; b < NB; ++b)
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < 2; ++r)
 #pragma unroll
-      for (int q = 0; q <= KQ + 1 + b; ++q) acc[b][r][q] = q == KQ ? 0.f : rows[(32 * b + r) * DG_SP + 32 * q];
-#pragma unroll 2
+      for (int q = 0; q <= KQ + 1 + b; ++q) {
+        const float* at = rows + (32 * b + 2 * r) * DG_SP + 32 * q;
+        acc[b][r][q] = q == KQ ? 0ull : pack2(at[0], at[DG_SP]);
+      }
+#pragma unroll 4
   for (int j = 0; j < 32; ++j) {
-    float pc[4];
+    f32x2 pc[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) pc[q] = P[j * DG_PP + lane + 32 * q];
+    for (int q = 0; q < 4; ++q) {
+      const float v = -P[j * DG_PP + lane + 32 * q];
+      pc[q] = pack2(v, v);
+    }
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
-      const float4 raw = *reinterpret_cast<const float4*>(P + j * DG_PP + 32 * (KQ + 1 + b) + 4 * warp);
-      const float pr[4] = {raw.x, raw.y, raw.z, raw.w};
+      const ulonglong2 pr = *reinterpret_cast<const ulonglong2*>(P + j * DG_PP + 32 * (KQ + 1 + b) + 4 * warp);
 #pragma unroll
-      for (int q = 0; q <= KQ + 1 + b; ++q)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) acc[b][r][q] = fmaf(-pr[r], pc[q], acc[b][r][q]);
+      for (int q = 0; q <= KQ + 1 + b; ++q) {
+        acc[b][0][q] = fma2(pr.x, pc[q], acc[b][0][q]);
+        acc[b][1][q] = fma2(pr.y, pc[q], acc[b][1][q]);
+      }
     }
   }
 #pragma unroll
   for (int b = 0; b < NB; ++b)
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < 2; ++r)
 #pragma unroll
-      for (int q = 0; q <= KQ + 1 + b; ++q) rows[(32 * b + r) * DG_SP + 32 * q] = acc[b][r][q];
+      for (int q = 0; q <= KQ + 1 + b; ++q) {
+        float* at = rows + (32 * b + 2 * r) * DG_SP + 32 * q;
+        unpack2(acc[b][r][q], at[0], at[DG_SP]);
+      }
 }
 
 // Factors the block that S (in shared memory, zeros above the diagonal, identity past the matrix) holds and stores its
@@ -245,52 +243,65 @@ __device__ __noinline__ void diag_block(uint8_t* image, int live, float* S, int 
     epi_sync();
     float* const P = P0 + (kb >> 5 & 1) * 32 * DG_PP;
     if (warp == 0) {
-      float a[32], o[32], last = 0.f;
+      DiagRow a;   // entries above the diagonal: not used
+      const float* from = S + (kb + lane) * DG_SP + kb;
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        a[i] = S[(kb + lane) * DG_SP + kb + i];   // i > lane: not used
-        o[i] = 0.f;
-      }
-      float iv = diag_pivot(__shfl_sync(0xffffffffu, a[0], 0), 0, bad);
+      for (int i = 0; i < 8; ++i) a.g[i] = from[i];
+#pragma unroll
+      for (int i = 0; i < 12; ++i) a.v[i] = pack2(from[8 + 2 * i], from[9 + 2 * i]);
+      float iv = diag_pivot(__shfl_sync(0xffffffffu, a.g[0], 0), bad);
 #pragma unroll 1
       for (int j8 = 0; j8 < 32; j8 += 8) {
-        diag_factor_step<0>(a, o, last, iv, Lk, inv, j8, lane, bad);
-        diag_factor_step<1>(a, o, last, iv, Lk, inv, j8, lane, bad);
-        diag_factor_step<2>(a, o, last, iv, Lk, inv, j8, lane, bad);
-        diag_factor_step<3>(a, o, last, iv, Lk, inv, j8, lane, bad);
-        diag_factor_step<4>(a, o, last, iv, Lk, inv, j8, lane, bad);
-        diag_factor_step<5>(a, o, last, iv, Lk, inv, j8, lane, bad);
-        diag_factor_step<6>(a, o, last, iv, Lk, inv, j8, lane, bad);
-        diag_factor_step<7>(a, o, last, iv, Lk, inv, j8, lane, bad);
-        diag_shift(a);
+        float l[8];
+        float* const column = Lk + j8 * DG_LP + lane;   // rows above a column's diagonal: not used
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          l[j] = a.g[j] * iv;
+          // all shuffles of the column first: they share the latency of the pivot's
+          float d = 0.f, row[8];
+          if (j < 7) d = __shfl_sync(0xffffffffu, fmaf(-l[j], l[j], a.g[j < 7 ? j + 1 : 7]), j8 + j + 1);
+#pragma unroll
+          for (int c = j + 1; c < 8; ++c) row[c] = __shfl_sync(0xffffffffu, l[j], j8 + c);
+          column[j * DG_LP] = l[j];
+          if (lane == 0) inv[j8 + j] = iv;
+          if (j < 7) iv = diag_pivot(d, bad);
+#pragma unroll
+          for (int c = j + 1; c < 8; ++c) a.g[c] = fmaf(-l[j], row[c], a.g[c]);
+        }
+        __syncwarp();
         asm volatile("barrier.cta.arrive %0, 160;" ::"r"(2 + (j8 >> 3)) : "memory");
+        if (j8 == 24) break;
+        a.apply(l, Lk + j8 * DG_LP + j8);
+        a.shift();
+        iv = diag_pivot(__shfl_sync(0xffffffffu, a.g[0], j8 + 8), bad);
       }
     } else {
       if (kb > 0) store(kb - 32, tid - 32, 224);
       if (panel >= 0) {
-        float v[32];
+        DiagRow v;
         const float* from = c >= kb + 32 ? S + c * DG_SP + kb : S + kb * DG_SP + c;
         const int pitch = c >= kb + 32 ? 1 : DG_SP;
+        // the block's own columns of the inverse start from the identity
+        auto entry = [&](int j) { return panel == kb / 32 ? (j == lane ? 1.f : 0.f) : from[j * pitch]; };
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = from[j * pitch];
-        if (panel == kb / 32) {   // the block's own columns of the inverse start from the identity
+        for (int i = 0; i < 8; ++i) v.g[i] = entry(i);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = lane == j ? 1.f : 0.f;
-        }
+        for (int i = 0; i < 12; ++i) v.v[i] = pack2(entry(8 + 2 * i), entry(9 + 2 * i));
 #pragma unroll 1
         for (int j8 = 0; j8 < 32; j8 += 8) {
           named_bar_sync(2 + (j8 >> 3), 160);
-          diag_panel_step<0>(v, Lk, inv, j8);
-          diag_panel_step<1>(v, Lk, inv, j8);
-          diag_panel_step<2>(v, Lk, inv, j8);
-          diag_panel_step<3>(v, Lk, inv, j8);
-          diag_panel_step<4>(v, Lk, inv, j8);
-          diag_panel_step<5>(v, Lk, inv, j8);
-          diag_panel_step<6>(v, Lk, inv, j8);
-          diag_panel_step<7>(v, Lk, inv, j8);
+          const float* const block = Lk + j8 * DG_LP + j8;
 #pragma unroll
-          for (int j = 0; j < 8; ++j) P[(j8 + j) * DG_PP + c] = v[j];
-          diag_shift(v);
+          for (int j = 0; j < 8; ++j) {
+            v.g[j] *= inv[j8 + j];
+#pragma unroll
+            for (int i = j + 1; i < 8; ++i) v.g[i] = fmaf(-v.g[j], block[j * DG_LP + i], v.g[i]);
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) P[(j8 + j) * DG_PP + c] = v.g[j];
+          if (j8 == 24) break;
+          v.apply(v.g, block);
+          v.shift();
         }
       }
     }
@@ -386,6 +397,17 @@ __device__ __forceinline__ bool epi_any(bool bad) {
   return r != 0;
 }
 
+__device__ __forceinline__ float4 lds4(uint32_t at) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+  return v;
+}
+__device__ __forceinline__ float lds(uint32_t at) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+  return v;
+}
+
 // A warp's 32 x 32 patch of fp32 values in its staging memory: rows of 128 bytes, the 16-byte pieces of a row exchanged.
 __device__ __forceinline__ void stage_patch(const float* v, uint8_t* stg, int lane) {
   __syncwarp();
@@ -395,39 +417,58 @@ __device__ __forceinline__ void stage_patch(const float* v, uint8_t* stg, int la
   __syncwarp();
 }
 // Three-way split of a staged patch, columns [32 h, 32 h + 32) of an image whose first row is at `base` (global or shared memory).
-// A lane splits eight values at a time.  The loop is not unrolled: code that runs once per tile is bound by instruction fetch
-// (unrolled over 64 values of a row per thread it took 5 us to split and store a tile).
-__device__ __noinline__ void split_patch(const uint8_t* stg, uint8_t* base, int h, int lane) {
+// A lane splits eight values at a time.  Code that runs once per tile is bound by instruction fetch (unrolled over the 64 values
+// of a row per thread it took 5 us to split and store a tile), so it is a function.
+__device__ __noinline__ void split_patch(uint32_t stg, uint8_t* base, int h, int lane) {
+  const int g = lane & 3;
 #pragma unroll 1
-  for (int i = 0; i < 4; ++i) {
-    const int r = i * 8 + (lane >> 2), g = lane & 3;
-    const float4 lo = *reinterpret_cast<const float4*>(stg + r * 128 + (((2 * g) ^ (r & 7)) << 4));
-    const float4 hi = *reinterpret_cast<const float4*>(stg + r * 128 + (((2 * g + 1) ^ (r & 7)) << 4));
-    float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-    uint8_t* at = base + r * 128 + (((4 * h + g) ^ (r & 7)) << 4);
+  for (int i = 0; i < 4; i += 2) {
+    float v[2][8];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int r = (i + u) * 8 + (lane >> 2);
+      const float4 lo = lds4(stg + r * 128 + (((2 * g) ^ (r & 7)) << 4)), hi = lds4(stg + r * 128 + (((2 * g + 1) ^ (r & 7)) << 4));
+      v[u][0] = lo.x, v[u][1] = lo.y, v[u][2] = lo.z, v[u][3] = lo.w, v[u][4] = hi.x, v[u][5] = hi.y, v[u][6] = hi.z, v[u][7] = hi.w;
+    }
 #pragma unroll
     for (int part = 0; part < 3; ++part) {
-      uint32_t w[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const __nv_bfloat16 b0 = __float2bfloat16_rn(v[2 * k]), b1 = __float2bfloat16_rn(v[2 * k + 1]);
-        w[k] = static_cast<uint32_t>(__bfloat16_as_ushort(b0)) | (static_cast<uint32_t>(__bfloat16_as_ushort(b1)) << 16);
-        v[2 * k] -= __bfloat162float(b0);
-        v[2 * k + 1] -= __bfloat162float(b1);
+      for (int u = 0; u < 2; ++u) {
+        const int r = (i + u) * 8 + (lane >> 2);
+        uint32_t w[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          float &x0 = v[u][2 * k], &x1 = v[u][2 * k + 1];
+          const __nv_bfloat162 b = __floats2bfloat162_rn(x0, x1);
+          w[k] = *reinterpret_cast<const uint32_t*>(&b);
+          x0 -= __uint_as_float(w[k] << 16);
+          x1 -= __uint_as_float(w[k] & 0xffff0000u);
+        }
+        *reinterpret_cast<uint4*>(base + part * PART_BYTES + r * 128 + (((4 * h + g) ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
       }
-      *reinterpret_cast<uint4*>(at + part * PART_BYTES) = make_uint4(w[0], w[1], w[2], w[3]);
     }
   }
 }
-// Stores a staged patch (element (r, c) at r * 32 + (c ^ r)) to out[row0 ..][col0 ..] and its mirror image.
-__device__ __noinline__ void store_patch(const float* stg, float* out, int n, int row0, int col0, bool diag, int lane) {
-  const int gc = col0 + lane, gr = row0 + lane;
-#pragma unroll 8
-  for (int r = 0; r < 32; ++r)
-    if (row0 + r < n && gc < n && (!diag || gc <= row0 + r)) out[static_cast<size_t>(row0 + r) * n + gc] = stg[r * 32 + (lane ^ r)];
-#pragma unroll 8
-  for (int c = 0; c < 32; ++c)
-    if (gr < n && col0 + c < n && (!diag || col0 + c < gr)) out[static_cast<size_t>(col0 + c) * n + gr] = stg[lane * 32 + (c ^ lane)];
+// Stores a staged patch (element (r, c) at r * 32 + (c ^ r)) to out[row0 ..][col0 ..], then its mirror image, eight loads in
+// flight.  Stores that alternate between the two take twice as long (9600 clocks a tile, in two passes 5100).
+__device__ __noinline__ void store_patch(uint32_t stg, float* out, int n, int row0, int col0, bool diag, int lane) {
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    const int first = pass == 0 ? row0 : col0, at = (pass == 0 ? col0 : row0) + lane;
+#pragma unroll 1
+    for (int i = 0; i < 32; i += 8) {
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        v[u] = lds(stg + (pass == 0 ? (i + u) * 32 + (lane ^ (i + u)) : lane * 32 + ((i + u) ^ lane)) * 4);
+      float* to = out + static_cast<size_t>(first + i) * n + at;
+#pragma unroll
+      for (int u = 0; u < 8; ++u, to += n) {
+        const int line = first + i + u;   // row of the output; the diagonal tile keeps its lower triangle
+        if (line < n && at < n && (!diag || (pass == 0 ? at <= line : line < at))) *to = v[u];
+      }
+    }
+  }
 }
 
 __global__ void __launch_bounds__(TC_THREADS, 1)
@@ -757,7 +798,7 @@ tc_tasks_kernel(const TcMat* __restrict__ mats, const Task* __restrict__ tasks, 
 #pragma unroll
           for (int c = 0; c < 32; ++c) stgf[lane * 32 + (c ^ lane)] = run[32 * h + c];
           __syncwarp();
-          store_patch(stgf, M.out, n, row0, col0 + 32 * h, diag, lane);
+          store_patch(smem_u32(stgf), M.out, n, row0, col0 + 32 * h, diag, lane);
         }
         continue;
       }
@@ -778,7 +819,7 @@ tc_tasks_kernel(const TcMat* __restrict__ mats, const Task* __restrict__ tasks, 
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         stage_patch(run + 32 * h, stg, lane);
-        split_patch(stg, operand, h, lane);
+        split_patch(smem_u32(stg), operand, h, lane);
       }
       proxy_fence();
       __syncwarp();
@@ -795,7 +836,7 @@ tc_tasks_kernel(const TcMat* __restrict__ mats, const Task* __restrict__ tasks, 
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         stage_patch(run + 32 * h, stg, lane);
-        split_patch(stg, image, h, lane);
+        split_patch(smem_u32(stg), image, h, lane);
       }
       proxy_fence();
       epi_sync();   // the release of one thread covers what the others stored before the barrier
