@@ -81,8 +81,9 @@ __host__ __device__ inline int task_blocks(int kind, int i, int j, int n) {
 //   factor   one warp, a row of the 32 x 32 block per lane, in registers.  Eight columns at a time: inside of the eight a column
 //            is passed on by shuffles, so the chain from pivot to pivot is a product, a shuffle and a reciprocal square root;
 //            then the eight are applied to the columns behind them;
-//   panel    four warps, one thread per row below (forward substitution with the block) and one per column of the inverse's
-//            rows [kb, be), eight columns behind the factor.  P[j][c] = T[kb + j][c] for c < be and L[c][kb + j] for c >= be;
+//   panel    two warps, a thread takes two of the rows below (forward substitution with the block) or of the columns of the
+//            inverse's rows [kb, be), eight columns behind the factor: with four warps of one row per thread, their loads took
+//            the shared memory pipe from the factor's shuffles.  P[j][c] = T[kb + j][c] for c < be and L[c][kb + j] for c >= be;
 //   update   S[i][c] -= sum_j P[j][i] P[j][c] for the rows i >= be: the trailing block right of be, the right-hand side of
 //            the inverse left of it.  Finished columns of the factor are dead (only the inverse leaves the kernel), so both
 //            share S.  A warp takes four rows of each row block, a lane one column of each column block up to the diagonal;
@@ -139,20 +140,28 @@ struct DiagRow {
 #pragma unroll
     for (int i = 0; i < 12; ++i) v[i] = i < 8 ? v[i + 4 < 12 ? i + 4 : 11] : 0ull;
   }
-  // columns from the ninth on -= x[j] * o[j * DG_LP + 8 ...] for the eight finished columns j, in their order
-  __device__ __forceinline__ void apply(const float (&x)[8], const float* o) {
+};
+
+// Columns from the ninth on -= x[j] * o[j * DG_LP + 8 ...] for the eight finished columns j, in their order; N rows share the
+// loads (a 16-byte load of a warp takes four clocks of the shared memory pipe even where all lanes read the same).
+template <int N>
+__device__ __forceinline__ void diag_apply(DiagRow (&row)[N], const float (&x)[N][8], const float* o) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const f32x2 m = pack2(-x[j], -x[j]);
+  for (int j = 0; j < 8; ++j) {
+    f32x2 m[N];
 #pragma unroll
-      for (int i = 0; i < 12; i += 2) {
-        const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(o + j * DG_LP + 8 + 2 * i);
-        v[i] = fma2(m, q.x, v[i]);
-        v[i + 1] = fma2(m, q.y, v[i + 1]);
+    for (int u = 0; u < N; ++u) m[u] = pack2(-x[u][j], -x[u][j]);
+#pragma unroll
+    for (int i = 0; i < 12; i += 2) {
+      const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(o + j * DG_LP + 8 + 2 * i);
+#pragma unroll
+      for (int u = 0; u < N; ++u) {
+        row[u].v[i] = fma2(m[u], q.x, row[u].v[i]);
+        row[u].v[i + 1] = fma2(m[u], q.y, row[u].v[i + 1]);
       }
     }
   }
-};
+}
 
 // Rows and columns behind stage KQ, whose columns are [32 KQ, 32 KQ + 32).
 template <int KQ>
@@ -205,9 +214,7 @@ __device__ __noinline__ void diag_block(uint8_t* image, int live, float* S, int 
   float* const Lk = P0 + 2 * 32 * DG_PP;
   float* const inv = Lk + 32 * DG_LP;
   const int lane = tid & 31, warp = tid >> 5;
-  // warp 0 factors; the panel is on four warps of the other schedulers
-  const int panel = warp == 5 ? 3 : (warp >= 1 && warp <= 3 ? warp - 1 : -1);
-  const int c = 32 * panel + lane;             // row or column of a panel thread
+  const int panel = warp == 1 || warp == 3 ? warp >> 1 : -1;   // warp 0 factors; the panel's warps are on other schedulers
   bool bad = false;
   auto store_row = [&](int r, int col, const uint32_t (&w)[3][2]) {   // columns col .. col + 3, col a multiple of four
     uint8_t* at = image + (col >> 6) * (3 * PART_BYTES) + r * 128 + ((((col & 63) >> 3) ^ (r & 7)) << 4) + (col & 4) * 2;
@@ -243,65 +250,78 @@ __device__ __noinline__ void diag_block(uint8_t* image, int live, float* S, int 
     epi_sync();
     float* const P = P0 + (kb >> 5 & 1) * 32 * DG_PP;
     if (warp == 0) {
-      DiagRow a;   // entries above the diagonal: not used
+      DiagRow a[1];   // entries above the diagonal: not used
       const float* from = S + (kb + lane) * DG_SP + kb;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) a.g[i] = from[i];
+      for (int i = 0; i < 8; ++i) a[0].g[i] = from[i];
 #pragma unroll
-      for (int i = 0; i < 12; ++i) a.v[i] = pack2(from[8 + 2 * i], from[9 + 2 * i]);
-      float iv = diag_pivot(__shfl_sync(0xffffffffu, a.g[0], 0), bad);
+      for (int i = 0; i < 12; ++i) a[0].v[i] = pack2(from[8 + 2 * i], from[9 + 2 * i]);
+      float iv = diag_pivot(__shfl_sync(0xffffffffu, a[0].g[0], 0), bad);
 #pragma unroll 1
       for (int j8 = 0; j8 < 32; j8 += 8) {
-        float l[8];
+        float l[1][8];
         float* const column = Lk + j8 * DG_LP + lane;   // rows above a column's diagonal: not used
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          l[j] = a.g[j] * iv;
+          l[0][j] = a[0].g[j] * iv;
           // all shuffles of the column first: they share the latency of the pivot's
           float d = 0.f, row[8];
-          if (j < 7) d = __shfl_sync(0xffffffffu, fmaf(-l[j], l[j], a.g[j < 7 ? j + 1 : 7]), j8 + j + 1);
+          if (j < 7) d = __shfl_sync(0xffffffffu, fmaf(-l[0][j], l[0][j], a[0].g[j < 7 ? j + 1 : 7]), j8 + j + 1);
 #pragma unroll
-          for (int c = j + 1; c < 8; ++c) row[c] = __shfl_sync(0xffffffffu, l[j], j8 + c);
-          column[j * DG_LP] = l[j];
+          for (int c = j + 1; c < 8; ++c) row[c] = __shfl_sync(0xffffffffu, l[0][j], j8 + c);
+          column[j * DG_LP] = l[0][j];
           if (lane == 0) inv[j8 + j] = iv;
           if (j < 7) iv = diag_pivot(d, bad);
 #pragma unroll
-          for (int c = j + 1; c < 8; ++c) a.g[c] = fmaf(-l[j], row[c], a.g[c]);
+          for (int c = j + 1; c < 8; ++c) a[0].g[c] = fmaf(-l[0][j], row[c], a[0].g[c]);
         }
         __syncwarp();
-        asm volatile("barrier.cta.arrive %0, 160;" ::"r"(2 + (j8 >> 3)) : "memory");
+        asm volatile("barrier.cta.arrive %0, 96;" ::"r"(2 + (j8 >> 3)) : "memory");
         if (j8 == 24) break;
-        a.apply(l, Lk + j8 * DG_LP + j8);
-        a.shift();
-        iv = diag_pivot(__shfl_sync(0xffffffffu, a.g[0], j8 + 8), bad);
+        diag_apply(a, l, Lk + j8 * DG_LP + j8);
+        a[0].shift();
+        iv = diag_pivot(__shfl_sync(0xffffffffu, a[0].g[0], j8 + 8), bad);
       }
     } else {
       if (kb > 0) store(kb - 32, tid - 32, 224);
       if (panel >= 0) {
-        DiagRow v;
-        const float* from = c >= kb + 32 ? S + c * DG_SP + kb : S + kb * DG_SP + c;
-        const int pitch = c >= kb + 32 ? 1 : DG_SP;
-        // the block's own columns of the inverse start from the identity
-        auto entry = [&](int j) { return panel == kb / 32 ? (j == lane ? 1.f : 0.f) : from[j * pitch]; };
+        DiagRow v[2];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v.g[i] = entry(i);
+        for (int u = 0; u < 2; ++u) {
+          const int block = 2 * panel + u, c = 32 * block + lane;
+          const float* from = c >= kb + 32 ? S + c * DG_SP + kb : S + kb * DG_SP + c;
+          const int pitch = c >= kb + 32 ? 1 : DG_SP;
+          // the block's own columns of the inverse start from the identity
+          auto entry = [&](int j) { return block == kb / 32 ? (j == lane ? 1.f : 0.f) : from[j * pitch]; };
 #pragma unroll
-        for (int i = 0; i < 12; ++i) v.v[i] = pack2(entry(8 + 2 * i), entry(9 + 2 * i));
+          for (int i = 0; i < 8; ++i) v[u].g[i] = entry(i);
+#pragma unroll
+          for (int i = 0; i < 12; ++i) v[u].v[i] = pack2(entry(8 + 2 * i), entry(9 + 2 * i));
+        }
 #pragma unroll 1
         for (int j8 = 0; j8 < 32; j8 += 8) {
-          named_bar_sync(2 + (j8 >> 3), 160);
+          named_bar_sync(2 + (j8 >> 3), 96);
           const float* const block = Lk + j8 * DG_LP + j8;
+          float x[2][8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            v.g[j] *= inv[j8 + j];
+            const float4 o0 = *reinterpret_cast<const float4*>(block + j * DG_LP), o1 = *reinterpret_cast<const float4*>(block + j * DG_LP + 4);
+            const float o[8] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w}, iv = inv[j8 + j];
 #pragma unroll
-            for (int i = j + 1; i < 8; ++i) v.g[i] = fmaf(-v.g[j], block[j * DG_LP + i], v.g[i]);
+            for (int u = 0; u < 2; ++u) {
+              x[u][j] = v[u].g[j] * iv;
+#pragma unroll
+              for (int i = j + 1; i < 8; ++i) v[u].g[i] = fmaf(-x[u][j], o[i], v[u].g[i]);
+            }
           }
 #pragma unroll
-          for (int j = 0; j < 8; ++j) P[(j8 + j) * DG_PP + c] = v.g[j];
+          for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) P[(j8 + j) * DG_PP + 64 * panel + 32 * u + lane] = x[u][j];
           if (j8 == 24) break;
-          v.apply(v.g, block);
-          v.shift();
+          diag_apply(v, x, block);
+          v[0].shift();
+          v[1].shift();
         }
       }
     }
@@ -876,9 +896,9 @@ PreparedCache<Prepared, 4>& g_cache = *new PreparedCache<Prepared, 4>;
 // DIAG).  In a slot every matrix may take one step, and the longest remaining chains always do; shorter ones join while the
 // slot has room, and OUT tiles, which nothing waits for, fill the rest.
 std::vector<Task> make_tasks(const std::vector<int>& sizes, int ctas) {
-  constexpr int STEP_US = 35, BLOCK_US = 1, TILE_US = 5, DIAG_US = 28;
+  constexpr int STEP_US = 35, BLOCK_US = 1, TILE_US = 5, DIAG_US = 28, AHEAD = 12;
   const int count = static_cast<int>(sizes.size());
-  std::vector<int> nb(count), step(count, 0), order(count), out_i(count, 0), out_j(count, 0);
+  std::vector<int> nb(count), step(count, 0), order(count), out_i(count, 0), out_j(count, 0), started(count, 0);
   for (int m = 0; m < count; ++m) {
     nb[m] = (sizes[m] + TB - 1) / TB;
     order[m] = m;
@@ -903,11 +923,19 @@ std::vector<Task> make_tasks(const std::vector<int>& sizes, int ctas) {
       used += work;
       taken.push_back(m);
     }
+    int ahead = 0;
     for (int m : taken) {
       const int j = step[m];
-      for (int i = j + 1; i < nb[m]; ++i) {
+      for (int i = started[m] > j ? j + 2 : j + 1; i < nb[m]; ++i) {
         tasks.push_back({m, TASK_FACTOR, i, j});
         if (i == j + 1) tasks.push_back({m, TASK_DIAG, i, i});
+      }
+      // the next step's first tile and diagonal block, so that they are not behind the rest of this slot
+      if (4 * (nb[m] - j) >= 3 * longest && ahead < AHEAD && j + 2 < nb[m]) {
+        tasks.push_back({m, TASK_FACTOR, j + 2, j + 1});
+        tasks.push_back({m, TASK_DIAG, j + 2, j + 2});
+        started[m] = j + 2;   // steps below this one have them
+        ++ahead;
       }
     }
     for (int m : taken)
