@@ -416,6 +416,8 @@ void gemm_batch_begin() {
   g_batch_open = true;
 }
 
+bool gemm_batch_is_open() { return g_batch_open; }
+
 // Launches what was recorded since gemm_batch_begin() on the current stream; returns the number of products.
 int64_t gemm_batch_end() {
   TORCH_CHECK(g_batch.active, "no GEMM batch is open");

@@ -357,7 +357,9 @@ IMPLICIT_IM2COL = os.environ.get('ASDL_B200_IMPLICIT_IM2COL', '1') != '0'
 #: explicit path is ahead on every layer measured (32 images): at 56 x 56 x 64 channels (110 MiB of patches) 0.099 ms for
 #: im2col + SYRK and 0.128 for the implicit SYRK; on the small maps of deep layers (14 x 14 x 256: 28 MiB) the 4-D boxes of
 #: 2 x 2 pixels x 16 images load at half the rate of the 2-D boxes of an explicit matrix (0.065 and 0.146 ms).
-IMPLICIT_IM2COL_MIN_MB = float(os.environ.get('ASDL_B200_IMPLICIT_IM2COL_MIN_MB', '64'))
+#: Products by tap difference (below) are faster than both and come first, unless a program has set another threshold than this.
+_IMPLICIT_IM2COL_DEFAULT_MB = 64.0
+IMPLICIT_IM2COL_MIN_MB = float(os.environ.get('ASDL_B200_IMPLICIT_IM2COL_MIN_MB', _IMPLICIT_IM2COL_DEFAULT_MB))
 
 
 def implicit_im2col_eligible(x: torch.Tensor, kernel, stride, dilation, padding, out_hw, khwc_order: bool) -> bool:
@@ -372,6 +374,38 @@ def implicit_im2col_eligible(x: torch.Tensor, kernel, stride, dilation, padding,
                 and n * ho * wo * c * kh * kw * 2 >= IMPLICIT_IM2COL_MIN_MB * 2 ** 20)
 
 
+def tap_difference_eligible(x: torch.Tensor, kernel, padding, out_hw, khwc_order: bool) -> bool:
+    """True when the input-side factor of a convolution without stride and dilation is formed from products by tap
+    difference (``csrc/conv_gram.cu``) instead of a patch matrix: filters of 3 x 3 to 5 x 5.
+
+    The rule is in patch elements P = rows x columns of the patch matrix that is not written (times in us, patches -> differences):
+      * fp32: channels that fill at least half of their 64-channel chunks (24 of 64: 54 -> 56; 32 of 64: 64 -> 41, 32 x 32 images);
+        3 x 3 from the smallest size on (4 x 64 x 7 x 7: 27 -> 25), but with more than 128 channels from P = 3e6 (192: P = 3.4e5
+        28 -> 35, 3.5e6 52 -> 50); larger filters, which have many corrections, from 1e7 (64: 3.3e6 47 -> 53, 1e7 84 -> 60;
+        192: 9.8e6 152 -> 199, 3e7 373 -> 254);
+      * bf16, order (kh, kw, c) with whole 64-channel chunks, where the result is assembled block by block: 3 x 3 always
+        (4 x 64 x 7 x 7: 23 -> 19, 32 x 256 x 14 x 14: 62 -> 42), larger filters from 6e6 (64: 3.3e6 31 -> 37; 128: 6.5e6 59 -> 48);
+      * bf16 otherwise: at least 64 channels and P = 2.5e7 (96: 5.4e6 30 -> 34, 2.8e7 63 -> 48).
+    Rows and columns outside of a tap's window are taken off from sums over the whole image: at least half of the image has to
+    be in the window, so that little cancels."""
+    (kh, kw), (ph, pw), (ho, wo) = kernel, padding, out_hw
+    n, c, h, w = x.shape
+    if not (TAP_DIFFERENCES and 3 <= kh <= 5 and 3 <= kw <= 5 and x.is_cuda and ph < kh and pw < kw and min(n, c, ho, wo) > 0
+            and 2 * ho * wo >= h * w):
+        return False
+    size, chunks = n * ho * wo * c * kh * kw, (c + 63) // 64
+    small_filter = kh * kw <= 9
+    if _use_x3(x.dtype):
+        return c >= 32 * chunks and size >= ((0 if c <= 128 else 3e6) if small_filter else 1e7)
+    if khwc_order and c % 64 == 0:
+        return size >= (0 if small_filter else 6e6)
+    return c >= 64 and size >= 2.5e7
+
+
+#: form the factors of stride-1 convolutions from products by tap difference where that is the faster way
+TAP_DIFFERENCES = True
+
+
 def conv_patch_gram(x: torch.Tensor, conv: torch.nn.Conv2d, scale: float = 1.0,
                     out: Optional[torch.Tensor] = None, beta: float = 0.0,
                     channels_last_order: bool = False) -> torch.Tensor:
@@ -380,8 +414,9 @@ def conv_patch_gram(x: torch.Tensor, conv: torch.nn.Conv2d, scale: float = 1.0,
 
     ``channels_last_order=False`` orders rows/columns as (c, kh, kw) (matching
     ``weight.view(c_out, -1)``); ``True`` uses (kh, kw, c), the order of a channels_last weight.
-    CUDA: stride-1 convolutions on channels_last bf16 inputs with a multiple of 64 channels whose patch matrix
-    would take ``IMPLICIT_IM2COL_MIN_MB`` or more never form it - the SYRK's producer gathers 8 x 8 pixel blocks of one filter tap with 4-D TMA boxes, padding
+    CUDA: stride-1 convolutions with filters of 3 x 3 to 5 x 5 form it from products of the input with itself by tap
+    difference (``tap_difference_eligible``; not while a batch of products is recorded); other stride-1 convolutions on
+    channels_last bf16 inputs with a multiple of 64 channels whose patch matrix would take ``IMPLICIT_IM2COL_MIN_MB`` or more never form it - the SYRK's producer gathers 8 x 8 pixel blocks of one filter tap with 4-D TMA boxes, padding
     and image edges being TMA's zero fill (``IMPLICIT_IM2COL``); 1x1 stride-1 convolutions read the activations
     in place; everything else goes through a bf16 im2col kernel (vectorised for channels_last inputs).  fp32 inputs are
     staged as bf16 hi/lo patch pairs and multiplied in three passes (precision policy 'auto')."""
@@ -404,8 +439,15 @@ def conv_patch_gram(x: torch.Tensor, conv: torch.nn.Conv2d, scale: float = 1.0,
             and c % 8 == 0 and not _use_x3(x.dtype)):
         rows = x.permute(0, 2, 3, 1).reshape(n * h * w, c)  # a view: NHWC memory is already [rows, c]
         return gram(rows, scale=scale, out=out, beta=beta)
-    if (implicit_im2col_eligible(x, (kh, kw), (sh, sw), (dh, dw), (ph, pw), (ho, wo), channels_last_order)
-            and (out is None or (out.dtype == torch.float32 and out.stride(1) == 1))):
+    implicit = False
+    if sh == sw == dh == dw == 1 and kh * kw > 1 and (out is None or (out.dtype == torch.float32 and out.stride(1) == 1)):
+        implicit = channels_last_order and implicit_im2col_eligible(x, (kh, kw), (1, 1), (1, 1), (ph, pw), (ho, wo), True)
+        if tap_difference_eligible(x, (kh, kw), (ph, pw), (ho, wo), channels_last_order) and not (
+                implicit and IMPLICIT_IM2COL_MIN_MB != _IMPLICIT_IM2COL_DEFAULT_MB):
+            result, weight = (torch.empty(ncol, ncol, device=x.device, dtype=torch.float32), 0.0) if out is None else (out, beta)
+            if extension().conv_gram(x, result, kh, kw, ph, pw, float(scale), float(weight), channels_last_order, _use_x3(x.dtype)):
+                return result
+    if implicit:
         # no patch matrix: the SYRK's producer gathers its operand tiles from x with 4-D TMA boxes
         if out is None:
             out = torch.empty(ncol, ncol, device=x.device, dtype=torch.float32)

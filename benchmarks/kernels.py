@@ -192,20 +192,21 @@ def bench_lnstats(timer, rows, d, hbm, src):
 
 
 def bench_conv_syrk(timer, n, c, hw, k, flops_peak, src):
-    """Input-side factor of a stride-1 k x k convolution (padding k // 2) on a channels_last bf16 input: patches
-    gathered inside the SYRK by 4-D TMA boxes against the bf16 im2col kernel followed by the SYRK."""
+    """Input-side factor of a stride-1 k x k convolution (padding k // 2) on a channels_last bf16 input: products by tap
+    difference, patches gathered inside the SYRK by 4-D TMA boxes, and the bf16 im2col kernel followed by the SYRK."""
     conv = torch.nn.Conv2d(c, 8, k, padding=k // 2).cuda()
     x = torch.randn(n, c, hw, hw, device='cuda').to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
     ncol = c * k * k
     out = torch.empty(ncol, ncol, device='cuda')
+    ms_differences = timer(lambda: ops.conv_patch_gram(x, conv, out=out, channels_last_order=True))
     saved, saved_mb = ops.IMPLICIT_IM2COL, ops.IMPLICIT_IM2COL_MIN_MB
-    ops.IMPLICIT_IM2COL, ops.IMPLICIT_IM2COL_MIN_MB = True, 0.0
+    ops.IMPLICIT_IM2COL, ops.IMPLICIT_IM2COL_MIN_MB, ops.TAP_DIFFERENCES = True, 0.0, False
     ms = timer(lambda: ops.conv_patch_gram(x, conv, out=out, channels_last_order=True))
     ops.IMPLICIT_IM2COL = False
     ms_explicit = timer(lambda: ops.conv_patch_gram(x, conv, out=out, channels_last_order=True))
-    ops.IMPLICIT_IM2COL, ops.IMPLICIT_IM2COL_MIN_MB = saved, saved_mb
+    ops.IMPLICIT_IM2COL, ops.IMPLICIT_IM2COL_MIN_MB, ops.TAP_DIFFERENCES = saved, saved_mb, True
     fl = 2.0 * n * hw * hw * ncol * ncol
-    emit(case='conv_patch_syrk_bf16', n=n, c=c, hw=hw, k=k, ncol=ncol, implicit_ms=round(ms, 4),
+    emit(case='conv_patch_syrk_bf16', n=n, c=c, hw=hw, k=k, ncol=ncol, differences_ms=round(ms_differences, 4), implicit_ms=round(ms, 4),
          explicit_im2col_ms=round(ms_explicit, 4), speedup=round(ms_explicit / ms, 2),
          tflops_full_product=round(fl / ms / 1e9, 1), frac_of_peak_flops=round(fl / (ms * 1e-3) / flops_peak, 3),
          patch_matrix_mb=round(n * hw * hw * ncol * 2 / 2 ** 20, 1), peak_source=src)

@@ -191,6 +191,50 @@ def test_inverse_at_the_edges_of_the_diagonal_stages(n):
     ops.check_status()
 
 
+@pytest.mark.parametrize('kernel,padding', [((3, 3), (1, 1)), ((3, 3), (0, 0)), ((5, 5), (2, 2)), ((4, 3), (1, 2)), ((2, 2), (1, 0))])
+@pytest.mark.parametrize('shape', [(1, 64, 7, 7), (3, 24, 9, 6), (70, 65, 8, 8), (2, 192, 12, 13), (5, 128, 10, 10)])
+@pytest.mark.parametrize('dtype,layout', [(torch.float32, 'nchw'), (torch.bfloat16, 'nhwc'), (torch.float16, 'view')])
+def test_factor_by_tap_differences(kernel, padding, shape, dtype, layout):
+    """One, two and more chunks of channels, ragged ones, windows that cut both sides of the image, both column orders."""
+    n, c, h, w = shape
+    x = torch.randn(n, c + 1, h, w + 2, device=DEV, generator=_gen(3)).to(dtype)[:, 1:, :, 1:-1]
+    if layout != 'view':
+        x = x.contiguous(memory_format=torch.channels_last if layout == 'nhwc' else torch.contiguous_format)
+    taps = kernel[0] * kernel[1]
+    x3 = dtype == torch.float32
+    seen = (x if x3 else x.to(torch.bfloat16)).double()
+    patches = F.unfold(seen, kernel, padding=padding).transpose(1, 2).reshape(-1, c * taps)
+    for khwc in (True, False):
+        m = patches.view(-1, c, taps).transpose(1, 2).reshape(patches.shape) if khwc else patches
+        before = torch.randn(c * taps, c * taps, device=DEV, generator=_gen(4))
+        before += before.T.clone()
+        out = torch.full((c * taps, c * taps + 3), 2.0, device=DEV)[:, :c * taps]   # rows of any alignment
+        out.copy_(before)
+        assert ops.extension().conv_gram(x, out, *kernel, *padding, 1 / n, 0.5, khwc, x3)
+        want = m.T @ m / n + 0.5 * before.double()
+        # 2^-16 of a product of bf16 pairs (exact ones for bf16) and fp32 sums, over the whole image where the window is a part of it
+        bound = ((2.0 ** -15 if x3 else 0.0) + 64 * 2.0 ** -24) * h * w * seen.square().amax().item() + 2.0 ** -22 * before.abs().max()
+        assert (out.double() - want).abs().max() <= bound
+        assert torch.equal(out, out.T)
+        got = ops.extension().conv_gram(x, out, *kernel, *padding, 1 / n, 0.0, khwc, x3)
+        assert got and (out.double() - m.T @ m / n).abs().max() <= bound
+    ops.check_status()
+
+
+def test_the_rule_for_tap_differences_gives_what_patches_give(monkeypatch):
+    for shape, k, p, mode, dtype in [((4, 64, 7, 7), 3, 1, 'zeros', torch.float32), ((8, 32, 16, 16), 3, 1, 'reflect', torch.float32),
+                                     ((32, 64, 14, 14), 5, 2, 'zeros', torch.bfloat16), ((4, 128, 9, 9), 3, 0, 'zeros', torch.bfloat16)]:
+        x = torch.randn(*shape, device=DEV, generator=_gen(8)).to(dtype)
+        last = dtype == torch.bfloat16
+        x = x.contiguous(memory_format=torch.channels_last) if last else x
+        conv = torch.nn.Conv2d(shape[1], 4, k, padding=p, padding_mode=mode, bias=False).to(DEV)
+        got = ops.conv_patch_gram(x, conv, scale=1e-3, channels_last_order=last)
+        with monkeypatch.context() as m:
+            m.setattr(ops, 'TAP_DIFFERENCES', False)
+            want = ops.conv_patch_gram(x, conv, scale=1e-3, channels_last_order=last)
+        assert (got - want).norm() <= (4e-5 if dtype == torch.float32 else 5e-6) * want.norm()
+
+
 @pytest.mark.parametrize('sizes', [(1, 128, 129, 256, 384, 385), (640, 8, 513, 64, 257, 191, 1), (1153, 1024), (130,) * 90 + (400,) * 40])
 def test_grouped_inverse_of_mixed_sizes(sizes):
     """Tiles at and past the edges, chains of several lengths side by side, more tasks than CTAs; inputs with a row pitch."""
