@@ -111,6 +111,25 @@ void g2_launch_reduce_list(const GemmProblem2* d_probs, const GemmWork2* d_work,
     launch_reduce<128>(n_work, dummy, d_probs, d_work, nullptr, 0, stream);
 }
 
+// K ranges of the x3wide flavour, whose CTAs fill an SM each: the count with the least expected time of all waves and of the
+// reduction.  A K block of 128 x 256 tiles takes 0.85 us (three part products of 512 clocks), a tile 6 us around its sum, a
+// reduction 6 us and 0.04 us for each partial tile.  Two ranges for as many CTAs as two per SM had room for, whatever the waves,
+// took 1024 x 4096 through two waves of each product and a reduction each: 210 us for both products and their casts, one range
+// @K_NEW@.
+static int split_in_waves(int tiles, int kb_total, int n_sms) {
+  int best = 1;
+  double least = 1e30;
+  for (int s = 1; s <= 32 && (s == 1 || kb_total / s >= 4); ++s) {
+    const int waves = (tiles * s + n_sms - 1) / n_sms;
+    const double us = waves * (0.85 * ((kb_total + s - 1) / s) + 6.0) + (s > 1 ? 6.0 + 0.04 * tiles * s : 0.0);
+    if (us < 0.98 * least) {   // a tie goes to fewer ranges
+      least = us;
+      best = s;
+    }
+  }
+  return best;
+}
+
 // Fills the scalar fields of a problem and encodes its tensor maps.
 void gemm_fill_problem(GemmProblem2& P, const std::vector<at::Tensor>& a_segs,
                        const std::vector<at::Tensor>& b_segs, bool a_kmajor, bool b_kmajor,
@@ -205,7 +224,9 @@ void gemm_fill_problem(GemmProblem2& P, const std::vector<at::Tensor>& a_segs,
   P.ntiles = tile_count(P.tiles_m, P.tiles_n, sym, bn_grid);
   const int kb_total = (P.K + G2_BK - 1) / G2_BK;
   int nsplit = split3 ? 1 : static_cast<int>(nsplit_req);  // the chunked sum of a split3 product is not split
-  if (nsplit <= 0) {
+  if (nsplit <= 0 && x3wide) {
+    nsplit = split_in_waves(P.ntiles, kb_total, n_sms);
+  } else if (nsplit <= 0) {
     const int target = 2 * n_sms;
     nsplit = target / (P.ntiles > 0 ? P.ntiles : 1);
     const int max_by_k = kb_total / 8;
