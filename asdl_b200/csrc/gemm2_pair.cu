@@ -12,21 +12,29 @@ int g2_pair_tiles(const GemmProblem2& P) {
   return (P.flags & G2F_SYM) ? T * (T + 1) / 2 : T * P.tiles_n;
 }
 
-void g2_run_pair(const GemmProblem2& single, int n_work, int n_sms, cudaStream_t stream) {
-  if (n_work <= 0) return;
+template <int PARTS>
+static void run_pair(const GemmProblem2& single, int n_work, int n_sms, cudaStream_t stream) {
   static bool attr_set_on[64] = {false};
   int dev = 0;
   B200_CUDA_CHECK(cudaGetDevice(&dev));
   bool& attr_set = attr_set_on[dev & 63];
   if (!attr_set) {
-    B200_CUDA_CHECK(cudaFuncSetAttribute(umma_gemm2_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    B200_CUDA_CHECK(cudaFuncSetAttribute(umma_gemm2_pair_kernel<PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          G2P_SMEM_BYTES));
     attr_set = true;
   }
   const int pairs = std::max(1, std::min(n_work, n_sms / 2));
-  umma_gemm2_pair_kernel<<<2 * pairs, G2P_THREADS, G2P_SMEM_BYTES, stream>>>(single, n_work);
+  umma_gemm2_pair_kernel<PARTS><<<2 * pairs, G2P_THREADS, G2P_SMEM_BYTES, stream>>>(single, n_work);
   B200_CUDA_CHECK(cudaGetLastError());
   count_launch();
+}
+
+void g2_run_pair(const GemmProblem2& single, int n_work, int n_sms, cudaStream_t stream) {
+  if (n_work <= 0) return;
+  if (single.flags & G2F_SPLIT2)
+    run_pair<2>(single, n_work, n_sms, stream);
+  else
+    run_pair<1>(single, n_work, n_sms, stream);
 }
 
 }  // namespace b200

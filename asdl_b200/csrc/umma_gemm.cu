@@ -111,17 +111,28 @@ void g2_launch_reduce_list(const GemmProblem2* d_probs, const GemmWork2* d_work,
     launch_reduce<128>(n_work, dummy, d_probs, d_work, nullptr, 0, stream);
 }
 
-// K ranges of the x3wide flavour, whose CTAs fill an SM each: the count with the least expected time of all waves and of the
-// reduction.  A K block of 128 x 256 tiles takes 0.85 us (three part products of 512 clocks), a tile 6 us around its sum, a
-// reduction 6 us and 0.04 us for each partial tile.  Two ranges for as many CTAs as two per SM had room for, whatever the waves,
-// took 1024 x 4096 through two waves of each product and a reduction each: 210 us for both products and their casts, one range
-// @K_NEW@.
-static int split_in_waves(int tiles, int kb_total, int n_sms) {
+// bf16x3 products on CTA pairs: single ones (the tiles of a plan or a batch run on one kernel) of more than one 128-wide tile
+// each way, unless the tile policy asks for something else.
+static bool x3_takes_pairs(int64_t m, int64_t n) { return g_wide_mode >= 3 && !g_batch_open && m > 128 && n > 128; }
+
+// Symmetric ones: from 24 K blocks on, and where the lower 256 x 256 tiles cover little more than the lower 128 x 128 tiles do.
+// us, three segments of the plain flavour -> pairs: 3000 x 1000 42 -> 28, 8192 x 1500 102 -> 75, 8192 x 2048 114 -> 103,
+// 12608 x 768 47 -> 44.5; but 1000 x 2048 31 -> 39, 300 x 1000 22 -> 27, and 8192 x 384 (twice the area) 23.5 -> 24.7.
+static bool x3_syrk_takes_pairs(int64_t n, int64_t k) {
+  const int64_t t = (n + 127) / 128, p = (t + 1) / 2;
+  return x3_takes_pairs(n, n) && k >= 24 * G2_BK && 4.0 * (p * (p + 1) / 2) <= 1.35 * (t * (t + 1) / 2);
+}
+
+// K ranges of bf16x3 products on pairs (`slots` of them, `tiles` for them, `partials` 128 x 256 tiles): the count with the least
+// expected time of all waves and of the reduction.  A K block takes 0.9 us (three part products of 512 clocks), a tile 6 us around
+// its sum, a reduction 6 us and 0.04 us for each partial tile.  A count for two CTAs per SM took 1024 x 4096 through two waves of
+// each product and a reduction each.
+static int split_in_waves(int tiles, int partials, int kb_total, int slots) {
   int best = 1;
   double least = 1e30;
   for (int s = 1; s <= 32 && (s == 1 || kb_total / s >= 4); ++s) {
-    const int waves = (tiles * s + n_sms - 1) / n_sms;
-    const double us = waves * (0.85 * ((kb_total + s - 1) / s) + 6.0) + (s > 1 ? 6.0 + 0.04 * tiles * s : 0.0);
+    const int waves = (tiles * s + slots - 1) / slots;
+    const double us = waves * (0.9 * ((kb_total + s - 1) / s) + 6.0) + (s > 1 ? 6.0 + 0.04 * partials * s : 0.0);
     if (us < 0.98 * least) {   // a tie goes to fewer ranges
       least = us;
       best = s;
@@ -152,14 +163,15 @@ void gemm_fill_problem(GemmProblem2& P, const std::vector<at::Tensor>& a_segs,
   TORCH_CHECK(K == Kb, "contraction sizes differ: ", K, " vs ", Kb);
   TORCH_CHECK(M > 0 && N > 0 && M < (1 << 30) && N < (1 << 30) && K < (1ll << 31) - 64, "matrix sizes out of range");
   if (sym) TORCH_CHECK(M == N, "symmetric mode needs a square output");
-  const bool wide = x3wide || (!split3 && (g_wide_mode == 2 || (g_wide_mode == 1 && N >= 1024 && M >= 1024)));
+  const bool x3_pair = x3wide && x3_takes_pairs(M, N);
+  const bool wide = !x3_pair && (x3wide || (!split3 && (g_wide_mode == 2 || (g_wide_mode == 1 && N >= 1024 && M >= 1024))));
   // CTA pairs pay from outputs of 2048 x 2048 and about 2e10 multiply-adds on (measured: 20 % faster than
   // 128-wide tiles at 4096 x 4096 x 8192, slower below 2048 x 2048 where a launch is a wave or less).  While a
   // batch is recording, a product leaves the batch for a pair launch of its own only from 1e11 multiply-adds
   // on: smaller ones fill the GPU better together with the rest of the batch.
   const double macs = static_cast<double>(M) * static_cast<double>(N) * static_cast<double>(K);
-  const bool pair = !wide && !split3 &&
-                    (g_wide_mode == 4 || (g_wide_mode == 3 && N >= 2048 && M >= 2048 && macs >= (g_batch_open ? 1e11 : 2e10)));
+  const bool pair = x3_pair || (!wide && !split3 &&
+                    (g_wide_mode == 4 || (g_wide_mode == 3 && N >= 2048 && M >= 2048 && macs >= (g_batch_open ? 1e11 : 2e10))));
   const int bn = wide ? 256 : 128;        // B rows of a tensor-map box
   const int bn_grid = pair ? 256 : bn;    // tile width of the grid and of the split-K scratch
   for (int s = 0; s < nseg; ++s) {
@@ -224,8 +236,8 @@ void gemm_fill_problem(GemmProblem2& P, const std::vector<at::Tensor>& a_segs,
   P.ntiles = tile_count(P.tiles_m, P.tiles_n, sym, bn_grid);
   const int kb_total = (P.K + G2_BK - 1) / G2_BK;
   int nsplit = split3 ? 1 : static_cast<int>(nsplit_req);  // the chunked sum of a split3 product is not split
-  if (nsplit <= 0 && x3wide) {
-    nsplit = split_in_waves(P.ntiles, kb_total, n_sms);
+  if (nsplit <= 0 && x3_pair) {
+    nsplit = split_in_waves(g2_pair_tiles(P), P.ntiles, kb_total, n_sms / 2);
   } else if (nsplit <= 0) {
     const int target = 2 * n_sms;
     nsplit = target / (P.ntiles > 0 ? P.ntiles : 1);
@@ -283,7 +295,7 @@ void gemm_launch_single(const GemmProblem2& P, int dev, cudaStream_t stream) {
   const int n_work = P.ntiles * P.nsplit;
   const int n_sms = g2_sm_count(dev);
   const bool wide = (P.flags & (G2F_WIDE | G2F_PAIR)) != 0;   // layout of the split-K scratch
-  if (P.flags & G2F_PAIR)
+  if (P.flags & G2F_PAIR)   // plain or bf16x3
     g2_run_pair(P, g2_pair_tiles(P) * P.nsplit, n_sms, stream);
   else if (P.flags & G2F_SPLIT3)
     g2_run_split3(P, nullptr, nullptr, n_work, n_sms, stream);
@@ -472,6 +484,13 @@ void umma_gemm(std::vector<at::Tensor> a_segs, std::vector<at::Tensor> b_segs, b
   TORCH_CHECK(!a_segs.empty(), "no operands");
   const int dev = a_segs[0].get_device();
   c10::cuda::CUDAGuard guard(dev);
+  if (x3wide && sym && !x3_syrk_takes_pairs(a_segs[0].size(a_kmajor ? 0 : 1), a_segs[0].size(a_kmajor ? 1 : 0))) {
+    // symmetric ones that do not take pairs: three segments of the plain flavour, which batches record
+    TORCH_CHECK(a_segs.size() == 2 && b_segs.size() == 2, "an x3wide product takes the (hi, lo) parts of both operands");
+    a_segs = {a_segs[0], a_segs[0], a_segs[1]};
+    b_segs = {b_segs[0], b_segs[1], b_segs[0]};
+    x3wide = false;
+  }
   GemmProblem2 P;
   gemm_fill_problem(P, a_segs, b_segs, a_kmajor, b_kmajor, C, alpha, beta, sym, out_hi, out_mid, out_lo,
                     nsplit, split3, g2_sm_count(dev), false, x3wide);

@@ -2,10 +2,19 @@
 //
 // Two CTAs of a cluster - on the two SMs of one TPC - share every tile.  A pair tile is 256 x 256:
 // CTA r of the pair stages rows [128 r, 128 r + 128) of the A tile and columns [128 r, 128 r + 128) of
-// the B tile in its own shared memory (32 KiB per 64-wide K block, a six-stage ring), the leader CTA
+// the B tile in its own shared memory (32 KiB per 64-wide K block, a ring of six stages), the leader CTA
 // (rank 0) issues one 256 x 256 x 16 MMA per K step that reads both CTAs' shared memory, and every
 // CTA ends up with its 128 rows of the 256-column accumulator in its own TMEM.  Per FLOP a pair
 // moves two thirds of the shared-memory bytes of a 128 x 256 tile and half those of a 128 x 128 tile.
+//
+// With PARTS = 2 ("bf16x3" products of (hi, lo) pairs, G2F_SPLIT2) a stage holds both parts of both operands, loaded once
+// (64 KiB per CTA and K block, a ring of three), and three part products are issued from it: (lo, hi) (hi, lo) (hi, hi).
+// 128 x 256 tiles of single CTAs take 96 KiB for the same work in a ring of two, which left the load latency exposed (1.6 us per
+// K block against 0.83 of the tensor cores); three segments of the plain flavour load both operands for each part product.
+// (lo, hi) and (hi, lo) go to an accumulator of their own, which the epilogue adds: the tensor core truncates with every addition,
+// by a last bit of the accumulator, and so only a third of the additions meet the large one.  The two accumulators of a tile
+// take all of TMEM, so a pair's next tile waits for its epilogue; most launches are one wave.
+// 1024 x 4096 between fp32 factors: 183 -> 137 us with the casts (graph replay), error against 64 bits 1.0e-5 -> 8.1e-6.
 //
 // Signals inside a pair:
 //   full[s]      lives in the leader.  The leader's producer arms it with the bytes of BOTH CTAs'
@@ -28,12 +37,15 @@
 
 namespace b200 {
 
-constexpr int G2P_STAGES = 6;
-constexpr int G2P_STAGE_BYTES = 2 * G2_A_BYTES;             // this CTA's A rows and B columns of one K block
+template <int PARTS>
+struct G2PairCfg {
+  static constexpr int STAGES = 6 / PARTS;
+  static constexpr int STAGE_BYTES = PARTS * 2 * G2_A_BYTES;   // this CTA's A rows and B columns of one K block
+};
 constexpr int G2P_EPI_WARPS = 8;
 constexpr int G2P_THREADS = 64 + 32 * G2P_EPI_WARPS;
 constexpr int G2P_TMEM_COLS = 512;                          // two 256-column accumulators
-constexpr int G2P_SMEM_BYTES = G2P_STAGES * G2P_STAGE_BYTES + 1024 + 256;
+constexpr int G2P_SMEM_BYTES = 6 * 2 * G2_A_BYTES + 1024 + 256;
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -121,14 +133,15 @@ __device__ __forceinline__ G2PairItem g2_pair_decode(const GemmProblem2& P, int 
   return it;
 }
 
+template <int PARTS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G2P_THREADS, 1)
 umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
-  constexpr int STAGES = G2P_STAGES;
+  constexpr int STAGES = G2PairCfg<PARTS>::STAGES, STAGE_BYTES = G2PairCfg<PARTS>::STAGE_BYTES;
   constexpr int BN = 256;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * G2P_STAGE_BYTES);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* acc_full = empty_bar + STAGES;
   uint64_t* acc_empty = acc_full + 2;
@@ -173,7 +186,8 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
         const G2PairItem w = g2_pair_decode(P, wi);
         const int a_mn = w.TM * 256 + static_cast<int>(rank) * G2_BM;
         const int b_mn = w.TN * 256 + static_cast<int>(rank) * G2_BM;
-        for (int seg = 0; seg < P.nseg && ok; ++seg) {
+        const int nseg = PARTS > 1 ? 1 : P.nseg;
+        for (int seg = 0; seg < nseg && ok; ++seg) {
           for (int kb = 0; kb < w.nkb; ++kb, ++it) {
             const int s = it % STAGES;
             const uint32_t ph = (it / STAGES) & 1;
@@ -182,22 +196,27 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
               ok = false;
               break;
             }
-            uint8_t* sA = smem + s * G2P_STAGE_BYTES;
-            uint8_t* sB = sA + G2_A_BYTES;
-            if (leader) mbar_expect_tx(&full_bar[s], 2 * G2P_STAGE_BYTES);
+            if (leader) mbar_expect_tx(&full_bar[s], 2 * STAGE_BYTES);
             const uint32_t bar = mapa_shared(smem_u32(&full_bar[s]), 0);
             const int k = (w.kb0 + kb) * G2_BK;
-            if (a_k) {
-              tma_load_2d_pair(sA, &P.tmA[seg], bar, k, a_mn);
-            } else {
-              tma_load_2d_pair(sA, &P.tmA[seg], bar, a_mn, k);
-              tma_load_2d_pair(sA + G2_BK * 128, &P.tmA[seg], bar, a_mn + 64, k);
-            }
-            if (b_k) {
-              tma_load_2d_pair(sB, &P.tmB[seg], bar, k, b_mn);
-            } else {
-              tma_load_2d_pair(sB, &P.tmB[seg], bar, b_mn, k);
-              tma_load_2d_pair(sB + G2_BK * 128, &P.tmB[seg], bar, b_mn + 64, k);
+#pragma unroll
+            for (int part = 0; part < PARTS; ++part) {
+              const CUtensorMap* ta = &P.tmA[PARTS > 1 ? part : seg];
+              const CUtensorMap* tb = &P.tmB[PARTS > 1 ? part : seg];
+              uint8_t* sA = smem + s * STAGE_BYTES + part * G2_A_BYTES;
+              uint8_t* sB = sA + PARTS * G2_A_BYTES;
+              if (a_k) {
+                tma_load_2d_pair(sA, ta, bar, k, a_mn);
+              } else {
+                tma_load_2d_pair(sA, ta, bar, a_mn, k);
+                tma_load_2d_pair(sA + G2_BK * 128, ta, bar, a_mn + 64, k);
+              }
+              if (b_k) {
+                tma_load_2d_pair(sB, tb, bar, k, b_mn);
+              } else {
+                tma_load_2d_pair(sB, tb, bar, b_mn, k);
+                tma_load_2d_pair(sB + G2_BK * 128, tb, bar, b_mn + 64, k);
+              }
             }
           }
         }
@@ -222,8 +241,8 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
       for (int wi = pair_id; wi < n_work && ok; wi += n_pairs) {
         const G2PairItem w = g2_pair_decode(P, wi);
         if (w.nkb <= 0) continue;
-        const uint32_t ab = ch & 1;
-        if (!mbar_wait(&acc_empty[ab], ((ch >> 1) & 1) ^ 1)) {
+        const uint32_t ab = PARTS > 1 ? 0 : ch & 1;
+        if (!mbar_wait(&acc_empty[ab], (PARTS > 1 ? ch & 1 : (ch >> 1) & 1) ^ 1)) {
           set_error(P.status, ERR_WAIT_ACC);
           ok = false;
           break;
@@ -231,7 +250,8 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
         tc_fence_after_sync();
         const uint32_t tacc = tmem_base + ab * BN;
         uint32_t first = 1;
-        for (int seg = 0; seg < P.nseg && ok; ++seg) {
+        const int nseg = PARTS > 1 ? 1 : P.nseg;
+        for (int seg = 0; seg < nseg && ok; ++seg) {
           for (int kb = 0; kb < w.nkb; ++kb, ++it) {
             const int s = it % STAGES;
             if (!mbar_wait(&full_bar[s], (it / STAGES) & 1)) {
@@ -240,16 +260,27 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
               break;
             }
             tc_fence_after_sync();
-            const uint32_t aA = smem_u32(smem + s * G2P_STAGE_BYTES);
-            const uint32_t aB = aA + G2_A_BYTES;
+            constexpr int NPROD = PARTS > 1 ? 3 : 1;
+            constexpr int PART_A[3] = {PARTS - 1, 0, 0};   // (lo, hi) (hi, lo) (hi, hi)
+            constexpr int PART_B[3] = {0, PARTS - 1, 0};
 #pragma unroll
-            for (int k = 0; k < G2_BK / 16; ++k) {
-              const uint64_t da = a_k ? make_smem_desc_sw128(aA + k * 32, 16, 1024)
-                                      : make_smem_desc_sw128(aA + k * 16 * 128, G2_BK * 128, 1024);
-              const uint64_t db = b_k ? make_smem_desc_sw128(aB + k * 32, 16, 1024)
-                                      : make_smem_desc_sw128(aB + k * 16 * 128, G2_BK * 128, 1024);
-              umma_bf16_pair(tacc, da, db, idesc, first ? 0u : 1u);
-              first = 0;
+            for (int pr = 0; pr < NPROD; ++pr) {
+              const uint32_t aA = smem_u32(smem + s * STAGE_BYTES) + PART_A[pr] * G2_A_BYTES;
+              const uint32_t aB = smem_u32(smem + s * STAGE_BYTES) + (PARTS + PART_B[pr]) * G2_A_BYTES;
+#pragma unroll
+              for (int k = 0; k < G2_BK / 16; ++k) {
+                const uint64_t da = a_k ? make_smem_desc_sw128(aA + k * 32, 16, 1024)
+                                        : make_smem_desc_sw128(aA + k * 16 * 128, G2_BK * 128, 1024);
+                const uint64_t db = b_k ? make_smem_desc_sw128(aB + k * 32, 16, 1024)
+                                        : make_smem_desc_sw128(aB + k * 16 * 128, G2_BK * 128, 1024);
+                if (PARTS > 1) {
+                  const bool begins = kb == 0 && k == 0 && pr != 1;
+                  umma_bf16_pair(tacc + (pr < 2 ? BN : 0), da, db, idesc, begins ? 0u : 1u);
+                } else {
+                  umma_bf16_pair(tacc, da, db, idesc, first ? 0u : 1u);
+                  first = 0;
+                }
+              }
             }
             umma_commit_pair(&empty_bar[s]);
           }
@@ -280,9 +311,9 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
       const int tile_id = sym ? w.TM * (w.TM + 1) + static_cast<int>(rank) * (w.TM + 1) + w.TN : tm * E.full->tiles_n + w.TN;
       const int gr = c_row + row;
       const bool have = w.nkb > 0;
-      const uint32_t ab = ch & 1;
+      const uint32_t ab = PARTS > 1 ? 0 : ch & 1;
       if (have) {
-        ok = mbar_wait(&acc_full[ab], (ch >> 1) & 1);
+        ok = mbar_wait(&acc_full[ab], PARTS > 1 ? ch & 1 : (ch >> 1) & 1);
         if (!ok) set_error(P.status, ERR_WAIT_ACC);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
@@ -301,6 +332,16 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
           for (int j = 0; j < 32; ++j) {
             v[j] = __uint_as_float(r0[j]);
             v[32 + j] = __uint_as_float(r1[j]);
+          }
+          if constexpr (PARTS > 1) {   // the accumulator of the small part products
+            tmem_ld_32x32(tmem_base + lane_addr + BN + col0, r0);
+            tmem_ld_32x32(tmem_base + lane_addr + BN + col0 + 32, r1);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              v[j] += __uint_as_float(r0[j]);
+              v[32 + j] += __uint_as_float(r1[j]);
+            }
           }
           if (pass == PASSES - 1) {  // this warp's share is in registers: hand the accumulator back to the leader
             tc_fence_before_sync();

@@ -187,6 +187,12 @@ def matmul_fp32_tc(a_parts, b_parts, a_kmajor: bool, b_kmajor: bool, out=None, a
     return out
 
 
+def _syrk(hi, lo, out, scale, beta):
+    """``out = scale * x^T x + beta * out`` of staged samples; with a ``lo`` part three part products."""
+    parts = [hi] if lo is None else [hi, lo]
+    extension().umma_gemm(parts, parts, False, False, out, float(scale), float(beta), True, None, None, 0, None, False, lo is not None)
+
+
 def gram(x: torch.Tensor, scale: float = 1.0, out: Optional[torch.Tensor] = None,
          beta: float = 0.0) -> torch.Tensor:
     """``scale * x^T x (+ beta * out)`` for a sample matrix x [rows, n] -> [n, n].
@@ -211,9 +217,7 @@ def gram(x: torch.Tensor, scale: float = 1.0, out: Optional[torch.Tensor] = None
     if out is None:
         out = torch.empty(n, n, device=x.device, dtype=torch.float32)
         beta = 0.0
-    a_segs, b_segs = _segments(hi, lo, hi, lo)
-    extension().umma_gemm(a_segs, b_segs, False, False, out, float(scale), float(beta), True,
-                          None, None, 0)
+    _syrk(hi, lo, out, scale, beta)
     return out
 
 
@@ -466,8 +470,7 @@ def conv_patch_gram(x: torch.Tensor, conv: torch.nn.Conv2d, scale: float = 1.0,
     if out is None:
         out = torch.empty(ncol, ncol, device=x.device, dtype=torch.float32)
         beta = 0.0
-    extension().umma_gemm([hi, hi, lo], [hi, lo, hi], False, False, out, float(scale), float(beta),
-                          True, None, None, 0)
+    _syrk(hi, lo, out, scale, beta)
     return out
 
 

@@ -191,6 +191,47 @@ def test_inverse_at_the_edges_of_the_diagonal_stages(n):
     ops.check_status()
 
 
+@pytest.mark.parametrize('m,n', [(129, 129), (256, 300), (257, 640), (1000, 520)])
+@pytest.mark.parametrize('k', [2, 64, 200, 1600])
+def test_bf16x3_products_on_pairs(m, n, k):
+    """Odd and even counts of 128-row tiles, ragged edges, one K block, several K ranges, operands of either order, hi and lo images."""
+    a, b = torch.randn(k, m, device=DEV, generator=_gen(1)), torch.randn(k, n, device=DEV, generator=_gen(2))
+    (ah, al), (bh, bl) = ops._stage_bf16(a, True), ops._stage_bf16(b, True)
+    (akh, akl), (bkh, bkl) = ops._stage_bf16(a.T.contiguous(), True), ops._stage_bf16(b.T.contiguous(), True)
+    want = a.double().T @ b.double()
+    # 2^-16 of each product from the bf16 pairs, fp32 sums
+    bound = (a.abs().double().T @ b.abs().double()) * (2.0 ** -15 + k * 2.0 ** -24) + 1e-6
+    for (p, pk), (q, qk) in [(((ah, al), False), ((bh, bl), False)), (((akh, akl), True), ((bkh, bkl), True))]:
+        for nsplit in (0, 1, 3):
+            out = torch.full((m, n), float('nan'), device=DEV)
+            ops.extension().umma_gemm(list(p), list(q), pk, qk, out, 1.0, 0.0, False, None, None, nsplit, None, False, True)
+            assert ((out.double() - want).abs() <= bound).all()
+            hi = torch.empty(m, (n + 7) // 8 * 8, device=DEV, dtype=torch.bfloat16)
+            lo = torch.empty_like(hi)
+            ops.extension().umma_gemm(list(p), list(q), pk, qk, None, 1.0, 0.0, False, hi, lo, nsplit, None, False, True)
+            assert ((hi[:, :n].double() + lo[:, :n].double() - want).abs() <= bound + 2.0 ** -15 * want.abs()).all()
+    ops.check_status()
+
+
+@pytest.mark.parametrize('rows', [1535, 1536, 4001])
+@pytest.mark.parametrize('n', [128, 200, 256, 385, 520, 1000])
+def test_fp32_factor_on_pairs(rows, n):
+    """Both sides of the rule that takes a symmetric bf16x3 product to CTA pairs, also while a batch is recorded."""
+    x = torch.randn(rows, n, device=DEV, generator=_gen(5))
+    before = torch.eye(n, device=DEV)
+    want = x.double().T @ x.double() / rows + 0.5 * before.double()
+    bound = 2.0 ** -15 + 3 * rows * 2.0 ** -24 + 1e-6
+    out = before.clone()
+    ops.gram(x, scale=1 / rows, out=out, beta=0.5)
+    assert (out.double() - want).abs().max() <= bound * want.abs().max() and torch.equal(out, out.T)
+    out = before.clone()
+    ops.extension().gemm_batch_begin()
+    ops.gram(x, scale=1 / rows, out=out, beta=0.5)
+    ops.extension().gemm_batch_end()
+    assert (out.double() - want).abs().max() <= bound * want.abs().max() and torch.equal(out, out.T)
+    ops.check_status()
+
+
 @pytest.mark.parametrize('kernel,padding', [((3, 3), (1, 1)), ((3, 3), (0, 0)), ((5, 5), (2, 2)), ((4, 3), (1, 2)), ((2, 2), (1, 0))])
 @pytest.mark.parametrize('shape', [(1, 64, 7, 7), (3, 24, 9, 6), (70, 65, 8, 8), (2, 192, 12, 13), (5, 128, 10, 10)])
 @pytest.mark.parametrize('dtype,layout', [(torch.float32, 'nchw'), (torch.bfloat16, 'nhwc'), (torch.float16, 'view')])
