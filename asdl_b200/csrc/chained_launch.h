@@ -1,0 +1,33 @@
+// Kernels that follow each other on a stream with a programmatic dependency: the next one is brought onto the SMs while the one
+// before it finishes, and waits there before it touches memory, so the few microseconds between two kernels overlap.
+//
+// Every kernel launched this way calls chain_wait() before its first access to global memory, reads and writes alike.  The wait
+// ends when the kernel before it has finished and its writes are visible; since that one waited in the same way, everything
+// before it has finished too.  chain_next() lets the next kernel come as soon as all CTAs of this one have called it.
+// A kernel that is launched plainly behind a chain waits for its end as usual; a captured chain becomes programmatic edges.
+#pragma once
+#include <utility>
+
+#include "host_utils.h"
+
+namespace b200 {
+
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... Params, typename... Args>
+void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute = {};
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  B200_CUDA_CHECK(cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...));
+}
+
+}  // namespace b200

@@ -328,29 +328,9 @@ def kron_apply(left: torch.Tensor, mid: torch.Tensor, right: torch.Tensor) -> to
     if not cuda_kernels_enabled(left, mid, right) or mid.numel() == 0:
         dt = mid.dtype
         return left.to(dt) @ mid @ right.to(dt)
-    ext = extension()
-    m, n = mid.shape
     x3 = _use_x3(torch.float32) if (left.dtype == torch.float32 or mid.dtype == torch.float32) \
         else _use_x3(mid.dtype)
-    # A factor stored column by column is not copied: its transpose is row-major, and the GEMM takes that as the K-major
-    # operand.  Both orders of storage give the same product of the same entries, bit for bit.
-    l_col, r_col = (t.stride(1) != 1 and t.stride(0) == 1 for t in (left, right))
-    l_hi, l_lo = _stage_bf16(left.t() if l_col else left, x3)
-    g_hi, g_lo = _stage_bf16(mid, x3)
-    r_hi, r_lo = _stage_bf16(right.t() if r_col else right, x3)
-    ld = _round_up(max(n, 8), 8)
-    t_hi = torch.empty(m, ld, device=mid.device, dtype=torch.bfloat16)
-    t_lo = torch.empty_like(t_hi) if x3 else None
-    # T = left^T-as-stored . mid : A operand = left ([k=m, m] row-major, symmetric), B = mid [k=m, n]
-    out = torch.empty(m, n, device=mid.device, dtype=torch.float32)
-    if x3:   # (hi, lo) parts, loaded once per K block by the x3wide flavour
-        ext.umma_gemm([l_hi, l_lo], [g_hi, g_lo], l_col, False, None, 1.0, 0.0, False, t_hi, t_lo, 0, None, False, True)
-        ext.umma_gemm([t_hi[:, :n], t_lo[:, :n]], [r_hi, r_lo], True, r_col, out, 1.0, 0.0, False, None, None, 0,
-                      None, False, True)
-        return out.to(mid.dtype) if mid.dtype != torch.float32 else out
-    ext.umma_gemm([l_hi], [g_hi], l_col, False, None, 1.0, 0.0, False, t_hi, t_lo, 0)
-    # Y = T . right : A operand = T ([m, k=n] K-major), B = right ([k=n, n] row-major, symmetric)
-    ext.umma_gemm([t_hi[:, :n]], [r_hi], True, r_col, out, 1.0, 0.0, False, None, None, 0)
+    out = extension().kron_staged(left, mid, right, x3)
     return out.to(mid.dtype) if mid.dtype != torch.float32 else out
 
 
