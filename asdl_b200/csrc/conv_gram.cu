@@ -29,6 +29,7 @@
 // what is taken off is not finite either: more entries are affected.
 #include <cstring>
 
+#include "chained_launch.h"
 #include "gemm2_host.h"
 
 namespace b200 {
@@ -103,6 +104,7 @@ cg_stage_kernel(const T* __restrict__ x, const __grid_constant__ StageShape s, _
                 __nv_bfloat16* __restrict__ lo, int ld) {
   __shared__ float tile[64][65];   // [channel][row]
   __shared__ long long base[64];
+  chain_next();
   const int r0 = blockIdx.x * 64, c0 = blockIdx.y * 64;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x < 64) {
@@ -224,6 +226,7 @@ cg_product_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid_consta
     dst = g.nsplit > 1 ? partials + static_cast<size_t>(blockIdx.x) * CG_TILE : tiles + static_cast<size_t>(tile) * CG_TILE;
   } else {
     const int item = blockIdx.x - n_main, per = g.tc * g.tc, p = item / per, t = item - p * per;
+    if (tab.memory != nullptr) chain_wait();   // the tables were written by a kernel before
     const Correction q = tab.memory != nullptr ? Correction{tab.memory[2 * p], tab.memory[2 * p + 1]} : Correction{tab.words[2 * p], tab.words[2 * p + 1]};
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
@@ -253,6 +256,8 @@ cg_product_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid_consta
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  chain_next();
+  chain_wait();   // for the staged rows, and for tables in memory
 
   if (warp == 0) {
     const bool lead = elect_one();
@@ -351,6 +356,8 @@ cg_product_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid_consta
 // Sums the K ranges of the main tiles, in order.  grid: (16, tiles), a thread has four values and eight ranges in flight.
 __global__ void __launch_bounds__(256)
 cg_reduce_kernel(const float4* __restrict__ partials, float4* __restrict__ tiles, int nsplit) {
+  chain_next();
+  chain_wait();
   const int at = blockIdx.x * 256 + threadIdx.x;
   const float4* from = partials + static_cast<size_t>(blockIdx.y) * nsplit * (CG_TILE / 4) + at;
   float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -388,6 +395,7 @@ cg_assemble_kernel(const float* __restrict__ tiles, const __grid_constant__ Asse
                    float* __restrict__ out, long long ldc) {
   extern __shared__ int tab[];
   __shared__ float patch[32][33];
+  chain_wait();
   const int pairs = a.taps * (a.taps + 1) / 2, words = 3 * a.n_products + pairs + 1 + (a.n_terms + 1) / 2;
   for (int i = threadIdx.x; i < words; i += 256)
     tab[i] = tables.memory != nullptr ? tables.memory[tables.corr_words + i] : tables.words[tables.corr_words + i];
@@ -445,6 +453,7 @@ __global__ void __launch_bounds__(256)
 cg_assemble_blocks_kernel(const float* __restrict__ tiles, const __grid_constant__ AssembleShape a, const __grid_constant__ CgTables tables,
                           float* __restrict__ out, long long ldc, bool vec) {
   __shared__ float patch[64][65];
+  chain_wait();
   const int* tab = tables.memory != nullptr ? tables.memory + tables.corr_words : tables.words + tables.corr_words;
   const ProductAt* products = reinterpret_cast<const ProductAt*>(tab);
   const int pairs = a.taps * (a.taps + 1) / 2;
@@ -762,7 +771,7 @@ bool conv_gram(at::Tensor x, at::Tensor out, int64_t kh, int64_t kw, int64_t ph,
   float* dp = g.nsplit > 1 ? partials.data_ptr<float>() : nullptr;
   auto run = [&](auto kernel, int smem) {
     B200_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    kernel<<<items, 192, smem, stream>>>(tm_hi, tm_lo, g, tables, dp, tiles.data_ptr<float>(), status);
+    launch_chained(kernel, dim3(items), dim3(192), smem, stream, tm_hi, tm_lo, g, tables, dp, tiles.data_ptr<float>(), status);
   };
   if (x3)
     run(cg_product_kernel<2>, CgCfg<2>::SMEM_BYTES);
@@ -771,8 +780,8 @@ bool conv_gram(at::Tensor x, at::Tensor out, int64_t kh, int64_t kw, int64_t ph,
   B200_CUDA_CHECK(cudaGetLastError());
   count_launch();
   if (g.nsplit > 1) {
-    cg_reduce_kernel<<<dim3(CG_TILE / 4 / 256, main_tiles), 256, 0, stream>>>(reinterpret_cast<const float4*>(dp),
-                                                                             reinterpret_cast<float4*>(tiles.data_ptr<float>()), g.nsplit);
+    launch_chained(cg_reduce_kernel, dim3(CG_TILE / 4 / 256, main_tiles), dim3(256), 0, stream, reinterpret_cast<const float4*>(dp),
+                   reinterpret_cast<float4*>(tiles.data_ptr<float>()), g.nsplit);
     B200_CUDA_CHECK(cudaGetLastError());
     count_launch();
   }
@@ -789,10 +798,10 @@ bool conv_gram(at::Tensor x, at::Tensor out, int64_t kh, int64_t kw, int64_t ph,
   if (khwc && c % 64 == 0) {
     const int nb = a.n / 64;
     const bool vec = out.stride(0) % 4 == 0 && (reinterpret_cast<uintptr_t>(result) & 15) == 0;
-    cg_assemble_blocks_kernel<<<nb * (nb + 1) / 2, 256, 0, stream>>>(tiles.data_ptr<float>(), a, tables, result, out.stride(0), vec);
+    launch_chained(cg_assemble_blocks_kernel, dim3(nb * (nb + 1) / 2), dim3(256), 0, stream, tiles.data_ptr<float>(), a, tables, result, out.stride(0), vec);
   } else {
     const int nb = (a.n + 31) / 32, tab_bytes = static_cast<int>(host.size() - asm_at) * 4;
-    cg_assemble_kernel<<<nb * (nb + 1) / 2, 256, tab_bytes, stream>>>(tiles.data_ptr<float>(), a, tables, result, out.stride(0));
+    launch_chained(cg_assemble_kernel, dim3(nb * (nb + 1) / 2), dim3(256), tab_bytes, stream, tiles.data_ptr<float>(), a, tables, result, out.stride(0));
   }
   B200_CUDA_CHECK(cudaGetLastError());
   count_launch();

@@ -93,9 +93,9 @@ static void launch_reduce(int tiles, const GemmProblem2& single, const GemmProbl
                           const int* prefix, int n_probs, cudaStream_t stream) {
   // 50000 x 64 bf16, one tile of 32 splits: 21.6 -> 18.6 us with the product; 4096 x 512, ten tiles of 8 splits: 13.4 -> 14.9
   if (tiles * g2_reduce_patches<BN, 16>() <= 148)
-    splitk_reduce2_kernel<BN, 16><<<dim3(tiles, g2_reduce_patches<BN, 16>()), 256, 0, stream>>>(single, probs, work, prefix, n_probs);
+    launch_chained(splitk_reduce2_kernel<BN, 16>, dim3(tiles, g2_reduce_patches<BN, 16>()), dim3(256), 0, stream, single, probs, work, prefix, n_probs);
   else
-    splitk_reduce2_kernel<BN, 32><<<dim3(tiles, g2_reduce_patches<BN, 32>()), 256, 0, stream>>>(single, probs, work, prefix, n_probs);
+    launch_chained(splitk_reduce2_kernel<BN, 32>, dim3(tiles, g2_reduce_patches<BN, 32>()), dim3(256), 0, stream, single, probs, work, prefix, n_probs);
   B200_CUDA_CHECK(cudaGetLastError());
   count_launch();
 }

@@ -36,6 +36,7 @@
 // time; on expiry the status word is set and the CTA unwinds.  TMA loads only ever read this GPU's
 // memory; peer memory is written with per-thread stores from the epilogue.
 #pragma once
+#include "chained_launch.h"
 #include "sm100_ptx.cuh"
 
 namespace b200 {
@@ -843,6 +844,7 @@ template <int BN, int ROWS>
 __global__ void __launch_bounds__(256)
 splitk_reduce2_kernel(const __grid_constant__ GemmProblem2 single, const GemmProblem2* __restrict__ probs,
                       const GemmWork2* __restrict__ work, const int* __restrict__ tile_prefix, int n_probs) {
+  chain_wait();   // for the products
   constexpr int R = ROWS / 16, SPLITS = 8 / R;   // rows of a thread, splits in flight
   __shared__ float tile[ROWS][G2_RED_COLS + 1];
   GemmWork2 w;
