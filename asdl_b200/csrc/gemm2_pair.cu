@@ -24,7 +24,7 @@ static void run_pair(const GemmProblem2& single, int n_work, int n_sms, cudaStre
     attr_set = true;
   }
   const int pairs = std::max(1, std::min(n_work, n_sms / 2));
-  umma_gemm2_pair_kernel<PARTS><<<2 * pairs, G2P_THREADS, G2P_SMEM_BYTES, stream>>>(single, n_work);
+  launch_chained(umma_gemm2_pair_kernel<PARTS>, dim3(2 * pairs), dim3(G2P_THREADS), G2P_SMEM_BYTES, stream, single, n_work);
   B200_CUDA_CHECK(cudaGetLastError());
   count_launch();
 }

@@ -3,6 +3,7 @@
 //                      ("lo") so that hi+lo carries ~16 mantissa bits.
 //   * im2col_bf16    : conv input (any strides: NCHW or channels_last) -> patch matrix
 //                      [N*Ho*Wo, ld] bf16, columns ordered (kh, kw, c) or (c, kh, kw).
+#include "chained_launch.h"
 #include "host_utils.h"
 #include "row_walk.h"
 #include <cuda_bf16.h>
@@ -31,6 +32,7 @@ __global__ void __launch_bounds__(256)
 cast_parts_kernel(const T* __restrict__ src, long long lds, float scale, __nv_bfloat16* __restrict__ p0,
                   __nv_bfloat16* __restrict__ p1, __nv_bfloat16* __restrict__ p2, long long ldo, long long rows, int n,
                   int groups, int lanes) {
+  chain_next();
   const int lane = threadIdx.x / groups;
   const long long c0 = (static_cast<long long>(blockIdx.y) * groups + threadIdx.x % groups) * 8;
   if (lane >= lanes || c0 >= ldo) return;

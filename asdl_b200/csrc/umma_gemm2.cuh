@@ -470,9 +470,6 @@ umma_gemm2_kernel(const __grid_constant__ GemmProblem2 single, const GemmProblem
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  if (prefix_g != nullptr)
-    for (int i = threadIdx.x; i <= n_probs && i <= G2_MAX_BATCH; i += blockDim.x) prefix[i] = prefix_g[i];
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
@@ -488,6 +485,9 @@ umma_gemm2_kernel(const __grid_constant__ GemmProblem2 single, const GemmProblem
     tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
     tmem_relinquish();
   }
+  chain_wait();   // operands, tables and outputs: nothing is touched before
+  if (prefix_g != nullptr)
+    for (int i = threadIdx.x; i <= n_probs && i <= G2_MAX_BATCH; i += blockDim.x) prefix[i] = prefix_g[i];
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();

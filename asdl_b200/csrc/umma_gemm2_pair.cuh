@@ -170,6 +170,7 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
     tmem_alloc_pair(tmem_slot, G2P_TMEM_COLS);
     tmem_relinquish_pair();
   }
+  chain_wait();   // operands and outputs: nothing is touched before
   tc_fence_before_sync();
   cluster_sync_all();   // barriers of both CTAs are initialised before anything arrives on them
   tc_fence_after_sync();
