@@ -25,7 +25,7 @@
 // operand traffic of the ring, 96 KiB per K block of 1536 tensor cycles.  The former version ran the same arithmetic
 // right-looking in 28 (six factors up to 784) to 121 (the 107 factors of ResNet-50) dependent launches: every K = 128 update
 // read and wrote the fp32 matrix, each lane a row of its own, and every launch drained before the next began.
-// Six factors 784, 4 x 512, 10: 600 -> 263 us; ResNet-50's 107 factors: 8.08 -> 3.63 ms.
+// Six factors 784, 4 x 512, 10: 597 -> 251 us; ResNet-50's 107 factors: 8.04 -> 3.52 ms.
 //
 // Tables, task lists and the bf16 split buffers depend only on the addresses and sizes of the matrices; they are built once
 // and cached (prepared_cache.h), so a repeated call (the K-FAC state) issues no host-to-device copy and can be captured in a
@@ -91,7 +91,7 @@ __host__ __device__ inline int task_blocks(int kind, int i, int j, int n) {
 // Every entry sees the same roundings in the same order as a column-by-column elimination, and gives the same bits.  Two things
 // bound it: the chain of pivots (80 clocks each), and the number of instructions that a single warp per scheduler issues:
 // products are taken in pairs (fma.f32x2), and loops over groups of eight columns are not unrolled.  With each column applied at
-// once to all behind it, in single products, the block took 49 000 clocks, 27 800 of them to factor; now 44 000.
+// once to all behind it, in single products, the block took 49 000 clocks, 27 800 of them to factor; now 41 000.
 constexpr int DG_SP = TB + 1;   // pitch of S: lanes on consecutive rows of a column, or on consecutive columns
 constexpr int DG_PP = TB + 4;   // pitches of P and of the factored block: 16-byte reads
 constexpr int DG_LP = 64;       // the entries from 32 on are zeros: what shifted registers past the block are updated with
