@@ -18,8 +18,9 @@ namespace b200 {
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// `chained` false: an ordinary launch of the same kernel, whose wait then ends at once.
 template <typename... Params, typename... Args>
-void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+void launch_behind(bool chained, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t config = {};
   config.gridDim = grid;
   config.blockDim = block;
@@ -29,8 +30,13 @@ void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t sme
   attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute.val.programmaticStreamSerializationAllowed = 1;
   config.attrs = &attribute;
-  config.numAttrs = 1;
+  config.numAttrs = chained ? 1 : 0;
   B200_CUDA_CHECK(cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...));
+}
+
+template <typename... Params, typename... Args>
+void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  launch_behind(true, kernel, grid, block, smem, stream, std::forward<Args>(args)...);
 }
 
 }  // namespace b200

@@ -19,6 +19,11 @@ void g2_encode_operand(CUtensorMap* tm, const void* base, int64_t mn, int64_t k,
 // SM count of a device (cached).
 int g2_sm_count(int dev);
 
+// A problem passed by value is launched behind a chain (chained_launch.h): its tensor maps are kernel parameters.  Problems in a
+// table are not: the kernel reads their tensor maps from memory that a kernel or copy just before may have written, in place of
+// an earlier table, and griddepcontrol.wait is not specified to order that proxy as the boundary of two kernels does.
+inline bool g2_may_chain(const GemmProblem2* table) { return table == nullptr; }
+
 // One launch of a kernel flavour: either `single` (work == nullptr; its tiles are decoded from the
 // work index), a device-resident problem table with a work list, or such a table with an item
 // prefix per problem (`prefix`, `n_probs` <= G2_MAX_BATCH; `work` null).  Defined in gemm2_<flavour>.cu.

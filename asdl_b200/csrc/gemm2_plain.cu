@@ -19,7 +19,7 @@ void g2_run_plain(const GemmProblem2& single, const GemmProblem2* probs, const G
     attr_set = true;
   }
   const int grid = std::min(n_work, 2 * n_sms);
-  launch_chained(umma_gemm2_kernel<128, 4, 2, 1>, dim3(grid), dim3(G2Plain::THREADS), G2Plain::SMEM_BYTES, stream, single, probs, work, n_work, prefix, n_probs);
+  launch_behind(g2_may_chain(probs), umma_gemm2_kernel<128, 4, 2, 1>, dim3(grid), dim3(G2Plain::THREADS), G2Plain::SMEM_BYTES, stream, single, probs, work, n_work, prefix, n_probs);
   B200_CUDA_CHECK(cudaGetLastError());
   count_launch();
 }

@@ -19,7 +19,7 @@ void g2_run_split3(const GemmProblem2& single, const GemmProblem2* probs, const 
     attr_set = true;
   }
   const int grid = std::min(n_work, 1 * n_sms);
-  launch_chained(umma_gemm2_kernel<128, 8, 1, 3>, dim3(grid), dim3(G2Split3::THREADS), G2Split3::SMEM_BYTES, stream, single, probs, work, n_work, prefix, n_probs);
+  launch_behind(g2_may_chain(probs), umma_gemm2_kernel<128, 8, 1, 3>, dim3(grid), dim3(G2Split3::THREADS), G2Split3::SMEM_BYTES, stream, single, probs, work, n_work, prefix, n_probs);
   B200_CUDA_CHECK(cudaGetLastError());
   count_launch();
 }

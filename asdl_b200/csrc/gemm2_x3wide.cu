@@ -19,7 +19,7 @@ void g2_run_x3wide(const GemmProblem2& single, const GemmProblem2* probs, const 
     attr_set = true;
   }
   const int grid = std::min(n_work, n_sms);
-  launch_chained(umma_gemm2_kernel<256, 8, 1, 2>, dim3(grid), dim3(G2X3Wide::THREADS), G2X3Wide::SMEM_BYTES, stream, single, probs, work, n_work, prefix, n_probs);
+  launch_behind(g2_may_chain(probs), umma_gemm2_kernel<256, 8, 1, 2>, dim3(grid), dim3(G2X3Wide::THREADS), G2X3Wide::SMEM_BYTES, stream, single, probs, work, n_work, prefix, n_probs);
   B200_CUDA_CHECK(cudaGetLastError());
   count_launch();
 }

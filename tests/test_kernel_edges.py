@@ -232,6 +232,24 @@ def test_fp32_factor_on_pairs(rows, n):
     ops.check_status()
 
 
+def test_batches_whose_tables_take_each_others_place(ext):
+    """Problem tables of one batch after another lie at the same address and hold other tensor maps."""
+    for turn in range(6):
+        n = 64 + 72 * turn
+        xs = [torch.randn(300 + 50 * i, n, device=DEV, generator=_gen(10 * turn + i)).to(torch.bfloat16) for i in range(8)]
+        outs = [torch.empty(n, n, device=DEV) for _ in xs]
+        ext.gemm_batch_begin()
+        for x, out in zip(xs, outs):
+            ops.gram(x, out=out)
+        ext.gemm_batch_end()
+        del x
+        for x, out in zip(xs, outs):
+            want = x.double().T @ x.double()
+            # products of bf16 values are exact in fp32; the sums are not
+            assert (out.double() - want).abs().max() <= x.shape[0] * 2.0 ** -24 * want.abs().max()
+    ops.check_status()
+
+
 @pytest.mark.parametrize('kernel,padding', [((3, 3), (1, 1)), ((3, 3), (0, 0)), ((5, 5), (2, 2)), ((4, 3), (1, 2)), ((2, 2), (1, 0))])
 @pytest.mark.parametrize('shape', [(1, 64, 7, 7), (3, 24, 9, 6), (70, 65, 8, 8), (2, 192, 12, 13), (5, 128, 10, 10)])
 @pytest.mark.parametrize('dtype,layout', [(torch.float32, 'nchw'), (torch.bfloat16, 'nhwc'), (torch.float16, 'view')])
