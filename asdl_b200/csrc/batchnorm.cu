@@ -126,7 +126,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 // One warp per channel: the lanes stride over the splits, combine in double precision.
 __global__ void __launch_bounds__(256)
-bn_fwd_finalize(const float* __restrict__ part, const float* __restrict__ weight,
+bn_fwd_finalize(const float* part, const float* __restrict__ weight,
                 const float* __restrict__ bias, float* __restrict__ running_mean,
                 float* __restrict__ running_var, float* __restrict__ mean_out,
                 float* __restrict__ invstd_out, float* __restrict__ coef, long long* __restrict__ tracked,
@@ -177,7 +177,7 @@ constexpr int APPLY_ROWS_PLAIN = 4, APPLY_ROWS_RES = 3;   // fit 64 registers: f
 template <bool RES, bool RELU>
 __global__ void __launch_bounds__(256, 4)
 bn_apply(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
-         const float* __restrict__ scale, const float* __restrict__ shift, __nv_bfloat16* __restrict__ y,
+         const float* scale, const float* shift, __nv_bfloat16* __restrict__ y,
          long long rows, int channels, int groups, int lanes) {
   chain_wait();
   constexpr int APPLY_ROWS = RES ? APPLY_ROWS_RES : APPLY_ROWS_PLAIN;
@@ -232,9 +232,7 @@ constexpr int DX_ROWS = 2;
 template <int MASK, bool DRES>
 __global__ void __launch_bounds__(256, 3)
 bn_dx(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-      const __nv_bfloat16* __restrict__ y, const float* __restrict__ scale, const float* __restrict__ shift,
-      const float* __restrict__ k_dy, const float* __restrict__ k_x,
-      const float* __restrict__ k_const, __nv_bfloat16* __restrict__ dx, __nv_bfloat16* __restrict__ dres,
+      const __nv_bfloat16* __restrict__ y, const float* scale, const float* shift, const float* k_dy, const float* k_x, const float* k_const, __nv_bfloat16* __restrict__ dx, __nv_bfloat16* __restrict__ dres,
       long long rows, int channels, int groups, int lanes) {
   chain_wait();
   const int lane = threadIdx.x / groups;
@@ -376,7 +374,7 @@ bn_bwd_sums(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict
 //    = dy * k_dy + x * k_x + k_const  with
 //   k_dy = w*invstd, k_x = -k_dy * invstd * m2, k_const = -k_dy * (m1 - mean * invstd * m2)
 __global__ void __launch_bounds__(256)
-bn_bwd_finalize(const float* __restrict__ part, const float* __restrict__ weight, const float* __restrict__ bias,
+bn_bwd_finalize(const float* part, const float* __restrict__ weight, const float* __restrict__ bias,
                 const float* __restrict__ mean, const float* __restrict__ invstd,
                 float* __restrict__ dweight, float* __restrict__ dbias,
                 float* __restrict__ coef, int channels, int splits, long long rows) {

@@ -3,7 +3,9 @@
 //
 // Every kernel launched this way calls chain_wait() before its first access to global memory, reads and writes alike.  The wait
 // ends when the kernel before it has finished and its writes are visible; since that one waited in the same way, everything
-// before it has finished too.  chain_next() lets the next kernel come as soon as all CTAs of this one have called it.
+// before it has finished too.  What a kernel of the chain has written is read by ordinary loads, not through __ldg or a
+// const __restrict__ parameter: the read-only path is for data that nobody writes while the kernel is resident, and the compiler
+// may move such loads ahead of the wait.  __ldcg takes its pointer from after_wait().  chain_next() lets the next kernel come as soon as all CTAs of this one have called it.
 // With the split-K reduction and the kernels of a convolution factor chained: 8192 x 1024 bf16 samples 27.5 -> 24.6 us,
 // 32 x 256 x 14 x 14 bf16 45.1 -> 39.8, 128 x 64 x 32 x 32 fp32 84.7 -> 77.8; with the GEMMs behind their casts: 24.6 -> 22.7 for the
 // first, 12608 x 768 fp32 samples 48.9 -> 47.5, 1024 x 4096 between fp32 factors 159 -> 155.
@@ -17,6 +19,13 @@ namespace b200 {
 
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// The same pointer, for loads that the compiler would move ahead of chain_wait().
+template <typename T>
+__device__ __forceinline__ T* after_wait(T* p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
 
 // `chained` false: an ordinary launch of the same kernel, whose wait then ends at once.
 template <typename... Params, typename... Args>

@@ -355,7 +355,7 @@ cg_product_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid_consta
 
 // Sums the K ranges of the main tiles, in order.  grid: (16, tiles), a thread has four values and eight ranges in flight.
 __global__ void __launch_bounds__(256)
-cg_reduce_kernel(const float4* __restrict__ partials, float4* __restrict__ tiles, int nsplit) {
+cg_reduce_kernel(const float4* partials, float4* tiles, int nsplit) {
   chain_next();
   chain_wait();
   const int at = blockIdx.x * 256 + threadIdx.x;
@@ -365,7 +365,7 @@ cg_reduce_kernel(const float4* __restrict__ partials, float4* __restrict__ tiles
     float4 v[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u)
-      v[u] = s + u < nsplit ? __ldcs(from + static_cast<size_t>(s + u) * (CG_TILE / 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[u] = s + u < nsplit ? from[static_cast<size_t>(s + u) * (CG_TILE / 4)] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       sum.x += v[u].x;
@@ -391,8 +391,8 @@ struct AssembleShape {
 // 32 x 32 patches on or below the diagonal; tables: [ProductAt x products][first term of tap pair t (t + 1) / 2 + t', and one
 // past the last][terms: product, + 0x8000 for those that are taken off].
 __global__ void __launch_bounds__(256)
-cg_assemble_kernel(const float* __restrict__ tiles, const __grid_constant__ AssembleShape a, const __grid_constant__ CgTables tables,
-                   float* __restrict__ out, long long ldc) {
+cg_assemble_kernel(const float* tiles, const __grid_constant__ AssembleShape a, const __grid_constant__ CgTables tables,
+                   float* out, long long ldc) {
   extern __shared__ int tab[];
   __shared__ float patch[32][33];
   chain_wait();
@@ -429,7 +429,7 @@ cg_assemble_kernel(const float* __restrict__ tiles, const __grid_constant__ Asse
         const int ca = p.a0 + (row >> 6), cb = p.b0 + (col >> 6);
         const int r = (ca & 1) * 64 + (row & 63), c = (cb & 1) * 64 + (col & 63);
         const float* tile = tiles + static_cast<size_t>(p.tile0 + (ca >> 1) * p.tiles_b + (cb >> 1)) * CG_TILE;
-        const float w = __ldg(tile + r * 128 + ((((c >> 2) ^ (r & 7)) << 2) | (c & 3)));
+        const float w = tile[r * 128 + ((((c >> 2) ^ (r & 7)) << 2) | (c & 3))];
         sum += term & 0x8000 ? -w : w;
       }
       v = a.scale * sum;
@@ -450,8 +450,8 @@ cg_assemble_kernel(const float* __restrict__ tiles, const __grid_constant__ Asse
 // chunks.  The terms belong to the whole block, and all accesses have 16 bytes: 32 x 256 x 14 x 14, 2304 x 2304 result:
 // 26 us with a look-up per entry, 8.7 so.
 __global__ void __launch_bounds__(256)
-cg_assemble_blocks_kernel(const float* __restrict__ tiles, const __grid_constant__ AssembleShape a, const __grid_constant__ CgTables tables,
-                          float* __restrict__ out, long long ldc, bool vec) {
+cg_assemble_blocks_kernel(const float* tiles, const __grid_constant__ AssembleShape a, const __grid_constant__ CgTables tables,
+                          float* out, long long ldc, bool vec) {
   __shared__ float patch[64][65];
   chain_wait();
   const int* tab = tables.memory != nullptr ? tables.memory + tables.corr_words : tables.words + tables.corr_words;
@@ -485,7 +485,7 @@ cg_assemble_blocks_kernel(const float* __restrict__ tiles, const __grid_constant
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int r = ty + 16 * k;
-      w[k] = __ldg(reinterpret_cast<const float4*>(tile + r * 128 + ((((cb & 1) * 16 + tx) ^ (r & 7)) << 2)));
+      w[k] = *reinterpret_cast<const float4*>(tile + r * 128 + ((((cb & 1) * 16 + tx) ^ (r & 7)) << 2));
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {

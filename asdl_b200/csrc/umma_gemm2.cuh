@@ -844,7 +844,7 @@ template <int BN, int ROWS>
 __global__ void __launch_bounds__(256)
 splitk_reduce2_kernel(const __grid_constant__ GemmProblem2 single, const GemmProblem2* __restrict__ probs,
                       const GemmWork2* __restrict__ work, const int* __restrict__ tile_prefix, int n_probs) {
-  chain_wait();   // for the products
+  chain_wait();   // for the products; tables are older than their launch, which is a plain one (g2_may_chain)
   constexpr int R = ROWS / 16, SPLITS = 8 / R;   // rows of a thread, splits in flight
   __shared__ float tile[ROWS][G2_RED_COLS + 1];
   GemmWork2 w;
@@ -882,7 +882,7 @@ splitk_reduce2_kernel(const __grid_constant__ GemmProblem2 single, const GemmPro
   if (row0 >= P.M || col0 >= P.N) return;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   constexpr size_t SPLIT = static_cast<size_t>(G2_BM) * BN;   // floats of one split's partial tile
-  const float* p0 = P.ws + static_cast<size_t>(w.tile_id) * P.nsplit * SPLIT +
+  const float* p0 = after_wait(P.ws) + static_cast<size_t>(w.tile_id) * P.nsplit * SPLIT +
                     static_cast<size_t>(sub_r * ROWS + ty) * BN + sub_c * G2_RED_COLS + tx * 4;
   const int gc = col0 + tx * 4;
   const bool full = gc + 4 <= P.N;

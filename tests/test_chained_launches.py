@@ -19,3 +19,47 @@ def test_kernels_that_take_problem_tables_from_memory_are_launched_plainly(flavo
     launches = re.findall(r'launch_\w+\(([^,]*),', _source(f'gemm2_{flavour}.cu'))
     assert launches == ['g2_may_chain(probs)']
     assert re.search(r'g2_may_chain\(const GemmProblem2\* table\) \{ return table == nullptr; \}', _source('gemm2_host.h'))
+
+
+#: read-only parameters of kernels that wait on a chain: written before the chain's first kernel, which is launched plainly
+OLDER_THAN_THE_CHAIN = {'x', 'dy', 'y', 'res', 'weight', 'bias', 'mean', 'invstd', 'probs', 'work', 'prefix_g', 'tile_prefix'}
+
+
+def _kernels(name):
+    """(name, parameters, body) of the kernels of a file."""
+    text = re.sub(r'__(launch_bounds|cluster_dims)__\([^()]*\)', '', _source(name))
+    for head in re.finditer(r'__global__\s+void\s+(\w+)\(', text):
+        start = text.index('{', head.end())
+        depth, end = 1, start + 1
+        while depth:
+            depth += {'{': 1, '}': -1}.get(text[end], 0)
+            end += 1
+        yield head.group(1), text[head.end():start], text[start:end]
+
+
+def test_what_a_chain_has_written_is_read_by_ordinary_loads():
+    """The read-only path is for data that nobody writes while the kernel is resident, and a chained kernel is resident early."""
+    found = set()
+    for name in sorted(f for f in os.listdir(CSRC) if f.endswith(('.cu', '.cuh'))):
+        for kernel, params, body in _kernels(name):
+            if 'chain_wait()' not in body:
+                continue
+            found.add(kernel)
+            read_only = set(re.findall(r'const [\w:]+\* __restrict__ (\w+)', params))
+            assert read_only <= OLDER_THAN_THE_CHAIN, (kernel, read_only - OLDER_THAN_THE_CHAIN)
+            assert '__ldg(' not in body and '__ldcs(' not in body, kernel
+            if '__ldcg(' in body:
+                assert 'after_wait(' in body, kernel
+    assert found >= {'bn_fwd_finalize', 'bn_apply', 'bn_bwd_finalize', 'bn_dx', 'cg_product_kernel', 'cg_reduce_kernel',
+                     'umma_gemm2_kernel', 'umma_gemm2_pair_kernel', 'splitk_reduce2_kernel'}
+
+
+def test_every_kernel_of_a_chain_waits():
+    """A kernel that ends without waiting would let the kernel behind it run ahead of the one in front."""
+    chained = set()
+    for name in sorted(f for f in os.listdir(CSRC) if f.endswith(('.cu', '.cuh'))):
+        chained |= {k for k in re.findall(r'launch_chained\((\w+)', _source(name)) if k != 'kernel'}
+        chained |= set(re.findall(r'launch_behind\([^,]*, (\w+)', _source(name))) - {'kernel'}
+    waiting = {k for name in os.listdir(CSRC) if name.endswith(('.cu', '.cuh')) for k, _, body in _kernels(name)
+               if 'chain_wait()' in body}
+    assert chained and chained <= waiting
