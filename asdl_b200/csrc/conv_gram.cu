@@ -553,6 +553,7 @@ bool gemm_batch_is_open();
 bool conv_gram(at::Tensor x, at::Tensor out, int64_t kh, int64_t kw, int64_t ph, int64_t pw, double scale, double beta, bool khwc,
                bool x3) {
   TORCH_CHECK(x.is_cuda() && x.dim() == 4, "x must be a 4-d CUDA tensor");
+  TORCH_CHECK(x.scalar_type() == at::kFloat || x.scalar_type() == at::kBFloat16 || x.scalar_type() == at::kHalf, "x must be fp32, bf16 or fp16");
   const int64_t n = x.size(0), c = x.size(1), h = x.size(2), w = x.size(3);
   const int64_t ho = h + 2 * ph - kh + 1, wo = w + 2 * pw - kw + 1, taps = kh * kw, ncol = taps * c;
   if (gemm_batch_is_open() || kh < 1 || kw < 1 || kh > CG_MAX_K || kw > CG_MAX_K || taps < 2 || ph < 0 || pw < 0 || ph >= kh ||
@@ -756,10 +757,8 @@ bool conv_gram(at::Tensor x, at::Tensor out, int64_t kh, int64_t kw, int64_t ph,
     stage(x.data_ptr<float>());
   else if (x.scalar_type() == at::kBFloat16)
     stage(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()));
-  else if (x.scalar_type() == at::kHalf)
-    stage(x.data_ptr<at::Half>());
   else
-    TORCH_CHECK(false, "x must be fp32, bf16 or fp16");
+    stage(x.data_ptr<at::Half>());
   B200_CUDA_CHECK(cudaGetLastError());
   count_launch();
 

@@ -280,6 +280,15 @@ def test_factor_by_tap_differences(kernel, padding, shape, dtype, layout):
     ops.check_status()
 
 
+def test_a_refused_factor_by_tap_differences_launches_nothing(ext):
+    """5 x 5 filters have tables that a kernel writes first; a refused call stops ahead of it."""
+    x, out = torch.zeros(2, 8, 9, 9, device=DEV, dtype=torch.float64), torch.zeros(200, 200, device=DEV)
+    before = ext.launch_count()
+    with pytest.raises(RuntimeError, match='fp32, bf16 or fp16'):
+        ext.conv_gram(x, out, 5, 5, 2, 2, 1.0, 0.0, True, False)
+    assert ext.launch_count() == before
+
+
 def test_the_rule_for_tap_differences_gives_what_patches_give(monkeypatch):
     for shape, k, p, mode, dtype in [((4, 64, 7, 7), 3, 1, 'zeros', torch.float32), ((8, 32, 16, 16), 3, 1, 'reflect', torch.float32),
                                      ((32, 64, 14, 14), 5, 2, 'zeros', torch.bfloat16), ((4, 128, 9, 9), 3, 0, 'zeros', torch.bfloat16)]:
