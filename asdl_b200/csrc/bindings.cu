@@ -61,6 +61,7 @@ void symm_reduce_slots(at::Tensor local, at::Tensor table, int64_t world, int64_
                        double beta);
 at::Tensor kron_staged(at::Tensor left, at::Tensor mid, at::Tensor right, bool x3);
 bool conv_gram(at::Tensor x, at::Tensor out, int64_t kh, int64_t kw, int64_t ph, int64_t pw, double scale, double beta, bool khwc, bool x3);
+std::vector<std::vector<int64_t>> conv_gram_plan(int64_t n, int64_t c, int64_t h, int64_t w, int64_t kh, int64_t kw, int64_t ph, int64_t pw, int64_t sms, bool x3);
 void chol_inverse(std::vector<at::Tensor> mats, std::vector<at::Tensor> outs, at::Tensor damping);
 std::pair<int64_t, int64_t> chol_inverse_cache_info();
 void chol_inverse_tc(std::vector<at::Tensor> mats, std::vector<at::Tensor> outs, at::Tensor damping);
@@ -132,6 +133,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("symm_pull_slots", &b200::symm_pull_slots);
   m.def("kron_staged", &b200::kron_staged, "left * mid * right of symmetric outer matrices, staging included");
   m.def("conv_gram", &b200::conv_gram, "input-side factor of a stride-1 convolution from products by tap difference");
+  m.def("conv_gram_plan", &b200::conv_gram_plan, "staged rows and products of conv_gram for a shape");
   m.def("chol_inverse", &b200::chol_inverse, "grouped damped SPD inverse (fp32, CUDA cores)");
   m.def("chol_inverse_cache_info", &b200::chol_inverse_cache_info, "(entries, entries that captured graphs keep)");
   m.def("chol_inverse_tc", &b200::chol_inverse_tc, "grouped damped SPD inverse (fp32-accurate, tensor cores)");

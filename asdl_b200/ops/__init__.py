@@ -362,28 +362,43 @@ def tap_difference_eligible(x: torch.Tensor, kernel, padding, out_hw, khwc_order
     """True when the input-side factor of a convolution without stride and dilation is formed from products by tap
     difference (``csrc/conv_gram.cu``) instead of a patch matrix: filters of 3 x 3 to 5 x 5.
 
-    The rule is in patch elements P = rows x columns of the patch matrix that is not written (times in us, patches -> differences):
-      * fp32: channels that fill at least half of their 64-channel chunks (24 of 64: 54 -> 56; 32 of 64: 64 -> 41, 32 x 32 images);
-        3 x 3 from the smallest size on (4 x 64 x 7 x 7: 27 -> 25), but with more than 128 channels from P = 3e6 (192: P = 3.4e5
-        28 -> 35, 3.5e6 52 -> 50); larger filters, which have many corrections, from 1e7 (64: 3.3e6 47 -> 53, 1e7 84 -> 60;
-        192: 9.8e6 152 -> 199, 3e7 373 -> 254);
-      * bf16, order (kh, kw, c) with whole 64-channel chunks, where the result is assembled block by block: 3 x 3 always
-        (4 x 64 x 7 x 7: 23 -> 19, 32 x 256 x 14 x 14: 62 -> 42), larger filters from 6e6 (64: 3.3e6 31 -> 37; 128: 6.5e6 59 -> 48);
-      * bf16 otherwise: at least 64 channels and P = 2.5e7 (96: 5.4e6 30 -> 34, 2.8e7 63 -> 48).
-    Rows and columns outside of a tap's window are taken off from sums over the whole image: at least half of the image has to
-    be in the window, so that little cancels."""
+    The rule is in patch elements P = rows x columns of the patch matrix that is not written, chunks of 64 channels, and padding: "same"
+    keeps the size of the image; with less, more image rows and columns are outside of some tap's window and have products of their
+    own (times in us, patches -> differences):
+      * fp32, channels that fill at least half of their chunks.  3 x 3 with same padding from P = 3.5e6 (64 channels: 1.2e6 27 -> 32, 3.6e6
+        37 -> 36, 7.2e6 51 -> 41), with more than 128 channels from 8e6 (192: 3.5e6 44 -> 49, 1.1e7 87 -> 64); padding 2 from 1e6 (1.5e6
+        29 -> 22); padding 0 from 1.2e7 (128: 5.3e6 46 -> 48, 1.4e7 84 -> 66).  Larger filters from 2e7 per chunk (5 x 5, 64: 1e7
+        78 -> 76, 2e7 131 -> 90; 128: 2e7 201 -> 194, 4e7 345 -> 262; 256: 4e7 573 -> 594, 2.1e8 2874 -> 1029), with more padding from 8e6
+        per chunk (64: 4.2e6 46 -> 47, 9.9e6 132 -> 47), with less never (5 x 5 without padding, 128: 8e7 645 -> 631);
+      * bf16, order (kh, kw, c) with whole chunks, where the result is assembled block by block: from 1.4e7 / chunks (3 x 3, 64: 7.2e6
+        27 -> 31, 1.9e7 40 -> 35; 128: 4.7e6 25 -> 26, 7.2e6 29 -> 28; 256: 4.7e6 44 -> 32, 1.4e7 58 -> 36; 5 x 5, 64: 1e7 38 -> 43,
+        2e7 57 -> 50; 128: 6.6e6 57 -> 50); with more padding from 9e6 / chunks, 3 x 3 always (1.5e6 22 -> 17); with less 3 x 3 from 1.7e7
+        (128: 7.4e6 29 -> 36, 3.3e7 67 -> 50), larger filters from 4e7 (5 x 5, padding 1, 128: 1.5e7 82 -> 82, 3.9e7 179 -> 113);
+      * bf16 otherwise: at least 64 channels, P = 2.5e7 and same padding (96: 5.4e6 26 -> 31, 2.8e7 58 -> 47);
+      * calls that the host bounds, 3 x 3 up to P = 5e5 (4 x 64 x 7 x 7: 26 -> 23 and 22 -> 18; but 96 channels in fp32 27 -> 33).
+    The images' rows, of all images together, are padded to a multiple of 64 pixels; where that doubles them, patches are faster
+    (2 x 128 x 512 x 4: 44 -> 62)."""
     (kh, kw), (ph, pw), (ho, wo) = kernel, padding, out_hw
     n, c, h, w = x.shape
+    edge = max(kh - 1 - ph, kw - 1 - pw)
     if not (TAP_DIFFERENCES and 3 <= kh <= 5 and 3 <= kw <= 5 and x.is_cuda and ph < kh and pw < kw and min(n, c, ho, wo) > 0
-            and 2 * ho * wo >= h * w):
+            and min(h, w) >= 2 * edge):
         return False
-    size, chunks = n * ho * wo * c * kh * kw, (c + 63) // 64
+    size, chunks, x3 = n * ho * wo * c * kh * kw, (c + 63) // 64, _use_x3(x.dtype)
+    blocks = not x3 and khwc_order and c % 64 == 0
     small_filter = kh * kw <= 9
-    if _use_x3(x.dtype):
-        return c >= 32 * chunks and size >= ((0 if c <= 128 else 3e6) if small_filter else 1e7)
-    if khwc_order and c % 64 == 0:
-        return size >= (0 if small_filter else 6e6)
-    return c >= 64 and size >= 2.5e7
+    padded = (2 * edge > max(kh, kw) - 1) - (2 * edge < max(kh, kw) - 1)   # -1: more than "same", 0: same, 1: less
+    if small_filter and size <= 5e5 and padded <= 0 and (blocks or (x3 and 32 <= c <= 64)):
+        return True
+    if _round_up(n * (w + kw - 1), 64) > 2 * n * w:
+        return False
+    if x3:
+        least = (3.5e6 if c <= 128 else 8e6, 1.2e7, 1e6) if small_filter else (2e7 * chunks, float('inf'), 8e6 * chunks)
+        return c >= 32 * chunks and size >= least[padded]
+    if blocks:
+        least = (1.4e7 / chunks, 1.7e7 if small_filter else 4e7, 0 if small_filter else 9e6 / chunks)
+        return edge < 4 and size >= least[padded]
+    return c >= 64 and size >= 2.5e7 and padded <= 0
 
 
 #: form the factors of stride-1 convolutions from products by tap difference where that is the faster way

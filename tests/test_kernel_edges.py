@@ -250,7 +250,8 @@ def test_batches_whose_tables_take_each_others_place(ext):
     ops.check_status()
 
 
-@pytest.mark.parametrize('kernel,padding', [((3, 3), (1, 1)), ((3, 3), (0, 0)), ((5, 5), (2, 2)), ((4, 3), (1, 2)), ((2, 2), (1, 0))])
+@pytest.mark.parametrize('kernel,padding', [((3, 3), (1, 1)), ((3, 3), (0, 0)), ((5, 5), (2, 2)), ((5, 5), (0, 0)), ((5, 5), (1, 0)),
+                                            ((4, 3), (1, 2)), ((2, 2), (1, 0))])
 @pytest.mark.parametrize('shape', [(1, 64, 7, 7), (3, 24, 9, 6), (70, 65, 8, 8), (2, 192, 12, 13), (5, 128, 10, 10)])
 @pytest.mark.parametrize('dtype,layout', [(torch.float32, 'nchw'), (torch.bfloat16, 'nhwc'), (torch.float16, 'view')])
 def test_factor_by_tap_differences(kernel, padding, shape, dtype, layout):
@@ -269,15 +270,50 @@ def test_factor_by_tap_differences(kernel, padding, shape, dtype, layout):
         before += before.T.clone()
         out = torch.full((c * taps, c * taps + 3), 2.0, device=DEV)[:, :c * taps]   # rows of any alignment
         out.copy_(before)
-        assert ops.extension().conv_gram(x, out, *kernel, *padding, 1 / n, 0.5, khwc, x3)
+        done = ops.extension().conv_gram(x, out, *kernel, *padding, 1 / n, 0.5, khwc, x3)
+        # no plan where an image row or column would be among the first and among the last that a window leaves out
+        assert done == (h >= 2 * (kernel[0] - 1 - padding[0]) and w >= 2 * (kernel[1] - 1 - padding[1]))
+        if not done:
+            assert torch.equal(out, before)
+            return
         want = m.T @ m / n + 0.5 * before.double()
-        # 2^-16 of a product of bf16 pairs (exact ones for bf16) and fp32 sums, over the whole image where the window is a part of it
-        bound = ((2.0 ** -15 if x3 else 0.0) + 64 * 2.0 ** -24) * h * w * seen.square().amax().item() + 2.0 ** -22 * before.abs().max()
-        assert (out.double() - want).abs().max() <= bound
+        # 2^-16 of a product of bf16 pairs (exact ones for bf16) and an ulp for every sixteen rows of a sum; the products of an entry
+        # add up to at most the root of its two diagonal entries
+        energy = m.square().sum(0).sqrt() / n ** 0.5
+        bound = ((2.0 ** -15 + 3 / 16 * len(m) * 2.0 ** -23 if x3 else 1 / 16 * len(m) * 2.0 ** -23) + 2.0 ** -20) * torch.outer(energy, energy) + 2.0 ** -22 * before.abs()
+        assert ((out.double() - want).abs() <= bound).all()
         assert torch.equal(out, out.T)
         got = ops.extension().conv_gram(x, out, *kernel, *padding, 1 / n, 0.0, khwc, x3)
-        assert got and (out.double() - m.T @ m / n).abs().max() <= bound
+        assert got and ((out.double() - m.T @ m / n).abs() <= bound).all()
     ops.check_status()
+
+
+@pytest.mark.parametrize('dtype,last', [(torch.float32, False), (torch.bfloat16, True)])
+def test_a_factor_of_one_image_row_has_the_zeros_and_signs_of_a_gram_matrix(ext, dtype, last):
+    """Taps whose window leaves the only non-zero row out have exact zeros, and no diagonal entry is negative."""
+    x = torch.zeros(4, 64, 12, 12, device=DEV)
+    x[:, :, -1] = 100 * torch.randn(4, 64, 12, device=DEV, generator=_gen(11))
+    x = x.to(dtype)
+    out = torch.full((576, 576), float('nan'), device=DEV)
+    assert ext.conv_gram(x, out, 3, 3, 1, 1, 1.0, 0.0, last, dtype == torch.float32)
+    taps = out if last else out.view(64, 9, 64, 9).permute(1, 0, 3, 2).reshape(576, 576)
+    assert (taps[:192] == 0).all() and (taps[:, :192] == 0).all()
+    assert (out.diagonal() >= 0).all() and (taps.diagonal()[192:] > 0).all()
+
+
+@pytest.mark.parametrize('at', [(0, 0), (5, 0), (11, 7), (6, 6)])
+@pytest.mark.parametrize('value', [float('inf'), float('nan')])
+def test_a_value_that_is_not_finite_stays_in_its_channel(ext, at, value):
+    """Taps that see the value have diagonal entries that are not finite, and other channels have what they have without it."""
+    x = torch.randn(3, 70, 12, 12, device=DEV, generator=_gen(12))
+    clean, out = torch.empty(630, 630, device=DEV), torch.empty(630, 630, device=DEV)
+    ext.conv_gram(x, clean, 3, 3, 1, 1, 1.0, 0.0, False, True)
+    x[1, 20, at[0], at[1]] = value
+    ext.conv_gram(x, out, 3, 3, 1, 1, 1.0, 0.0, False, True)
+    seen = ~F.unfold(x, 3, padding=1).isfinite().all(2).all(0)
+    assert 4 <= seen.sum() <= 9 and not out.diagonal()[seen].isfinite().any()
+    others = torch.arange(630, device=DEV) // 9 != 20
+    assert torch.equal(out[others][:, others], clean[others][:, others])
 
 
 def test_a_refused_factor_by_tap_differences_launches_nothing(ext):
@@ -296,9 +332,10 @@ def test_the_rule_for_tap_differences_gives_what_patches_give(monkeypatch):
         last = dtype == torch.bfloat16
         x = x.contiguous(memory_format=torch.channels_last) if last else x
         conv = torch.nn.Conv2d(shape[1], 4, k, padding=p, padding_mode=mode, bias=False).to(DEV)
-        got = ops.conv_patch_gram(x, conv, scale=1e-3, channels_last_order=last)
         with monkeypatch.context() as m:
-            m.setattr(ops, 'TAP_DIFFERENCES', False)
+            m.setattr(ops, 'tap_difference_eligible', lambda *args: True)   # whatever is the faster one
+            got = ops.conv_patch_gram(x, conv, scale=1e-3, channels_last_order=last)
+            m.setattr(ops, 'tap_difference_eligible', lambda *args: False)
             want = ops.conv_patch_gram(x, conv, scale=1e-3, channels_last_order=last)
         assert (got - want).norm() <= (4e-5 if dtype == torch.float32 else 5e-6) * want.norm()
 
