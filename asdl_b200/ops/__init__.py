@@ -341,9 +341,10 @@ IMPLICIT_IM2COL = os.environ.get('ASDL_B200_IMPLICIT_IM2COL', '1') != '0'
 #: explicit path is ahead on every layer measured (32 images): at 56 x 56 x 64 channels (110 MiB of patches) 0.099 ms for
 #: im2col + SYRK and 0.128 for the implicit SYRK; on the small maps of deep layers (14 x 14 x 256: 28 MiB) the 4-D boxes of
 #: 2 x 2 pixels x 16 images load at half the rate of the 2-D boxes of an explicit matrix (0.065 and 0.146 ms).
-#: Products by tap difference (below) are faster than both and come first, unless a program has set another threshold than this.
-_IMPLICIT_IM2COL_DEFAULT_MB = 64.0
-IMPLICIT_IM2COL_MIN_MB = float(os.environ.get('ASDL_B200_IMPLICIT_IM2COL_MIN_MB', _IMPLICIT_IM2COL_DEFAULT_MB))
+#: None: from 64 MiB on, and products by tap difference (below), which are faster than both, come first where they are eligible.
+#: A number, 64 too, asks for implicit im2col from that size on, whatever is faster.
+_mb = os.environ.get('ASDL_B200_IMPLICIT_IM2COL_MIN_MB')
+IMPLICIT_IM2COL_MIN_MB: Optional[float] = None if _mb is None else float(_mb)
 
 
 def implicit_im2col_eligible(x: torch.Tensor, kernel, stride, dilation, padding, out_hw, khwc_order: bool) -> bool:
@@ -355,7 +356,7 @@ def implicit_im2col_eligible(x: torch.Tensor, kernel, stride, dilation, padding,
     return bool(IMPLICIT_IM2COL and khwc_order and x.is_cuda and x.dtype == torch.bfloat16 and not _use_x3(x.dtype)
                 and sh == sw == dh == dw == 1 and c % 64 == 0 and kh * kw <= 12 and ph < kh and pw < kw
                 and ho > ph and wo > pw and x.is_contiguous(memory_format=torch.channels_last)
-                and n * ho * wo * c * kh * kw * 2 >= IMPLICIT_IM2COL_MIN_MB * 2 ** 20)
+                and n * ho * wo * c * kh * kw * 2 >= (64 if IMPLICIT_IM2COL_MIN_MB is None else IMPLICIT_IM2COL_MIN_MB) * 2 ** 20)
 
 
 def tap_difference_eligible(x: torch.Tensor, kernel, padding, out_hw, khwc_order: bool) -> bool:
@@ -402,7 +403,7 @@ def tap_difference_eligible(x: torch.Tensor, kernel, padding, out_hw, khwc_order
 
 
 #: form the factors of stride-1 convolutions from products by tap difference where that is the faster way
-TAP_DIFFERENCES = True
+TAP_DIFFERENCES = os.environ.get('ASDL_B200_TAP_DIFFERENCES', '1') != '0'
 
 
 def conv_patch_gram(x: torch.Tensor, conv: torch.nn.Conv2d, scale: float = 1.0,
@@ -415,7 +416,8 @@ def conv_patch_gram(x: torch.Tensor, conv: torch.nn.Conv2d, scale: float = 1.0,
     ``weight.view(c_out, -1)``); ``True`` uses (kh, kw, c), the order of a channels_last weight.
     CUDA: stride-1 convolutions with filters of 3 x 3 to 5 x 5 form it from products of the input with itself by tap
     difference (``tap_difference_eligible``; not while a batch of products is recorded); other stride-1 convolutions on
-    channels_last bf16 inputs with a multiple of 64 channels whose patch matrix would take ``IMPLICIT_IM2COL_MIN_MB`` or more never form it - the SYRK's producer gathers 8 x 8 pixel blocks of one filter tap with 4-D TMA boxes, padding
+    channels_last bf16 inputs with a multiple of 64 channels whose patch matrix would take 64 MiB
+    (``IMPLICIT_IM2COL_MIN_MB``) or more never form it - the SYRK's producer gathers 8 x 8 pixel blocks of one filter tap with 4-D TMA boxes, padding
     and image edges being TMA's zero fill (``IMPLICIT_IM2COL``); 1x1 stride-1 convolutions read the activations
     in place; everything else goes through a bf16 im2col kernel (vectorised for channels_last inputs).  fp32 inputs are
     staged as bf16 hi/lo patch pairs and multiplied in three passes (precision policy 'auto')."""
@@ -441,8 +443,8 @@ def conv_patch_gram(x: torch.Tensor, conv: torch.nn.Conv2d, scale: float = 1.0,
     implicit = False
     if sh == sw == dh == dw == 1 and kh * kw > 1 and (out is None or (out.dtype == torch.float32 and out.stride(1) == 1)):
         implicit = channels_last_order and implicit_im2col_eligible(x, (kh, kw), (1, 1), (1, 1), (ph, pw), (ho, wo), True)
-        if tap_difference_eligible(x, (kh, kw), (ph, pw), (ho, wo), channels_last_order) and not (
-                implicit and IMPLICIT_IM2COL_MIN_MB != _IMPLICIT_IM2COL_DEFAULT_MB):
+        asked = implicit and IMPLICIT_IM2COL_MIN_MB is not None
+        if not asked and tap_difference_eligible(x, (kh, kw), (ph, pw), (ho, wo), channels_last_order):
             result, weight = (torch.empty(ncol, ncol, device=x.device, dtype=torch.float32), 0.0) if out is None else (out, beta)
             if extension().conv_gram(x, result, kh, kw, ph, pw, float(scale), float(weight), channels_last_order, _use_x3(x.dtype)):
                 return result

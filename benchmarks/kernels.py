@@ -199,12 +199,12 @@ def bench_conv_syrk(timer, n, c, hw, k, flops_peak, src):
     ncol = c * k * k
     out = torch.empty(ncol, ncol, device='cuda')
     ms_differences = timer(lambda: ops.conv_patch_gram(x, conv, out=out, channels_last_order=True))
-    saved, saved_mb = ops.IMPLICIT_IM2COL, ops.IMPLICIT_IM2COL_MIN_MB
+    saved = ops.IMPLICIT_IM2COL, ops.IMPLICIT_IM2COL_MIN_MB, ops.TAP_DIFFERENCES
     ops.IMPLICIT_IM2COL, ops.IMPLICIT_IM2COL_MIN_MB, ops.TAP_DIFFERENCES = True, 0.0, False
     ms = timer(lambda: ops.conv_patch_gram(x, conv, out=out, channels_last_order=True))
     ops.IMPLICIT_IM2COL = False
     ms_explicit = timer(lambda: ops.conv_patch_gram(x, conv, out=out, channels_last_order=True))
-    ops.IMPLICIT_IM2COL, ops.IMPLICIT_IM2COL_MIN_MB, ops.TAP_DIFFERENCES = saved, saved_mb, True
+    ops.IMPLICIT_IM2COL, ops.IMPLICIT_IM2COL_MIN_MB, ops.TAP_DIFFERENCES = saved
     fl = 2.0 * n * hw * hw * ncol * ncol
     emit(case='conv_patch_syrk_bf16', n=n, c=c, hw=hw, k=k, ncol=ncol, differences_ms=round(ms_differences, 4), implicit_ms=round(ms, 4),
          explicit_im2col_ms=round(ms_explicit, 4), speedup=round(ms_explicit / ms, 2),

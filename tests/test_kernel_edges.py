@@ -340,6 +340,18 @@ def test_the_rule_for_tap_differences_gives_what_patches_give(monkeypatch):
         assert (got - want).norm() <= (4e-5 if dtype == torch.float32 else 5e-6) * want.norm()
 
 
+@pytest.mark.parametrize('threshold,implicit', [(None, False), (0.0, True), (64.0, True), (63.9, True), (200.0, False)])
+def test_a_threshold_that_is_set_asks_for_implicit_im2col(ext, monkeypatch, threshold, implicit):
+    """110 MiB of patches, which both ways can take: a number asks for one of them, also the number that holds by default."""
+    conv = torch.nn.Conv2d(64, 8, 3, padding=1, bias=False).to(DEV)
+    x = torch.randn(32, 64, 56, 56, device=DEV, generator=_gen(9)).to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
+    monkeypatch.setattr(ops, 'IMPLICIT_IM2COL_MIN_MB', threshold)
+    monkeypatch.setattr(ops, 'TAP_DIFFERENCES', True)
+    before = ext.launch_count()
+    ops.conv_patch_gram(x, conv, channels_last_order=True)
+    assert (ext.launch_count() - before <= 2) == implicit   # the product and its split-K reduction
+
+
 @pytest.mark.parametrize('sizes', [(1, 128, 129, 256, 384, 385), (640, 8, 513, 64, 257, 191, 1), (1153, 1024), (130,) * 90 + (400,) * 40])
 def test_grouped_inverse_of_mixed_sizes(sizes):
     """Tiles at and past the edges, chains of several lengths side by side, more tasks than CTAs; inputs with a row pitch."""
