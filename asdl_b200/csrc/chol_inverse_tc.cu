@@ -46,8 +46,8 @@ constexpr int TB = 128;  // tile
 
 enum : int { TASK_DIAG = 0, TASK_FACTOR = 1, TASK_INV = 2, TASK_OUT = 3, TASK_END = 4 };
 
-// L and X are kept as the images that the products want in shared memory.  Tile (i, j), j <= i, has index i (i + 1) / 2 + j and
-// consists of two halves of 64 columns; a half is three parts (hi, mid, lo) of 128 rows of 128 bytes, the 16-byte pieces of a row
+// L and X are kept as the images that the products want in shared memory.  Tile (i, j) of X, j <= i, has index i (i + 1) / 2 + j; L
+// is kept below the diagonal only, tile (i, j), j < i, at i (i - 1) / 2 + j.  A tile consists of two halves of 64 columns; a half is three parts (hi, mid, lo) of 128 rows of 128 bytes, the 16-byte pieces of a row
 // exchanged as the 128-byte swizzle does it.  A half of a part is a K block of a K-major operand (16 KiB, one copy); its rows
 // [64 b, 64 b + 64) are 64 columns of K block b of an MN-major operand (8 KiB).  Rows and columns past the matrix are stored too.
 constexpr int PART_BYTES = 128 * 128, TILE_BYTES = 6 * PART_BYTES;
@@ -55,7 +55,7 @@ constexpr int PART_BYTES = 128 * 128, TILE_BYTES = 6 * PART_BYTES;
 struct TcMat {
   const float* A;          // input n x n (pitch lda)
   float* out;              // n x n
-  uint8_t* L;              // tiles of L; those of the diagonal are not used
+  uint8_t* L;              // tiles of L below the diagonal
   uint8_t* X;              // tiles of X
   int* row_l;              // finished tiles of block row i of L
   int* col_x;              // block column j of X is finished down to (not including) this block row
@@ -64,6 +64,9 @@ struct TcMat {
 
 __device__ __forceinline__ uint8_t* tile_at(uint8_t* base, int i, int j) {
   return base + (static_cast<size_t>(i) * (i + 1) / 2 + j) * TILE_BYTES;
+}
+__device__ __forceinline__ uint8_t* below_at(uint8_t* base, int i, int j) {
+  return base + (static_cast<size_t>(i) * (i - 1) / 2 + j) * TILE_BYTES;
 }
 
 struct Task {
@@ -569,9 +572,7 @@ tc_tasks_kernel(const TcMat* __restrict__ mats, const Task* __restrict__ tasks, 
         const int* wb = t.kind == TASK_INV || t.kind == TASK_OUT ? M.col_x + t.j : M.row_l + t.j;
         int seen_a = -1, seen_b = -1;
         const int nkb = task_blocks(t.kind, t.i, t.j, M.n), total = nkb + (two ? 2 : 0);
-        uint8_t* const la = t.kind == TASK_OUT ? M.X : M.L;                              // operands of the sum
-        uint8_t* const lb = t.kind == TASK_INV || t.kind == TASK_OUT ? M.X : M.L;
-        const bool a_k = t.kind != TASK_OUT, b_k = t.kind == TASK_FACTOR;
+        const bool a_k = t.kind != TASK_OUT, b_k = t.kind == TASK_FACTOR;   // operands of the sum: rows of L, columns of X
         for (int kb = 0; kb < total && ok; ++kb, ++it) {
           const uint32_t s = it % TC_STAGES, parity = ((it / TC_STAGES) & 1) ^ 1;
           const uint8_t *src_a = nullptr, *src_b = nullptr;   // null: nothing to load (shared, or written by the epilogue)
@@ -583,9 +584,9 @@ tc_tasks_kernel(const TcMat* __restrict__ mats, const Task* __restrict__ tasks, 
               ok = false;
               break;
             }
-            src_a = a_k ? tile_at(la, t.i, panel) + hb * 3 * PART_BYTES : tile_at(la, panel, t.i) + hb * (PART_BYTES / 2);
+            src_a = a_k ? below_at(M.L, t.i, panel) + hb * 3 * PART_BYTES : tile_at(M.X, panel, t.i) + hb * (PART_BYTES / 2);
             if (!shared_ab)
-              src_b = b_k ? tile_at(lb, t.j, panel) + hb * 3 * PART_BYTES : tile_at(lb, panel, t.j) + hb * (PART_BYTES / 2);
+              src_b = b_k ? below_at(M.L, t.j, panel) + hb * 3 * PART_BYTES : tile_at(M.X, panel, t.j) + hb * (PART_BYTES / 2);
           } else {   // T, the other operand of the second product
             const int d = t.kind == TASK_FACTOR ? t.j : t.i;
             int seen = -1;
@@ -852,7 +853,7 @@ tc_tasks_kernel(const TcMat* __restrict__ mats, const Task* __restrict__ tasks, 
         for (int c = 0; c < 64; ++c) run[c] = -run[c];
       }
       // parts of the result: this warp's 32 rows of a half are 4 KiB in a row
-      uint8_t* const image = tile_at(t.kind == TASK_FACTOR ? M.L : M.X, t.i, t.j) + half * (3 * PART_BYTES) + q * 32 * 128;
+      uint8_t* const image = (t.kind == TASK_FACTOR ? below_at(M.L, t.i, t.j) : tile_at(M.X, t.i, t.j)) + half * (3 * PART_BYTES) + q * 32 * 128;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         stage_patch(run + 32 * h, stg, lane);
@@ -1003,7 +1004,7 @@ void chol_inverse_tc(std::vector<at::Tensor> mats, std::vector<at::Tensor> outs,
       const int64_t nb = (mats[i].size(0) + TB - 1) / TB;
       sizes[i] = static_cast<int>(mats[i].size(0));
       base[i] = total;
-      total += 2 * (nb * (nb + 1) / 2) * TILE_BYTES;
+      total += nb * nb * TILE_BYTES;   // X with, L without the diagonal
       words += 2 * nb;
     }
     P.splits = at::empty({total}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, dev));
@@ -1025,7 +1026,7 @@ void chol_inverse_tc(std::vector<at::Tensor> mats, std::vector<at::Tensor> outs,
       M.col_x = progress + M.nb;
       progress += 2 * M.nb;
       M.L = sp + base[i];
-      M.X = M.L + static_cast<size_t>(M.nb) * (M.nb + 1) / 2 * TILE_BYTES;
+      M.X = M.L + static_cast<size_t>(M.nb) * (M.nb - 1) / 2 * TILE_BYTES;
     }
     const std::vector<Task> tasks = make_tasks(sizes, g2_sm_count(dev));
     P.n_tasks = static_cast<int>(tasks.size());

@@ -375,6 +375,22 @@ def test_grouped_inverse_of_mixed_sizes(sizes):
         assert torch.equal(o, o.T)
 
 
+def test_a_set_of_small_inverses_keeps_one_tile_for_each(ext):
+    """Up to 128 rows there is nothing below the diagonal: three 32 KiB parts of the inverse's factor, and the tables."""
+    ext.chol_inverse_tc_clear_cache()
+    mats = [torch.eye(10, device=DEV) * (i + 1) for i in range(200)]
+    outs = [torch.empty_like(m) for m in mats]
+    damp = torch.zeros(200, device=DEV)
+    ext.read_status(0)
+    before = torch.cuda.memory_allocated()
+    ext.chol_inverse_tc(mats, outs, damp)
+    assert torch.cuda.memory_allocated() - before <= 200 * (96 * 1024 + 512) + 4096
+    for i, out in enumerate(outs):
+        assert (out - torch.eye(10, device=DEV) / (i + 1)).abs().max() <= 2.0 ** -21
+    ops.check_status()
+    ext.chol_inverse_tc_clear_cache()
+
+
 @pytest.mark.parametrize('n,at', [(40, 35), (128, 0), (128, 100), (200, 150)])
 def test_a_negative_pivot_in_any_stage_is_reported(n, at):
     a = torch.eye(n, device=DEV)
