@@ -1,6 +1,5 @@
-// Host-side interface of the persistent tcgen05 GEMM (umma_gemm2.cuh) for the other translation
-// units of the extension (the tensor-core Cholesky inverse builds its own problem tables and work
-// lists and runs them through these launchers).
+// Host-side interface of the persistent tcgen05 GEMM (umma_gemm2.cuh): the launchers of its flavours, each in a translation unit of its
+// own, and what the inverse and the convolution factor share with it (tensor maps, SM count).
 #pragma once
 #include "host_utils.h"
 #include "umma_gemm2.cuh"

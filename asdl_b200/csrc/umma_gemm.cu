@@ -476,7 +476,8 @@ void gemm_batch_abort() {
 // Python entry: C = alpha * A^T B (+ beta C), optionally symmetric, optionally bf16 split outputs.
 // `split3`: the three segments are the (hi, mid, lo) parts of fp32 operands and the product is
 // formed fp32-grade (six part products, one accumulation chunk per K block; see umma_gemm2.cuh).
-// `x3wide`: the two segments are the (hi, lo) parts of both operands (bf16x3 on 128 x 256 tiles).
+// `x3wide`: the two segments are the (hi, lo) parts of both operands (bf16x3): on CTA pairs (x3_takes_pairs, x3_syrk_takes_pairs),
+// otherwise 128 x 256 tiles, or three segments of the plain flavour for symmetric products.
 void umma_gemm(std::vector<at::Tensor> a_segs, std::vector<at::Tensor> b_segs, bool a_kmajor,
                bool b_kmajor, c10::optional<at::Tensor> C, double alpha, double beta, bool sym,
                c10::optional<at::Tensor> out_hi, c10::optional<at::Tensor> out_lo,

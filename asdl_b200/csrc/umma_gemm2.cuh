@@ -88,11 +88,6 @@ enum : int {
 // the extents belong to output pixels that do not exist - TMA fills both with zeros.  The shared-memory image of a
 // box is exactly the MN-major tile of the explicit patch matrix, so the MMA side does not change.
 
-
-enum : int {
-  G2W_NO_SPLIT_OUT = 1,  // work item: do not write the bf16 outputs of the problem for this tile
-};
-
 struct alignas(64) GemmProblem2 {
   CUtensorMap tmA[G2_MAX_SEG];
   CUtensorMap tmB[G2_MAX_SEG];
@@ -127,8 +122,6 @@ struct GemmWork2 {
   int c_row, c_col; // output origin
   int tile_id;      // index of the tile inside the problem's split-K scratch
   int split;        // split-K slice
-  int wflags;
-  int pad;
 };
 
 // What the epilogue needs of a problem, read once per work item into registers: a problem of a
@@ -195,8 +188,6 @@ __device__ __forceinline__ GemmWork2 g2_decode(const GemmProblem2& P, int idx) {
   w.c_row = w.a_mn;
   w.c_col = w.b_mn;
   w.tile_id = t;
-  w.wflags = 0;
-  w.pad = 0;
   return w;
 }
 
@@ -285,8 +276,7 @@ __device__ __forceinline__ void g2_reduce_chunk(const G2Epi& P, const float* v, 
 }
 
 // Final store of 32 consecutive columns of one row held by this thread.
-__device__ __forceinline__ void g2_store_chunk(const G2Epi& P, const float* v, int gr, int gc0,
-                                               bool diag_tile, bool split_out) {
+__device__ __forceinline__ void g2_store_chunk(const G2Epi& P, const float* v, int gr, int gc0, bool diag_tile) {
   if (gr >= P.M) return;
   const bool sym = (P.flags & G2F_SYM) != 0;
   const float alpha = P.alpha, beta = P.beta;
@@ -366,7 +356,7 @@ __device__ __forceinline__ void g2_store_chunk(const G2Epi& P, const float* v, i
         if (gc0 + j < P.N) c[j] = out[j];
     }
   }
-  if (P.out_hi != nullptr && split_out) {
+  if (P.out_hi != nullptr) {
     const size_t o = static_cast<size_t>(gr) * P.ld_out + gc0;
     // a symmetric problem's bf16 images are consumed as full matrices: write the mirror image too
     const bool mirror = sym && !(P.flags & G2F_LOWER);
@@ -727,7 +717,6 @@ umma_gemm2_kernel(const __grid_constant__ GemmProblem2 single, const GemmProblem
       const bool sym = (P.flags & G2F_SYM) != 0;
       const bool atomic = (P.flags & G2F_ATOMIC) != 0;
       const bool to_ws = P.nsplit > 1 && !atomic;
-      const bool split_out = !(w.wflags & G2W_NO_SPLIT_OUT);
       const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
 
       auto finish = [&](const float* v, int col0) {
@@ -750,7 +739,7 @@ umma_gemm2_kernel(const __grid_constant__ GemmProblem2 single, const GemmProblem
             if (atomic)
               g2_reduce_chunk(P, v + c * 32, gr, gc0, diag);
             else
-              g2_store_chunk(P, v + c * 32, gr, gc0, diag, split_out);
+              g2_store_chunk(P, v + c * 32, gr, gc0, diag);
           }
         }
       };

@@ -372,7 +372,7 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
             if (atomic)
               g2_reduce_chunk(E, v + c * 32, gr, gc0, diag);
             else
-              g2_store_chunk(E, v + c * 32, gr, gc0, diag, true);
+              g2_store_chunk(E, v + c * 32, gr, gc0, diag);
           }
         }
       }
