@@ -112,27 +112,31 @@ void g2_launch_reduce_list(const GemmProblem2* d_probs, const GemmWork2* d_work,
 }
 
 // bf16x3 products on CTA pairs: single ones (the tiles of a plan or a batch run on one kernel) of more than one 128-wide tile
-// each way, unless the tile policy asks for something else.
+// each way, unless the tile policy asks for something else.  us of one product, M x N x K, 128 x 256 tiles of single CTAs -> pairs:
+// 129 x 129 x 1024 19.6 -> 14.2, 256^3 12.4 -> 13.4, 300 x 1000 x 1000 20.6 -> 16.5, 384^3 16.6 -> 14.5, 512 x 2048 x 2048 22.2 -> 22.8,
+// 2048 x 1024 x 1024 23.2 -> 24.2, 1024 x 4096 x 1024 41.4 -> 25.5, 2048^3 59.3 -> 39.0.
 static bool x3_takes_pairs(int64_t m, int64_t n) { return g_wide_mode >= 3 && !g_batch_open && m > 128 && n > 128; }
 
 // Symmetric ones: from 24 K blocks on, and where the lower 256 x 256 tiles cover little more than the lower 128 x 128 tiles do.
-// us, three segments of the plain flavour -> pairs: 3000 x 1000 42 -> 28, 8192 x 1500 102 -> 75, 8192 x 2048 114 -> 103,
-// 12608 x 768 47 -> 44.5; but 1000 x 2048 31 -> 39, 300 x 1000 22 -> 27, and 8192 x 384 (twice the area) 23.5 -> 24.7.
+// us of the product, three segments of the plain flavour -> pairs: 3000 x 1000 37.9 -> 23.0, 8192 x 1500 85 -> 56, 8192 x 2048 115 -> 83,
+// 12608 x 768 36 -> 32, 1536 x 1300 32 -> 23, 2000 x 1024 20.4 -> 21.0; outside of the rule 1000 x 2048 27.6 -> 35.5, 300 x 1000 21 -> 25,
+// 12608 x 640 (1.6 times the area) 30.7 -> 31.7.
 static bool x3_syrk_takes_pairs(int64_t n, int64_t k) {
   const int64_t t = (n + 127) / 128, p = (t + 1) / 2;
   return x3_takes_pairs(n, n) && k >= 24 * G2_BK && 4.0 * (p * (p + 1) / 2) <= 1.35 * (t * (t + 1) / 2);
 }
 
 // K ranges of bf16x3 products on pairs (`slots` of them, `tiles` for them, `partials` 128 x 256 tiles): the count with the least
-// expected time of all waves and of the reduction.  A K block takes 0.9 us (three part products of 512 clocks), a tile 6 us around
-// its sum, a reduction 6 us and 0.04 us for each partial tile.  A count for two CTAs per SM took 1024 x 4096 through two waves of
-// each product and a reduction each.
+// expected time of all waves and of the reduction.  Fitted to graph replays of 20 shapes, most within 1.5 us: a launch takes 4.5 us, a K
+// block 0.85 (three part products of 512 clocks), a tile 6 around its sum, a chained reduction 1 and 0.04 for each partial tile.
+// us of one product, one range -> the chosen count: 512^3 17.1 -> 14.2, 1024^3 23.8 -> 19.3, 256 x 256 x 4096 63.7 -> 16.0; 1024 x 4096 x
+// 1024 stays at one, 25.5 (two: 40.0).  With 6 us for a reduction, and ranges of four blocks at least, 1024^3 was not split.
 static int split_in_waves(int tiles, int partials, int kb_total, int slots) {
   int best = 1;
   double least = 1e30;
-  for (int s = 1; s <= 32 && (s == 1 || kb_total / s >= 4); ++s) {
+  for (int s = 1; s <= 32 && (s == 1 || kb_total / s >= 2); ++s) {
     const int waves = (tiles * s + slots - 1) / slots;
-    const double us = waves * (0.9 * ((kb_total + s - 1) / s) + 6.0) + (s > 1 ? 6.0 + 0.04 * partials * s : 0.0);
+    const double us = 4.5 + waves * (0.85 * ((kb_total + s - 1) / s) + 6.0) + (s > 1 ? 1.0 + 0.04 * partials * s : 0.0);
     if (us < 0.98 * least) {   // a tie goes to fewer ranges
       least = us;
       best = s;
