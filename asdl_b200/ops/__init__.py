@@ -328,6 +328,8 @@ def kron_apply(left: torch.Tensor, mid: torch.Tensor, right: torch.Tensor) -> to
     if not cuda_kernels_enabled(left, mid, right) or mid.numel() == 0:
         dt = mid.dtype
         return left.to(dt) @ mid @ right.to(dt)
+    if mid.ndim != 2:
+        raise ValueError(f'mid has to be 2-D. Got {mid.ndim}-D.')
     x3 = _use_x3(torch.float32) if (left.dtype == torch.float32 or mid.dtype == torch.float32) \
         else _use_x3(mid.dtype)
     out = extension().kron_staged(left, mid, right, x3)

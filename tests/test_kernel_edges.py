@@ -213,6 +213,13 @@ def test_bf16x3_products_on_pairs(m, n, k):
     ops.check_status()
 
 
+@pytest.mark.parametrize('shape', [(8,), (2, 8, 8)])
+def test_a_two_sided_product_of_something_else_than_a_matrix_is_a_value_error(shape):
+    eye = torch.eye(8, device=DEV)
+    with pytest.raises(ValueError):
+        ops.kron_apply(eye, torch.zeros(*shape, device=DEV), eye)
+
+
 @pytest.mark.parametrize('rows', [1535, 1536, 4001])
 @pytest.mark.parametrize('n', [128, 200, 256, 385, 520, 1000])
 def test_fp32_factor_on_pairs(rows, n):
