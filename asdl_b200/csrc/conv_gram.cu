@@ -13,7 +13,7 @@
 // pixel that is in some of them only is a product of its own.  These are few and short (3 x 3, padding 1: the first and last row for
 // d = (0, dx), the first and last column for d = (dy, 0), the corners for d = 0).  All terms are sums of products, nothing is taken
 // off: a tap that sees nothing but zeros has exact zeros, a diagonal entry is never negative, and an entry's error is relative to
-// what its own window holds.  (Sums over all pixels, less the edges, were 8 % faster and kept the rounding of the larger sum.)
+// what its own window holds.  (Sums over all pixels, less the edges, took as long and kept the rounding of the larger sum.)
 //
 //   stage     x -> bf16 (hi, or hi and lo) rows [pixel, channel], ordered image row, image, column, with kw - 1 zeros behind each
 //             image's row: a difference d is a constant offset of rows, and edge rows are K ranges.  Products that leave edge columns
@@ -27,7 +27,7 @@
 //   assemble  adds the terms of each entry and the moving average, writes entry and mirror image.
 //
 // The patch matrix was written and read before: 128 x 64 x 32 x 32 fp32, 3 x 3: 302 MB, 15 tiles of K = 131072 with three part
-// products, each loading both operands, 337 -> 85 us (staging 20, products 44, reduction 4, assembly 9); 32 x 256 x 14 x 14
+// products, each loading both operands, 337 -> 79 us (staging 20, products 44, reduction 4, assembly 9); 32 x 256 x 14 x 14
 // bf16: 63 -> 41 us (5, 18, 4, 9).  The fp32 products are bound by what L2 delivers (64 KiB per K block of 768 tensor clocks), the
 // staging by memory: each pixel is read once and written to all its places; strips that read their own pixels, 32 bytes of a
 // sector per channel, and copies of them took 11 us more.  Masking the edge columns in shared memory instead of in a copy
@@ -919,7 +919,9 @@ bool conv_gram(at::Tensor x, at::Tensor out, int64_t kh, int64_t kw, int64_t ph,
     launch_chained(cg_assemble_blocks_kernel, dim3(nb * (nb + 1) / 2), dim3(256), 0, stream, tiles.data_ptr<float>(), a, tables, result, out.stride(0), vec);
   } else {
     const int nb = (a.n + 31) / 32, tab_bytes = static_cast<int>(host.size() - P.assembly) * 4;
-    launch_chained(cg_assemble_kernel, dim3(nb * (nb + 1) / 2), dim3(256), tab_bytes, stream, tiles.data_ptr<float>(), a, tables, result, out.stride(0));
+    // launched plainly: resident beside the products, whose shared memory leaves little of an SM's memory to the L1 cache, its look-ups take
+    // longer than the launch (128 x 64 x 32 x 32 fp32: 85.3 us chained, 78.6 so; 8 x 64 x 16 x 16: 31.5 and 25.4)
+    launch_behind(false, cg_assemble_kernel, dim3(nb * (nb + 1) / 2), dim3(256), tab_bytes, stream, tiles.data_ptr<float>(), a, tables, result, out.stride(0));
   }
   B200_CUDA_CHECK(cudaGetLastError());
   count_launch();

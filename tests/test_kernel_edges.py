@@ -323,6 +323,27 @@ def test_a_value_that_is_not_finite_stays_in_its_channel(ext, at, value):
     assert torch.equal(out[others][:, others], clean[others][:, others])
 
 
+@pytest.mark.parametrize('k', [3, 5])
+def test_a_captured_factor_by_tap_differences_replays_on_new_inputs(ext, k):
+    """Tables that are kernel parameters (3 x 3) and tables that a kernel writes first (5 x 5)."""
+    x = torch.randn(4, 64, 16, 16, device=DEV, generator=_gen(13))
+    out, want = (torch.zeros(64 * k * k, 64 * k * k, device=DEV) for _ in range(2))
+    args = (k, k, k // 2, k // 2, 1.0, 0.0, False, True)
+    ext.conv_gram(x, out, *args)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(2):
+            ext.conv_gram(x, out, *args)
+    for seed in (14, 15):
+        x.copy_(torch.randn(4, 64, 16, 16, device=DEV, generator=_gen(seed)))
+        ext.conv_gram(x, want, *args)
+        out.fill_(float('nan'))
+        graph.replay()
+        assert torch.equal(out, want)
+    ops.check_status()
+
+
 def test_a_refused_factor_by_tap_differences_launches_nothing(ext):
     """5 x 5 filters have tables that a kernel writes first; a refused call stops ahead of it."""
     x, out = torch.zeros(2, 8, 9, 9, device=DEV, dtype=torch.float64), torch.zeros(200, 200, device=DEV)
