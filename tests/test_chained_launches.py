@@ -17,7 +17,7 @@ def _source(name):
 def test_kernels_that_take_problem_tables_from_memory_are_launched_plainly(flavour):
     """Tensor maps of a table are read through a proxy of their own, which griddepcontrol.wait is not specified to order."""
     launches = re.findall(r'launch_\w+\(([^,]*),', _source(f'gemm2_{flavour}.cu'))
-    assert launches == ['g2_may_chain(probs)']
+    assert len(launches) == 1 and re.fullmatch(r'g2_may_chain\(probs\)( && !\w+)?', launches[0])
     assert re.search(r'g2_may_chain\(const GemmProblem2\* table\) \{ return table == nullptr; \}', _source('gemm2_host.h'))
 
 

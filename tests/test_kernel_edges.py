@@ -191,6 +191,19 @@ def test_inverse_at_the_edges_of_the_diagonal_stages(n):
     ops.check_status()
 
 
+@pytest.mark.parametrize('n', [1537, 1601, 2000, 2001, 2100, 2101, 2177])
+def test_factors_of_about_as_many_tiles_as_sms(n):
+    """Both sides of the rule that launches products of unaligned outputs plainly, and the CTAs of one wave and a little more."""
+    x = torch.randn(70, n, device=DEV, generator=_gen(16)).to(torch.bfloat16)
+    want = x.double().T @ x.double()
+    out = torch.eye(n, device=DEV)
+    for turn in (1, 2):
+        ops.gram(x, out=out, beta=0.5)
+        assert (out.double() - want - 0.5 * (torch.eye(n, device=DEV) if turn == 1 else before)).abs().max() <= 1e-6 * want.abs().max()
+        before = out.clone()
+    ops.check_status()
+
+
 @pytest.mark.parametrize('m,n', [(129, 129), (256, 300), (257, 640), (1000, 520)])
 @pytest.mark.parametrize('k', [2, 64, 200, 1600])
 def test_bf16x3_products_on_pairs(m, n, k):
