@@ -21,10 +21,10 @@ void g2_run_plain(const GemmProblem2& single, const GemmProblem2* probs, const G
   const int grid = std::min(n_work, 2 * n_sms);
   // A chained launch fills the SMs as the kernel before leaves them, two CTAs on some and none on others, where a plain one gives each SM
   // one first.  That matters where about as many CTAs as SMs have long epilogues, of 4-byte stores: symmetric products of 64 rows, us
-  // plainly -> chained: n = 2001 (136 tiles) 37.5 -> 42.4, 2101 (153) 42.6 -> 51.5; but 1281 (66) 35.4 -> 32.2, 2501 (210) 58.8 -> 53.9, and
-  // with 16-byte stores 2000 18.7 -> 15.9.
+  // plainly -> chained: n = 1801 (120 tiles) 35.4 -> 37.5, 2001 (136) 37.5 -> 42.4, 2101 (153) 42.6 -> 51.5; but 1665 (105) 35.5 -> 33.5, 2177 (171) 55.8 ->
+  // 53.5, and with 16-byte stores 2000 18.7 -> 15.9.
   const bool uneven = probs == nullptr && single.nsplit == 1 && single.C != nullptr &&
-                      ((single.ldc & 3) != 0 || (reinterpret_cast<uintptr_t>(single.C) & 15) != 0) && 3 * n_work > 2 * n_sms &&
+                      ((single.ldc & 3) != 0 || (reinterpret_cast<uintptr_t>(single.C) & 15) != 0) && 4 * n_work > 3 * n_sms &&
                       8 * n_work <= 9 * n_sms;
   launch_behind(g2_may_chain(probs) && !uneven, umma_gemm2_kernel<128, 4, 2, 1>, dim3(grid), dim3(G2Plain::THREADS), G2Plain::SMEM_BYTES, stream, single, probs, work, n_work, prefix, n_probs);
   B200_CUDA_CHECK(cudaGetLastError());
