@@ -368,40 +368,42 @@ def tap_difference_eligible(x: torch.Tensor, kernel, padding, out_hw, khwc_order
     The rule is in patch elements P = rows x columns of the patch matrix that is not written, chunks of 64 channels, and padding: "same"
     keeps the size of the image; with less, more image rows and columns are outside of some tap's window and have products of their
     own (times in us, patches -> differences):
-      * fp32, channels that fill at least half of their chunks.  3 x 3 with same padding: up to 64 channels always (64: 1.2e6 27 -> 25, 3.6e6
-        37 -> 29; 32: 5.9e5 24 -> 25), up to 128 from P = 2.4e6 (96: 1.8e6 30 -> 31; 128: 2.4e6 34 -> 33, 7.2e6 56 -> 36), more from 8e6
-        (192: 3.5e6 44 -> 50, 1.1e7 87 -> 65); padding 2 from 1e6 (1.5e6 29 -> 23); padding 0 from 7e6 (64: 2.6e6 31 -> 35, 7e6 50 -> 41;
-        128: 7.4e6 60 -> 58), with more than 128 channels from 1.6e7 (256: 1.1e7 100 -> 113).  Larger filters from 2e7 per chunk (5 x 5,
-        64: 1e7 80 -> 73, 2e7 132 -> 88; 128: 2e7 200 -> 194, 4e7 342 -> 261; 256: 4e7 566 -> 587, 2.1e8 2821 -> 1026), with more padding
-        from 8e6 per chunk (64: 4.2e6 46 -> 48, 9.9e6 132 -> 48), with less never (5 x 5 without padding, 128: 8e7 625 -> 633);
+      * fp32, channels that fill at least half of their chunks.  3 x 3 with same padding: up to 64 channels from P = 1e6 (64: 1.1e5 25 -> 29,
+        1.2e6 28 -> 28, 3.6e6 37 -> 29), up to 128 from 2.4e6 (96: 1.8e6 30 -> 30; 128: 2.4e6 34 -> 33, 7.2e6 56 -> 37), more from 8e6
+        (192: 3.5e6 44 -> 51, 1.1e7 87 -> 65); padding 2 from 1e6 (1.2e6 27 -> 25); padding 0 from 7e6 (64: 2.6e6 31 -> 35, 7e6 50 -> 41;
+        128: 7.4e6 60 -> 58), with more than 128 channels from 1.6e7 (256: 1.1e7 100 -> 113).  Larger filters from 1e7 per chunk, 2e7 if
+        there are more than three (5 x 5, 64: 3.3e6 44 -> 68, 1e7 80 -> 76; 128: 1e7 133 -> 167, 2e7 200 -> 194; 192: 3e7 350 -> 345; 256: 4e7
+        566 -> 587, 2.1e8 2821 -> 1026), with more padding from 8e6 per chunk (64: 4.2e6 46 -> 48, 9.9e6 132 -> 48), with less never
+        (5 x 5 without padding, 128: 8e7 625 -> 633);
       * bf16, order (kh, kw, c) with whole chunks, where the result is assembled block by block: from 1.4e7 / chunks (3 x 3, 64: 7.2e6
         27 -> 31, 1.9e7 40 -> 35; 128: 4.7e6 25 -> 26, 7.2e6 29 -> 28; 256: 4.7e6 44 -> 32, 1.4e7 58 -> 36; 5 x 5, 64: 1e7 38 -> 43,
-        2e7 57 -> 50; 128: 6.6e6 57 -> 50); with more padding from 9e6 / chunks, 3 x 3 always (1.5e6 22 -> 17); with less 3 x 3 from 1.7e7
+        2e7 57 -> 50; 128: 6.6e6 57 -> 50); with more padding from 9e6 / chunks, 3 x 3 from 1e6 (1.2e6 27 -> 25); with less 3 x 3 from 1.7e7
         (128: 7.4e6 29 -> 36, 3.3e7 67 -> 50), larger filters from 4e7 (5 x 5, padding 1, 128: 1.5e7 82 -> 82, 3.9e7 179 -> 113);
-      * bf16 otherwise: at least 64 channels, P = 2.5e7 and same padding (96: 5.4e6 26 -> 31, 2.8e7 58 -> 47);
-      * calls that the host bounds, 3 x 3 with same padding: up to P = 5e5, bf16 by blocks 1.5e6 (4 x 64 x 7 x 7: 26 -> 23 and 22 -> 18;
-        8 x 64 x 16 x 16, bf16: 24 -> 19, 22 -> 21).
+      * bf16 otherwise: at least 64 channels, P = 2.5e7 and same padding (96: 5.4e6 26 -> 31, 2.8e7 58 -> 47).
+    Smaller ones are bound by the host, which has more to do for differences (4 x 64 x 7 x 7: 25 -> 29, bf16 24 -> 27).
     The images' rows, of all images together, are padded to a multiple of 64 pixels; where that doubles them, patches are faster
     (2 x 128 x 512 x 4: 44 -> 60)."""
     (kh, kw), (ph, pw), (ho, wo) = kernel, padding, out_hw
     n, c, h, w = x.shape
-    edge = max(kh - 1 - ph, kw - 1 - pw)
-    if not (TAP_DIFFERENCES and 3 <= kh <= 5 and 3 <= kw <= 5 and x.is_cuda and ph < kh and pw < kw and min(n, c, ho, wo) > 0
-            and min(h, w) >= 2 * edge):
+    taps = kh * kw
+    size = n * ho * wo * c * taps
+    if size < 1e6 or taps < 9 or not (TAP_DIFFERENCES and kh <= 5 and kw <= 5 and kh >= 3 and kw >= 3 and ph < kh and pw < kw and x.is_cuda):
         return False
-    size, chunks, x3 = n * ho * wo * c * kh * kw, (c + 63) // 64, _use_x3(x.dtype)
+    x3 = _use_x3(x.dtype)
+    chunks, small_filter = (c + 63) // 64, taps == 9
     blocks = not x3 and khwc_order and c % 64 == 0
-    small_filter = kh * kw <= 9
-    padded = (2 * edge > max(kh, kw) - 1) - (2 * edge < max(kh, kw) - 1)   # -1: more than "same", 0: same, 1: less
-    if small_filter and padded <= 0 and size <= (1.5e6 if blocks else 5e5) and (blocks or (x3 and 32 <= c <= 64)):
-        return True
-    if _round_up(n * (w + kw - 1), 64) > 2 * n * w:
+    if blocks and size * chunks < 1.4e7 and ph < 2:   # with padding 0 or 1 nothing smaller is taken
         return False
+    edge = max(kh - 1 - ph, kw - 1 - pw)
+    if min(h, w) < 2 * edge or _round_up(n * (w + kw - 1), 64) > 2 * n * w:
+        return False
+    padded = (2 * edge > max(kh, kw) - 1) - (2 * edge < max(kh, kw) - 1)   # -1: more than "same", 0: same, 1: less
     if x3:
-        least = ((0, 2.4e6, 8e6)[min(chunks, 3) - 1], 7e6 if c <= 128 else 1.6e7, 1e6) if small_filter else (2e7 * chunks, float('inf'), 8e6 * chunks)
+        least = ((1e6, 2.4e6, 8e6)[min(chunks, 3) - 1], 7e6 if c <= 128 else 1.6e7, 1e6) if small_filter else (
+            (1e7 if chunks <= 3 else 2e7) * chunks, float('inf'), 8e6 * chunks)
         return c >= 32 * chunks and size >= least[padded]
     if blocks:
-        least = (1.4e7 / chunks, 1.7e7 if small_filter else 4e7, 0 if small_filter else 9e6 / chunks)
+        least = (1.4e7 / chunks, 1.7e7 if small_filter else 4e7, 1e6 if small_filter else 9e6 / chunks)
         return edge < 4 and size >= least[padded]
     return c >= 64 and size >= 2.5e7 and padded <= 0
 
