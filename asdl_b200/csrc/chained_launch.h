@@ -6,9 +6,10 @@
 // before it has finished too.  What a kernel of the chain has written is read by ordinary loads, not through __ldg or a
 // const __restrict__ parameter: the read-only path is for data that nobody writes while the kernel is resident, and the compiler
 // may move such loads ahead of the wait.  __ldcg takes its pointer from after_wait().  chain_next() lets the next kernel come as soon as all CTAs of this one have called it.
-// With the split-K reduction and the kernels of a convolution factor chained: 8192 x 1024 bf16 samples 27.5 -> 24.6 us,
-// 32 x 256 x 14 x 14 bf16 45.1 -> 39.8, 128 x 64 x 32 x 32 fp32 84.7 -> 77.8; with the GEMMs behind their casts: 24.6 -> 22.7 for the
-// first, 12608 x 768 fp32 samples 48.9 -> 47.5, 1024 x 4096 between fp32 factors 159 -> 155.
+// Launched plainly -> chained, passes in turn: 8192 x 1024 bf16 samples 27.3 -> 22.9 us, 12608 x 768 fp32 samples 52.9 -> 46.9, the
+// convolution factors of 32 x 256 x 14 x 14 bf16 47.7 -> 41.7 and of 128 x 64 x 32 x 32 fp32 82.6 -> 78.6, 1024 x 4096 between fp32 factors 153 -> 149.
+// What a chained kernel gets of the SMs while the one before it still runs can be uneven or short of L1 cache: two launches are
+// plain for that reason (gemm2_plain.cu, conv_gram.cu).
 // A kernel that is launched plainly behind a chain waits for its end as usual; a captured chain becomes programmatic edges.
 #pragma once
 #include <utility>

@@ -25,7 +25,7 @@
 // operand traffic of the ring, 96 KiB per K block of 1536 tensor cycles.  The former version ran the same arithmetic
 // right-looking in 28 (six factors up to 784) to 121 (the 107 factors of ResNet-50) dependent launches: every K = 128 update
 // read and wrote the fp32 matrix, each lane a row of its own, and every launch drained before the next began.
-// Six factors 784, 4 x 512, 10: 597 -> 251 us; ResNet-50's 107 factors: 8.04 -> 3.52 ms.
+// Six factors 784, 4 x 512, 10: 597 -> 252 us; ResNet-50's 107 factors, pass after pass at the power limit: 8.04 -> 3.55 ms.
 //
 // Tables, task lists and the bf16 split buffers depend only on the addresses and sizes of the matrices; they are built once
 // and cached (prepared_cache.h), so a repeated call (the K-FAC state) issues no host-to-device copy and can be captured in a
@@ -895,7 +895,9 @@ PreparedCache<Prepared, 4>& g_cache = *new PreparedCache<Prepared, 4>;
 // The task list of matrices of `sizes` for `ctas` CTAs.  Any order in which a task follows what it needs is correct; this one
 // is made for speed.  Time is cut into slots of one step of a chain (DIAG, FACTOR of the next row, last panel of the next
 // DIAG).  In a slot every matrix may take one step, and the longest remaining chains always do; shorter ones join while the
-// slot has room, and OUT tiles, which nothing waits for, fill the rest.
+// slot has room, and OUT tiles, which nothing waits for, fill the rest.  The durations are rough (a step takes 34 us, a diagonal block 22)
+// and the list does not depend on them much: STEP_US from 20 to 100, DIAG_US from 15 to 45 and AHEAD from 4 to 200 gave 256.5 - 256.9 us for
+// six factors up to 784 (257.8 with nothing ahead) and 3.47 - 3.65 ms, in no order, for ResNet-50's 107.
 std::vector<Task> make_tasks(const std::vector<int>& sizes, int ctas) {
   constexpr int STEP_US = 35, BLOCK_US = 1, TILE_US = 5, DIAG_US = 28, AHEAD = 12;
   const int count = static_cast<int>(sizes.size());
