@@ -22,12 +22,15 @@
 //   products  128 x 128 tiles of 64-channel chunks.  Each chunk is a TMA box with a row offset of its own, so a tile holds the
 //             chunks of several differences.  Where one chunk holds all channels, B is two chunks too, the second with the row
 //             before: it gives the difference next to that of the first;
-//             a CTA takes one K range of a tile; hi and lo parts are loaded once for the three part products;
+//             a CTA takes one K range of a tile; hi and lo parts are loaded once for the three part products, of which (lo, hi) and
+//             (hi, lo) have an accumulator of their own.  The tensor core truncates with every addition, so few of them should meet a
+//             large sum: with one accumulator and ranges of any length 32 x 96 x 32 x 32, 5 x 5, had an error of 1.0e-4 against 64 bits
+//             (patches in three segments 9.7e-5), with the second accumulator 4.5e-5, with ranges of 128 K blocks besides 6.8e-6;
 //   reduce    sums the K ranges in order;
 //   assemble  adds the terms of each entry and the moving average, writes entry and mirror image.
 //
 // The patch matrix was written and read before: 128 x 64 x 32 x 32 fp32, 3 x 3: 302 MB, 15 tiles of K = 131072 with three part
-// products, each loading both operands, 337 -> 79 us (staging 20, products 44, reduction 4, assembly 9); 32 x 256 x 14 x 14
+// products, each loading both operands, 337 -> 80 us (staging 20, products 44, reduction 4, assembly 9); 32 x 256 x 14 x 14
 // bf16: 63 -> 41 us (5, 18, 4, 9).  The fp32 products are bound by what L2 delivers (64 KiB per K block of 768 tensor clocks), the
 // staging by memory: each pixel is read once and written to all its places; strips that read their own pixels, 32 bytes of a
 // sector per channel, and copies of them took 11 us more.  Masking the edge columns in shared memory instead of in a copy
@@ -214,6 +217,7 @@ struct CgCfg {
   static constexpr int STAGES = 3;
   static constexpr int STAGE_BYTES = PARTS * 2 * G2_A_BYTES;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+  static constexpr int TMEM_COLS = PARTS * 128;   // (lo, hi) and (hi, lo) have an accumulator of their own
 };
 
 // Tables: [Grid x n_grids, and one behind the last][rows of the slots][tables of the assembly].  Those of up to CG_SMALL words are
@@ -286,7 +290,7 @@ cg_product_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid_consta
     mbar_fence_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 128);
+    tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
     tmem_relinquish();
   }
   tc_fence_before_sync();
@@ -351,7 +355,7 @@ cg_product_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid_consta
         const uint64_t db = desc_b + ((s * Cfg::STAGE_BYTES + PART_B[pr] * G2_A_BYTES) >> 4);
 #pragma unroll
         for (int k = 0; k < G2_BK / 16; ++k)
-          if (lead) umma_bf16(tmem_base, da + k * 128, db + k * 128, idesc, (kb | pr | k) ? 1u : 0u);
+          if (lead) umma_bf16(tmem_base + (pr < NPROD - 1 ? 128 : 0), da + k * 128, db + k * 128, idesc, (kb | k) || pr == 1 ? 1u : 0u);
       }
       if (lead) umma_commit(&empty_bar[s]);
       __syncwarp();
@@ -369,6 +373,13 @@ cg_product_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid_consta
       uint32_t v[32];
       tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + 32 * h, v);
       tmem_ld_wait();
+      if constexpr (PARTS > 1) {
+        uint32_t small[32];
+        tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + 128 + 32 * h, small);
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(__uint_as_float(v[c]) + __uint_as_float(small[c]));
+      }
 #pragma unroll
       for (int p = 0; p < 8; ++p)
         *reinterpret_cast<uint4*>(smem + row * 512 + (((8 * h + p) ^ (row & 7)) << 4)) = make_uint4(v[4 * p], v[4 * p + 1], v[4 * p + 2], v[4 * p + 3]);
@@ -386,7 +397,7 @@ cg_product_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid_consta
   __syncthreads();
   if (warp == 1) {
     __syncwarp();
-    tmem_dealloc(tmem_base, 128);
+    tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
   }
 }
 
@@ -588,7 +599,7 @@ struct Plan {
 };
 
 // False: the shape is outside of what the tables hold.
-bool make_plan(Plan& P, int64_t n, int64_t c, int64_t h, int64_t w, int kh, int kw, int ph, int pw, int resident) {
+bool make_plan(Plan& P, int64_t n, int64_t c, int64_t h, int64_t w, int kh, int kw, int ph, int pw, int resident, int longest_sum) {
   const int64_t ho = h + 2 * ph - kh + 1, wo = w + 2 * pw - kw + 1;
   const int taps = kh * kw;
   if (kh < 1 || kw < 1 || kh > CG_MAX_K || kw > CG_MAX_K || taps < 2 || ph < 0 || pw < 0 || ph >= kh || pw >= kw || ho < 1 || wo < 1 ||
@@ -721,7 +732,7 @@ bool make_plan(Plan& P, int64_t n, int64_t c, int64_t h, int64_t w, int kh, int 
       first.push_back(static_cast<int>(terms.size()));
     }
 
-  // ---- tiles and items: long grids first, K ranges as short as it takes to give every resident CTA one
+  // ---- tiles and items: long grids first, K ranges as short as it takes to give every resident CTA one, or equal parts of them
   const int nb = cc == 1 ? 2 : 1, tiles_b = (nb * cc + 1) / 2;
   std::vector<int> order;
   int64_t tiles = 0, blocks = 0;
@@ -736,13 +747,16 @@ bool make_plan(Plan& P, int64_t n, int64_t c, int64_t h, int64_t w, int kh, int 
   }
   if (order.empty() || products.size() > CG_MAX_PRODUCTS || terms.size() > CG_MAX_TERMS || tiles > CG_MAX_TILES) return false;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return grids[a].nkb > grids[b].nkb; });
-  auto ranges = [&](const HostGrid& g, int64_t len) { return static_cast<int>(std::min<int64_t>(64, (g.nkb + len - 1) / len)); };
+  auto ranges = [&](const HostGrid& g, int64_t len) { return static_cast<int>((g.nkb + len - 1) / len); };
   int64_t len = std::max<int64_t>(4, blocks / resident);
   for (; len < longest; len += 1 + len / 32) {
     int64_t items = 0;
     for (int g : order) items += grid_tiles(grids[g]) * ranges(grids[g], len);
     if (items <= resident) break;
   }
+  // a longer sum loses more to the tensor core's truncation than patches did: the same share of every CTA in equal parts
+  len = std::min<int64_t>(len, longest);
+  len = (len + (len + longest_sum - 1) / longest_sum - 1) / ((len + longest_sum - 1) / longest_sum);
   P.n_grids = static_cast<int>(order.size());
   P.tiles = P.split_tiles = P.partial_tiles = P.items = 0;
   std::vector<Grid> out(P.n_grids + 1);
@@ -784,6 +798,10 @@ bool make_plan(Plan& P, int64_t n, int64_t c, int64_t h, int64_t w, int kh, int 
 }
 
 int resident_ctas(int sms, bool x3) { return sms * (x3 ? 1 : 2); }
+// K blocks of a range, for the error of the sums (above); the shorter ranges also fill the last wave of many tiles: 32 x 128 x 32 x 32,
+// 5 x 5, 157 tiles, 462 -> 274 us, 32 x 192 x 32 x 32, 3 x 3, 181 -> 147.  bf16 products have a third of the additions; their errors are below
+// those of patches with ranges of any length.
+int longest_sum_of(bool x3) { return x3 ? 128 : 1 << 30; }
 
 }  // namespace
 
@@ -794,7 +812,7 @@ std::vector<std::vector<int64_t>> conv_gram_plan(int64_t n, int64_t c, int64_t h
                                                  int64_t sms, bool x3) {
   Plan P;
   if (!make_plan(P, n, c, h, w, static_cast<int>(kh), static_cast<int>(kw), static_cast<int>(ph), static_cast<int>(pw),
-                 resident_ctas(static_cast<int>(sms), x3)))
+                 resident_ctas(static_cast<int>(sms), x3), longest_sum_of(x3)))
     return {};
   const StageShape& s = P.s;
   // every row that is staged, with what it holds: (row, image, y, x), image -1: zeros
@@ -819,7 +837,7 @@ bool conv_gram(at::Tensor x, at::Tensor out, int64_t kh, int64_t kw, int64_t ph,
   Plan P;
   if (gemm_batch_is_open() || kh > CG_MAX_K || kw > CG_MAX_K ||
       !make_plan(P, x.size(0), c, x.size(2), x.size(3), static_cast<int>(kh), static_cast<int>(kw), static_cast<int>(ph), static_cast<int>(pw),
-                 resident_ctas(g2_sm_count(dev), x3)))
+                 resident_ctas(g2_sm_count(dev), x3), longest_sum_of(x3)))
     return false;
   TORCH_CHECK(out.is_cuda() && out.scalar_type() == at::kFloat && out.dim() == 2 && out.size(0) == ncol && out.size(1) == ncol &&
                   out.stride(1) == 1, "out must be a [c kh kw, c kh kw] fp32 CUDA matrix with unit column stride");

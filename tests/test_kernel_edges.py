@@ -336,6 +336,24 @@ def test_a_value_that_is_not_finite_stays_in_its_channel(ext, at, value):
     assert torch.equal(out[others][:, others], clean[others][:, others])
 
 
+@pytest.mark.parametrize('shape,k', [((32, 96, 32, 32), 5), ((32, 256, 28, 28), 3), ((16, 130, 30, 31), 5)])
+def test_long_sums_of_fp32_factors_by_tap_differences(ext, shape, k):
+    """K ranges of hundreds of blocks: the tensor core truncates with each of its additions of 16 rows."""
+    n, c, h, w = shape
+    x = torch.relu(torch.randn(*shape, device=DEV, generator=_gen(17)))
+    out = torch.empty(c * k * k, c * k * k, device=DEV)
+    assert ext.conv_gram(x, out, k, k, k // 2, k // 2, 1.0, 0.0, False, True)
+    want = torch.zeros(c * k * k, c * k * k, device=DEV, dtype=torch.float64)
+    for part in x.split(4):
+        m = F.unfold(part.double(), k, padding=k // 2).transpose(1, 2).reshape(-1, c * k * k)
+        want += m.T @ m
+    (_, _, n_grids, *_), words, _ = ext.conv_gram_plan(n, c, h, w, k, k, k // 2, k // 2, torch.cuda.get_device_properties(0).multi_processor_count, True)
+    blocks = max(-(-words[8 * g + 2] // words[8 * g + 3]) for g in range(n_grids))
+    # 2^-16 of a product, and half a last bit of half the sum, on average, for each addition to the large accumulator; a third accumulating
+    # product in it would be three times that
+    assert (out - want).norm() <= (2.0 ** -16 + 4 * blocks * 2.0 ** -25) * want.norm()
+
+
 @pytest.mark.parametrize('k', [3, 5])
 def test_a_captured_factor_by_tap_differences_replays_on_new_inputs(ext, k):
     """Tables that are kernel parameters (3 x 3) and tables that a kernel writes first (5 x 5)."""
