@@ -368,8 +368,8 @@ def tap_difference_eligible(x: torch.Tensor, kernel, padding, out_hw, khwc_order
     The rule is in patch elements P = rows x columns of the patch matrix that is not written, chunks of 64 channels, and padding: "same"
     keeps the size of the image; with less, more image rows and columns are outside of some tap's window and have products of their
     own (times in us, patches -> differences):
-      * fp32, channels that fill at least half of their chunks.  3 x 3 with same padding: up to 64 channels from P = 1e6 (64: 1.1e5 25 -> 29,
-        1.2e6 28 -> 28, 3.6e6 37 -> 29), up to 128 from 2.4e6 (96: 1.8e6 30 -> 30; 128: 2.4e6 34 -> 33, 7.2e6 56 -> 37), more from 8e6
+      * fp32, channels that fill at least half of their chunks.  3 x 3 with same padding: up to 64 channels from P = 2e6 (64: 1.1e5 25 -> 29,
+        1.8e6 29 -> 29, 3.6e6 37 -> 29; 32: 1.2e6 32 -> 35), up to 128 from 2.4e6 (96: 1.8e6 30 -> 30; 128: 2.4e6 34 -> 33, 7.2e6 56 -> 37), more from 8e6
         (192: 3.5e6 44 -> 51, 1.1e7 87 -> 65); padding 2 from 1e6 (1.2e6 27 -> 25); padding 0 from 7e6 (64: 2.6e6 31 -> 35, 7e6 50 -> 41;
         128: 7.4e6 60 -> 58), with more than 128 channels from 1.6e7 (256: 1.1e7 100 -> 113).  Larger filters from 1e7 per chunk, 2e7 if
         there are more than three (5 x 5, 64: 3.3e6 44 -> 68, 1e7 80 -> 76; 128: 1e7 133 -> 167, 2e7 200 -> 194; 192: 3e7 350 -> 345; 256: 4e7
@@ -399,7 +399,7 @@ def tap_difference_eligible(x: torch.Tensor, kernel, padding, out_hw, khwc_order
         return False
     padded = (2 * edge > max(kh, kw) - 1) - (2 * edge < max(kh, kw) - 1)   # -1: more than "same", 0: same, 1: less
     if x3:
-        least = ((1e6, 2.4e6, 8e6)[min(chunks, 3) - 1], 7e6 if c <= 128 else 1.6e7, 1e6) if small_filter else (
+        least = ((2e6, 2.4e6, 8e6)[min(chunks, 3) - 1], 7e6 if c <= 128 else 1.6e7, 1e6) if small_filter else (
             (1e7 if chunks <= 3 else 2e7) * chunks, float('inf'), 8e6 * chunks)
         return c >= 32 * chunks and size >= least[padded]
     if blocks:
