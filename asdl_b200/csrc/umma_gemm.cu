@@ -131,10 +131,13 @@ static bool x3_syrk_takes_pairs(int64_t n, int64_t k) {
 // block 0.85 (three part products of 512 clocks), a tile 6 around its sum, a chained reduction 1 and 0.04 for each partial tile.
 // us of one product, one range -> the chosen count: 512^3 17.1 -> 14.2, 1024^3 23.8 -> 19.3, 256 x 256 x 4096 63.7 -> 16.0; 1024 x 4096 x
 // 1024 stays at one, 25.5 (two: 40.0).  With 6 us for a reduction, and ranges of four blocks at least, 1024^3 was not split.
+// A range has at most 256 K blocks: the tensor core truncates with each of its additions (60000 x 2048 samples in two ranges: error
+// against 64 bits 1.2e-4, three segments of the plain kernels 1.0e-4).
 static int split_in_waves(int tiles, int partials, int kb_total, int slots) {
-  int best = 1;
+  const int first = std::max(1, (kb_total + 255) / 256);
+  int best = first;
   double least = 1e30;
-  for (int s = 1; s <= 32 && (s == 1 || kb_total / s >= 2); ++s) {
+  for (int s = first; s <= std::max(32, first) && (s == first || kb_total / s >= 2); ++s) {
     const int waves = (tiles * s + slots - 1) / slots;
     const double us = 4.5 + waves * (0.85 * ((kb_total + s - 1) / s) + 6.0) + (s > 1 ? 1.0 + 0.04 * partials * s : 0.0);
     if (us < 0.98 * least) {   // a tie goes to fewer ranges

@@ -354,6 +354,14 @@ def test_long_sums_of_fp32_factors_by_tap_differences(ext, shape, k):
     assert (out - want).norm() <= (2.0 ** -16 + 4 * blocks * 2.0 ** -25) * want.norm()
 
 
+@pytest.mark.parametrize('rows,n', [(60000, 2048), (20000, 1100)])
+def test_long_sums_of_fp32_factors_on_pairs(rows, n):
+    x = torch.randn(rows, n, device=DEV, generator=_gen(18))
+    want = x.double().T @ x.double()
+    # 2^-16 of a product, and a last bit of half the sum for each of the additions of a range of 256 K blocks
+    assert (ops.gram(x) - want).norm() <= (2.0 ** -16 + 4 * 256 * 2.0 ** -24) * want.norm()
+
+
 @pytest.mark.parametrize('k', [3, 5])
 def test_a_captured_factor_by_tap_differences_replays_on_new_inputs(ext, k):
     """Tables that are kernel parameters (3 x 3) and tables that a kernel writes first (5 x 5)."""
