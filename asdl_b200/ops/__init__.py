@@ -582,7 +582,7 @@ def batchnorm_unitwise_stats(y: torch.Tensor, g: torch.Tensor, weight: torch.Ten
     return out.mul_(beta).add_(new, alpha=alpha)
 
 
-#: ReLU mask of the fused BatchNorm backward: recomputed from x (True) or read from the saved output (False)
+#: ReLU mask of the fused BatchNorm backward: recomputed from x (True) or left by the forward pass as bits (False)
 BN_RELU_MASK_FROM_X = os.environ.get('ASDL_B200_BN_MASK_FROM_X', '1') != '0'
 
 
@@ -592,14 +592,15 @@ class _BatchNormTrain(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, running_mean, running_var, num_batches_tracked, momentum, eps,
                 residual, relu):
-        y, mean, invstd = extension().bn_forward_train(x, weight.detach(), bias.detach(), running_mean,
-                                                       running_var, num_batches_tracked, float(momentum),
-                                                       float(eps), residual, bool(relu))
         ctx.relu, ctx.has_residual = bool(relu), residual is not None
-        # ReLU without a residual: y > 0 exactly when x * scale + shift > 0, so the backward kernels recompute the
-        # mask from x (which they read anyway) and the bias, instead of reading y once more in each pass
+        # ReLU without a residual: y > 0 exactly when x * scale + shift > 0, so the backward kernel recomputes the
+        # mask from x (which it reads anyway) and the bias; with one the forward kernel leaves a bit per value
         ctx.mask_from_x = ctx.relu and not ctx.has_residual and BN_RELU_MASK_FROM_X
-        ctx.save_for_backward(x, weight, mean, invstd, *([bias] if ctx.mask_from_x else ([y] if relu else [])))
+        want_mask = ctx.relu and not ctx.mask_from_x and any(ctx.needs_input_grad)
+        y, mean, invstd, *mask = extension().bn_forward_train(x, weight.detach(), bias.detach(), running_mean,
+                                                              running_var, num_batches_tracked, float(momentum),
+                                                              float(eps), residual, ctx.relu, want_mask)
+        ctx.save_for_backward(x, weight, mean, invstd, *([bias] if ctx.mask_from_x else mask))
         ctx.mark_non_differentiable(mean, invstd)
         ctx.set_materialize_grads(False)   # no zero tensors for the statistics on every backward pass
         return y, mean, invstd
@@ -611,9 +612,9 @@ class _BatchNormTrain(torch.autograd.Function):
             dy = torch.zeros_like(x)
         if not dy.is_contiguous(memory_format=torch.channels_last):
             dy = dy.contiguous(memory_format=torch.channels_last)
-        y = rest[0] if (ctx.relu and not ctx.mask_from_x) else None
+        mask = rest[0] if (ctx.relu and not ctx.mask_from_x) else None
         bias = rest[0].detach() if ctx.mask_from_x else None
-        out = extension().bn_backward_train(x, dy, weight.detach(), mean, invstd, y, ctx.has_residual, bias)
+        out = extension().bn_backward_train(x, dy, weight.detach(), mean, invstd, mask, ctx.has_residual, bias)
         dx, dweight, dbias = out[:3]
         dres = None
         if ctx.has_residual:
@@ -637,8 +638,8 @@ def batch_norm_train(x, weight, bias, running_mean=None, running_var=None, momen
                      residual=None, relu=False, num_batches_tracked=None, return_stats=False):
     """``act(batch_norm(x) + residual)`` with batch statistics (running statistics and the batch
     counter updated in place), differentiable in x, weight, bias and residual.  CUDA, channels_last
-    bf16 activations with fp32 parameters: three kernels forward (sums, finalize, transform) and
-    three backward, each pass reading / writing every activation once with 16-byte accesses;
+    bf16 activations with fp32 parameters: one kernel forward and one backward, which keep what they have
+    summed on the chip for the transform;
     anything else: ``F.batch_norm`` followed by the add and the ReLU.  With ``return_stats`` the
     result is ``(y, mean, invstd)`` (``None`` statistics on the PyTorch path)."""
     if batch_norm_train_supported(x, weight, bias, residual):

@@ -529,6 +529,26 @@ def test_batch_norm_row_walk(n, c, h, w, relu, residual):
         assert ((got.double() - ref).abs() <= 2.0 ** -8 * (ref.abs() + ref.abs().max()) + 1e-5).all()
 
 
+@pytest.mark.parametrize('relu,residual', [(False, False), (True, False), (True, True)])
+@pytest.mark.parametrize('n,c,h,w', [(1, 8, 1, 384), (1, 136, 1, 385), (2, 72, 3, 64), (1, 24, 7, 55), (1, 40, 16, 32), (3, 16, 19, 27)])
+def test_batch_norm_rows_around_a_ring(n, c, h, w, relu, residual):
+    """12 rows per lane fill the ring of the forward pass, 6 that of the backward pass; 512 rows are one split."""
+    test_batch_norm_row_walk(n, c, h, w, relu, residual)
+
+
+@pytest.mark.parametrize('c', [8, 72])
+def test_batch_norm_mask_of_special_values(c):
+    """The gradient passes where the stored output is above zero: not at zeros of either sign, nor where it is NaN."""
+    values = torch.tensor([0.0, -0.0, 1.0, -1.0, float('inf'), float('-inf'), float('nan'), 2.0 ** -133], device=DEV)
+    res = values.repeat(64 * c // 8 * 3)[:64 * c].view(1, 64, 1, c).roll(1, 1).permute(0, 3, 1, 2).to(torch.bfloat16).requires_grad_(True)
+    x = torch.zeros_like(res)                  # normalised to zeros: the output is the ReLU of the residual
+    y = ops.batch_norm_train(x, torch.ones(c, device=DEV), torch.zeros(c, device=DEV), residual=res, relu=True)
+    dy = torch.randn_like(y)
+    grad, = torch.autograd.grad(y, res, dy)
+    assert torch.equal(y.float(), torch.nan_to_num(res.detach().float(), posinf=float('inf'), neginf=0.0).clamp(min=0))
+    assert torch.equal(grad, torch.where(y > 0, dy, torch.zeros_like(dy)))
+
+
 class _Cut(torch.autograd.Function):
     """Identity whose backward gives no gradient."""
 
