@@ -44,6 +44,13 @@ std::vector<at::Tensor> bn_backward_train(at::Tensor x, at::Tensor dy, at::Tenso
                                           c10::optional<at::Tensor> bias_for_mask);
 void bn_unitwise_stats_xhat(at::Tensor x, at::Tensor dy, c10::optional<at::Tensor> y, at::Tensor mean,
                             at::Tensor invstd, at::Tensor stats, double alpha, double beta);
+std::tuple<at::Tensor, at::Tensor, at::Tensor> batch_norm_autograd(at::Tensor x, at::Tensor weight, at::Tensor bias,
+                                                                   c10::optional<at::Tensor> running_mean,
+                                                                   c10::optional<at::Tensor> running_var,
+                                                                   c10::optional<at::Tensor> num_batches_tracked, double momentum,
+                                                                   double eps, c10::optional<at::Tensor> residual, bool relu,
+                                                                   bool mask_from_x);
+at::Tensor layer_norm_autograd(at::Tensor x, at::Tensor weight, at::Tensor bias, double eps);
 bool ln_supported_size(int64_t d);
 std::vector<at::Tensor> ln_forward(at::Tensor x, at::Tensor weight, at::Tensor bias, double eps);
 std::vector<at::Tensor> ln_backward(at::Tensor x, at::Tensor dy, at::Tensor weight, at::Tensor mean,
@@ -117,6 +124,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("bn_unitwise_stats", &b200::bn_unitwise_stats);
   m.def("bn_forward_train", &b200::bn_forward_train);
   m.def("bn_backward_train", &b200::bn_backward_train);
+  m.def("batch_norm_autograd", &b200::batch_norm_autograd);
+  m.def("layer_norm_autograd", &b200::layer_norm_autograd);
   m.def("bn_unitwise_stats_xhat", &b200::bn_unitwise_stats_xhat);
   m.def("ln_supported_size", &b200::ln_supported_size);
   m.def("ln_forward", &b200::ln_forward);

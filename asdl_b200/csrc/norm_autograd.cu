@@ -1,0 +1,92 @@
+// BatchNorm and LayerNorm as differentiable functions: the saved tensors and both passes without the interpreter, whose lock the
+// autograd thread has to wait for.  Host time of a forward and a backward pass, which bounds small and medium layers: BatchNorm with
+// a residual and ReLU 120 -> 100 us, LayerNorm with its curvature blocks 117 -> 98 (about 50 of each are PyTorch's own engine).
+#include <torch/extension.h>
+
+namespace b200 {
+
+std::vector<at::Tensor> bn_forward_train(at::Tensor x, at::Tensor weight, at::Tensor bias, c10::optional<at::Tensor> running_mean,
+                                         c10::optional<at::Tensor> running_var, c10::optional<at::Tensor> num_batches_tracked,
+                                         double momentum, double eps, c10::optional<at::Tensor> residual, bool relu, bool want_mask);
+std::vector<at::Tensor> bn_backward_train(at::Tensor x, at::Tensor dy, at::Tensor weight, at::Tensor mean, at::Tensor invstd,
+                                          c10::optional<at::Tensor> mask, bool want_dres, c10::optional<at::Tensor> bias_for_mask);
+std::vector<at::Tensor> ln_forward(at::Tensor x, at::Tensor weight, at::Tensor bias, double eps);
+std::vector<at::Tensor> ln_backward(at::Tensor x, at::Tensor dy, at::Tensor weight, at::Tensor mean, at::Tensor rstd);
+
+namespace {
+
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+struct BatchNormTrain : torch::autograd::Function<BatchNormTrain> {
+  static variable_list forward(AutogradContext* ctx, const at::Tensor& x, const at::Tensor& weight, const at::Tensor& bias,
+                               const c10::optional<at::Tensor>& running_mean, const c10::optional<at::Tensor>& running_var,
+                               const c10::optional<at::Tensor>& tracked, double momentum, double eps,
+                               const c10::optional<at::Tensor>& residual, bool relu, bool mask_from_x, bool differentiable) {
+    const bool bits = relu && !mask_from_x;
+    auto out = bn_forward_train(x, weight, bias, running_mean, running_var, tracked, momentum, eps, residual, relu, bits && differentiable);
+    variable_list saved = {x, weight, out[1], out[2]};
+    if (mask_from_x) saved.push_back(bias);
+    if (out.size() > 3) saved.push_back(out[3]);
+    ctx->save_for_backward(saved);
+    ctx->saved_data["residual"] = residual.has_value();
+    ctx->saved_data["bits"] = bits;
+    ctx->saved_data["from_x"] = mask_from_x;
+    ctx->set_materialize_grads(false);   // no zero tensors for the statistics on every backward pass
+    ctx->mark_non_differentiable({out[1], out[2]});
+    return {out[0], out[1], out[2]};
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const at::Tensor& x = saved[0];
+    at::Tensor dy = grads[0];
+    if (!dy.defined()) dy = at::zeros_like(x);   // an undefined gradient of y counts as zeros
+    dy = dy.contiguous(at::MemoryFormat::ChannelsLast);
+    const bool residual = ctx->saved_data["residual"].toBool(), bits = ctx->saved_data["bits"].toBool();
+    c10::optional<at::Tensor> mask, bias;
+    if (bits) mask = saved[4];
+    if (ctx->saved_data["from_x"].toBool()) bias = saved[4];
+    auto out = bn_backward_train(x, dy, saved[1], saved[2], saved[3], mask, residual, bias);
+    at::Tensor dres;
+    if (residual) dres = bits ? out[3] : dy;
+    const at::Tensor none;
+    return {out[0], out[1], out[2], none, none, none, none, none, dres, none, none, none};
+  }
+};
+
+struct LayerNorm : torch::autograd::Function<LayerNorm> {
+  static at::Tensor forward(AutogradContext* ctx, const at::Tensor& x, const at::Tensor& weight, const at::Tensor& bias, double eps) {
+    auto out = ln_forward(x, weight, bias, eps);
+    ctx->save_for_backward({x, weight, out[1], out[2]});
+    return out[0];
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    auto out = ln_backward(saved[0], grads[0].contiguous(), saved[1], saved[2], saved[3]);
+    return {out[0], out[1], out[2], at::Tensor()};
+  }
+};
+
+}  // namespace
+
+// (y, mean, invstd) of a training-mode BatchNorm, y = act(batch_norm(x) (+ residual)).
+std::tuple<at::Tensor, at::Tensor, at::Tensor> batch_norm_autograd(at::Tensor x, at::Tensor weight, at::Tensor bias,
+                                                                   c10::optional<at::Tensor> running_mean,
+                                                                   c10::optional<at::Tensor> running_var,
+                                                                   c10::optional<at::Tensor> num_batches_tracked, double momentum,
+                                                                   double eps, c10::optional<at::Tensor> residual, bool relu,
+                                                                   bool mask_from_x) {
+  const bool differentiable = at::GradMode::is_enabled() && (x.requires_grad() || weight.requires_grad() || bias.requires_grad() ||
+                                                             (residual.has_value() && residual->requires_grad()));
+  auto out = BatchNormTrain::apply(x, weight, bias, running_mean, running_var, num_batches_tracked, momentum, eps, residual, relu,
+                                   relu && !residual.has_value() && mask_from_x, differentiable);
+  return {out[0], out[1], out[2]};
+}
+
+at::Tensor layer_norm_autograd(at::Tensor x, at::Tensor weight, at::Tensor bias, double eps) {
+  return LayerNorm::apply(x, weight, bias, eps);
+}
+
+}  // namespace b200

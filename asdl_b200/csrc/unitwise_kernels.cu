@@ -305,12 +305,12 @@ int current_device() {
 
 void ln_unitwise_stats(at::Tensor y, at::Tensor g, at::Tensor weight, at::Tensor bias, at::Tensor stats, double alpha,
                        double beta) {
-  TORCH_CHECK(y.is_cuda() && g.is_cuda() && y.dim() == 2 && y.sizes() == g.sizes() && y.is_contiguous() &&
-                  g.is_contiguous() && y.scalar_type() == g.scalar_type(), "y and g must be contiguous [rows, d] CUDA tensors");
+  TORCH_CHECK(y.is_cuda() && g.is_cuda() && y.dim() >= 1 && y.numel() == g.numel() && y.is_contiguous() &&
+                  g.is_contiguous() && y.scalar_type() == g.scalar_type(), "y and g must be contiguous [..., d] CUDA tensors");
   const bool bf16 = y.scalar_type() == at::kBFloat16;
   TORCH_CHECK(bf16 || y.scalar_type() == at::kFloat, "y must be bf16 or fp32");
-  const long long rows = y.size(0);
-  const int d = static_cast<int>(y.size(1));
+  const int d = static_cast<int>(y.size(-1));
+  const long long rows = d == 0 ? 0 : y.numel() / d;
   TORCH_CHECK(weight.is_cuda() && bias.is_cuda() && weight.scalar_type() == at::kFloat && bias.scalar_type() == at::kFloat &&
                   weight.is_contiguous() && bias.is_contiguous() && weight.numel() == d && bias.numel() == d,
               "weight / bias must be contiguous fp32 [d]");

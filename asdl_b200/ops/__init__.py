@@ -587,7 +587,8 @@ BN_RELU_MASK_FROM_X = os.environ.get('ASDL_B200_BN_MASK_FROM_X', '1') != '0'
 
 
 class _BatchNormTrain(torch.autograd.Function):
-    """Training-mode batch normalisation (+ residual add, + ReLU) on the library's NHWC bf16 kernels."""
+    """Training-mode batch normalisation (+ residual add, + ReLU) on the library's NHWC bf16 kernels, for ``torch.jit.trace``, which
+    records a function of Python as a call and would only see the allocations of a native one."""
 
     @staticmethod
     def forward(ctx, x, weight, bias, running_mean, running_var, num_batches_tracked, momentum, eps,
@@ -643,8 +644,12 @@ def batch_norm_train(x, weight, bias, running_mean=None, running_var=None, momen
     anything else: ``F.batch_norm`` followed by the add and the ReLU.  With ``return_stats`` the
     result is ``(y, mean, invstd)`` (``None`` statistics on the PyTorch path)."""
     if batch_norm_train_supported(x, weight, bias, residual):
-        y, mean, invstd = _BatchNormTrain.apply(x, weight, bias, running_mean, running_var,
-                                                num_batches_tracked, momentum, eps, residual, relu)
+        if torch._C._get_tracing_state() is None:
+            y, mean, invstd = extension().batch_norm_autograd(x, weight, bias, running_mean, running_var, num_batches_tracked,
+                                                              momentum, eps, residual, relu, BN_RELU_MASK_FROM_X)
+        else:
+            y, mean, invstd = _BatchNormTrain.apply(x, weight, bias, running_mean, running_var,
+                                                    num_batches_tracked, momentum, eps, residual, relu)
         return (y, mean, invstd) if return_stats else y
     if num_batches_tracked is not None:
         num_batches_tracked.add_(1)
@@ -679,7 +684,7 @@ def batchnorm_unitwise_stats_from_input(x, dy, y, mean, invstd, out, alpha=1.0, 
 
 
 class _LayerNormFn(torch.autograd.Function):
-    """LayerNorm over the last dimension on the library's bf16 kernels."""
+    """LayerNorm over the last dimension on the library's bf16 kernels, for ``torch.jit.trace`` (see ``_BatchNormTrain``)."""
 
     @staticmethod
     def forward(ctx, x, weight, bias, eps):
@@ -710,6 +715,8 @@ def layer_norm(x, weight, bias, eps=1e-5):
     backward (the input gradient and the weight / bias gradients come out of one pass over dy and
     x); anything else: ``F.layer_norm``."""
     if layer_norm_supported(x, weight, bias):
+        if torch._C._get_tracing_state() is None:
+            return extension().layer_norm_autograd(x, weight, bias, eps)
         return _LayerNormFn.apply(x, weight, bias, eps)
     return torch.nn.functional.layer_norm(x, (weight.numel(),) if weight is not None else x.shape[-1:],
                                           weight, bias, eps)
@@ -756,8 +763,7 @@ def layernorm_unitwise_stats(y: torch.Tensor, g: torch.Tensor, weight: torch.Ten
         beta = 0.0
     if (cuda_kernels_enabled(y, g) and weight.ndim == 1 and y.shape[-1] == d and y.dtype == g.dtype
             and y.dtype in (torch.bfloat16, torch.float32) and weight.dtype == torch.float32 and out.is_contiguous()):
-        extension().ln_unitwise_stats(y.reshape(-1, d).contiguous(), g.reshape(-1, d).contiguous(),
-                                      weight.detach().contiguous(), bias.detach().contiguous(), out,
+        extension().ln_unitwise_stats(y.contiguous(), g.contiguous(), weight.contiguous(), bias.contiguous(), out,
                                       float(alpha), float(beta))
         return out
     k = weight.ndim

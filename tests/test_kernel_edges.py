@@ -549,6 +549,53 @@ def test_batch_norm_mask_of_special_values(c):
     assert torch.equal(grad, torch.where(y > 0, dy, torch.zeros_like(dy)))
 
 
+def _norm_calls():
+    def act(*shape):
+        return torch.randn(*shape, device=DEV, generator=_gen(30)).to(torch.bfloat16)
+    x, res = (act(4, 16, 5, 5).contiguous(memory_format=torch.channels_last).requires_grad_(True) for _ in range(2))
+    weight, bias = (torch.rand(16, device=DEV, generator=_gen(31)).requires_grad_(True) for _ in range(2))
+    wide, gain, shift = act(6, 256).requires_grad_(True), torch.ones(256, device=DEV).requires_grad_(True), torch.zeros(256, device=DEV)
+    return [(lambda x, w, b: ops.batch_norm_train(x, w, b, relu=True), (x, weight, bias)),
+            (lambda x, w, b, r: ops.batch_norm_train(x, w, b, residual=r, relu=True), (x, weight, bias, res)),
+            (lambda x, w, b, r: ops.batch_norm_train(x, w, b, residual=r), (x, weight, bias, res)),
+            (lambda x, w, b: ops.layer_norm(x, w, b), (wide, gain, shift))]
+
+
+@pytest.mark.parametrize('which', range(4))
+def test_native_norm_functions_keep_the_rules_of_autograd(which):
+    fn, args = _norm_calls()[which]
+    leaves = [a for a in args if a.requires_grad]
+    y = fn(*args)
+    dy = torch.randn_like(y)
+    want = torch.autograd.grad(y, leaves, dy)
+    # saved tensors go through hooks, and are gone after the first pass
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t) or len(packed) - 1, lambda i: packed[i].clone()):
+        y2 = fn(*args)
+    assert packed
+    for a, b in zip(torch.autograd.grad(y2, leaves, dy), want):
+        assert torch.equal(a, b)
+    with pytest.raises(RuntimeError, match='second time'):
+        torch.autograd.grad(y2, leaves, dy)
+    # a trace runs the kernels again instead of returning what its allocations hold
+    if which < 3:   # sizes are tensors in a trace, so that a LayerNorm goes to PyTorch's, which refuses bf16 with fp32 parameters
+        traced = torch.jit.trace(fn, tuple(a.detach() for a in args), check_trace=False)
+        assert torch.equal(traced(*(2 * a.detach() for a in args)), fn(*(2 * a.detach() for a in args)))
+    # transforms that a kernel has no rule for are refused
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda x: fn(x, *args[1:]).float().sum())(args[0])
+    with pytest.raises(RuntimeError), torch.autograd.forward_ad.dual_level():
+        fn(torch.autograd.forward_ad.make_dual(args[0].detach(), torch.ones_like(args[0])), *args[1:])
+    with torch.no_grad():
+        assert not fn(*args).requires_grad and torch.equal(fn(*args), y)
+    args[0].data.add_(0)   # not seen by autograd
+    y3 = fn(*args)
+    with torch.no_grad():
+        args[0].mul_(1)
+    with pytest.raises(RuntimeError, match='inplace'):
+        torch.autograd.grad(y3, leaves, dy)
+
+
 class _Cut(torch.autograd.Function):
     """Identity whose backward gives no gradient."""
 
