@@ -51,6 +51,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> batch_norm_autograd(at::Tensor x,
                                                                    double eps, c10::optional<at::Tensor> residual, bool relu,
                                                                    bool mask_from_x);
 at::Tensor layer_norm_autograd(at::Tensor x, at::Tensor weight, at::Tensor bias, double eps);
+at::Tensor max_pool_autograd(at::Tensor x, int64_t pad);
 bool ln_supported_size(int64_t d);
 std::vector<at::Tensor> ln_forward(at::Tensor x, at::Tensor weight, at::Tensor bias, double eps);
 std::vector<at::Tensor> ln_backward(at::Tensor x, at::Tensor dy, at::Tensor weight, at::Tensor mean,
@@ -126,6 +127,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("bn_backward_train", &b200::bn_backward_train);
   m.def("batch_norm_autograd", &b200::batch_norm_autograd);
   m.def("layer_norm_autograd", &b200::layer_norm_autograd);
+  m.def("max_pool_autograd", &b200::max_pool_autograd);
   m.def("bn_unitwise_stats_xhat", &b200::bn_unitwise_stats_xhat);
   m.def("ln_supported_size", &b200::ln_supported_size);
   m.def("ln_forward", &b200::ln_forward);

@@ -4,7 +4,7 @@ import torch.nn as nn
 
 from .. import ops
 
-__all__ = ['FusedBatchNorm2d', 'FusedLayerNorm', 'grouped_bf16_weights']
+__all__ = ['FusedBatchNorm2d', 'FusedLayerNorm', 'FusedMaxPool2d', 'grouped_bf16_weights']
 
 
 class FusedBatchNorm2d(nn.BatchNorm2d):
@@ -87,6 +87,27 @@ class FusedLayerNorm(nn.LayerNorm):
             xb = xb if xb.is_contiguous() else xb.contiguous()
             if ops.layer_norm_supported(xb, self.weight, self.bias):
                 return ops.layer_norm(xb, self.weight, self.bias, self.eps)
+        return super().forward(x)
+
+
+class FusedMaxPool2d(nn.MaxPool2d):
+    """``nn.MaxPool2d`` whose forward / backward run on the library's NHWC kernels for 3 x 3 windows with stride 2 and channels_last
+    bf16 CUDA inputs with a multiple of 8 channels, and exactly like the parent otherwise, traced and under ``torch.func`` or
+    forward-mode differentiation too.  Same values and gradients."""
+
+    def _native(self, x):
+        p = self.padding
+        return (self.kernel_size == 3 and self.stride == 2 and (p == 0 or p == 1) and self.dilation == 1 and not self.return_indices
+                and not self.ceil_mode and x.is_cuda and x.dtype == torch.bfloat16 and x.ndim == 4
+                and torch._C._get_tracing_state() is None and not torch._C._are_functorch_transforms_active()
+                and not torch.compiler.is_compiling()
+                and torch.autograd.forward_ad._current_level < 0 and ops.cuda_kernels_enabled(x) and x.numel() > 0
+                and x.shape[1] % 8 == 0 and x.shape[0] <= 65535 and min(x.shape[2:]) + 2 * p >= 3 and max(x.shape[2:]) < 2 ** 30
+                and x.shape[1] * (x.shape[3] + 2) < 2 ** 33 and x.is_contiguous(memory_format=torch.channels_last) and x.data_ptr() % 16 == 0)
+
+    def forward(self, x):
+        if self._native(x):
+            return ops.extension().max_pool_autograd(x, self.padding)
         return super().forward(x)
 
 

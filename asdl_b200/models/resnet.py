@@ -7,7 +7,7 @@ ResNets of its own (examples/arxiv_results/models/resnet.py)."""
 import torch
 import torch.nn as nn
 
-from .layers import FusedBatchNorm2d, grouped_bf16_weights
+from .layers import FusedBatchNorm2d, FusedMaxPool2d, grouped_bf16_weights
 
 __all__ = ['ResNet', 'Bottleneck', 'resnet50', 'resnet_tiny']
 
@@ -51,7 +51,7 @@ class ResNet(nn.Module):
         self.conv1 = nn.Conv2d(in_channels, width, 7, stride=2, padding=3, bias=False)
         self.bn1 = FusedBatchNorm2d(width, act='relu' if fused else None)
         self.relu = nn.ReLU(inplace=False)
-        self.maxpool = nn.MaxPool2d(3, stride=2, padding=1)
+        self.maxpool = FusedMaxPool2d(3, stride=2, padding=1)
         self.layer1 = self._make_layer(width, layers[0])
         self.layer2 = self._make_layer(width * 2, layers[1], stride=2)
         self.layer3 = self._make_layer(width * 4, layers[2], stride=2)

@@ -4,6 +4,7 @@ import torch
 import torch.nn.functional as F
 
 from asdl_b200 import ops
+from asdl_b200.models.layers import FusedMaxPool2d
 
 pytestmark = pytest.mark.gpu
 DEV = 'cuda'
@@ -547,6 +548,32 @@ def test_batch_norm_mask_of_special_values(c):
     grad, = torch.autograd.grad(y, res, dy)
     assert torch.equal(y.float(), torch.nan_to_num(res.detach().float(), posinf=float('inf'), neginf=0.0).clamp(min=0))
     assert torch.equal(grad, torch.where(y > 0, dy, torch.zeros_like(dy)))
+
+
+@pytest.mark.parametrize('padding', [0, 1])
+@pytest.mark.parametrize('n,c,h,w', [(2, 64, 17, 18), (1, 8, 3, 3), (3, 24, 16, 33), (2, 264, 15, 40), (1, 16, 32, 4)])
+def test_max_pool_gives_the_bits_of_pytorch(padding, n, c, h, w):
+    kernel, stride = 3, 2
+    pool = FusedMaxPool2d(kernel, stride=stride, padding=padding)
+    x = torch.randn(n, c, h, w, device=DEV, generator=_gen(32)).mul_(2).round_().to(torch.bfloat16)   # many equal values
+    x.view(-1)[::97] = float('nan')
+    x.view(-1)[::61] = float('-inf')
+    x[0, :, :8, :8] = float('-inf')   # whole windows
+    x = x.contiguous(memory_format=torch.channels_last).requires_grad_(True)
+    assert pool._native(x)
+    y, want = pool(x), F.max_pool2d(x, kernel, stride, padding)
+    assert y.shape == want.shape and y.is_contiguous(memory_format=torch.channels_last)
+    assert torch.equal(y.nan_to_num(nan=1e4), want.nan_to_num(nan=1e4))
+    dy = torch.randn_like(want)
+    got, ref = torch.autograd.grad(y, x, dy, retain_graph=True)[0], torch.autograd.grad(want, x, dy)[0]
+    assert torch.equal(got, ref)
+    # twice differentiable: the second pass is the gather of what the first one scatters
+    g = dy.clone().requires_grad_(True)
+    back, = torch.autograd.grad(y, x, g, create_graph=True)
+    v = torch.randn_like(back)
+    again, = torch.autograd.grad(back, g, v)
+    _, where = F.max_pool2d(x.detach(), kernel, stride, padding, return_indices=True)
+    assert torch.equal(again, v.flatten(2).gather(2, where.flatten(2)).view_as(again))
 
 
 def _norm_calls():
