@@ -96,7 +96,7 @@ struct alignas(64) GemmProblem2 {
   __nv_bfloat16* out_hi;  // optional bf16 image of the result
   __nv_bfloat16* out_mid; // optional second part of a three-way split (needs out_hi and out_lo)
   __nv_bfloat16* out_lo;  // optional residual
-  float* ws;              // split-K scratch: [tile][split][128][BN] fp32
+  float* ws;              // split-K scratch: [tile][split][BN / 4][128][4] fp32
   int* status;            // device error word
   float* C_extra[G2_MAX_EXTRA];  // plain copies of the fp32 result (same ldc), e.g. peer GPUs
   int n_extra;
@@ -273,6 +273,17 @@ __device__ __forceinline__ void g2_reduce_chunk(const G2Epi& P, const float* v, 
         g2_red_add_f32(P.C + static_cast<size_t>(gc) * P.ldc + gr, alpha * v[j]);
     }
   }
+}
+
+// Partial tiles of split-K lie as [columns / 4][128 rows][4 columns]: a warp, whose lanes hold a row each, stores 512 bytes in a row, and
+// the reduction loads them the same way.  With rows of the tile in memory every store instruction touched 32 half sectors: product
+// and reduction of 8192 x 1024 bf16 samples 22.6 -> 19.1 us, of 8192 x 2048 45.5 -> 41.3, of 12608 x 768 fp32 samples with their cast 45.0 -> 41.9,
+// a 768 x 768 gradient between fp32 factors 38.8 -> 33.1.
+__device__ __forceinline__ void g2_store_partial(float* tile, const float (&v)[64], int row, int col0) {
+  float* at = tile + (col0 / 4 * G2_BM + row) * 4;
+#pragma unroll
+  for (int j = 0; j < 16; ++j)
+    *reinterpret_cast<float4*>(at + j * G2_BM * 4) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
 }
 
 // Final store of 32 consecutive columns of one row held by this thread.
@@ -719,14 +730,10 @@ umma_gemm2_kernel(const __grid_constant__ GemmProblem2 single, const GemmProblem
       const bool to_ws = P.nsplit > 1 && !atomic;
       const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
 
-      auto finish = [&](const float* v, int col0) {
+      auto finish = [&](const float (&v)[64], int col0) {
         // v: 64 consecutive columns of this thread's row starting at tile column col0
         if (to_ws) {
-          float* part = P.ws + (static_cast<size_t>(w.tile_id) * P.nsplit + w.split) * (G2_BM * BN) +
-                        static_cast<size_t>(row) * BN + col0;
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            *reinterpret_cast<float4*>(part + 4 * j) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          g2_store_partial(P.ws + (static_cast<size_t>(w.tile_id) * P.nsplit + w.split) * (G2_BM * BN), v, row, col0);
           return;
         }
 #pragma unroll
@@ -818,10 +825,11 @@ umma_gemm2_kernel(const __grid_constant__ GemmProblem2 single, const GemmProblem
   }
 }
 
-// Sums split-K partials and applies the epilogue.  One block handles a ROWS x 64 patch of one tile; a thread owns four
-// consecutive columns of ROWS / 16 rows, and eight 16-byte loads of partials are in flight (the kernel reads nsplit times what
-// it writes and does nothing else; with 4-byte loads of one split at a time it ran at 1.3 TB/s).  The mirrored store goes
-// through shared memory.  Partials are added in split order.  Patches have 32 rows, or 16 where those still leave SMs without a
+// Sums split-K partials and applies the epilogue.  One block handles a ROWS x 64 patch of one tile; a thread adds up four
+// consecutive columns of ROWS / 16 row positions, and eight 16-byte loads of partials are in flight (the kernel reads nsplit times
+// what it writes and does nothing else; with 4-byte loads of one split at a time it ran at 1.3 TB/s).  The sums change hands through
+// shared memory, since partials are stored column by column and the result row by row; the mirrored store reads them there too.
+// Partials are added in split order.  Patches have 32 rows, or 16 where those still leave SMs without a
 // block: what one SM can load bounds it then.
 // grid: (work items, 128 / ROWS * BN / 64).
 constexpr int G2_RED_COLS = 64;
@@ -871,8 +879,10 @@ splitk_reduce2_kernel(const __grid_constant__ GemmProblem2 single, const GemmPro
   if (row0 >= P.M || col0 >= P.N) return;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   constexpr size_t SPLIT = static_cast<size_t>(G2_BM) * BN;   // floats of one split's partial tile
+  const int pr = threadIdx.x & (ROWS - 1), pq = threadIdx.x / ROWS;   // row and first group of four columns of this thread's partials
+  constexpr int GROUP = 256 / ROWS;                                   // to the next one
   const float* p0 = after_wait(P.ws) + static_cast<size_t>(w.tile_id) * P.nsplit * SPLIT +
-                    static_cast<size_t>(sub_r * ROWS + ty) * BN + sub_c * G2_RED_COLS + tx * 4;
+                    static_cast<size_t>(((sub_c * (G2_RED_COLS / 4) + pq) * G2_BM + sub_r * ROWS + pr) * 4);
   const int gc = col0 + tx * 4;
   const bool full = gc + 4 <= P.N;
   const bool vec_in = full && g2_vec_ok(P.Cin, P.ldc), vec_out = full && g2_vec_ok(P.C, P.ldc);
@@ -907,7 +917,7 @@ splitk_reduce2_kernel(const __grid_constant__ GemmProblem2 single, const GemmPro
 #pragma unroll
       for (int i = 0; i < R; ++i)
         v[i][u] = all || s + u < P.nsplit
-                      ? __ldcg(reinterpret_cast<const float4*>(p0 + static_cast<size_t>(16 * i) * BN + static_cast<size_t>(s + u) * SPLIT))
+                      ? __ldcg(reinterpret_cast<const float4*>(p0 + GROUP * i * G2_BM * 4 + static_cast<size_t>(s + u) * SPLIT))
                       : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int u = 0; u < SPLITS; ++u)
@@ -925,6 +935,11 @@ splitk_reduce2_kernel(const __grid_constant__ GemmProblem2 single, const GemmPro
   if constexpr (ROWS == 16)   // many splits: 1 us of 19 less; with few splits per tile it costs as much
     for (; s + SPLITS <= P.nsplit; s += SPLITS) add_round(std::true_type{}, s);
   for (; s < P.nsplit; s += SPLITS) add_round(std::false_type{}, s);
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) tile[pr][(pq + GROUP * i) * 4 + j] = acc[i][j];
+  __syncthreads();
   const bool mirror_bf16 = sym && !(P.flags & G2F_LOWER);
 #pragma unroll
   for (int i = 0; i < R; ++i) {
@@ -932,7 +947,7 @@ splitk_reduce2_kernel(const __grid_constant__ GemmProblem2 single, const GemmPro
     float val[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      val[j] = P.alpha * acc[i][j];
+      val[j] = P.alpha * tile[lr][tx * 4 + j];
       if (P.beta != 0.f) val[j] += P.beta * cin[i][j];
       tile[lr][tx * 4 + j] = val[j];
     }

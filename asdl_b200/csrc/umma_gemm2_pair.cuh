@@ -355,11 +355,7 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
         }
         if (c_row >= E.M) continue;   // the lower half of the last pair row of an odd tile count: nothing to write
         if (to_ws) {
-          float* part = E.ws + (static_cast<size_t>(tile_id) * E.nsplit + w.split) * (G2_BM * BN) +
-                        static_cast<size_t>(row) * BN + col0;
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            *reinterpret_cast<float4*>(part + 4 * j) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          g2_store_partial(E.ws + (static_cast<size_t>(tile_id) * E.nsplit + w.split) * (G2_BM * BN), v, row, col0);
           continue;
         }
 #pragma unroll
