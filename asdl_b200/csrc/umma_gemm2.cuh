@@ -47,16 +47,20 @@ constexpr int G2_MAX_SEG = 6;
 constexpr int G2_MAX_EXTRA = 7;
 constexpr int G2_MAX_BATCH = 256;   // problems of one launch in batch mode
 constexpr int G2_A_BYTES = G2_BM * G2_BK * 2;  // 16 KiB
+constexpr int G2_PATCH = 16;        // columns of a result that an epilogue warp stages at a time (two CTAs per SM leave 3 KiB per warp)
 
 template <int BN, int EPI_WARPS, int MINB, int PARTS>
 struct G2Cfg {
+  // results go out by way of shared memory where statistics are formed; in the flavours of two-sided products, whose results are
+  // bf16 images or only written, the second path through the epilogue cost 3 - 10 us (1024 x 4096: 134.9 -> 144.6)
+  static constexpr bool STAGED = PARTS == 1 && BN == 128;
   static constexpr int STAGES = PARTS > 1 ? 2 : (BN == 256 ? 4 : (MINB == 2 ? 3 : 6));
   static constexpr int B_BYTES = BN * G2_BK * 2;
   static constexpr int STAGE_BYTES = PARTS * (G2_A_BYTES + B_BYTES);
   static constexpr int TMEM_COLS = 2 * BN;
   static constexpr int THREADS = 64 + 32 * EPI_WARPS;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align slack*/ + 256 /*barriers*/ +
-                                    4 * (G2_MAX_BATCH + 4) /*item prefix of a batch*/;
+                                    4 * (G2_MAX_BATCH + 4) /*item prefix of a batch*/ + (STAGED ? EPI_WARPS * 32 * G2_PATCH * 4 : 0);
 };
 using G2Plain = G2Cfg<128, 4, 2, 1>;
 using G2Wide = G2Cfg<256, 8, 1, 1>;
@@ -449,6 +453,140 @@ __device__ __forceinline__ void g2_store_chunk(const G2Epi& P, const float* v, i
   }
 }
 
+// ---- results that only go to C: by way of shared memory ----
+// A lane holds a row of the accumulator, so that its stores (and loads of C for beta) touch 32 rows each, half a sector of every one, and
+// code that handles 64 columns in a straight line is bound by instruction fetch where a CTA has one tile: 18 000 of the 26 500 clocks of a
+// 784 x 784 factor of 128 samples were its epilogue, now 5 000.  A warp stages 32 rows x COLS columns at a time in one loop, stores whole segments of rows, then the mirror image; C for beta comes in
+// one patch ahead.  Graph replay: 128 x 784 fp32 samples 16.5 -> 12.9 us, 600 x 512 25.1 -> 20.1, 64 x 2000 bf16 16.0 -> 12.3, 64 x 1801 31.9 -> 18.3,
+// 2048 x 3072 47.0 -> 37.5, 8192 x 4096 (CTA pairs) 118 -> 112.  Rows of the patch are COLS * 4 bytes, their 16-byte pieces exchanged so that neither order of access conflicts.
+template <int COLS>
+__device__ __forceinline__ uint32_t g2_patch_at(uint32_t stg, int r, int piece) {
+  return stg + r * (COLS * 4) + ((piece ^ (COLS == 16 ? (r >> 1) & 3 : r & 7)) << 4);
+}
+__device__ __forceinline__ float4 g2_lds(uint32_t at) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+  return v;
+}
+__device__ __forceinline__ void g2_sts(uint32_t at, float x, float y, float z, float w) {
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
+// What this store takes; the rest (bf16 images, copies on peers, reductions into C) goes out from registers, and so does a result that
+// is only written, 16 bytes at a time: nothing waits for those stores.
+__device__ __forceinline__ bool g2_staged(const G2Epi& P) {
+  return P.C != nullptr && P.out_hi == nullptr && P.n_extra == 0 && !(P.flags & G2F_ATOMIC) &&
+         ((P.flags & G2F_SYM) || P.beta != 0.f || !g2_vec_ok(P.C, P.ldc));
+}
+// p[index * ldc], one instruction for the address
+__device__ __forceinline__ float* g2_line(float* p, int ldc, int index) {
+  return reinterpret_cast<float*>(reinterpret_cast<char*>(p) + static_cast<long long>(ldc) * (4 * index));
+}
+// Columns [gc_first, gc_first + TOTAL) of a tile whose rows begin at c_row, this warp's 32 rows from row0 on.  ready(): waits for the
+// accumulator (false: give up); read(c, v): columns c .. c + COLS of this lane's row; release(): everything has been read.
+// Few instructions matter: the epilogue has one warp per scheduler, so each of them takes its full latency.
+template <int COLS, int TOTAL, typename Ready, typename Read, typename Release>
+__device__ __forceinline__ bool g2_store_columns(const G2Epi& P, uint32_t stg, int c_row, int row0, int gc_first, int lane, Ready ready, Read read,
+                                                 Release release) {
+  constexpr int PIECES = COLS / 4, STEP = 32 / PIECES, TURNS = PIECES;   // lanes of a row, rows of an access, accesses
+  const float alpha = P.alpha, beta = P.beta;
+  const int M = P.M, N = P.N, ldc = P.ldc;
+  const bool sym = (P.flags & G2F_SYM) != 0, mirror = sym && !(P.flags & G2F_LOWER);
+  const int piece = lane % PIECES, r0 = lane / PIECES, gr0 = row0 + r0;
+  float* const C = P.C + static_cast<size_t>(gr0) * ldc + 4 * piece;
+  float* const Cin = const_cast<float*>(P.Cin) + static_cast<size_t>(gr0) * ldc + 4 * piece;
+  const bool vec_out = g2_vec_ok(P.C, ldc), vec_in = g2_vec_ok(P.Cin, ldc), rows_in = row0 + 32 <= M;
+  // columns to store: inside the matrix, and of a symmetric result (wide tiles may reach past the diagonal) up to the diagonal
+  const int end = row0 >= M ? 0 : min(N, sym ? min((c_row / G2_BM + 1) * G2_BM, row0 + 32) : N) - gc_first;
+  float4 ahead[TURNS];
+  auto fetch = [&](int gc0) {
+    const int gc = gc0 + 4 * piece;
+    if (rows_in && vec_in && gc0 + COLS <= N) {
+#pragma unroll
+      for (int u = 0; u < TURNS; ++u) ahead[u] = *reinterpret_cast<const float4*>(g2_line(Cin + gc0, ldc, u * STEP));
+      return;
+    }
+#pragma unroll
+    for (int u = 0; u < TURNS; ++u) {
+      const float* from = g2_line(Cin + gc0, ldc, u * STEP);
+      const bool there = gr0 + u * STEP < M;
+      ahead[u].x = there && gc < N ? from[0] : 0.f;
+      ahead[u].y = there && gc + 1 < N ? from[1] : 0.f;
+      ahead[u].z = there && gc + 2 < N ? from[2] : 0.f;
+      ahead[u].w = there && gc + 3 < N ? from[3] : 0.f;
+    }
+  };
+  if (beta != 0.f && end > 0) fetch(gc_first);
+  if (!ready()) return false;
+  if (end <= 0) release();
+#pragma unroll 1
+  for (int c = 0; c < TOTAL && c < end; c += COLS) {
+    const int gc0 = gc_first + c;
+    const bool diag = sym && gc0 / G2_BM == c_row / G2_BM;   // keep the lower triangle
+    float v[COLS];
+    read(c, v);
+    if (c + COLS >= TOTAL || c + COLS >= end) release();
+    if (beta == 0.f) {
+#pragma unroll
+      for (int k = 0; k < COLS; ++k) v[k] *= alpha;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < PIECES; ++k) g2_sts(g2_patch_at<COLS>(stg, lane, k), v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+    __syncwarp();
+    float4 w[TURNS], old[TURNS];
+#pragma unroll
+    for (int u = 0; u < TURNS; ++u) old[u] = ahead[u];
+    if (beta != 0.f && c + COLS < TOTAL && c + COLS < end) fetch(gc0 + COLS);
+#pragma unroll
+    for (int u = 0; u < TURNS; ++u) w[u] = g2_lds(g2_patch_at<COLS>(stg, r0 + u * STEP, piece));
+    if (beta != 0.f) {
+#pragma unroll
+      for (int u = 0; u < TURNS; ++u) {
+        w[u] = make_float4(fmaf(beta, old[u].x, alpha * w[u].x), fmaf(beta, old[u].y, alpha * w[u].y),
+                           fmaf(beta, old[u].z, alpha * w[u].z), fmaf(beta, old[u].w, alpha * w[u].w));
+        if (mirror) g2_sts(g2_patch_at<COLS>(stg, r0 + u * STEP, piece), w[u].x, w[u].y, w[u].z, w[u].w);
+      }
+    }
+    if (rows_in && vec_out && gc0 + COLS <= N && !(diag && gc0 + COLS - 1 > row0)) {
+#pragma unroll
+      for (int u = 0; u < TURNS; ++u) *reinterpret_cast<float4*>(g2_line(C + gc0, ldc, u * STEP)) = w[u];
+    } else {
+      const int gc = gc0 + 4 * piece;
+#pragma unroll
+      for (int u = 0; u < TURNS; ++u) {
+        const int gr = gr0 + u * STEP, stop = gr < M ? min(N, diag ? gr + 1 : N) - gc : 0;
+        float* to = g2_line(C + gc0, ldc, u * STEP);
+        if (stop > 0) to[0] = w[u].x;
+        if (stop > 1) to[1] = w[u].y;
+        if (stop > 2) to[2] = w[u].z;
+        if (stop > 3) to[3] = w[u].w;
+      }
+    }
+    if (mirror) {   // so that the result is exactly symmetric
+      if (beta != 0.f) {
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < PIECES; ++k) {
+          const float4 x = g2_lds(g2_patch_at<COLS>(stg, lane, k));
+          v[4 * k] = x.x, v[4 * k + 1] = x.y, v[4 * k + 2] = x.z, v[4 * k + 3] = x.w;
+        }
+      }
+      const int gr = row0 + lane;
+      float* const to = P.C + static_cast<size_t>(gc0) * ldc + gr;
+      if (rows_in && gc0 + COLS <= N && !(diag && gc0 + COLS > row0)) {
+#pragma unroll
+        for (int k = 0; k < COLS; ++k) *g2_line(to, ldc, k) = v[k];
+      } else {
+        const int stop = gr < M ? min(N, diag ? gr : N) - gc0 : 0;
+#pragma unroll
+        for (int k = 0; k < COLS; ++k)
+          if (k < stop) *g2_line(to, ldc, k) = v[k];
+      }
+    }
+  }
+  return true;
+}
+
 template <int BN, int EPI_WARPS, int MINB, int PARTS>
 __global__ void __launch_bounds__(64 + 32 * EPI_WARPS, MINB)
 umma_gemm2_kernel(const __grid_constant__ GemmProblem2 single, const GemmProblem2* __restrict__ probs,
@@ -716,6 +854,7 @@ umma_gemm2_kernel(const __grid_constant__ GemmProblem2 single, const GemmProblem
     const int col_base = ((warp - 2) >> 2) * COLS;            // first column of this warp's share
     constexpr int PASSES = COLS / 64;
     const int row = q * 32 + lane;
+    const uint32_t stg = smem_u32(smem + STAGES * Cfg::STAGE_BYTES + 256 + 4 * (G2_MAX_BATCH + 4)) + (warp - 2) * 32 * G2_PATCH * 4;
     uint32_t ch = 0;
     bool ok = true;
     for (int wi = blockIdx.x; wi < n_work && ok; wi += gridDim.x) {
@@ -753,6 +892,32 @@ umma_gemm2_kernel(const __grid_constant__ GemmProblem2 single, const GemmProblem
 
       if constexpr (!SPLIT3) {
         const uint32_t ab = ch & 1;
+        if (Cfg::STAGED && !to_ws && nchunks == 1 && g2_staged(P)) {
+          const uint32_t from = tmem_base + lane_addr + ab * BN + col_base;
+          ok = g2_store_columns<G2_PATCH, COLS>(
+              P, stg, w.c_row, w.c_row + q * 32, w.c_col + col_base, lane,
+              [&] {
+                bool there = mbar_wait(&acc_full[ab], (ch >> 1) & 1);
+                if (!there) set_error(status, ERR_WAIT_ACC);
+                there = __all_sync(0xffffffffu, there);
+                tc_fence_after_sync();
+                return there;
+              },
+              [&](int c, float (&v)[G2_PATCH]) {
+                uint32_t r[G2_PATCH];
+                tmem_ld_32x16(from + c, r);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < G2_PATCH; ++j) v[j] = __uint_as_float(r[j]);
+              },
+              [&] {
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_empty[ab]);
+              });
+          ++ch;
+          continue;
+        }
         if (nchunks == 1) {
           ok = mbar_wait(&acc_full[ab], (ch >> 1) & 1);
           if (!ok) set_error(status, ERR_WAIT_ACC);

@@ -45,7 +45,9 @@ struct G2PairCfg {
 constexpr int G2P_EPI_WARPS = 8;
 constexpr int G2P_THREADS = 64 + 32 * G2P_EPI_WARPS;
 constexpr int G2P_TMEM_COLS = 512;                          // two 256-column accumulators
+constexpr int G2P_PATCH = 32;                               // columns of a result that an epilogue warp stages at a time
 constexpr int G2P_SMEM_BYTES = 6 * 2 * G2_A_BYTES + 1024 + 256;
+constexpr int G2P_STAGED_BYTES = G2P_EPI_WARPS * 32 * G2P_PATCH * 4;   // of the flavour without parts (G2Cfg::STAGED)
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -300,7 +302,8 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
     const G2Epi E = g2_epi(P);
     const bool sym = (E.flags & G2F_SYM) != 0;
     const bool atomic = (E.flags & G2F_ATOMIC) != 0;
-    const bool to_ws = E.nsplit > 1 && !atomic;
+    const bool to_ws = E.nsplit > 1 && !atomic, staged = !to_ws && g2_staged(E);
+    const uint32_t stg = smem_u32(smem + STAGES * STAGE_BYTES + 256) + (warp - 2) * 32 * G2P_PATCH * 4;
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     uint32_t ch = 0;
     bool ok = true;
@@ -313,6 +316,32 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
       const int gr = c_row + row;
       const bool have = w.nkb > 0;
       const uint32_t ab = PARTS > 1 ? 0 : ch & 1;
+      if (PARTS == 1 && have && staged) {
+        const uint32_t from = tmem_base + lane_addr + ab * BN + col_base;
+        ok = g2_store_columns<G2P_PATCH, COLS>(
+            E, stg, c_row, c_row + q * 32, c_col + col_base, lane,
+            [&] {
+              bool there = mbar_wait(&acc_full[ab], (ch >> 1) & 1);
+              if (!there) set_error(P.status, ERR_WAIT_ACC);
+              there = __all_sync(0xffffffffu, there);
+              tc_fence_after_sync();
+              return there;
+            },
+            [&](int c, float (&v)[G2P_PATCH]) {
+              uint32_t r[G2P_PATCH];
+              tmem_ld_32x32(from + c, r);
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < G2P_PATCH; ++j) v[j] = __uint_as_float(r[j]);
+            },
+            [&] {   // this warp's share has been read: hand the accumulator back to the leader
+              tc_fence_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&acc_empty[ab]), 0));
+            });
+        ++ch;
+        continue;
+      }
       if (have) {
         ok = mbar_wait(&acc_full[ab], PARTS > 1 ? ch & 1 : (ch >> 1) & 1);
         if (!ok) set_error(P.status, ERR_WAIT_ACC);
