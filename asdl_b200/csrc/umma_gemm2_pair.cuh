@@ -16,6 +16,11 @@
 // take all of TMEM, so a pair's next tile waits for its epilogue; most launches are one wave.
 // 1024 x 4096 between fp32 factors: 183 -> 137 us with the casts (graph replay), error against 64 bits 1.0e-5 -> 8.1e-6.
 //
+// HALVES = 2: tiles of 256 x 512, whose two 256-column halves take the two accumulators.  Both CTAs bring 48 KiB per K block of 1024
+// tensor clocks instead of 32 KiB per 512, which is less than L2 delivers (53 bytes per clock and SM) instead of more; a half
+// past the diagonal of a symmetric result is neither loaded nor multiplied.  A pair's next tile waits for its epilogue; gemm2_pair.cu has
+// the rule and what it measured.
+//
 // Signals inside a pair:
 //   full[s]      lives in the leader.  The leader's producer arms it with the bytes of BOTH CTAs'
 //                loads; each CTA's TMA loads (no cluster multicast: every CTA fetches its own
@@ -37,10 +42,11 @@
 
 namespace b200 {
 
-template <int PARTS>
+template <int PARTS, int HALVES>
 struct G2PairCfg {
-  static constexpr int STAGES = 6 / PARTS;
-  static constexpr int STAGE_BYTES = PARTS * 2 * G2_A_BYTES;   // this CTA's A rows and B columns of one K block
+  static_assert(PARTS == 1 || HALVES == 1, "one or the other takes both accumulators");
+  static constexpr int STAGE_BYTES = PARTS * (1 + HALVES) * G2_A_BYTES;   // this CTA's A rows and B columns of one K block
+  static constexpr int STAGES = 6 * 2 * G2_A_BYTES / STAGE_BYTES;
 };
 constexpr int G2P_EPI_WARPS = 8;
 constexpr int G2P_THREADS = 64 + 32 * G2P_EPI_WARPS;
@@ -112,21 +118,23 @@ struct G2PairItem {
   int split;
 };
 
+template <int HALVES>
 __device__ __forceinline__ G2PairItem g2_pair_decode(const GemmProblem2& P, int idx) {
   G2PairItem it;
   const int t = idx / P.nsplit;
   it.split = idx - t * P.nsplit;
   if (P.flags & G2F_SYM) {
     int TM = 0, rem = t;
-    while (rem > TM) {   // row TM of the pair grid holds TM + 1 tiles
-      rem -= TM + 1;
+    while (rem > TM / HALVES) {   // row TM of the pair grid holds TM / HALVES + 1 tiles
+      rem -= TM / HALVES + 1;
       ++TM;
     }
     it.TM = TM;
     it.TN = rem;
   } else {
-    it.TM = t / P.tiles_n;
-    it.TN = t - it.TM * P.tiles_n;
+    const int across = (P.tiles_n + HALVES - 1) / HALVES;
+    it.TM = t / across;
+    it.TN = t - it.TM * across;
   }
   const int kb_total = (P.K + G2_BK - 1) / G2_BK;
   it.kb0 = static_cast<int>((static_cast<long long>(it.split) * kb_total) / P.nsplit);
@@ -135,10 +143,18 @@ __device__ __forceinline__ G2PairItem g2_pair_decode(const GemmProblem2& P, int 
   return it;
 }
 
-template <int PARTS>
+// Halves of a tile that have columns to compute
+template <int HALVES>
+__device__ __forceinline__ int g2_pair_halves(const GemmProblem2& P, const G2PairItem& w) {
+  if (HALVES == 1) return 1;
+  return (P.flags & G2F_SYM ? w.TN * HALVES + 1 <= w.TM : w.TN * HALVES + 1 < P.tiles_n) ? 2 : 1;
+}
+
+template <int PARTS, int HALVES>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G2P_THREADS, 1)
 umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
-  constexpr int STAGES = G2PairCfg<PARTS>::STAGES, STAGE_BYTES = G2PairCfg<PARTS>::STAGE_BYTES;
+  constexpr int STAGES = G2PairCfg<PARTS, HALVES>::STAGES, STAGE_BYTES = G2PairCfg<PARTS, HALVES>::STAGE_BYTES;
+  constexpr bool ALL_TMEM = PARTS > 1 || HALVES > 1;   // one tile takes both accumulators
   constexpr int BN = 256;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -186,9 +202,10 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
       uint32_t it = 0;
       bool ok = true;
       for (int wi = pair_id; wi < n_work && ok; wi += n_pairs) {
-        const G2PairItem w = g2_pair_decode(P, wi);
+        const G2PairItem w = g2_pair_decode<HALVES>(P, wi);
         const int a_mn = w.TM * 256 + static_cast<int>(rank) * G2_BM;
-        const int b_mn = w.TN * 256 + static_cast<int>(rank) * G2_BM;
+        const int b_mn = w.TN * 256 * HALVES + static_cast<int>(rank) * G2_BM;
+        const int halves = g2_pair_halves<HALVES>(P, w);
         const int nseg = PARTS > 1 ? 1 : P.nseg;
         for (int seg = 0; seg < nseg && ok; ++seg) {
           for (int kb = 0; kb < w.nkb; ++kb, ++it) {
@@ -199,7 +216,7 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
               ok = false;
               break;
             }
-            if (leader) mbar_expect_tx(&full_bar[s], 2 * STAGE_BYTES);
+            if (leader) mbar_expect_tx(&full_bar[s], HALVES > 1 ? 2 * (1 + halves) * G2_A_BYTES : 2 * STAGE_BYTES);
             const uint32_t bar = mapa_shared(smem_u32(&full_bar[s]), 0);
             const int k = (w.kb0 + kb) * G2_BK;
 #pragma unroll
@@ -214,11 +231,15 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
                 tma_load_2d_pair(sA, ta, bar, a_mn, k);
                 tma_load_2d_pair(sA + G2_BK * 128, ta, bar, a_mn + 64, k);
               }
-              if (b_k) {
-                tma_load_2d_pair(sB, tb, bar, k, b_mn);
-              } else {
-                tma_load_2d_pair(sB, tb, bar, b_mn, k);
-                tma_load_2d_pair(sB + G2_BK * 128, tb, bar, b_mn + 64, k);
+#pragma unroll
+              for (int h = 0; h < HALVES; ++h) {
+                if (h >= halves) break;
+                if (b_k) {
+                  tma_load_2d_pair(sB + h * G2_A_BYTES, tb, bar, k, b_mn + 256 * h);
+                } else {
+                  tma_load_2d_pair(sB + h * G2_A_BYTES, tb, bar, b_mn + 256 * h, k);
+                  tma_load_2d_pair(sB + h * G2_A_BYTES + G2_BK * 128, tb, bar, b_mn + 256 * h + 64, k);
+                }
               }
             }
           }
@@ -242,10 +263,11 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
       uint32_t it = 0, ch = 0;
       bool ok = true;
       for (int wi = pair_id; wi < n_work && ok; wi += n_pairs) {
-        const G2PairItem w = g2_pair_decode(P, wi);
+        const G2PairItem w = g2_pair_decode<HALVES>(P, wi);
         if (w.nkb <= 0) continue;
-        const uint32_t ab = PARTS > 1 ? 0 : ch & 1;
-        if (!mbar_wait(&acc_empty[ab], (PARTS > 1 ? ch & 1 : (ch >> 1) & 1) ^ 1)) {
+        const int halves = g2_pair_halves<HALVES>(P, w);
+        const uint32_t ab = ALL_TMEM ? 0 : ch & 1;
+        if (!mbar_wait(&acc_empty[ab], (ALL_TMEM ? ch & 1 : (ch >> 1) & 1) ^ 1)) {
           set_error(P.status, ERR_WAIT_ACC);
           ok = false;
           break;
@@ -281,6 +303,7 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
                   umma_bf16_pair(tacc + (pr < 2 ? BN : 0), da, db, idesc, begins ? 0u : 1u);
                 } else {
                   umma_bf16_pair(tacc, da, db, idesc, first ? 0u : 1u);
+                  if (HALVES > 1 && halves > 1) umma_bf16_pair(tacc + BN, da, db + (G2_A_BYTES >> 4), idesc, first ? 0u : 1u);
                   first = 0;
                 }
               }
@@ -295,7 +318,7 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
   } else {
     // ------------------------------ epilogue (both CTAs) ------------------------------
     const int q = warp & 3;                                   // TMEM lane quarter this warp may access
-    constexpr int COLS = BN / (G2P_EPI_WARPS / 4);            // 128 columns per warp
+    constexpr int COLS = HALVES * BN / (G2P_EPI_WARPS / 4);   // columns per warp
     const int col_base = ((warp - 2) >> 2) * COLS;
     constexpr int PASSES = COLS / 64;
     const int row = q * 32 + lane;
@@ -308,20 +331,20 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
     uint32_t ch = 0;
     bool ok = true;
     for (int wi = pair_id; wi < n_work && ok; wi += n_pairs) {
-      const G2PairItem w = g2_pair_decode(P, wi);
+      const G2PairItem w = g2_pair_decode<HALVES>(P, wi);
       const int c_row = w.TM * 256 + static_cast<int>(rank) * G2_BM;
-      const int c_col = w.TN * 256;
+      const int c_col = w.TN * 256 * HALVES;
       const int tm = 2 * w.TM + static_cast<int>(rank);
       const int tile_id = sym ? w.TM * (w.TM + 1) + static_cast<int>(rank) * (w.TM + 1) + w.TN : tm * E.full->tiles_n + w.TN;
       const int gr = c_row + row;
       const bool have = w.nkb > 0;
-      const uint32_t ab = PARTS > 1 ? 0 : ch & 1;
+      const uint32_t ab = ALL_TMEM ? 0 : ch & 1;
       if (PARTS == 1 && have && staged) {
         const uint32_t from = tmem_base + lane_addr + ab * BN + col_base;
         ok = g2_store_columns<G2P_PATCH, COLS>(
             E, stg, c_row, c_row + q * 32, c_col + col_base, lane,
             [&] {
-              bool there = mbar_wait(&acc_full[ab], (ch >> 1) & 1);
+              bool there = mbar_wait(&acc_full[ab], ALL_TMEM ? ch & 1 : (ch >> 1) & 1);
               if (!there) set_error(P.status, ERR_WAIT_ACC);
               there = __all_sync(0xffffffffu, there);
               tc_fence_after_sync();
@@ -343,7 +366,7 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
         continue;
       }
       if (have) {
-        ok = mbar_wait(&acc_full[ab], PARTS > 1 ? ch & 1 : (ch >> 1) & 1);
+        ok = mbar_wait(&acc_full[ab], ALL_TMEM ? ch & 1 : (ch >> 1) & 1);
         if (!ok) set_error(P.status, ERR_WAIT_ACC);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
@@ -383,7 +406,7 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
           for (int j = 0; j < 64; ++j) v[j] = 0.f;
         }
         if (c_row >= E.M) continue;   // the lower half of the last pair row of an odd tile count: nothing to write
-        if (to_ws) {
+        if (HALVES == 1 && to_ws) {   // tiles of 512 columns are not split
           g2_store_partial(E.ws + (static_cast<size_t>(tile_id) * E.nsplit + w.split) * (G2_BM * BN), v, row, col0);
           continue;
         }

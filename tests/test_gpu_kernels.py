@@ -862,6 +862,38 @@ def test_cta_pair_tiles_match_narrow_tiles(ext):
     ops.check_status()
 
 
+@pytest.mark.parametrize('rows,n,ny', [(4600, 2840, 2840), (4616, 2904, 2600), (4672, 3080, 2312), (5000, 4104, 1288)])
+def test_cta_pair_tiles_of_512_columns(ext, rows, n, ny):
+    """Long products of more 256 x 256 tiles than CTA pairs against the 128 x 128 flavour: odd and even counts of tiles and of their
+    halves, ragged edges, beta, bf16 images, several segments; the shorter of the row counts stays with 256 columns."""
+    torch.manual_seed(0)
+    x, x2 = (torch.randn(rows, n, device=DEV).to(torch.bfloat16) for _ in range(2))
+    y = torch.randn(rows, ny, device=DEV).to(torch.bfloat16)
+    try:
+        res = []
+        for mode in (0, 4):
+            ext.set_gemm_wide(mode)
+            c = torch.full((n, n), 2.0, device=DEV)
+            ext.umma_gemm([x], [x], False, False, c, 0.5, 0.25, True, None, None, 1)
+            g = torch.full((n, ny), float('nan'), device=DEV)
+            ext.umma_gemm([x], [y], False, False, g, 1.0, 0.0, False, None, None, 1)
+            gk = torch.full((n, ny + 1), float('nan'), device=DEV)[:, 1:]
+            ext.umma_gemm([x.T.contiguous()], [y.T.contiguous()], True, True, gk, 1.0, 0.0, False, None, None, 1)
+            s = torch.empty(n, n, device=DEV)
+            hi = torch.zeros(n, (n + 63) // 64 * 64, device=DEV, dtype=torch.bfloat16)
+            lo = torch.zeros_like(hi)
+            ext.umma_gemm([x, x2], [x, x2], False, False, s, 1.0, 0.0, True, hi, lo, 1)
+            res.append((c, g, gk, s, hi, lo))
+        (c0, g0, gk0, s0, hi0, lo0), (c1, g1, gk1, s1, hi1, lo1) = res
+        assert rel_err(c1, c0) < 1e-6 and torch.equal(c1, c1.T)
+        assert rel_err(g1, g0) < 1e-6 and rel_err(gk1, g0) < 1e-6
+        assert rel_err(s1, s0) < 1e-6 and torch.equal(s1, s1.T)
+        assert rel_err(hi1[:, :n].float() + lo1[:, :n].float(), s1) < 1e-4
+    finally:
+        ext.set_gemm_wide(-1)
+    ops.check_status()
+
+
 @pytest.mark.parametrize('backend', ['tensor_core', 'cuda_core'])
 @pytest.mark.parametrize('sizes', [[1], [128], [129, 300, 40], [1500, 640, 257], [2304, 576, 64, 64]])
 def test_chol_inverse_backends(backend, sizes):
