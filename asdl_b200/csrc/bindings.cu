@@ -32,6 +32,7 @@ void gemm_plan_run(int64_t id);
 void cast_pad_bf16_grouped(at::Tensor table, int64_t count, int64_t max_elems);
 void cast_split3(at::Tensor src, at::Tensor hi, at::Tensor mid, at::Tensor lo);
 void transpose_cast(at::Tensor src, at::Tensor dst);
+void cast_many(std::vector<at::Tensor> dst, std::vector<at::Tensor> src);
 void bn_unitwise_stats(at::Tensor y, at::Tensor g, at::Tensor weight, at::Tensor bias, at::Tensor stats,
                        double alpha, double beta);
 std::vector<at::Tensor> bn_forward_train(at::Tensor x, at::Tensor weight, at::Tensor bias,
@@ -122,6 +123,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("cast_pad_bf16_grouped", &b200::cast_pad_bf16_grouped, py::arg("table"), py::arg("count"), py::arg("max_elems") = 0);
   m.def("cast_split3", &b200::cast_split3);
   m.def("transpose_cast", &b200::transpose_cast);
+  m.def("cast_many", &b200::cast_many);
   m.def("bn_unitwise_stats", &b200::bn_unitwise_stats);
   m.def("bn_forward_train", &b200::bn_forward_train);
   m.def("bn_backward_train", &b200::bn_backward_train);

@@ -111,6 +111,14 @@ class FusedMaxPool2d(nn.MaxPool2d):
         return super().forward(x)
 
 
+def _copy_all(dst, src):
+    """``dst[i].copy_(src[i])``; conversions between fp32 and bf16 on the GPU in one launch."""
+    if src[0].is_cuda and ops.cuda_kernels_enabled(src[0]):
+        ops.extension().cast_many(dst, src)
+    else:
+        torch._foreach_copy_(dst, src)
+
+
 class _GroupedCast(torch.autograd.Function):
     """fp32 parameters -> bf16 copies that live in one flat buffer (a few multi-tensor launches
     instead of one cast kernel per parameter); the backward pass converts the bf16 gradients back to
@@ -126,7 +134,7 @@ class _GroupedCast(torch.autograd.Function):
             off += (w.numel() + 7) // 8 * 8
             outs.append(chunk.as_strided(w.shape, w.stride()) if w.is_contiguous() or _dense(w)
                         else chunk.view(w.shape))
-        torch._foreach_copy_(outs, [w.detach() for w in weights])
+        _copy_all(outs, [w.detach() for w in weights])
         ctx.meta = [(w.shape, w.stride()) for w in weights]
         return tuple(outs)
 
@@ -150,7 +158,7 @@ class _GroupedCast(torch.autograd.Function):
                     same.append(g)
                     same_dst.append(d)
             if same:
-                torch._foreach_copy_(same_dst, same)
+                _copy_all(same_dst, same)
             for (i, _), d in zip(present, dst):
                 outs[i] = d
         return tuple(outs)

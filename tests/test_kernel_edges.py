@@ -576,6 +576,32 @@ def test_max_pool_gives_the_bits_of_pytorch(padding, n, c, h, w):
     assert torch.equal(again, v.flatten(2).gather(2, where.flatten(2)).view_as(again))
 
 
+@pytest.mark.parametrize('up', [False, True])
+def test_casts_of_many_tensors(up):
+    """Sizes around a vector and a piece of 8192, layouts that are alike or not, unaligned views, more tensors than a table holds."""
+    src_type, dst_type = (torch.bfloat16, torch.float32) if up else (torch.float32, torch.bfloat16)
+    shapes = [(1,), (7,), (8,), (8191,), (8192,), (8193,), (3, 5, 7, 9), (64, 16, 1, 1), (0, 4), (40, 24, 3, 3), (100, 300)]
+    src, dst = [], []
+    for i, shape in enumerate(shapes * 13):
+        s = torch.randn(shape, device=DEV, generator=_gen(40 + i)).to(src_type)
+        if len(shape) == 4 and i % 2:
+            s = s.contiguous(memory_format=torch.channels_last)
+        if i % 5 == 4:   # a base that is not 16-byte aligned
+            s = torch.cat([s.new_zeros(1), s.flatten()])[1:].view(shape)
+        d = torch.full(shape, float('nan'), device=DEV, dtype=dst_type)
+        if len(shape) == 4 and i % 3:
+            d = d.contiguous(memory_format=torch.channels_last)
+        if len(shape) == 2 and i % 7 == 3:
+            s = s.T.contiguous().T
+        src.append(s)
+        dst.append(d)
+    src.append(torch.arange(9, device=DEV, dtype=torch.float32))
+    dst.append(torch.zeros(9, device=DEV, dtype=torch.float64))
+    ops.extension().cast_many(dst, src)
+    for s, d in zip(src, dst):
+        assert torch.equal(d, s.to(d.dtype))
+
+
 def _norm_calls():
     def act(*shape):
         return torch.randn(*shape, device=DEV, generator=_gen(30)).to(torch.bfloat16)
