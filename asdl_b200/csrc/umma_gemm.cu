@@ -512,6 +512,7 @@ void umma_gemm(std::vector<at::Tensor> a_segs, std::vector<at::Tensor> b_segs, b
 // ---- two-sided product: allocation, casts and both products behind one native call -----------------------------------------
 // Small ones are bound by the host: as calls from Python 10 x 32 took 55 us and 64 x 576 55, now 30 and 45.
 void cast_pad_bf16(at::Tensor src, at::Tensor hi, c10::optional<at::Tensor> lo, double scale);
+bool cast_jobs(const std::vector<at::Tensor>& src, const std::vector<at::Tensor>& hi, const std::vector<at::Tensor>& lo);
 
 // [rows, n] -> its bf16 parts (hi, or hi and lo) as [rows, n] views with a row pitch that TMA takes; bf16 that already has one is
 // not copied.
@@ -537,8 +538,26 @@ at::Tensor kron_staged(at::Tensor left, at::Tensor mid, at::Tensor right, bool x
   c10::cuda::CUDAGuard guard(mid.get_device());
   const int64_t m = mid.size(0), n = mid.size(1);
   const bool l_col = left.stride(1) != 1 && left.stride(0) == 1, r_col = right.stride(1) != 1 && right.stride(0) == 1;
-  const std::vector<at::Tensor> l = stage_parts(l_col ? left.t() : left, x3), g = stage_parts(mid, x3),
-                                r = stage_parts(r_col ? right.t() : right, x3);
+  std::vector<at::Tensor> l, g, r;
+  const bool all_fp32 = left.scalar_type() == at::kFloat && mid.scalar_type() == at::kFloat && right.scalar_type() == at::kFloat &&
+                        left.device() == mid.device() && right.device() == mid.device();
+  if (x3 && all_fp32 && mid.numel() > 0 && left.numel() > 0 && right.numel() > 0 && right.size(1) < (1LL << 27) && n < (1LL << 27)) {
+    const auto rows = [](const at::Tensor& x) { return x.stride(1) == 1 ? x : x.contiguous(); };
+    const std::vector<at::Tensor> src = {rows(l_col ? left.t() : left), rows(mid), rows(r_col ? right.t() : right)};
+    std::vector<at::Tensor> hi, lo;
+    for (const at::Tensor& x : src)
+      for (std::vector<at::Tensor>* parts : {&hi, &lo})
+        parts->push_back(at::empty({x.size(0), std::max<int64_t>(8, (x.size(1) + 7) / 8 * 8)}, x.options().dtype(at::kBFloat16)));
+    cast_jobs(src, hi, lo);
+    const auto part = [&](int i) {
+      const int64_t width = src[i].size(1);
+      return hi[i].size(1) == width ? std::vector<at::Tensor>{hi[i], lo[i]}
+                                    : std::vector<at::Tensor>{hi[i].narrow(1, 0, width), lo[i].narrow(1, 0, width)};
+    };
+    l = part(0), g = part(1), r = part(2);
+  } else {
+    l = stage_parts(l_col ? left.t() : left, x3), g = stage_parts(mid, x3), r = stage_parts(r_col ? right.t() : right, x3);
+  }
   const int64_t ld = std::max<int64_t>(8, (n + 7) / 8 * 8);
   const auto options = mid.options().dtype(at::kBFloat16);
   std::vector<at::Tensor> t = {at::empty({m, ld}, options)};

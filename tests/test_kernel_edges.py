@@ -576,6 +576,22 @@ def test_max_pool_gives_the_bits_of_pytorch(padding, n, c, h, w):
     assert torch.equal(again, v.flatten(2).gather(2, where.flatten(2)).view_as(again))
 
 
+@pytest.mark.parametrize('m,n', [(1, 1), (8, 8), (7, 9), (1, 300), (129, 2049), (640, 24)])
+def test_two_sided_product_stages_its_operands_together(m, n):
+    """Pitches that are padded or not, rows that are aligned or not, strided and transposed operands."""
+    def spd(k, seed):
+        x = torch.randn(2 * k, k, device=DEV, generator=_gen(seed))
+        return x.T @ x / (2 * k)
+    left, right = spd(m, 50), spd(n, 51)
+    for mid in (torch.randn(m, n, device=DEV, generator=_gen(52)), torch.randn(n, m, device=DEV, generator=_gen(53)).T,
+                torch.randn(m, 2 * n + 1, device=DEV, generator=_gen(54))[:, 1::2], torch.randn(m, n + 3, device=DEV, generator=_gen(55))[:, 3:]):
+        want = left.double() @ mid.double() @ right.double()
+        for r in (right, right.T.contiguous().T):
+            got = ops.kron_apply(left, mid, r)
+            # hi and lo parts carry 2^-16 of every operand of the two products
+            assert (got.double() - want).norm() <= 4 * 2.0 ** -16 * want.norm()
+
+
 @pytest.mark.parametrize('up', [False, True])
 def test_casts_of_many_tensors(up):
     """Sizes around a vector and a piece of 8192, layouts that are alike or not, unaligned views, more tensors than a table holds."""
