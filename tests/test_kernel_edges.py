@@ -576,7 +576,7 @@ def test_max_pool_gives_the_bits_of_pytorch(padding, n, c, h, w):
     assert torch.equal(again, v.flatten(2).gather(2, where.flatten(2)).view_as(again))
 
 
-@pytest.mark.parametrize('m,n', [(1, 1), (8, 8), (7, 9), (1, 300), (129, 2049), (640, 24)])
+@pytest.mark.parametrize('m,n', [(1, 2), (2, 2), (8, 8), (7, 9), (1, 300), (129, 2049), (640, 24)])
 def test_two_sided_product_stages_its_operands_together(m, n):
     """Pitches that are padded or not, rows that are aligned or not, strided and transposed operands."""
     def spd(k, seed):
