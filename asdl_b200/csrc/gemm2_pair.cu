@@ -27,17 +27,16 @@ static int wide_tiles(const GemmProblem2& P, int pairs) {
 
 template <int PARTS, int HALVES>
 static void run_pair(const GemmProblem2& single, int n_work, int n_sms, cudaStream_t stream) {
-  constexpr int smem = G2P_SMEM_BYTES + (PARTS == 1 ? G2P_STAGED_BYTES : 0);
   static bool attr_set_on[64] = {false};
   int dev = 0;
   B200_CUDA_CHECK(cudaGetDevice(&dev));
   bool& attr_set = attr_set_on[dev & 63];
   if (!attr_set) {
-    B200_CUDA_CHECK(cudaFuncSetAttribute(umma_gemm2_pair_kernel<PARTS, HALVES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    B200_CUDA_CHECK(cudaFuncSetAttribute(umma_gemm2_pair_kernel<PARTS, HALVES>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2P_SMEM_BYTES));
     attr_set = true;
   }
   const int pairs = std::max(1, std::min(n_work, n_sms / 2));
-  launch_chained(umma_gemm2_pair_kernel<PARTS, HALVES>, dim3(2 * pairs), dim3(G2P_THREADS), smem, stream, single, n_work);
+  launch_chained(umma_gemm2_pair_kernel<PARTS, HALVES>, dim3(2 * pairs), dim3(G2P_THREADS), G2P_SMEM_BYTES, stream, single, n_work);
   B200_CUDA_CHECK(cudaGetLastError());
   count_launch();
 }

@@ -283,10 +283,11 @@ __device__ __forceinline__ void g2_reduce_chunk(const G2Epi& P, const float* v, 
 // the reduction loads them the same way.  With rows of the tile in memory every store instruction touched 32 half sectors: product
 // and reduction of 8192 x 1024 bf16 samples 22.6 -> 19.1 us, of 8192 x 2048 45.5 -> 41.3, of 12608 x 768 fp32 samples with their cast 45.0 -> 41.9,
 // a 768 x 768 gradient between fp32 factors 38.8 -> 33.1.
-__device__ __forceinline__ void g2_store_partial(float* tile, const float (&v)[64], int row, int col0) {
+template <int COLS>
+__device__ __forceinline__ void g2_store_partial(float* tile, const float (&v)[COLS], int row, int col0) {
   float* at = tile + (col0 / 4 * G2_BM + row) * 4;
 #pragma unroll
-  for (int j = 0; j < 16; ++j)
+  for (int j = 0; j < COLS / 4; ++j)
     *reinterpret_cast<float4*>(at + j * G2_BM * 4) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
 }
 
@@ -473,9 +474,11 @@ __device__ __forceinline__ void g2_sts(uint32_t at, float x, float y, float z, f
 }
 // What this store takes; the rest (bf16 images, copies on peers, reductions into C) goes out from registers, and so does a result that
 // is only written, 16 bytes at a time: nothing waits for those stores.
+__device__ __forceinline__ bool g2_only_c(const G2Epi& P) {
+  return P.C != nullptr && P.out_hi == nullptr && P.n_extra == 0 && !(P.flags & G2F_ATOMIC);
+}
 __device__ __forceinline__ bool g2_staged(const G2Epi& P) {
-  return P.C != nullptr && P.out_hi == nullptr && P.n_extra == 0 && !(P.flags & G2F_ATOMIC) &&
-         ((P.flags & G2F_SYM) || P.beta != 0.f || !g2_vec_ok(P.C, P.ldc));
+  return g2_only_c(P) && ((P.flags & G2F_SYM) || P.beta != 0.f || !g2_vec_ok(P.C, P.ldc));
 }
 // p[index * ldc], one instruction for the address
 __device__ __forceinline__ float* g2_line(float* p, int ldc, int index) {

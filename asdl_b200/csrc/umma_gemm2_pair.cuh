@@ -52,8 +52,7 @@ constexpr int G2P_EPI_WARPS = 8;
 constexpr int G2P_THREADS = 64 + 32 * G2P_EPI_WARPS;
 constexpr int G2P_TMEM_COLS = 512;                          // two 256-column accumulators
 constexpr int G2P_PATCH = 32;                               // columns of a result that an epilogue warp stages at a time
-constexpr int G2P_SMEM_BYTES = 6 * 2 * G2_A_BYTES + 1024 + 256;
-constexpr int G2P_STAGED_BYTES = G2P_EPI_WARPS * 32 * G2P_PATCH * 4;   // of the flavour without parts (G2Cfg::STAGED)
+constexpr int G2P_SMEM_BYTES = 6 * 2 * G2_A_BYTES + 1024 + 256 + G2P_EPI_WARPS * 32 * G2P_PATCH * 4;
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -141,6 +140,49 @@ __device__ __forceinline__ G2PairItem g2_pair_decode(const GemmProblem2& P, int 
   const int kb1 = static_cast<int>((static_cast<long long>(it.split + 1) * kb_total) / P.nsplit);
   it.nkb = kb1 - it.kb0;
   return it;
+}
+
+// The intermediate of a two-sided product: its two bf16 parts and nothing else.  32 rows x 32 columns of a warp, one row per lane, are
+// staged and leave as 16 bytes of eight columns, four lanes to a row.
+__device__ __forceinline__ bool g2_only_images(const G2Epi& P) {
+  return P.C == nullptr && P.out_hi != nullptr && P.out_lo != nullptr && P.out_mid == nullptr && P.n_extra == 0 && P.beta == 0.f &&
+         !(P.flags & (G2F_ATOMIC | G2F_SYM)) && (P.ld_out & 7) == 0 &&
+         ((reinterpret_cast<uintptr_t>(P.out_hi) | reinterpret_cast<uintptr_t>(P.out_lo)) & 15) == 0;
+}
+__device__ __forceinline__ void g2_store_images(const G2Epi& P, uint32_t stg, const float (&v)[32], int row0, int gc0, int lane) {
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 8; ++k) g2_sts(g2_patch_at<32>(stg, lane, k), v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+  __syncwarp();
+  const int oct = lane & 3, gc = gc0 + 8 * oct;
+#pragma unroll 2
+  for (int r = lane >> 2; r < 32; r += 8) {
+    const int gr = row0 + r;
+    const float4 a = g2_lds(g2_patch_at<32>(stg, r, 2 * oct)), b = g2_lds(g2_patch_at<32>(stg, r, 2 * oct + 1));
+    const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float x0 = P.alpha * x[2 * k], x1 = P.alpha * x[2 * k + 1];
+      const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
+      hi[k] = reinterpret_cast<const uint32_t&>(h);
+      const __nv_bfloat162 l = __floats2bfloat162_rn(x0 - __uint_as_float(hi[k] << 16), x1 - __uint_as_float(hi[k] & 0xffff0000u));
+      lo[k] = reinterpret_cast<const uint32_t&>(l);
+    }
+    if (gr >= P.M) continue;
+    const size_t at = static_cast<size_t>(gr) * P.ld_out + gc;
+    if (gc + 8 <= P.N) {
+      *reinterpret_cast<uint4*>(P.out_hi + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+      *reinterpret_cast<uint4*>(P.out_lo + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (gc + k < P.N) {
+          P.out_hi[at + k] = __ushort_as_bfloat16(static_cast<unsigned short>(hi[k / 2] >> (16 * (k & 1))));
+          P.out_lo[at + k] = __ushort_as_bfloat16(static_cast<unsigned short>(lo[k / 2] >> (16 * (k & 1))));
+        }
+    }
+  }
 }
 
 // Halves of a tile that have columns to compute
@@ -320,12 +362,11 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
     const int q = warp & 3;                                   // TMEM lane quarter this warp may access
     constexpr int COLS = HALVES * BN / (G2P_EPI_WARPS / 4);   // columns per warp
     const int col_base = ((warp - 2) >> 2) * COLS;
-    constexpr int PASSES = COLS / 64;
     const int row = q * 32 + lane;
     const G2Epi E = g2_epi(P);
     const bool sym = (E.flags & G2F_SYM) != 0;
     const bool atomic = (E.flags & G2F_ATOMIC) != 0;
-    const bool to_ws = E.nsplit > 1 && !atomic, staged = !to_ws && g2_staged(E);
+    const bool to_ws = E.nsplit > 1 && !atomic, staged = !to_ws && (PARTS > 1 ? g2_only_c(E) : g2_staged(E)), images = g2_only_images(E);
     const uint32_t stg = smem_u32(smem + STAGES * STAGE_BYTES + 256) + (warp - 2) * 32 * G2P_PATCH * 4;
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     uint32_t ch = 0;
@@ -339,90 +380,66 @@ umma_gemm2_pair_kernel(const __grid_constant__ GemmProblem2 P0, int n_work) {
       const int gr = c_row + row;
       const bool have = w.nkb > 0;
       const uint32_t ab = ALL_TMEM ? 0 : ch & 1;
-      if (PARTS == 1 && have && staged) {
-        const uint32_t from = tmem_base + lane_addr + ab * BN + col_base;
-        ok = g2_store_columns<G2P_PATCH, COLS>(
-            E, stg, c_row, c_row + q * 32, c_col + col_base, lane,
-            [&] {
-              bool there = mbar_wait(&acc_full[ab], ALL_TMEM ? ch & 1 : (ch >> 1) & 1);
-              if (!there) set_error(P.status, ERR_WAIT_ACC);
-              there = __all_sync(0xffffffffu, there);
-              tc_fence_after_sync();
-              return there;
-            },
-            [&](int c, float (&v)[G2P_PATCH]) {
-              uint32_t r[G2P_PATCH];
-              tmem_ld_32x32(from + c, r);
-              tmem_ld_wait();
-#pragma unroll
-              for (int j = 0; j < G2P_PATCH; ++j) v[j] = __uint_as_float(r[j]);
-            },
-            [&] {   // this warp's share has been read: hand the accumulator back to the leader
-              tc_fence_before_sync();
-              __syncwarp();
-              if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&acc_empty[ab]), 0));
-            });
-        ++ch;
-        continue;
-      }
-      if (have) {
-        ok = mbar_wait(&acc_full[ab], ALL_TMEM ? ch & 1 : (ch >> 1) & 1);
-        if (!ok) set_error(P.status, ERR_WAIT_ACC);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
+      const uint32_t from = tmem_base + lane_addr + ab * BN + col_base;
+      auto ready = [&] {
+        bool there = !have || mbar_wait(&acc_full[ab], ALL_TMEM ? ch & 1 : (ch >> 1) & 1);
+        if (!there) set_error(P.status, ERR_WAIT_ACC);
+        there = __all_sync(0xffffffffu, there);
         tc_fence_after_sync();
-      }
-#pragma unroll
-      for (int pass = 0; pass < PASSES; ++pass) {
-        float v[64];
-        const int col0 = col_base + pass * 64;
+        return there;
+      };
+      auto read = [&](int c, float (&v)[G2P_PATCH]) {
+        uint32_t r[G2P_PATCH] = {};
         if (have) {
-          uint32_t r0[32], r1[32];
-          tmem_ld_32x32(tmem_base + lane_addr + ab * BN + col0, r0);
-          tmem_ld_32x32(tmem_base + lane_addr + ab * BN + col0 + 32, r1);
+          tmem_ld_32x32(from + c, r);
+          tmem_ld_wait();
+        }
+#pragma unroll
+        for (int j = 0; j < G2P_PATCH; ++j) v[j] = __uint_as_float(r[j]);
+        if (PARTS > 1 && have) {   // the accumulator of the small part products
+          tmem_ld_32x32(from + BN + c, r);
           tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            v[j] = __uint_as_float(r0[j]);
-            v[32 + j] = __uint_as_float(r1[j]);
-          }
-          if constexpr (PARTS > 1) {   // the accumulator of the small part products
-            tmem_ld_32x32(tmem_base + lane_addr + BN + col0, r0);
-            tmem_ld_32x32(tmem_base + lane_addr + BN + col0 + 32, r1);
-            tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              v[j] += __uint_as_float(r0[j]);
-              v[32 + j] += __uint_as_float(r1[j]);
-            }
-          }
-          if (pass == PASSES - 1) {  // this warp's share is in registers: hand the accumulator back to the leader
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&acc_empty[ab]), 0));
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 64; ++j) v[j] = 0.f;
+          for (int j = 0; j < G2P_PATCH; ++j) v[j] += __uint_as_float(r[j]);
         }
+      };
+      auto release = [&] {   // this warp's share has been read: hand the accumulator back to the leader
+        tc_fence_before_sync();
+        __syncwarp();
+        if (have && lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&acc_empty[ab]), 0));
+      };
+      if (staged) {
+        ok = g2_store_columns<G2P_PATCH, COLS>(E, stg, c_row, c_row + q * 32, c_col + col_base, lane, ready, read, release);
+        if (have) ++ch;
+        continue;
+      }
+      ok = ready();
+      if (!ok) break;
+      float* const part = E.ws + (static_cast<size_t>(tile_id) * E.nsplit + w.split) * (G2_BM * BN);
+      // one patch after the other: unrolled, each kind of output is too much code for a tile (instruction fetch)
+#pragma unroll 1
+      for (int c = 0; c < COLS; c += G2P_PATCH) {
+        float v[G2P_PATCH];
+        read(c, v);
+        if (c + G2P_PATCH == COLS) release();
         if (c_row >= E.M) continue;   // the lower half of the last pair row of an odd tile count: nothing to write
+        const int col0 = col_base + c, gc0 = c_col + col0;
         if (HALVES == 1 && to_ws) {   // tiles of 512 columns are not split
-          g2_store_partial(E.ws + (static_cast<size_t>(tile_id) * E.nsplit + w.split) * (G2_BM * BN), v, row, col0);
+          g2_store_partial(part, v, row, col0);
           continue;
         }
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int gc0 = c_col + col0 + c * 32;
-          // a symmetric problem's pair tile on the diagonal reaches past the diagonal block: skip that part
-          const bool beyond = sym && (gc0 / G2_BM) > (c_row / G2_BM);
-          const bool diag = sym && (gc0 / G2_BM) == (c_row / G2_BM);
-          if (gc0 < E.N && !beyond && !(diag && gc0 > gr)) {
-            if (atomic)
-              g2_reduce_chunk(E, v + c * 32, gr, gc0, diag);
-            else
-              g2_store_chunk(E, v + c * 32, gr, gc0, diag);
-          }
-        }
+        // a symmetric problem's pair tile on the diagonal reaches past the diagonal block: skip that part
+        const bool beyond = sym && (gc0 / G2_BM) > (c_row / G2_BM);
+        const bool diag = sym && (gc0 / G2_BM) == (c_row / G2_BM);
+        if (gc0 >= E.N || beyond) continue;
+        if (PARTS > 1 && images)
+          g2_store_images(E, stg, v, c_row + q * 32, gc0, lane);
+        else if (diag && gc0 > gr)
+          continue;
+        else if (atomic)
+          g2_reduce_chunk(E, v, gr, gc0, diag);
+        else
+          g2_store_chunk(E, v, gr, gc0, diag);
       }
       if (have) ++ch;
     }
