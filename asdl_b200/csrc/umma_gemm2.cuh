@@ -47,20 +47,19 @@ constexpr int G2_MAX_SEG = 6;
 constexpr int G2_MAX_EXTRA = 7;
 constexpr int G2_MAX_BATCH = 256;   // problems of one launch in batch mode
 constexpr int G2_A_BYTES = G2_BM * G2_BK * 2;  // 16 KiB
-constexpr int G2_PATCH = 16;        // columns of a result that an epilogue warp stages at a time (two CTAs per SM leave 3 KiB per warp)
 
 template <int BN, int EPI_WARPS, int MINB, int PARTS>
 struct G2Cfg {
-  // results go out by way of shared memory where statistics are formed; in the flavours of two-sided products, whose results are
-  // bf16 images or only written, the second path through the epilogue cost 3 - 10 us (1024 x 4096: 134.9 -> 144.6)
-  static constexpr bool STAGED = PARTS == 1 && BN == 128;
+  // results go out by way of shared memory, in patches of so many columns (two CTAs of the plain flavour leave 3 KiB per warp)
+  static constexpr int PATCH = PARTS == 2 ? 32 : 16;
+  static constexpr bool STAGED = PARTS == 2 || (PARTS == 1 && BN == 128);
   static constexpr int STAGES = PARTS > 1 ? 2 : (BN == 256 ? 4 : (MINB == 2 ? 3 : 6));
   static constexpr int B_BYTES = BN * G2_BK * 2;
   static constexpr int STAGE_BYTES = PARTS * (G2_A_BYTES + B_BYTES);
   static constexpr int TMEM_COLS = 2 * BN;
   static constexpr int THREADS = 64 + 32 * EPI_WARPS;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align slack*/ + 256 /*barriers*/ +
-                                    4 * (G2_MAX_BATCH + 4) /*item prefix of a batch*/ + (STAGED ? EPI_WARPS * 32 * G2_PATCH * 4 : 0);
+                                    4 * (G2_MAX_BATCH + 4) /*item prefix of a batch*/ + (STAGED ? EPI_WARPS * 32 * PATCH * 4 : 0);
 };
 using G2Plain = G2Cfg<128, 4, 2, 1>;
 using G2Wide = G2Cfg<256, 8, 1, 1>;
@@ -590,6 +589,49 @@ __device__ __forceinline__ bool g2_store_columns(const G2Epi& P, uint32_t stg, i
   return true;
 }
 
+// The intermediate of a two-sided product: its two bf16 parts and nothing else.  32 rows x 32 columns of a warp, one row per lane, are
+// staged and leave as 16 bytes of eight columns, four lanes to a row.
+__device__ __forceinline__ bool g2_only_images(const G2Epi& P) {
+  return P.C == nullptr && P.out_hi != nullptr && P.out_lo != nullptr && P.out_mid == nullptr && P.n_extra == 0 && P.beta == 0.f &&
+         !(P.flags & (G2F_ATOMIC | G2F_SYM)) && (P.ld_out & 7) == 0 &&
+         ((reinterpret_cast<uintptr_t>(P.out_hi) | reinterpret_cast<uintptr_t>(P.out_lo)) & 15) == 0;
+}
+__device__ __forceinline__ void g2_store_images(const G2Epi& P, uint32_t stg, const float (&v)[32], int row0, int gc0, int lane) {
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 8; ++k) g2_sts(g2_patch_at<32>(stg, lane, k), v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+  __syncwarp();
+  const int oct = lane & 3, gc = gc0 + 8 * oct;
+#pragma unroll 2
+  for (int r = lane >> 2; r < 32; r += 8) {
+    const int gr = row0 + r;
+    const float4 a = g2_lds(g2_patch_at<32>(stg, r, 2 * oct)), b = g2_lds(g2_patch_at<32>(stg, r, 2 * oct + 1));
+    const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float x0 = P.alpha * x[2 * k], x1 = P.alpha * x[2 * k + 1];
+      const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
+      hi[k] = reinterpret_cast<const uint32_t&>(h);
+      const __nv_bfloat162 l = __floats2bfloat162_rn(x0 - __uint_as_float(hi[k] << 16), x1 - __uint_as_float(hi[k] & 0xffff0000u));
+      lo[k] = reinterpret_cast<const uint32_t&>(l);
+    }
+    if (gr >= P.M) continue;
+    const size_t at = static_cast<size_t>(gr) * P.ld_out + gc;
+    if (gc + 8 <= P.N) {
+      *reinterpret_cast<uint4*>(P.out_hi + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+      *reinterpret_cast<uint4*>(P.out_lo + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (gc + k < P.N) {
+          P.out_hi[at + k] = __ushort_as_bfloat16(static_cast<unsigned short>(hi[k / 2] >> (16 * (k & 1))));
+          P.out_lo[at + k] = __ushort_as_bfloat16(static_cast<unsigned short>(lo[k / 2] >> (16 * (k & 1))));
+        }
+    }
+  }
+}
+
 template <int BN, int EPI_WARPS, int MINB, int PARTS>
 __global__ void __launch_bounds__(64 + 32 * EPI_WARPS, MINB)
 umma_gemm2_kernel(const __grid_constant__ GemmProblem2 single, const GemmProblem2* __restrict__ probs,
@@ -855,9 +897,8 @@ umma_gemm2_kernel(const __grid_constant__ GemmProblem2 single, const GemmProblem
     const int q = warp & 3;                                   // TMEM lane quarter this warp may access
     constexpr int COLS = BN / (EPI_WARPS / 4);                // columns per warp
     const int col_base = ((warp - 2) >> 2) * COLS;            // first column of this warp's share
-    constexpr int PASSES = COLS / 64;
     const int row = q * 32 + lane;
-    const uint32_t stg = smem_u32(smem + STAGES * Cfg::STAGE_BYTES + 256 + 4 * (G2_MAX_BATCH + 4)) + (warp - 2) * 32 * G2_PATCH * 4;
+    const uint32_t stg = smem_u32(smem + STAGES * Cfg::STAGE_BYTES + 256 + 4 * (G2_MAX_BATCH + 4)) + (warp - 2) * 32 * Cfg::PATCH * 4;
     uint32_t ch = 0;
     bool ok = true;
     for (int wi = blockIdx.x; wi < n_work && ok; wi += gridDim.x) {
@@ -872,89 +913,89 @@ umma_gemm2_kernel(const __grid_constant__ GemmProblem2 single, const GemmProblem
       const bool to_ws = P.nsplit > 1 && !atomic;
       const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
 
-      auto finish = [&](const float (&v)[64], int col0) {
-        // v: 64 consecutive columns of this thread's row starting at tile column col0
-        if (to_ws) {
-          g2_store_partial(P.ws + (static_cast<size_t>(w.tile_id) * P.nsplit + w.split) * (G2_BM * BN), v, row, col0);
-          return;
-        }
+      if constexpr (!SPLIT3) {
+        const uint32_t ab = ch & 1;
+        const bool have = nchunks == 1;
+        const uint32_t from = tmem_base + lane_addr + ab * BN + col_base;
+        auto ready = [&] {
+          bool there = !have || mbar_wait(&acc_full[ab], (ch >> 1) & 1);
+          if (!there) set_error(status, ERR_WAIT_ACC);
+          there = __all_sync(0xffffffffu, there);
+          tc_fence_after_sync();
+          return there;
+        };
+        auto release = [&] {   // everything this warp needs has been read: free the accumulator
+          tc_fence_before_sync();
+          __syncwarp();
+          if (have && lane == 0) mbar_arrive(&acc_empty[ab]);
+        };
+        auto read = [&](int c, auto& v) {
+          constexpr int COUNT = sizeof(v) / sizeof(float);
+          uint32_t r[COUNT] = {};
+          if (have) {
+            if constexpr (COUNT == 16)
+              tmem_ld_32x16(from + c, r);
+            else
+              tmem_ld_32x32(from + c, r);
+            tmem_ld_wait();
+          }
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int gc0 = w.c_col + col0 + c * 32;
+          for (int j = 0; j < COUNT; ++j) v[j] = __uint_as_float(r[j]);
+        };
+        if (Cfg::STAGED && !to_ws && (PARTS == 2 ? g2_only_c(P) : g2_staged(P))) {
+          ok = g2_store_columns<Cfg::PATCH, COLS>(P, stg, w.c_row, w.c_row + q * 32, w.c_col + col_base, lane, ready, read, release);
+          if (have) ++ch;
+          continue;
+        }
+        ok = ready();
+        if (!ok) break;
+        const bool images = PARTS == 2 && g2_only_images(P);
+        // one patch after the other: unrolled, each kind of output is too much code for a tile (instruction fetch)
+#pragma unroll 1
+        for (int c = 0; c < COLS; c += 32) {
+          float v[32];
+          read(c, v);
+          if (c + 32 == COLS) release();
+          const int col0 = col_base + c, gc0 = w.c_col + col0;
+          if (to_ws) {
+            g2_store_partial(P.ws + (static_cast<size_t>(w.tile_id) * P.nsplit + w.split) * (G2_BM * BN), v, row, col0);
+            continue;
+          }
           // with wide tiles a symmetric problem's tile may reach past the diagonal block: skip that part
           const bool beyond = sym && (gc0 / G2_BM) > (w.c_row / G2_BM);
           const bool diag = sym && (gc0 / G2_BM) == (w.c_row / G2_BM);
-          if (gc0 < P.N && !beyond && !(diag && gc0 > gr)) {
-            if (atomic)
-              g2_reduce_chunk(P, v + c * 32, gr, gc0, diag);
-            else
-              g2_store_chunk(P, v + c * 32, gr, gc0, diag);
-          }
-        }
-      };
-
-      if constexpr (!SPLIT3) {
-        const uint32_t ab = ch & 1;
-        if (Cfg::STAGED && !to_ws && nchunks == 1 && g2_staged(P)) {
-          const uint32_t from = tmem_base + lane_addr + ab * BN + col_base;
-          ok = g2_store_columns<G2_PATCH, COLS>(
-              P, stg, w.c_row, w.c_row + q * 32, w.c_col + col_base, lane,
-              [&] {
-                bool there = mbar_wait(&acc_full[ab], (ch >> 1) & 1);
-                if (!there) set_error(status, ERR_WAIT_ACC);
-                there = __all_sync(0xffffffffu, there);
-                tc_fence_after_sync();
-                return there;
-              },
-              [&](int c, float (&v)[G2_PATCH]) {
-                uint32_t r[G2_PATCH];
-                tmem_ld_32x16(from + c, r);
-                tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < G2_PATCH; ++j) v[j] = __uint_as_float(r[j]);
-              },
-              [&] {
-                tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&acc_empty[ab]);
-              });
-          ++ch;
-          continue;
-        }
-        if (nchunks == 1) {
-          ok = mbar_wait(&acc_full[ab], (ch >> 1) & 1);
-          if (!ok) set_error(status, ERR_WAIT_ACC);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          tc_fence_after_sync();
-        }
-#pragma unroll
-        for (int pass = 0; pass < PASSES; ++pass) {
-          float v[64];
-          const int col0 = col_base + pass * 64;
-          if (nchunks == 1) {
-            uint32_t r0[32], r1[32];
-            tmem_ld_32x32(tmem_base + lane_addr + ab * BN + col0, r0);
-            tmem_ld_32x32(tmem_base + lane_addr + ab * BN + col0 + 32, r1);
-            tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              v[j] = __uint_as_float(r0[j]);
-              v[32 + j] = __uint_as_float(r1[j]);
-            }
-            if (pass == PASSES - 1) {  // everything this warp needs is in registers: free the accumulator
-              tc_fence_before_sync();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&acc_empty[ab]);
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 64; ++j) v[j] = 0.f;
-          }
-          finish(v, col0);
+          if (gc0 >= P.N || beyond) continue;
+          if (PARTS == 2 && images)
+            g2_store_images(P, stg, v, w.c_row + q * 32, gc0, lane);
+          else if (diag && gc0 > gr)
+            continue;
+          else if (atomic)
+            g2_reduce_chunk(P, v, gr, gc0, diag);
+          else
+            g2_store_chunk(P, v, gr, gc0, diag);
         }
         if (nchunks == 1) ++ch;
       } else {
+        auto finish = [&](const float (&v)[64], int col0) {
+          // v: 64 consecutive columns of this thread's row starting at tile column col0
+          if (to_ws) {
+            g2_store_partial(P.ws + (static_cast<size_t>(w.tile_id) * P.nsplit + w.split) * (G2_BM * BN), v, row, col0);
+            return;
+          }
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const int gc0 = w.c_col + col0 + c * 32;
+            // with wide tiles a symmetric problem's tile may reach past the diagonal block: skip that part
+            const bool beyond = sym && (gc0 / G2_BM) > (w.c_row / G2_BM);
+            const bool diag = sym && (gc0 / G2_BM) == (w.c_row / G2_BM);
+            if (gc0 < P.N && !beyond && !(diag && gc0 > gr)) {
+              if (atomic)
+                g2_reduce_chunk(P, v + c * 32, gr, gc0, diag);
+              else
+                g2_store_chunk(P, v + c * 32, gr, gc0, diag);
+            }
+          }
+        };
         // one chunk per K block: running fp32 sum in registers
         float run[64];
 #pragma unroll

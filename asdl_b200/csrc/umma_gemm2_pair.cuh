@@ -142,49 +142,6 @@ __device__ __forceinline__ G2PairItem g2_pair_decode(const GemmProblem2& P, int 
   return it;
 }
 
-// The intermediate of a two-sided product: its two bf16 parts and nothing else.  32 rows x 32 columns of a warp, one row per lane, are
-// staged and leave as 16 bytes of eight columns, four lanes to a row.
-__device__ __forceinline__ bool g2_only_images(const G2Epi& P) {
-  return P.C == nullptr && P.out_hi != nullptr && P.out_lo != nullptr && P.out_mid == nullptr && P.n_extra == 0 && P.beta == 0.f &&
-         !(P.flags & (G2F_ATOMIC | G2F_SYM)) && (P.ld_out & 7) == 0 &&
-         ((reinterpret_cast<uintptr_t>(P.out_hi) | reinterpret_cast<uintptr_t>(P.out_lo)) & 15) == 0;
-}
-__device__ __forceinline__ void g2_store_images(const G2Epi& P, uint32_t stg, const float (&v)[32], int row0, int gc0, int lane) {
-  __syncwarp();
-#pragma unroll
-  for (int k = 0; k < 8; ++k) g2_sts(g2_patch_at<32>(stg, lane, k), v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-  __syncwarp();
-  const int oct = lane & 3, gc = gc0 + 8 * oct;
-#pragma unroll 2
-  for (int r = lane >> 2; r < 32; r += 8) {
-    const int gr = row0 + r;
-    const float4 a = g2_lds(g2_patch_at<32>(stg, r, 2 * oct)), b = g2_lds(g2_patch_at<32>(stg, r, 2 * oct + 1));
-    const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    uint32_t hi[4], lo[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float x0 = P.alpha * x[2 * k], x1 = P.alpha * x[2 * k + 1];
-      const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
-      hi[k] = reinterpret_cast<const uint32_t&>(h);
-      const __nv_bfloat162 l = __floats2bfloat162_rn(x0 - __uint_as_float(hi[k] << 16), x1 - __uint_as_float(hi[k] & 0xffff0000u));
-      lo[k] = reinterpret_cast<const uint32_t&>(l);
-    }
-    if (gr >= P.M) continue;
-    const size_t at = static_cast<size_t>(gr) * P.ld_out + gc;
-    if (gc + 8 <= P.N) {
-      *reinterpret_cast<uint4*>(P.out_hi + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-      *reinterpret_cast<uint4*>(P.out_lo + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        if (gc + k < P.N) {
-          P.out_hi[at + k] = __ushort_as_bfloat16(static_cast<unsigned short>(hi[k / 2] >> (16 * (k & 1))));
-          P.out_lo[at + k] = __ushort_as_bfloat16(static_cast<unsigned short>(lo[k / 2] >> (16 * (k & 1))));
-        }
-    }
-  }
-}
-
 // Halves of a tile that have columns to compute
 template <int HALVES>
 __device__ __forceinline__ int g2_pair_halves(const GemmProblem2& P, const G2PairItem& w) {
