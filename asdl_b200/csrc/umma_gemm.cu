@@ -176,9 +176,15 @@ void gemm_fill_problem(GemmProblem2& P, const std::vector<at::Tensor>& a_segs,
   // 128-wide tiles at 4096 x 4096 x 8192, slower below 2048 x 2048 where a launch is a wave or less).  While a
   // batch is recording, a product leaves the batch for a pair launch of its own only from 1e11 multiply-adds
   // on: smaller ones fill the GPU better together with the rest of the batch.
+  // Symmetric products of at least 3000 x 3000 gain from 1.5e10 on (us, narrow -> pairs: 2048 rows x 3072 45.4 -> 38.7, 1024 x 4096 46.7 -> 37.1; but
+  // 1024 x 3072 24.6 -> 26.5, 2048 x 2560 23.9 -> 31.3), and from about 3750 on with any number of rows if they add to C: narrow tiles then
+  // bring C in pieces of 64 bytes (64 x 4096 48.0 -> 30.6, 512 x 4096 50.0 -> 33.9; without C 16.5 -> 19.4 and 22.3 -> 23.3, 64 x 3072 with it
+  // 25.5 -> 25.3).
   const double macs = static_cast<double>(M) * static_cast<double>(N) * static_cast<double>(K);
+  const double outputs = static_cast<double>(M) * static_cast<double>(N);
+  const double least = g_batch_open ? 1e11 : sym && beta != 0.0 && outputs >= 1.4e7 ? 0.0 : sym && outputs >= 9e6 ? 1.5e10 : 2e10;
   const bool pair = x3_pair || (!wide && !split3 &&
-                    (g_wide_mode == 4 || (g_wide_mode == 3 && N >= 2048 && M >= 2048 && macs >= (g_batch_open ? 1e11 : 2e10))));
+                    (g_wide_mode == 4 || (g_wide_mode == 3 && N >= 2048 && M >= 2048 && macs >= least)));
   const int bn = wide ? 256 : 128;        // B rows of a tensor-map box
   const int bn_grid = pair ? 256 : bn;    // tile width of the grid and of the split-K scratch
   for (int s = 0; s < nseg; ++s) {
