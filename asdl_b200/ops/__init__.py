@@ -639,8 +639,8 @@ def batch_norm_train(x, weight, bias, running_mean=None, running_var=None, momen
                      residual=None, relu=False, num_batches_tracked=None, return_stats=False):
     """``act(batch_norm(x) + residual)`` with batch statistics (running statistics and the batch
     counter updated in place), differentiable in x, weight, bias and residual.  CUDA, channels_last
-    bf16 activations with fp32 parameters: one kernel forward and one backward, which keep what they have
-    summed on the chip for the transform;
+    bf16 activations with fp32 parameters: three kernels forward (sums, finalize, transform) and
+    three backward, with 16-byte accesses; the transforms find part of what the sums have read in L2;
     anything else: ``F.batch_norm`` followed by the add and the ReLU.  With ``return_stats`` the
     result is ``(y, mean, invstd)`` (``None`` statistics on the PyTorch path)."""
     if batch_norm_train_supported(x, weight, bias, residual):
