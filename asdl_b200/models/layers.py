@@ -97,7 +97,8 @@ class FusedMaxPool2d(nn.MaxPool2d):
 
     def _native(self, x):
         p = self.padding
-        return (self.kernel_size == 3 and self.stride == 2 and (p == 0 or p == 1) and self.dilation == 1 and not self.return_indices
+        # a subclass (a fake tensor, say) need not have memory
+        return (type(x) is torch.Tensor and self.kernel_size == 3 and self.stride == 2 and (p == 0 or p == 1) and self.dilation == 1 and not self.return_indices
                 and not self.ceil_mode and x.is_cuda and x.dtype == torch.bfloat16 and x.ndim == 4
                 and torch._C._get_tracing_state() is None and not torch._C._are_functorch_transforms_active()
                 and not torch.compiler.is_compiling()

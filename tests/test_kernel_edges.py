@@ -618,6 +618,13 @@ def test_casts_of_many_tensors(up):
         assert torch.equal(d, s.to(d.dtype))
 
 
+def test_max_pool_leaves_tensors_without_memory_to_pytorch():
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    with FakeTensorMode():
+        x = torch.empty(2, 8, 9, 9, device=DEV, dtype=torch.bfloat16).contiguous(memory_format=torch.channels_last)
+        assert FusedMaxPool2d(3, stride=2, padding=1)(x).shape == (2, 8, 5, 5)
+
+
 def _norm_calls():
     def act(*shape):
         return torch.randn(*shape, device=DEV, generator=_gen(30)).to(torch.bfloat16)
