@@ -33,6 +33,8 @@ void cast_pad_bf16_grouped(at::Tensor table, int64_t count, int64_t max_elems);
 void cast_split3(at::Tensor src, at::Tensor hi, at::Tensor mid, at::Tensor lo);
 void transpose_cast(at::Tensor src, at::Tensor dst);
 void cast_many(std::vector<at::Tensor> dst, std::vector<at::Tensor> src);
+void stage_gradients(std::vector<at::Tensor> grads, std::vector<at::Tensor> staged, std::vector<at::Tensor> hi,
+                     std::vector<at::Tensor> lo, double scale);
 void bn_unitwise_stats(at::Tensor y, at::Tensor g, at::Tensor weight, at::Tensor bias, at::Tensor stats,
                        double alpha, double beta);
 std::vector<at::Tensor> bn_forward_train(at::Tensor x, at::Tensor weight, at::Tensor bias,
@@ -124,6 +126,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("cast_split3", &b200::cast_split3);
   m.def("transpose_cast", &b200::transpose_cast);
   m.def("cast_many", &b200::cast_many);
+  m.def("stage_gradients", &b200::stage_gradients);
   m.def("bn_unitwise_stats", &b200::bn_unitwise_stats);
   m.def("bn_forward_train", &b200::bn_forward_train);
   m.def("bn_backward_train", &b200::bn_backward_train);

@@ -87,10 +87,9 @@ cast_parts_kernel(const T* __restrict__ src, long long lds, float scale, __nv_bf
                            static_cast<long long>(gridDim.x) * lanes);
 }
 
-// The operands of a two-sided product, fp32 -> hi, lo, in one launch: one wave of blocks, shared out by size.  1024 x 4096 with its
-// factors (168 MB) 151.0 -> 146.4 us pass after pass, 768 x 768 in graphs 33.4 -> 31.2 us, 1000 x 333 37.4 -> 29.8, 10 x 32 14.9 -> 11.8; each
-// launch is 2 us of the host's time besides (10 x 32: 33 -> 26 us).
-constexpr int CAST_JOBS = 3;
+// Several fp32 matrices -> hi, lo in one launch: one wave of blocks, shared out by size.  The operands of a two-sided product:
+// 1024 x 4096 with its factors (168 MB) 151.0 -> 146.4 us pass after pass, 768 x 768 in graphs 33.4 -> 31.2 us, 1000 x 333
+// 37.4 -> 29.8, 10 x 32 14.9 -> 11.8; each launch is 2 us of the host's time besides (10 x 32: 33 -> 26 us).
 struct CastJob {
   const float* src;
   __nv_bfloat16 *hi, *lo;
@@ -98,57 +97,110 @@ struct CastJob {
   int n, groups, lanes, across, first;   // blocks beside each other, first block
   bool vec;
 };
+template <int JOBS>
 struct CastJobs {
-  CastJob job[CAST_JOBS];
-  int blocks;
+  CastJob job[JOBS];
+  int count, blocks;
+  float scale;
 };
-__global__ void __launch_bounds__(256) cast_jobs_kernel(const __grid_constant__ CastJobs t) {
+template <int JOBS>
+__global__ void __launch_bounds__(256) cast_jobs_kernel(const __grid_constant__ CastJobs<JOBS> t) {
   chain_next();
-  int k = 0;
-#pragma unroll
-  for (int i = 1; i < CAST_JOBS; ++i) k += static_cast<int>(blockIdx.x) >= t.job[i].first;
+  int k = 0, past = t.count;   // the last job whose first block is not past this one
+  while (past - k > 1) {
+    const int mid = (k + past) / 2;
+    (t.job[mid].first <= static_cast<int>(blockIdx.x) ? k : past) = mid;
+  }
   const CastJob& j = t.job[k];
-  const int end = k + 1 < CAST_JOBS ? t.job[k + 1].first : t.blocks, block = blockIdx.x - j.first, down = (end - j.first) / j.across;
+  const int end = k + 1 < t.count ? t.job[k + 1].first : t.blocks, block = blockIdx.x - j.first, down = (end - j.first) / j.across;
   const int lane = threadIdx.x / j.groups;
   const long long c0 = (static_cast<long long>(block % j.across) * j.groups + threadIdx.x % j.groups) * 8;
   if (lane >= j.lanes || c0 >= j.ldo) return;
   const long long first = static_cast<long long>(block / j.across) * j.lanes + lane, step = static_cast<long long>(down) * j.lanes;
   if (j.vec)
-    cast_rows<float, 2, true>(j.src, j.lds, 1.f, j.hi, j.lo, nullptr, j.ldo, j.rows, j.n, c0, first, step);
+    cast_rows<float, 2, true>(j.src, j.lds, t.scale, j.hi, j.lo, nullptr, j.ldo, j.rows, j.n, c0, first, step);
   else
-    cast_rows<float, 2, false>(j.src, j.lds, 1.f, j.hi, j.lo, nullptr, j.ldo, j.rows, j.n, c0, first, step);
+    cast_rows<float, 2, false>(j.src, j.lds, t.scale, j.hi, j.lo, nullptr, j.ldo, j.rows, j.n, c0, first, step);
 }
 
-// src[i] -> hi[i], lo[i]: fp32 matrices with unit column stride, contiguous bf16 ones of a pitch that is a multiple of eight.  False,
-// with nothing done, where there is nothing to cast.
-bool cast_jobs(const std::vector<at::Tensor>& src, const std::vector<at::Tensor>& hi, const std::vector<at::Tensor>& lo) {
-  TORCH_CHECK(src.size() == CAST_JOBS && hi.size() == CAST_JOBS && lo.size() == CAST_JOBS, "three matrices");
-  CastJobs t;
+static CastJob cast_job(const float* src, long long lds, int64_t rows, int64_t n, const at::Tensor& hi, const at::Tensor& lo) {
+  TORCH_CHECK(hi.is_contiguous() && lo.is_contiguous() && hi.scalar_type() == at::kBFloat16 && lo.scalar_type() == at::kBFloat16 &&
+                  hi.dim() == 2 && hi.size(1) % 8 == 0 && hi.size(1) < (1LL << 31) && hi.sizes() == lo.sizes() &&
+                  hi.size(0) == rows && hi.size(1) >= n, "parts must match their matrix");
+  CastJob j;
+  j.src = src;
+  j.hi = reinterpret_cast<__nv_bfloat16*>(hi.data_ptr());
+  j.lo = reinterpret_cast<__nv_bfloat16*>(lo.data_ptr());
+  TORCH_CHECK(((reinterpret_cast<uintptr_t>(j.hi) | reinterpret_cast<uintptr_t>(j.lo)) & 15) == 0, "parts must be 16-byte aligned");
+  j.lds = lds, j.ldo = hi.size(1), j.rows = rows, j.n = static_cast<int>(n);
+  j.vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && lds % 4 == 0;
+  return j;
+}
+template <int JOBS>
+static void launch_cast_jobs(CastJobs<JOBS>& t, double scale, cudaStream_t stream) {
+  if (t.count == 0) return;
   double elements = 0;
-  for (const at::Tensor& h : hi) elements += static_cast<double>(h.numel());
-  t.blocks = 0;
-  for (int i = 0; i < CAST_JOBS; ++i) {
-    TORCH_CHECK(src[i].scalar_type() == at::kFloat && src[i].stride(1) == 1 && hi[i].is_contiguous() && lo[i].is_contiguous() &&
-                    hi[i].size(1) % 8 == 0 && hi[i].size(1) < (1LL << 31) && hi[i].sizes() == lo[i].sizes() && hi[i].size(0) == src[i].size(0) &&
-                    hi[i].size(1) >= src[i].size(1), "parts must match their matrix");
-    if (hi[i].numel() == 0) return false;
+  for (int i = 0; i < t.count; ++i) elements += static_cast<double>(t.job[i].rows) * t.job[i].ldo;
+  t.blocks = 0, t.scale = static_cast<float>(scale);
+  for (int i = 0; i < t.count; ++i) {
     CastJob& j = t.job[i];
-    j.src = src[i].data_ptr<float>();
-    j.hi = reinterpret_cast<__nv_bfloat16*>(hi[i].data_ptr());
-    j.lo = reinterpret_cast<__nv_bfloat16*>(lo[i].data_ptr());
-    TORCH_CHECK(((reinterpret_cast<uintptr_t>(j.hi) | reinterpret_cast<uintptr_t>(j.lo)) & 15) == 0, "parts must be 16-byte aligned");
-    j.lds = src[i].stride(0), j.ldo = hi[i].size(1), j.rows = src[i].size(0), j.n = static_cast<int>(src[i].size(1));
-    j.vec = (reinterpret_cast<uintptr_t>(j.src) & 15) == 0 && j.lds % 4 == 0;
     const Walk w = walk_plan(static_cast<int>(j.ldo / 8));
     j.groups = w.groups, j.lanes = w.lanes, j.across = w.chunks, j.first = t.blocks;
     const long long most = (j.rows + w.lanes - 1) / w.lanes;
-    const long long share = static_cast<long long>(148 * 6 * (hi[i].numel() / elements) / w.chunks + 0.999);
+    const long long share = static_cast<long long>(148 * 6 * (j.rows * j.ldo / elements) / w.chunks + 0.999);
     t.blocks += static_cast<int>(std::max(1LL, std::min(most, share))) * w.chunks;
   }
-  cast_jobs_kernel<<<t.blocks, 256, 0, at::cuda::getCurrentCUDAStream(src[0].get_device()).stream()>>>(t);
+  cast_jobs_kernel<JOBS><<<t.blocks, 256, 0, stream>>>(t);
   B200_CUDA_CHECK(cudaGetLastError());
   count_launch();
-  return true;
+}
+
+// src[i] -> hi[i], lo[i]: fp32 matrices with unit column stride, contiguous bf16 ones of a pitch that is a multiple of eight.
+void cast_jobs(const std::vector<at::Tensor>& src, const std::vector<at::Tensor>& hi, const std::vector<at::Tensor>& lo) {
+  TORCH_CHECK(src.size() == 3 && hi.size() == 3 && lo.size() == 3, "three matrices");
+  CastJobs<3> t;
+  t.count = 0;
+  for (int i = 0; i < 3; ++i) {
+    TORCH_CHECK(src[i].scalar_type() == at::kFloat && src[i].stride(1) == 1, "fp32 with unit column stride");
+    if (hi[i].numel() > 0) t.job[t.count++] = cast_job(src[i].data_ptr<float>(), src[i].stride(0), src[i].size(0), src[i].size(1), hi[i], lo[i]);
+  }
+  launch_cast_jobs(t, 1.0, at::cuda::getCurrentCUDAStream(src[0].get_device()).stream());
+}
+
+// scale * grads[i] -> hi[i], lo[i].  staged[i] is the dense fp32 view, of the gradient's shape, whose memory is the matrix [rows, n]
+// of the factor's order: a gradient of the same strides is read where it lies, another one is copied there first.  Up to 64
+// gradients share a launch, whose table travels as an argument: they lie elsewhere in each step. Bound by memory; ResNet-50's
+// 54 matrices (188 MB with the parts) take 11 us from L2 and HBM together, with the copy ahead of them it was 30: ten steps
+// 24.13 -> 23.94 ms.
+void stage_gradients(std::vector<at::Tensor> grads, std::vector<at::Tensor> staged, std::vector<at::Tensor> hi,
+                     std::vector<at::Tensor> lo, double scale) {
+  constexpr int JOBS = 64;
+  TORCH_CHECK(grads.size() == staged.size() && grads.size() == hi.size() && grads.size() == lo.size(), "one of each per gradient");
+  if (grads.empty()) return;
+  const auto device = staged[0].device();
+  TORCH_CHECK(device.is_cuda(), "CUDA gradients");
+  c10::cuda::CUDAGuard guard(device);
+  const cudaStream_t stream = at::cuda::getCurrentCUDAStream(device.index()).stream();
+  CastJobs<JOBS> t;
+  t.count = 0;
+  for (size_t i = 0; i < grads.size(); ++i) {
+    const at::Tensor &g = grads[i], &v = staged[i];
+    TORCH_CHECK(v.scalar_type() == at::kFloat && v.is_non_overlapping_and_dense() && v.device() == device && hi[i].device() == device &&
+                    lo[i].device() == device && v.dim() > 0, "dense fp32 matrices on one device");
+    bool in_place = g.layout() == at::kStrided && g.device() == device && g.scalar_type() == at::kFloat && !g.is_neg() &&
+                    !g.key_set().has(c10::DispatchKey::Python) && g.sizes() == v.sizes();
+    for (int64_t d = 0; in_place && d < v.dim(); ++d) in_place = v.size(d) == 1 || g.stride(d) == v.stride(d);
+    if (!in_place) v.copy_(g);
+    if (v.numel() == 0) continue;
+    const int64_t rows = v.size(0), n = v.numel() / rows;
+    TORCH_CHECK(rows == 1 || v.stride(0) == n, "rows of the matrix in the order of the first dimension");
+    t.job[t.count++] = cast_job(in_place ? g.data_ptr<float>() : v.data_ptr<float>(), n, rows, n, hi[i], lo[i]);
+    if (t.count == JOBS) {
+      launch_cast_jobs(t, scale, stream);
+      t.count = 0;
+    }
+  }
+  launch_cast_jobs(t, scale, stream);
 }
 
 // The same for what the vector kernel does not take (launch_cast): one element per thread.

@@ -518,7 +518,7 @@ void umma_gemm(std::vector<at::Tensor> a_segs, std::vector<at::Tensor> b_segs, b
 // ---- two-sided product: allocation, casts and both products behind one native call -----------------------------------------
 // Small ones are bound by the host: as calls from Python 10 x 32 took 55 us and 64 x 576 55, now 30 and 45.
 void cast_pad_bf16(at::Tensor src, at::Tensor hi, c10::optional<at::Tensor> lo, double scale);
-bool cast_jobs(const std::vector<at::Tensor>& src, const std::vector<at::Tensor>& hi, const std::vector<at::Tensor>& lo);
+void cast_jobs(const std::vector<at::Tensor>& src, const std::vector<at::Tensor>& hi, const std::vector<at::Tensor>& lo);
 
 // [rows, n] -> its bf16 parts (hi, or hi and lo) as [rows, n] views with a row pitch that TMA takes; bf16 that already has one is
 // not copied.

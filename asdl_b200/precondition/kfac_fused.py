@@ -1166,7 +1166,8 @@ class FusedKfacGradientMaker(KfacGradientMaker):
         table = torch.tensor(rows, dtype=torch.int64, device=dev)
         max_elems = max(r[3] * r[6] for r in rows)
         return dict(key=tuple(id(st) for st in todo), views=views, table=table, plans=(plan1, plan2), max_elems=max_elems,
-                    keep=keep, flat=None if arena is not None else flat)
+                    parts=([k[0] for k in keep], [k[1] for k in keep]) if x3 else None, keep=keep,
+                    flat=None if arena is not None else flat)
 
     def _precondition_kron_grouped(self, todo, grad_scale):
         ext = ops.extension()
@@ -1175,11 +1176,15 @@ class FusedKfacGradientMaker(KfacGradientMaker):
             group = self._group = self._build_group(todo)
         grads = [st.module.weight.grad for st in todo]
         moved = [(v, g) for v, g in zip(group['views'], grads) if g.data_ptr() != v.data_ptr()]
-        if moved:
-            torch._foreach_copy_([v for v, _ in moved], [g for _, g in moved])
-        if grad_scale != 1:
-            torch._foreach_mul_(group['views'], grad_scale)
-        ext.cast_pad_bf16_grouped(group['table'], len(todo), group['max_elems'])
+        if group['parts'] is not None:
+            # the gradients are read where they lie: 94 MB of ResNet-50's are not written and read once more
+            ext.stage_gradients(grads, group['views'], *group['parts'], grad_scale)
+        else:
+            if moved:
+                torch._foreach_copy_([v for v, _ in moved], [g for _, g in moved])
+            if grad_scale != 1:
+                torch._foreach_mul_(group['views'], grad_scale)
+            ext.cast_pad_bf16_grouped(group['table'], len(todo), group['max_elems'])
         ext.gemm_plan_run(group['plans'][0])
         ext.gemm_plan_run(group['plans'][1])
         if moved:

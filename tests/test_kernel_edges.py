@@ -618,6 +618,35 @@ def test_casts_of_many_tensors(up):
         assert torch.equal(d, s.to(d.dtype))
 
 
+@pytest.mark.parametrize('scale', [1.0, -0.375])
+@pytest.mark.parametrize('count', [1, 3, 64, 131])
+def test_stage_gradients(ext, count, scale):
+    shapes = [(1, 1), (64, 3, 7, 7), (37, 65), (130, 8), (3, 2056), (5, 24, 3, 3), (2, 16, 1, 1), (700, 40)]
+    grads, staged, want = [], [], []
+    for i in range(count):
+        shape = shapes[i % len(shapes)]
+        numel = torch.Size(shape).numel()
+        rows, last = shape[0], i % 3 == 1 and len(shape) == 4                 # in the factor's order, or copied into it
+        fmt = torch.channels_last if len(shape) == 4 else torch.contiguous_format
+        v = torch.zeros(shape, device=DEV).contiguous(memory_format=fmt)
+        flat = torch.randn(numel + 1, device=DEV, generator=_gen(i))[i % 2:i % 2 + numel]   # on and off 16 bytes
+        if last or len(shape) == 2:
+            g = flat.view(shape)
+        else:
+            g = flat.as_strided(v.shape, v.stride())
+        grads.append(g.half() if i % 11 == 10 else g)
+        staged.append(v)
+        x = grads[-1].float().mul(scale)
+        want.append((x.permute(0, 2, 3, 1) if len(shape) == 4 else x).reshape(rows, -1))
+    hi, lo = ([torch.full((w.shape[0], (w.shape[1] + 7) // 8 * 8), 9.0, device=DEV, dtype=torch.bfloat16) for w in want] for _ in range(2))
+    kept = [g.clone() for g in grads]
+    ext.stage_gradients(grads, staged, hi, lo, scale)
+    for w, h, l, g, k in zip(want, hi, lo, grads, kept):
+        w = F.pad(w, (0, h.shape[1] - w.shape[1]))
+        assert torch.equal(h, w.bfloat16()) and torch.equal(l, (w - w.bfloat16().float()).bfloat16())
+        assert torch.equal(g, k)
+
+
 def test_max_pool_leaves_tensors_without_memory_to_pytorch():
     from torch._subclasses.fake_tensor import FakeTensorMode
     with FakeTensorMode():
