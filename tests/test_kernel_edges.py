@@ -647,6 +647,15 @@ def test_stage_gradients(ext, count, scale):
         assert torch.equal(g, k)
 
 
+@pytest.mark.parametrize('n', [1, 31, 33, 511, 513, 1000, 1031])
+def test_bias_products(ext, n):
+    inverse, bias, scratch = (torch.randn(shape, device=DEV, generator=_gen(n)) for shape in ((n, n), (n,), (n,)))
+    want = 0.5 * (inverse.double() @ bias.double())
+    bound = 0.5 * (inverse.double().abs() @ bias.double().abs()) * (n / 32 + 7) * 2.0 ** -24   # a lane's chain, then the lanes' sums
+    ext.bias_precondition_mt([[inverse.data_ptr(), bias.data_ptr(), scratch.data_ptr(), n]], 0.5)
+    assert bool(((bias.double() - want).abs() <= bound).all())
+
+
 def test_max_pool_leaves_tensors_without_memory_to_pytorch():
     from torch._subclasses.fake_tensor import FakeTensorMode
     with FakeTensorMode():
