@@ -448,8 +448,15 @@ __global__ void __launch_bounds__(256) cast_many_kernel(const __grid_constant__ 
 void cast_many(std::vector<at::Tensor> dst, std::vector<at::Tensor> src) {
   TORCH_CHECK(dst.size() == src.size(), "dst and src must have the same length");
   if (dst.empty()) return;
-  const auto alike = [](const at::Tensor& a, const at::Tensor& b) {
-    if (!a.is_cuda() || a.device() != b.device() || a.sizes() != b.sizes() || !a.is_non_overlapping_and_dense() || !b.is_non_overlapping_and_dense()) return false;
+  // what PyTorch has to look into: subclasses (a fake tensor has no memory), batches of vmap, values that are the negative of their memory
+  const auto plain = [](const at::Tensor& t) {
+    return t.layout() == at::kStrided && t.has_storage() &&
+           !t.key_set().has_any(c10::DispatchKeySet({c10::DispatchKey::Python, c10::DispatchKey::Batched, c10::DispatchKey::FuncTorchBatched,
+                                                     c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Functionalize,
+                                                     c10::DispatchKey::Negative, c10::DispatchKey::ZeroTensor}));
+  };
+  const auto alike = [&](const at::Tensor& a, const at::Tensor& b) {
+    if (!plain(a) || !plain(b) || !a.is_cuda() || a.device() != b.device() || a.sizes() != b.sizes() || !a.is_non_overlapping_and_dense() || !b.is_non_overlapping_and_dense()) return false;
     for (int64_t k = 0; k < a.dim(); ++k)
       if (a.size(k) > 1 && a.stride(k) != b.stride(k)) return false;
     return true;

@@ -104,6 +104,19 @@ def cuda_kernels_enabled(*tensors):
         t.dtype in (torch.float32, torch.bfloat16, torch.float16) for t in tensors)
 
 
+_PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
+
+
+def unobserved(*tensors):
+    """True when a native call on these tensors may stand in for PyTorch operations: they have memory of their own, which a fake
+    tensor has not, nor need any other subclass, and nothing records or transforms operations (a trace, a compilation, a dispatch
+    mode, ``torch.func``, forward-mode differentiation): it would see the call's allocations, but not the kernels that fill them."""
+    return (not torch.compiler.is_compiling() and torch._C._len_torch_dispatch_stack() == 0
+            and torch._ops._len_torch_dispatch_stack_pre_dispatch() == 0 and torch._C._get_tracing_state() is None
+            and not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0
+            and all(type(t) in _PLAIN_TYPES for t in tensors))
+
+
 def check_status(device=None):
     """Raises if a kernel reported a problem (timed-out wait, non-SPD matrix) since the last
     check.  Synchronises the current stream."""

@@ -1,0 +1,85 @@
+"""Native calls that stand in for PyTorch operations: only where nobody looks on who would see the allocations of the call and not
+its kernel, and only on tensors with memory of their own."""
+import types
+
+import pytest
+import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+from torch.fx.experimental.proxy_tensor import make_fx
+
+from asdl_b200 import ops
+from asdl_b200.models import layers, resnet_tiny
+
+
+class _NoExtension:
+    """In the place of the extension: every native call fails, before it can touch an address."""
+
+    def __getattr__(self, name):
+        def call(*args):
+            raise AssertionError(f'native call {name}')
+        return call
+
+
+def test_casts_of_tensors_without_memory_are_left_to_pytorch(monkeypatch):
+    monkeypatch.setattr(ops, 'extension', _NoExtension)
+    with FakeTensorMode(), torch.device('cuda'):
+        model = resnet_tiny(fused=True).eval()
+        x = torch.empty(2, 3, 64, 64, dtype=torch.bfloat16).contiguous(memory_format=torch.channels_last)
+        with layers.grouped_bf16_weights(model):
+            assert model.conv1.weight.dtype == torch.bfloat16 and model(x).shape == (2, 10)
+        # the way back: a gradient of a linear layer (transposed) and one of a convolution
+        shapes = [(32, 16), (8, 4, 3, 3)]
+        ctx = types.SimpleNamespace(meta=[(torch.Size(s), torch.empty(s).stride()) for s in shapes])
+        grads = [torch.empty(16, 32, dtype=torch.bfloat16).t(), torch.empty(8, 4, 3, 3, dtype=torch.bfloat16)]
+        back = layers._GroupedCast.backward(ctx, *grads)
+        assert all(g.dtype == torch.float32 and g.shape == s for g, s in zip(back, shapes))
+
+
+def test_calls_that_are_looked_at_are_not_native():
+    seen = []
+
+    def look(x):
+        seen.append(ops.unobserved(x))
+        return x * 2
+
+    x = torch.ones(3)
+    assert ops.unobserved(x) and ops.unobserved(torch.nn.Parameter(x))
+    for options in ({'tracing_mode': 'real'}, {'tracing_mode': 'fake'}, {'pre_dispatch': True}):
+        make_fx(look, **options)(x)
+    torch.jit.trace(look, (x,), check_trace=False)
+    torch.func.vmap(look)(x)
+    torch.func.jvp(look, (x,), (x,))
+    with torch.autograd.forward_ad.dual_level():
+        look(torch.autograd.forward_ad.make_dual(x, x))
+    with FakeTensorMode():
+        fake = torch.empty(3)
+    look(fake)   # outlives its mode
+    assert len(seen) == 8 and not any(seen)
+
+
+@pytest.mark.gpu
+def test_recorded_graphs_hold_the_casts():
+    """A graph that is recorded on real tensors computes with the weights of the model."""
+    model = resnet_tiny(fused=True).to('cuda').to(memory_format=torch.channels_last).eval()
+
+    def call(inp):
+        with layers.grouped_bf16_weights(model):
+            return model(inp)
+
+    with torch.no_grad():
+        x = [torch.randn(2, 3, 64, 64, device='cuda').to(torch.bfloat16).contiguous(memory_format=torch.channels_last) for _ in range(2)]
+        graph = make_fx(call)(x[0])
+        assert any('copy' in str(n.target) for n in graph.graph.nodes)
+        for inp in x:
+            torch.testing.assert_close(graph(inp), call(inp), rtol=2e-2, atol=2e-2)   # cuDNN may take another kernel
+
+
+@pytest.mark.gpu
+def test_casts_of_tensors_that_pytorch_has_to_look_into():
+    x = torch.randn(64, device='cuda')
+    got = torch.empty(64, device='cuda', dtype=torch.bfloat16)
+    ops.extension().cast_many([got], [torch._neg_view(x)])
+    assert torch.equal(got, -x.bfloat16())
+    with FakeTensorMode():
+        fake = [torch.empty(64, device='cuda', dtype=t) for t in (torch.bfloat16, torch.float32)]
+        ops.extension().cast_many(fake[:1], fake[1:])
