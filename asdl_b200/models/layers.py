@@ -92,17 +92,14 @@ class FusedLayerNorm(nn.LayerNorm):
 
 class FusedMaxPool2d(nn.MaxPool2d):
     """``nn.MaxPool2d`` whose forward / backward run on the library's NHWC kernels for 3 x 3 windows with stride 2 and channels_last
-    bf16 CUDA inputs with a multiple of 8 channels, and exactly like the parent otherwise, traced and under ``torch.func`` or
-    forward-mode differentiation too.  Same values and gradients."""
+    bf16 CUDA inputs with a multiple of 8 channels, and exactly like the parent otherwise, also where something records or transforms
+    operations (:func:`asdl_b200.ops.unobserved`).  Same values and gradients."""
 
     def _native(self, x):
         p = self.padding
-        # a subclass (a fake tensor, say) need not have memory
-        return (type(x) is torch.Tensor and self.kernel_size == 3 and self.stride == 2 and (p == 0 or p == 1) and self.dilation == 1 and not self.return_indices
+        return (ops.unobserved(x) and self.kernel_size == 3 and self.stride == 2 and (p == 0 or p == 1) and self.dilation == 1 and not self.return_indices
                 and not self.ceil_mode and x.is_cuda and x.dtype == torch.bfloat16 and x.ndim == 4
-                and torch._C._get_tracing_state() is None and not torch._C._are_functorch_transforms_active()
-                and not torch.compiler.is_compiling()
-                and torch.autograd.forward_ad._current_level < 0 and ops.cuda_kernels_enabled(x) and x.numel() > 0
+                and ops.cuda_kernels_enabled(x) and x.numel() > 0
                 and x.shape[1] % 8 == 0 and x.shape[0] <= 65535 and min(x.shape[2:]) + 2 * p >= 3 and max(x.shape[2:]) < 2 ** 30
                 and x.shape[1] * (x.shape[3] + 2) < 2 ** 33 and x.is_contiguous(memory_format=torch.channels_last) and x.data_ptr() % 16 == 0)
 

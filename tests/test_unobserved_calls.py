@@ -4,6 +4,7 @@ import types
 
 import pytest
 import torch
+import torch.nn.functional as F
 from torch._subclasses.fake_tensor import FakeTensorMode
 from torch.fx.experimental.proxy_tensor import make_fx
 
@@ -83,3 +84,16 @@ def test_casts_of_tensors_that_pytorch_has_to_look_into():
     with FakeTensorMode():
         fake = [torch.empty(64, device='cuda', dtype=t) for t in (torch.bfloat16, torch.float32)]
         ops.extension().cast_many(fake[:1], fake[1:])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('options', [{'tracing_mode': 'real'}, {'pre_dispatch': True}])
+def test_recorded_graphs_hold_the_pooling(options):
+    """A graph that is recorded on real tensors pools the activations that it is given."""
+    pool = layers.FusedMaxPool2d(3, stride=2, padding=1)
+    with torch.no_grad():
+        x = [torch.randn(2, 8, 9, 9, device='cuda').to(torch.bfloat16).contiguous(memory_format=torch.channels_last) for _ in range(2)]
+        assert pool._native(x[0])
+        graph = make_fx(lambda inp: pool(inp), **options)(x[0])
+        for inp in x:
+            assert torch.equal(graph(inp), F.max_pool2d(inp, 3, 2, 1))
