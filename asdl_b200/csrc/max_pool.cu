@@ -168,11 +168,12 @@ struct MaxPool : torch::autograd::Function<MaxPool> {
 
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
     const at::Tensor code = ctx->get_saved_variables()[0];
-    const at::Tensor dy = grads[0].contiguous(at::MemoryFormat::ChannelsLast);
+    at::Tensor dy = grads[0].contiguous(at::MemoryFormat::ChannelsLast);
     const auto sizes = ctx->saved_data["sizes"].toIntVector();
     const int64_t pad = ctx->saved_data["pad"].toInt();
     c10::cuda::CUDAGuard guard(dy.get_device());
     if (at::GradMode::is_enabled() && dy.requires_grad()) return {differentiable(dy, code, sizes, pad), at::Tensor()};
+    if ((reinterpret_cast<uintptr_t>(dy.data_ptr()) & 15) != 0) dy = dy.clone();   // a view into another gradient
     auto dx = at::empty(sizes, dy.options(), at::MemoryFormat::ChannelsLast);
     const Pool s = shape(dx, pad);
     TORCH_CHECK(plain(dy) && dy.size(2) == s.oh && dy.size(3) == s.ow && code.is_cuda() && code.get_device() == dy.get_device() &&

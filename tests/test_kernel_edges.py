@@ -656,6 +656,14 @@ def test_bias_products(ext, n):
     assert bool(((bias.double() - want).abs() <= bound).all())
 
 
+def test_max_pool_takes_gradients_at_any_address():
+    x = torch.randn(2, 8, 9, 9, device=DEV, generator=_gen(33)).to(torch.bfloat16).contiguous(memory_format=torch.channels_last).requires_grad_(True)
+    y, want = FusedMaxPool2d(3, stride=2, padding=1)(x), F.max_pool2d(x, 3, 2, 1)
+    dy = torch.randn(y.numel() + 1, device=DEV, generator=_gen(34)).to(torch.bfloat16)[1:].view(2, 5, 5, 8).permute(0, 3, 1, 2)
+    assert dy.data_ptr() % 16 and dy.is_contiguous(memory_format=torch.channels_last)
+    assert torch.equal(torch.autograd.grad(y, x, dy)[0], torch.autograd.grad(want, x, dy)[0])
+
+
 def test_max_pool_leaves_tensors_without_memory_to_pytorch():
     from torch._subclasses.fake_tensor import FakeTensorMode
     with FakeTensorMode():
