@@ -61,18 +61,18 @@ def test_calls_that_are_looked_at_are_not_native():
 @pytest.mark.gpu
 def test_recorded_graphs_hold_the_casts():
     """A graph that is recorded on real tensors computes with the weights of the model."""
-    model = resnet_tiny(fused=True).to('cuda').to(memory_format=torch.channels_last).eval()
+    model = torch.nn.Sequential(torch.nn.Linear(32, 64, bias=False), torch.nn.Linear(64, 16, bias=False)).to('cuda')
 
     def call(inp):
         with layers.grouped_bf16_weights(model):
             return model(inp)
 
     with torch.no_grad():
-        x = [torch.randn(2, 3, 64, 64, device='cuda').to(torch.bfloat16).contiguous(memory_format=torch.channels_last) for _ in range(2)]
+        x = [torch.randn(8, 32, device='cuda').to(torch.bfloat16) for _ in range(2)]
         graph = make_fx(call)(x[0])
         assert any('copy' in str(n.target) for n in graph.graph.nodes)
         for inp in x:
-            torch.testing.assert_close(graph(inp), call(inp), rtol=2e-2, atol=2e-2)   # cuDNN may take another kernel
+            assert torch.equal(graph(inp), call(inp))
 
 
 @pytest.mark.gpu
