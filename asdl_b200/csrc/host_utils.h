@@ -57,6 +57,15 @@ inline void encode_tmap_bf16_2d(CUtensorMap* out, const void* base, uint64_t inn
   TORCH_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed with code ", static_cast<int>(r));
 }
 
+// Whether the values of a tensor are what lies at its address.  PyTorch has to look into the others: subclasses with a dispatch of their
+// own (a fake tensor has no memory), batches of vmap, wrappers of torch.func, values that are the negative of their memory.
+inline bool values_in_memory(const at::Tensor& t) {
+  return t.layout() == at::kStrided && t.has_storage() &&
+         !t.key_set().has_any(c10::DispatchKeySet({c10::DispatchKey::Python, c10::DispatchKey::Batched, c10::DispatchKey::FuncTorchBatched,
+                                                   c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Functionalize,
+                                                   c10::DispatchKey::Negative, c10::DispatchKey::ZeroTensor}));
+}
+
 // Number of kernels of this extension launched so far in this process (all devices).
 inline std::atomic<long long>& launch_counter() {
   static std::atomic<long long> n{0};

@@ -9,6 +9,7 @@
 // The bytes (51 MB of activations, 13 pooled, 6 of positions) bound both: 32 x 64 x 112 x 112 in graphs forward 112.7 (PyTorch's
 // kernels) -> 20.2 us, backward 237.3 -> 19.4; 24 x 32 x 96 x 96 45.1 -> 7.0 and 107.4 -> 8.2, 4 x 16 x 32 x 32 9.8 -> 3.7 and 8.4 -> 2.0.  With
 // a thread per input pixel, one window loaded after the other, the backward pass took 58.6.
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <cuda_bf16.h>
 #include <torch/extension.h>
 
@@ -140,8 +141,13 @@ dim3 pool_grid(int width, int height, int vecs, int64_t images) {
               static_cast<unsigned>(images));
 }
 
-// The backward pass as a function that can be differentiated again: PyTorch's, on its indices.
-at::Tensor differentiable(const at::Tensor& dy, const at::Tensor& code, const std::vector<int64_t>& sizes, int64_t pad) {
+// The backward pass in operations of PyTorch, on its indices: for a gradient that is differentiated again, in reverse or by a tangent,
+// that is a batch (is_grads_batched) or a subclass, or while operations are recorded.
+bool needs_operations(const at::Tensor& dy) {
+  return (at::GradMode::is_enabled() && dy.requires_grad()) || c10::impl::TorchDispatchModeTLS::any_modes_set() || !values_in_memory(dy) ||
+         dy._fw_grad(0).defined();
+}
+at::Tensor backward_operations(const at::Tensor& dy, const at::Tensor& code, const std::vector<int64_t>& sizes, int64_t pad) {
   const auto place = code.view({dy.size(0), dy.size(2), dy.size(3), dy.size(1)}).permute({0, 3, 1, 2}).to(at::kLong);
   const auto options = place.options();
   const auto top = (at::arange(dy.size(2), options) * S - pad).view({-1, 1}), left = at::arange(dy.size(3), options) * S - pad;
@@ -168,11 +174,12 @@ struct MaxPool : torch::autograd::Function<MaxPool> {
 
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
     const at::Tensor code = ctx->get_saved_variables()[0];
-    at::Tensor dy = grads[0].contiguous(at::MemoryFormat::ChannelsLast);
+    at::Tensor dy = grads[0];
     const auto sizes = ctx->saved_data["sizes"].toIntVector();
     const int64_t pad = ctx->saved_data["pad"].toInt();
     c10::cuda::CUDAGuard guard(dy.get_device());
-    if (at::GradMode::is_enabled() && dy.requires_grad()) return {differentiable(dy, code, sizes, pad), at::Tensor()};
+    if (needs_operations(dy)) return {backward_operations(dy, code, sizes, pad), at::Tensor()};
+    dy = dy.contiguous(at::MemoryFormat::ChannelsLast);
     if ((reinterpret_cast<uintptr_t>(dy.data_ptr()) & 15) != 0) dy = dy.clone();   // a view into another gradient
     auto dx = at::empty(sizes, dy.options(), at::MemoryFormat::ChannelsLast);
     const Pool s = shape(dx, pad);

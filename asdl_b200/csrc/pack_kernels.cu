@@ -187,8 +187,7 @@ void stage_gradients(std::vector<at::Tensor> grads, std::vector<at::Tensor> stag
     const at::Tensor &g = grads[i], &v = staged[i];
     TORCH_CHECK(v.scalar_type() == at::kFloat && v.is_non_overlapping_and_dense() && v.device() == device && hi[i].device() == device &&
                     lo[i].device() == device && v.dim() > 0, "dense fp32 matrices on one device");
-    bool in_place = g.layout() == at::kStrided && g.device() == device && g.scalar_type() == at::kFloat && !g.is_neg() &&
-                    !g.key_set().has(c10::DispatchKey::Python) && g.sizes() == v.sizes();
+    bool in_place = values_in_memory(g) && g.device() == device && g.scalar_type() == at::kFloat && g.sizes() == v.sizes();
     for (int64_t d = 0; in_place && d < v.dim(); ++d) in_place = v.size(d) == 1 || g.stride(d) == v.stride(d);
     if (!in_place) v.copy_(g);
     if (v.numel() == 0) continue;
@@ -448,15 +447,8 @@ __global__ void __launch_bounds__(256) cast_many_kernel(const __grid_constant__ 
 void cast_many(std::vector<at::Tensor> dst, std::vector<at::Tensor> src) {
   TORCH_CHECK(dst.size() == src.size(), "dst and src must have the same length");
   if (dst.empty()) return;
-  // what PyTorch has to look into: subclasses (a fake tensor has no memory), batches of vmap, values that are the negative of their memory
-  const auto plain = [](const at::Tensor& t) {
-    return t.layout() == at::kStrided && t.has_storage() &&
-           !t.key_set().has_any(c10::DispatchKeySet({c10::DispatchKey::Python, c10::DispatchKey::Batched, c10::DispatchKey::FuncTorchBatched,
-                                                     c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Functionalize,
-                                                     c10::DispatchKey::Negative, c10::DispatchKey::ZeroTensor}));
-  };
-  const auto alike = [&](const at::Tensor& a, const at::Tensor& b) {
-    if (!plain(a) || !plain(b) || !a.is_cuda() || a.device() != b.device() || a.sizes() != b.sizes() || !a.is_non_overlapping_and_dense() || !b.is_non_overlapping_and_dense()) return false;
+  const auto alike = [](const at::Tensor& a, const at::Tensor& b) {
+    if (!values_in_memory(a) || !values_in_memory(b) || !a.is_cuda() || a.device() != b.device() || a.sizes() != b.sizes() || !a.is_non_overlapping_and_dense() || !b.is_non_overlapping_and_dense()) return false;
     for (int64_t k = 0; k < a.dim(); ++k)
       if (a.size(k) > 1 && a.stride(k) != b.stride(k)) return false;
     return true;

@@ -664,6 +664,25 @@ def test_max_pool_takes_gradients_at_any_address():
     assert torch.equal(torch.autograd.grad(y, x, dy)[0], torch.autograd.grad(want, x, dy)[0])
 
 
+def test_max_pool_gradients_that_pytorch_has_to_look_into():
+    """Batches of gradients, gradients with a tangent, negative views: the results of the parent."""
+    x = torch.randn(2, 8, 9, 9, device=DEV, generator=_gen(35)).to(torch.bfloat16).contiguous(memory_format=torch.channels_last).requires_grad_(True)
+    y, want = FusedMaxPool2d(3, stride=2, padding=1)(x), F.max_pool2d(x, 3, 2, 1)
+    dy, tangent = (torch.randn_like(want) for _ in range(2))
+
+    def back(out, g, **options):
+        return torch.autograd.grad(out, x, g, retain_graph=True, **options)[0]
+
+    batch = torch.stack([dy, tangent])
+    assert torch.equal(back(y, batch, is_grads_batched=True), back(want, batch, is_grads_batched=True))
+    assert torch.equal(torch.func.vmap(lambda g: back(y, g))(batch), torch.func.vmap(lambda g: back(want, g))(batch))
+    assert torch.equal(back(y, torch._neg_view(dy)), back(want, -dy))
+    ad = torch.autograd.forward_ad
+    with ad.dual_level():
+        got, ref = (ad.unpack_dual(back(out, ad.make_dual(dy, tangent))) for out in (y, want))
+        assert torch.equal(got.primal, ref.primal) and torch.equal(got.tangent, ref.tangent)
+
+
 def test_max_pool_leaves_tensors_without_memory_to_pytorch():
     from torch._subclasses.fake_tensor import FakeTensorMode
     with FakeTensorMode():
