@@ -78,8 +78,11 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> batch_norm_autograd(at::Tensor x,
                                                                    c10::optional<at::Tensor> num_batches_tracked, double momentum,
                                                                    double eps, c10::optional<at::Tensor> residual, bool relu,
                                                                    bool mask_from_x) {
-  const bool differentiable = at::GradMode::is_enabled() && (x.requires_grad() || weight.requires_grad() || bias.requires_grad() ||
-                                                             (residual.has_value() && residual->requires_grad()));
+  // whether there will be a backward pass, which reads the mask: any tensor among the arguments counts, as for the engine
+  bool differentiable = x.requires_grad() || weight.requires_grad() || bias.requires_grad();
+  for (const auto* t : {&running_mean, &running_var, &num_batches_tracked, &residual})
+    differentiable |= t->has_value() && (*t)->requires_grad();
+  differentiable &= at::GradMode::is_enabled();
   auto out = BatchNormTrain::apply(x, weight, bias, running_mean, running_var, num_batches_tracked, momentum, eps, residual, relu,
                                    relu && !residual.has_value() && mask_from_x, differentiable);
   return {out[0], out[1], out[2]};

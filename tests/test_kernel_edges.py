@@ -737,6 +737,16 @@ def test_native_norm_functions_keep_the_rules_of_autograd(which):
         torch.autograd.grad(y3, leaves, dy)
 
 
+def test_batch_norm_with_running_statistics_that_require_a_gradient():
+    """They make the output part of a graph, whose backward pass has a mask to read and no gradient for them."""
+    x = torch.randn(2, 8, 5, 5, device=DEV, generator=_gen(36)).to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
+    weight, bias, mean, var = (torch.ones(8, device=DEV) for _ in range(4))
+    y = ops.batch_norm_train(x, weight, bias, mean.requires_grad_(True), var, residual=x, relu=True)
+    assert y.requires_grad
+    y.float().sum().backward()
+    assert mean.grad is None
+
+
 class _Cut(torch.autograd.Function):
     """Identity whose backward gives no gradient."""
 
