@@ -66,6 +66,9 @@ inline bool values_in_memory(const at::Tensor& t) {
                                                    c10::DispatchKey::Negative, c10::DispatchKey::ZeroTensor}));
 }
 
+// Rows of consecutive values.  The stride of a single column is any number, which contiguous() leaves as it is.
+inline bool unit_columns(const at::Tensor& t) { return t.stride(1) == 1 || t.size(1) <= 1; }
+
 // Number of kernels of this extension launched so far in this process (all devices).
 inline std::atomic<long long>& launch_counter() {
   static std::atomic<long long> n{0};

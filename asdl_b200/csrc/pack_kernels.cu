@@ -161,7 +161,7 @@ void cast_jobs(const std::vector<at::Tensor>& src, const std::vector<at::Tensor>
   CastJobs<3> t;
   t.count = 0;
   for (int i = 0; i < 3; ++i) {
-    TORCH_CHECK(src[i].scalar_type() == at::kFloat && src[i].stride(1) == 1, "fp32 with unit column stride");
+    TORCH_CHECK(src[i].scalar_type() == at::kFloat && unit_columns(src[i]), "fp32 with unit column stride");
     if (hi[i].numel() > 0) t.job[t.count++] = cast_job(src[i].data_ptr<float>(), src[i].stride(0), src[i].size(0), src[i].size(1), hi[i], lo[i]);
   }
   launch_cast_jobs(t, 1.0, at::cuda::getCurrentCUDAStream(src[0].get_device()).stream());
@@ -250,7 +250,7 @@ void launch_cast(const T* src, long long lds, float scale, __nv_bfloat16* p0, __
 }
 
 void cast_pad_bf16(at::Tensor src, at::Tensor hi, c10::optional<at::Tensor> lo, double scale) {
-  TORCH_CHECK(src.is_cuda() && src.dim() == 2 && src.stride(1) == 1, "src must be 2-D, unit col stride");
+  TORCH_CHECK(src.is_cuda() && src.dim() == 2 && unit_columns(src), "src must be 2-D, unit col stride");
   TORCH_CHECK(hi.is_cuda() && hi.scalar_type() == at::kBFloat16 && hi.dim() == 2 &&
                   hi.is_contiguous() && hi.size(0) == src.size(0) && hi.size(1) >= src.size(1),
               "hi must be contiguous bf16 [rows, >= n]");
@@ -290,7 +290,7 @@ void cast_pad_bf16(at::Tensor src, at::Tensor hi, c10::optional<at::Tensor> lo, 
 // the full 24-bit significand of v.  Six tensor-core products of such parts (hi*hi, hi*mid, mid*hi,
 // hi*lo, mid*mid, lo*hi) reproduce an fp32 product to ~2^-24.
 void cast_split3(at::Tensor src, at::Tensor hi, at::Tensor mid, at::Tensor lo) {
-  TORCH_CHECK(src.is_cuda() && src.dim() == 2 && src.stride(1) == 1 && src.scalar_type() == at::kFloat,
+  TORCH_CHECK(src.is_cuda() && src.dim() == 2 && unit_columns(src) && src.scalar_type() == at::kFloat,
               "src must be a 2-D fp32 CUDA tensor with unit column stride");
   for (const at::Tensor* t : {&hi, &mid, &lo})
     TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kBFloat16 && t->dim() == 2 && t->is_contiguous() &&

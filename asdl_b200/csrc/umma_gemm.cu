@@ -531,7 +531,7 @@ static std::vector<at::Tensor> stage_parts(const at::Tensor& x, bool x3) {
   const auto options = x.options().dtype(at::kBFloat16);
   std::vector<at::Tensor> parts = {at::empty({rows, ld}, options)};
   if (x3) parts.push_back(at::empty({rows, ld}, options));
-  cast_pad_bf16(x.stride(1) == 1 ? x : x.contiguous(), parts[0], x3 ? c10::optional<at::Tensor>(parts[1]) : c10::nullopt, 1.0);
+  cast_pad_bf16(unit_columns(x) ? x : x.contiguous(), parts[0], x3 ? c10::optional<at::Tensor>(parts[1]) : c10::nullopt, 1.0);
   if (ld != n)
     for (at::Tensor& p : parts) p = p.narrow(1, 0, n);
   return parts;
@@ -548,7 +548,7 @@ at::Tensor kron_staged(at::Tensor left, at::Tensor mid, at::Tensor right, bool x
   const bool all_fp32 = left.scalar_type() == at::kFloat && mid.scalar_type() == at::kFloat && right.scalar_type() == at::kFloat &&
                         left.device() == mid.device() && right.device() == mid.device();
   if (x3 && all_fp32 && mid.numel() > 0 && left.numel() > 0 && right.numel() > 0 && right.size(1) < (1LL << 27) && n < (1LL << 27)) {
-    const auto rows = [](const at::Tensor& x) { return x.stride(1) == 1 ? x : x.contiguous(); };
+    const auto rows = [](const at::Tensor& x) { return unit_columns(x) ? x : x.contiguous(); };
     const std::vector<at::Tensor> src = {rows(l_col ? left.t() : left), rows(mid), rows(r_col ? right.t() : right)};
     std::vector<at::Tensor> hi, lo;
     for (const at::Tensor& x : src)

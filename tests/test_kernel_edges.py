@@ -576,7 +576,7 @@ def test_max_pool_gives_the_bits_of_pytorch(padding, n, c, h, w):
     assert torch.equal(again, v.flatten(2).gather(2, where.flatten(2)).view_as(again))
 
 
-@pytest.mark.parametrize('m,n', [(1, 2), (2, 2), (8, 8), (7, 9), (1, 300), (129, 2049), (640, 24)])
+@pytest.mark.parametrize('m,n', [(1, 1), (2, 1), (129, 1), (1, 2), (2, 2), (8, 8), (7, 9), (1, 300), (129, 2049), (640, 24)])
 def test_two_sided_product_stages_its_operands_together(m, n):
     """Pitches that are padded or not, rows that are aligned or not, strided and transposed operands."""
     def spd(k, seed):
@@ -590,6 +590,25 @@ def test_two_sided_product_stages_its_operands_together(m, n):
             got = ops.kron_apply(left, mid, r)
             # hi and lo parts carry 2^-16 of every operand of the two products
             assert (got.double() - want).norm() <= 4 * 2.0 ** -16 * want.norm()
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize('rows', [1, 7, 200])
+def test_one_column_of_any_stride(rows, dtype):
+    """contiguous() returns a column as it is, whatever the stride of its columns."""
+    wide = torch.randn(rows, 5, device=DEV, generator=_gen(56)).to(dtype)
+    other = torch.randn(rows, 3, device=DEV, generator=_gen(57)).to(dtype)
+    for x in (wide.T.contiguous().T[:, :1], wide[:, 1::5], wide[:, 3:]):
+        x = x[:, :1]
+        want, bound = x.double().T @ x.double(), 2.0 ** -15 * x.double().square().sum()   # hi and lo parts carry 2^-16 of every operand
+        assert ((ops.gram(x).double() - want).abs() <= bound).all()
+        with torch.no_grad():
+            got, ref = ops.matmul_tn(x, other).double(), x.double().T @ other.double()
+        assert ((got - ref).abs() <= 2.0 ** -15 * x.double().norm() * other.double().norm(dim=0)).all()
+        if dtype == torch.float32:
+            assert torch.equal(sum(p.float() for p in ops.split3(x)), x)
+            one = torch.ones(1, 1, device=DEV).T
+            assert (ops.kron_apply(torch.eye(rows, device=DEV), x, one).double() - x.double()).norm() <= 2.0 ** -14 * x.double().norm()
 
 
 @pytest.mark.parametrize('up', [False, True])
