@@ -96,15 +96,21 @@ def set_gemm_tiles(mode: int = -1):
     extension().set_gemm_wide(int(mode))
 
 
+_KERNEL_DTYPES = (torch.float32, torch.bfloat16, torch.float16)
+_PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
+
+
 def cuda_kernels_enabled(*tensors):
-    """True when the custom kernels should handle these tensors."""
+    """True when the custom kernels should handle these tensors: floating-point ones in the memory of a GPU (a fake tensor, or
+    another subclass with a dispatch of its own, need not have any)."""
     if _backend == 'torch':
         return False
-    return all(t.is_cuda for t in tensors) and all(
-        t.dtype in (torch.float32, torch.bfloat16, torch.float16) for t in tensors)
-
-
-_PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
+    for t in tensors:
+        if not t.is_cuda or t.dtype not in _KERNEL_DTYPES:
+            return False
+        if type(t) not in _PLAIN_TYPES and torch._C._dispatch_keys(t).has(torch._C.DispatchKey.Python):
+            return False
+    return True
 
 
 def unobserved(*tensors):

@@ -36,6 +36,19 @@ def test_casts_of_tensors_without_memory_are_left_to_pytorch(monkeypatch):
         assert all(g.dtype == torch.float32 and g.shape == s for g, s in zip(back, shapes))
 
 
+def test_tensors_without_memory_do_not_reach_a_kernel(monkeypatch):
+    monkeypatch.setattr(ops, 'extension', _NoExtension)
+    with FakeTensorMode(), torch.device('cuda'):
+        x, square = torch.empty(12, 8), torch.empty(8, 8)
+        assert ops.gram(x).shape == (8, 8) and ops.kron_apply(torch.empty(12, 12), x, square).shape == (12, 8)
+        assert ops.matmul_tn(x, x).shape == (8, 8) and ops.eigh(square)[0].shape == (8,)
+        norm = layers.FusedBatchNorm2d(8, act='relu')
+        act = torch.empty(2, 8, 5, 5, dtype=torch.bfloat16).contiguous(memory_format=torch.channels_last)
+        assert norm(act, residual=act).shape == act.shape
+        assert not ops.layer_norm_supported(torch.empty(4, 256, dtype=torch.bfloat16), torch.empty(256), torch.empty(256))
+        assert torch.nn.Parameter(x).is_cuda and not ops.cuda_kernels_enabled(torch.nn.Parameter(x))
+
+
 def test_calls_that_are_looked_at_are_not_native():
     seen = []
 
