@@ -356,7 +356,7 @@ bn_apply(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ 
   };
   fetch(std::integral_constant<int, 0>());
   fetch(std::integral_constant<int, 1>());
-  fetch(std::integral_constant<int, 2>());   // x and res are older than the chain, whose first kernel waits for all before it
+  fetch(std::integral_constant<int, 2>());   // x and res are older than the chain, whose first kernel, bn_sums, is launched plainly
   chain_wait();
   f32x2 a[4], b[4];
   load_pairs(scale + c0, a);
@@ -591,6 +591,7 @@ std::vector<at::Tensor> bn_forward_train(at::Tensor x, at::Tensor weight, at::Te
   auto part = at::empty({s.splits, s.channels, 2}, f32);
   auto coef = at::empty({2, s.channels}, f32);
   float* partp = part.data_ptr<float>();
+  // plainly: bn_apply reads x and the residual ahead of its wait
   bn_sums<false, MASK_NONE><<<dim3(s.chunks, s.splits), LANES * s.groups, 0, stream>>>(
       xp, xp, nullptr, nullptr, nullptr, nullptr, nullptr, partp, s.rows, s.channels, s.groups, s.rows_per_split);
   launch_chained(bn_fwd_finalize, dim3((s.channels + 7) / 8), dim3(256), 0, stream, partp, weight.data_ptr<float>(),
@@ -657,7 +658,7 @@ std::vector<at::Tensor> bn_backward_train(at::Tensor x, at::Tensor dy, at::Tenso
   auto part = at::empty({s.splits, s.channels, 2}, f32);
   auto coef = at::empty({5, s.channels}, f32);
   float* partp = part.data_ptr<float>();
-  auto sums = [&](auto kernel) {
+  auto sums = [&](auto kernel) {   // plainly: bn_dx reads x, dy and the mask ahead of its wait
     kernel<<<dim3(s.chunks, s.splits), LANES * s.groups, 0, stream>>>(xp, gp, maskp, mp, ip, wp, bp, partp, s.rows, s.channels, s.groups,
                                                                    s.rows_per_split);
   };

@@ -3,7 +3,9 @@
 //
 // Every kernel launched this way calls chain_wait() before its first access to global memory, reads and writes alike.  The wait
 // ends when the kernel before it has finished and its writes are visible; since that one waited in the same way, everything
-// before it has finished too.  What a kernel of the chain has written is read by ordinary loads, not through __ldg or a
+// before it has finished too.  One exception: the first kernel of a chain is launched plainly, so that all older work has finished
+// before any kernel of the chain is on an SM, and bn_apply and bn_dx (batchnorm.cu) read ahead of their wait what is older than
+// the chain.  That holds only as long as bn_sums, the first kernel there, is launched plainly.  What a kernel of the chain has written is read by ordinary loads, not through __ldg or a
 // const __restrict__ parameter: the read-only path is for data that nobody writes while the kernel is resident, and the compiler
 // may move such loads ahead of the wait.  __ldcg takes its pointer from after_wait().  chain_next() lets the next kernel come as soon as all CTAs of this one have called it.
 // Launched plainly -> chained, passes in turn: 8192 x 1024 bf16 samples 27.3 -> 22.9 us, 12608 x 768 fp32 samples 52.9 -> 46.9, the

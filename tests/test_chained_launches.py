@@ -63,3 +63,18 @@ def test_every_kernel_of_a_chain_waits():
     waiting = {k for name in os.listdir(CSRC) if name.endswith(('.cu', '.cuh')) for k, _, body in _kernels(name)
                if 'chain_wait()' in body}
     assert chained and chained <= waiting
+
+
+def test_chains_whose_kernels_read_ahead_of_the_wait_begin_with_a_plain_launch():
+    """Only the last kernels of BatchNorm do, and what they read there is older than the chain because bn_sums is launched plainly."""
+    ahead = {k for name in os.listdir(CSRC) if name.endswith(('.cu', '.cuh')) for k, _, body in _kernels(name)
+             if 'chain_wait()' in body and re.search(r'\bfetch\w*\(', body[:body.index('chain_wait()')])}
+    assert ahead == {'bn_apply', 'bn_dx'}
+    text = _source('batchnorm.cu')
+    launches = text[text.index('std::vector<at::Tensor> bn_forward_train('):]
+    for use in re.finditer(r'bn_sums<[^>]*>', launches):
+        assert launches[use.end():].startswith('<<<') or launches[:use.start()].endswith('sums(')
+    assert len(re.findall(r'auto sums = \[&\]\(auto kernel\) \{\s*kernel<<<', launches)) == 1
+    for name in ('bn_forward_train', 'bn_backward_train'):
+        body = launches[launches.index(name + '('):]
+        assert re.search(r'<<<|launch_chained\(', body).group() == '<<<'
