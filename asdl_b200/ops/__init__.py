@@ -702,27 +702,12 @@ def batchnorm_unitwise_stats_from_input(x, dy, y, mean, invstd, out, alpha=1.0, 
     return out.mul_(beta).add_(new, alpha=alpha)
 
 
-class _LayerNormFn(torch.autograd.Function):
-    """LayerNorm over the last dimension on the library's bf16 kernels, for ``torch.jit.trace`` (see ``_BatchNormTrain``)."""
-
-    @staticmethod
-    def forward(ctx, x, weight, bias, eps):
-        y, mean, rstd = extension().ln_forward(x, weight.detach(), bias.detach(), float(eps))
-        ctx.save_for_backward(x, weight, mean, rstd)
-        return y
-
-    @staticmethod
-    def backward(ctx, dy):
-        x, weight, mean, rstd = ctx.saved_tensors
-        dx, dweight, dbias = extension().ln_backward(x, dy.contiguous(), weight.detach(), mean, rstd)
-        return dx, dweight, dbias, None
-
-
 _LN_SIZES = {256 * v for v in (1, 2, 3, 4, 6, 8, 12, 16)}
 
 
 def layer_norm_supported(x: torch.Tensor, weight, bias) -> bool:
-    return (weight is not None and bias is not None and weight.ndim == 1 and cuda_kernels_enabled(x)
+    # a jit trace would see the allocations of the native function only
+    return (torch._C._get_tracing_state() is None and weight is not None and bias is not None and weight.ndim == 1 and cuda_kernels_enabled(x)
             and x.dtype == torch.bfloat16 and x.is_contiguous() and x.numel() > 0
             and x.shape[-1] == weight.numel() and weight.numel() in _LN_SIZES
             and weight.dtype == torch.float32 and bias.dtype == torch.float32)
@@ -734,9 +719,7 @@ def layer_norm(x, weight, bias, eps=1e-5):
     backward (the input gradient and the weight / bias gradients come out of one pass over dy and
     x); anything else: ``F.layer_norm``."""
     if layer_norm_supported(x, weight, bias):
-        if torch._C._get_tracing_state() is None:
-            return extension().layer_norm_autograd(x, weight, bias, eps)
-        return _LayerNormFn.apply(x, weight, bias, eps)
+        return extension().layer_norm_autograd(x, weight, bias, eps)
     return torch.nn.functional.layer_norm(x, (weight.numel(),) if weight is not None else x.shape[-1:],
                                           weight, bias, eps)
 
