@@ -138,15 +138,9 @@ __device__ __forceinline__ unsigned long long last_use() {
   asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
   return policy;
 }
-#ifndef BN_ST
-#define BN_ST 1
-#endif
+// Results are not read again in their direction: streaming stores.
 __device__ __forceinline__ void store(__nv_bfloat16* p, const uint32_t (&w)[4]) {
-#if BN_ST
   asm volatile("st.global.cs.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
-#else
-  *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
-#endif
 }
 
 // How the backward kernels find the ReLU mask: no activation, from the bits that the forward pass has left (a sixteenth of the
