@@ -56,9 +56,6 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> batch_norm_autograd(at::Tensor x,
 at::Tensor layer_norm_autograd(at::Tensor x, at::Tensor weight, at::Tensor bias, double eps);
 at::Tensor max_pool_autograd(at::Tensor x, int64_t pad);
 bool ln_supported_size(int64_t d);
-std::vector<at::Tensor> ln_forward(at::Tensor x, at::Tensor weight, at::Tensor bias, double eps);
-std::vector<at::Tensor> ln_backward(at::Tensor x, at::Tensor dy, at::Tensor weight, at::Tensor mean,
-                                    at::Tensor rstd);
 void symm_barrier(at::Tensor peers, int64_t rank, int64_t world, int64_t slot, int64_t wait_ms);
 void symm_reduce_segments(at::Tensor peers, int64_t rank, int64_t world, at::Tensor segs, double scale,
                           int64_t mc_ptr);
@@ -135,8 +132,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("max_pool_autograd", &b200::max_pool_autograd);
   m.def("bn_unitwise_stats_xhat", &b200::bn_unitwise_stats_xhat);
   m.def("ln_supported_size", &b200::ln_supported_size);
-  m.def("ln_forward", &b200::ln_forward);
-  m.def("ln_backward", &b200::ln_backward);
   m.def("symm_barrier", &b200::symm_barrier);
   m.def("symm_reduce_segments", &b200::symm_reduce_segments, py::arg("peers"), py::arg("rank"), py::arg("world"),
         py::arg("segs"), py::arg("scale"), py::arg("mc_ptr") = 0);
