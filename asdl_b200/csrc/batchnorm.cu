@@ -31,6 +31,7 @@
 
 #include "chained_launch.h"
 #include "host_utils.h"
+#include "packed_fp32.cuh"
 #include "row_walk.h"
 
 #include <type_traits>
@@ -44,43 +45,15 @@ constexpr int LANES = 32;    // row lanes of a split
 constexpr int THREADS = GROUPS * LANES;
 constexpr int MIN_ROWS = 512;   // of a split, where there are more
 
-// Two fp32 values in a register pair: the packed instructions round each as the scalar ones do and take half the issue slots, which
-// is what these kernels run out of beside the memory.
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pair(uint32_t lo, uint32_t hi) {
-  f32x2 v;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
-  return v;
-}
-__device__ __forceinline__ f32x2 pair(float lo, float hi) { return pair(__float_as_uint(lo), __float_as_uint(hi)); }
-__device__ __forceinline__ float2 split(f32x2 v) {
-  uint32_t lo, hi;
-  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
-  return make_float2(__uint_as_float(lo), __uint_as_float(hi));
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 v;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
-  return v;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 v;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
-  return v;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 v;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
-  return v;
-}
+// Sums and transforms work on packed pairs of values: issue slots are what these kernels run out of beside the memory.
 
 // 8 bf16 values as 4 words -> 4 pairs, and back
 __device__ __forceinline__ void unpack(const uint32_t (&w)[4], f32x2 (&out)[4]) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) out[i] = pair(w[i] << 16, w[i] & 0xffff0000u);
+  for (int i = 0; i < 4; ++i) out[i] = pack2(w[i] << 16, w[i] & 0xffff0000u);
 }
 __device__ __forceinline__ uint32_t pack(f32x2 v) {
-  const float2 f = split(v);
+  const float2 f = unpack2(v);
   const __nv_bfloat162 h = __floats2bfloat162_rn(f.x, f.y);
   return reinterpret_cast<const uint32_t&>(h);
 }
@@ -149,7 +122,7 @@ enum : int { MASK_NONE = 0, MASK_BITS = 1, MASK_FROM_X = 2 };
 __device__ __forceinline__ void mask_from_x(const f32x2 (&x)[4], const f32x2 (&scale)[4], const f32x2 (&shift)[4], uint32_t (&g)[4]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float2 y = split(fma2(x[i], scale[i], shift[i]));
+    const float2 y = unpack2(fma2(x[i], scale[i], shift[i]));
     g[i] = (y.x > 0.f ? g[i] & 0xffffu : 0u) | (y.y > 0.f ? g[i] & 0xffff0000u : 0u);
   }
 }
@@ -252,7 +225,7 @@ bn_sums(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ d
   float4* red = reinterpret_cast<float4*>(memory);   // [pair of channels][lane][group]
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float2 a = split(first[i]), b = split(second[i]);
+    const float2 a = unpack2(first[i]), b = unpack2(second[i]);
     red[i * THREADS + t] = make_float4(a.x, b.x, a.y, b.y);
   }
   __syncthreads();

@@ -36,6 +36,7 @@
 #include <cstring>
 
 #include "gemm2_host.h"
+#include "packed_fp32.cuh"
 #include "prepared_cache.h"
 
 namespace b200 {
@@ -102,20 +103,6 @@ constexpr int DG_SMEM = (TB * DG_SP + 2 * 32 * DG_PP + 32 * DG_LP + 32) * 4;
 
 // Barrier of the eight epilogue warps.
 __device__ __forceinline__ void epi_sync() { named_bar_sync(1, 256); }
-
-// Two fp32 values in one register pair; fma2: a * b + c of both, each rounded as fmaf does.
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
 
 // 1 / sqrt(pivot d); a pivot that is not positive is reported and replaced by 1.  The usual case has no branch in the chain:
 // rsqrt.approx.ftz is exact enough for the Newton step that follows, and subnormal pivots go another way.
