@@ -10,8 +10,8 @@
 // may move such loads ahead of the wait.  __ldcg takes its pointer from after_wait().  chain_next() lets the next kernel come as soon as all CTAs of this one have called it.
 // Launched plainly -> chained, passes in turn: 8192 x 1024 bf16 samples 27.3 -> 22.9 us, 12608 x 768 fp32 samples 52.9 -> 46.9, the
 // convolution factors of 32 x 256 x 14 x 14 bf16 47.7 -> 41.7 and of 128 x 64 x 32 x 32 fp32 82.6 -> 78.6, 1024 x 4096 between fp32 factors 153 -> 149.
-// What a chained kernel gets of the SMs while the one before it still runs can be uneven or short of L1 cache: two launches are
-// plain for that reason (gemm2_plain.cu, conv_gram.cu).
+// What a chained kernel gets of the SMs while the one before it still runs can be uneven (gemm2_plain.cu has what that costs) or short of
+// L1 cache: one launch is plain for that reason (conv_gram.cu).
 // A kernel that is launched plainly behind a chain waits for its end as usual; a captured chain becomes programmatic edges.
 #pragma once
 #include <utility>

@@ -19,13 +19,12 @@ void g2_run_plain(const GemmProblem2& single, const GemmProblem2* probs, const G
     attr_set = true;
   }
   const int grid = std::min(n_work, 2 * n_sms);
-  // A chained launch fills the SMs as the kernel before leaves them, two CTAs on some and none on others, where a plain one gives each SM
-  // one first.  That matters where a few more CTAs than SMs have long epilogues, of 4-byte stores: symmetric products of 64 rows with beta, us
-  // plainly -> chained: n = 2101 (153 tiles) 21.6 -> 22.9; but 1801 (120) 18.0 -> 17.5, 2001 (136) 18.5 -> 17.5 (beta 0: 15.4 -> 14.4), 2177 (171) 27.6 ->
-  // 27.2.
-  const bool uneven = probs == nullptr && single.nsplit == 1 && single.C != nullptr &&
-                      ((single.ldc & 3) != 0 || (reinterpret_cast<uintptr_t>(single.C) & 15) != 0) && n_work > n_sms && 8 * n_work <= 9 * n_sms;
-  launch_behind(g2_may_chain(probs) && !uneven, umma_gemm2_kernel<128, 4, 2, 1>, dim3(grid), dim3(G2Plain::THREADS), G2Plain::SMEM_BYTES, stream, single, probs, work, n_work, prefix, n_probs);
+  // Chained at any number of tiles.  Behind a chain two CTAs come to some SMs and none to others, and where a few more tiles than SMs
+  // have the longest epilogues, symmetric ones with beta and 4-byte stores, a plain launch is up to 1.5 us faster: 153 tiles, us plainly ->
+  // chained: 64 rows x 2057 17.6 -> 18.5, 64 x 2101 20.0 -> 21.5, 96 x 2101 20.3 -> 22.1, 128 x 2173 25.3 -> 25.8.  But 32 x 2101 19.8 -> 19.0,
+  // 192 x 2101 21.8 -> 20.7, 256 x 2101 22.5 -> 21.6, and everything else of 150 - 168 tiles gains as at other counts: 64 x 2101 and
+  // 2171 without beta 17.4 -> 17.4 and 20.8 -> 19.9, 1280 x 1793 of 64 rows 17.6 -> 16.2 and with beta 22.2 -> 21.0, 1408 x 1665 17.7 -> 16.7.
+  launch_behind(g2_may_chain(probs), umma_gemm2_kernel<128, 4, 2, 1>, dim3(grid), dim3(G2Plain::THREADS), G2Plain::SMEM_BYTES, stream, single, probs, work, n_work, prefix, n_probs);
   B200_CUDA_CHECK(cudaGetLastError());
   count_launch();
 }
