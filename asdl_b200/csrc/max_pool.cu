@@ -6,8 +6,8 @@
 // maximum a pixel is, so that every value is written once and needs no zeros first.  Comparisons and selections work on two values at
 // a time.  Values and gradients are PyTorch's: the first of equal values wins, a NaN wins over everything before it.
 //
-// The bytes (51 MB of activations, 13 pooled, 6 of positions) bound both: 32 x 64 x 112 x 112 in graphs forward 112.7 (PyTorch's
-// kernels) -> 20.2 us, backward 237.3 -> 19.4; 24 x 32 x 96 x 96 45.1 -> 7.0 and 107.4 -> 8.2, 4 x 16 x 32 x 32 9.8 -> 3.7 and 8.4 -> 2.0.  With
+// Instruction issue bounds both (62 and 76 % of the slots busy): 70 MB (51 of activations, 13 pooled, 6 of positions) would take memory
+// 11 us, and a pass over 32 x 64 x 112 x 112 runs at half that rate.  In graphs: forward 112.7 (PyTorch's kernels) -> 20.2 us, backward 237.3 -> 19.4; 24 x 32 x 96 x 96 45.1 -> 7.0 and 107.4 -> 8.2, 4 x 16 x 32 x 32 9.8 -> 3.7 and 8.4 -> 2.0.  With
 // a thread per input pixel, one window loaded after the other, the backward pass took 58.6.
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <cuda_bf16.h>

@@ -169,9 +169,9 @@ void cast_jobs(const std::vector<at::Tensor>& src, const std::vector<at::Tensor>
 
 // scale * grads[i] -> hi[i], lo[i].  staged[i] is the dense fp32 view, of the gradient's shape, whose memory is the matrix [rows, n]
 // of the factor's order: a gradient of the same strides is read where it lies, another one is copied there first.  Up to 64
-// gradients share a launch, whose table travels as an argument: they lie elsewhere in each step. Bound by memory; ResNet-50's
-// 54 matrices (188 MB with the parts) take 11 us from L2 and HBM together, with the copy ahead of them it was 30: ten steps
-// 24.13 -> 23.94 ms.
+// gradients share a launch, whose table travels as an argument: they lie elsewhere in each step. Bound by memory: ResNet-50's
+// 54 matrices (102 MB, 204 with the parts), two sets of them in turn in a graph, 97.0 us copied and split -> 38.2; the 18 of a
+// bottleneck ResNet of four blocks (80 MB with the parts) 41.1 -> 16.7, and ten K-FAC steps of that one 24.13 -> 23.94 ms.
 void stage_gradients(std::vector<at::Tensor> grads, std::vector<at::Tensor> staged, std::vector<at::Tensor> hi,
                      std::vector<at::Tensor> lo, double scale) {
   constexpr int JOBS = 64;

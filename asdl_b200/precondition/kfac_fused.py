@@ -1177,7 +1177,7 @@ class FusedKfacGradientMaker(KfacGradientMaker):
         grads = [st.module.weight.grad for st in todo]
         moved = [(v, g) for v, g in zip(group['views'], grads) if g.data_ptr() != v.data_ptr()]
         if group['parts'] is not None:
-            # the gradients are read where they lie: 94 MB of ResNet-50's are not written and read once more
+            # the gradients are read where they lie: 102 MB of ResNet-50's are not written and read once more
             ext.stage_gradients(grads, group['views'], *group['parts'], grad_scale)
         else:
             if moved:
