@@ -109,9 +109,16 @@ class FusedMaxPool2d(nn.MaxPool2d):
         return super().forward(x)
 
 
+def _native_casts(src):
+    """Whether casts of these tensors run on the library's kernels: not where the copies are differentiated, which PyTorch refuses for
+    lists of them and a kernel would drop."""
+    return (src[0].is_cuda and ops.cuda_kernels_enabled(src[0]) and ops.unobserved(*src)
+            and not (torch.is_grad_enabled() and any(t.requires_grad for t in src)))
+
+
 def _copy_all(dst, src):
     """``dst[i].copy_(src[i])``; conversions between fp32 and bf16 on the GPU in one launch."""
-    if src[0].is_cuda and ops.cuda_kernels_enabled(src[0]) and ops.unobserved(*src):
+    if _native_casts(src):
         ops.extension().cast_many(dst, src)
     else:
         torch._foreach_copy_(dst, src)
@@ -145,8 +152,7 @@ class _GroupedCast(torch.autograd.Function):
                    if _dense_meta(*ctx.meta[i]) else torch.empty(ctx.meta[i][0], device=g.device, dtype=torch.float32)
                    for i, g in present]
             same, same_dst = [], []
-            kernels = (present[0][1].is_cuda and ops.cuda_kernels_enabled(present[0][1])
-                       and ops.unobserved(*(g for _, g in present)))
+            kernels = _native_casts([g for _, g in present])
             for (i, g), d in zip(present, dst):
                 # autograd hands the weight gradient of a linear layer over as a transposed tensor: a
                 # tiled transposing cast instead of a strided element-wise copy

@@ -110,3 +110,17 @@ def test_recorded_graphs_hold_the_pooling(options):
         graph = make_fx(lambda inp: pool(inp), **options)(x[0])
         for inp in x:
             assert torch.equal(graph(inp), F.max_pool2d(inp, 3, 2, 1))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('layer,shape', [(torch.nn.Conv2d(8, 16, 3), (2, 8, 5, 5)), (torch.nn.Linear(32, 16), (4, 32))])
+def test_gradients_of_grouped_casts_are_not_differentiated_without_their_share(layer, shape):
+    """A second derivative through the casts is refused, as PyTorch refuses one of copies of tensor lists; the bias has one, and the
+    sum of both would be the bias's alone."""
+    layer = layer.to('cuda')
+    x = torch.randn(shape, device='cuda', dtype=torch.bfloat16)
+    with layers.grouped_bf16_weights(layer), torch.autocast('cuda', dtype=torch.bfloat16):
+        y = layer(x).float()
+    grads = torch.autograd.grad(y.square().sum(), (layer.weight, layer.bias), create_graph=True)
+    with pytest.raises(RuntimeError, match='_foreach_copy_'):
+        torch.autograd.grad(sum(g.sum() for g in grads), layer.weight)
