@@ -141,18 +141,18 @@ dim3 pool_grid(int width, int height, int vecs, int64_t images) {
               static_cast<unsigned>(images));
 }
 
-// The backward pass in operations of PyTorch, on its indices: for a gradient that is differentiated again, in reverse or by a tangent,
-// that is a batch (is_grads_batched) or a subclass, or while operations are recorded.
-bool needs_operations(const at::Tensor& dy) {
-  return (at::GradMode::is_enabled() && dy.requires_grad()) || c10::impl::TorchDispatchModeTLS::any_modes_set() || !values_in_memory(dy) ||
+// The backward pass in operations of PyTorch, on its indices: where it is differentiated again, by dy or (a derivative of zeros) by x, for a
+// gradient with a tangent, that is a batch (is_grads_batched) or a subclass, or while operations are recorded.
+bool needs_operations(const at::Tensor& dy, const at::Tensor& x) {
+  return (at::GradMode::is_enabled() && (dy.requires_grad() || x.requires_grad())) || c10::impl::TorchDispatchModeTLS::any_modes_set() || !values_in_memory(dy) ||
          dy._fw_grad(0).defined();
 }
-at::Tensor backward_operations(const at::Tensor& dy, const at::Tensor& code, const std::vector<int64_t>& sizes, int64_t pad) {
+at::Tensor backward_operations(const at::Tensor& dy, const at::Tensor& x, const at::Tensor& code, int64_t pad) {
   const auto place = code.view({dy.size(0), dy.size(2), dy.size(3), dy.size(1)}).permute({0, 3, 1, 2}).to(at::kLong);
   const auto options = place.options();
   const auto top = (at::arange(dy.size(2), options) * S - pad).view({-1, 1}), left = at::arange(dy.size(3), options) * S - pad;
-  const auto indices = ((place.floor_divide(K) + top) * sizes[3] + place.remainder(K) + left).masked_fill(place == 0xff, 0);
-  return at::max_pool2d_with_indices_backward(dy, at::empty(sizes, dy.options(), at::MemoryFormat::ChannelsLast), {K, K}, {S, S}, {pad, pad}, {1, 1},
+  const auto indices = ((place.floor_divide(K) + top) * x.size(3) + place.remainder(K) + left).masked_fill(place == 0xff, 0);
+  return at::max_pool2d_with_indices_backward(dy, x, {K, K}, {S, S}, {pad, pad}, {1, 1},
                                               false, indices.contiguous(at::MemoryFormat::ChannelsLast));
 }
 
@@ -166,22 +166,21 @@ struct MaxPool : torch::autograd::Function<MaxPool> {
         reinterpret_cast<const uint4*>(x.data_ptr()), reinterpret_cast<uint4*>(y.data_ptr()), reinterpret_cast<uint2*>(code.data_ptr()), s);
     B200_CUDA_CHECK(cudaGetLastError());
     count_launch();
-    ctx->save_for_backward({code});
-    ctx->saved_data["sizes"] = x.sizes().vec();
+    ctx->save_for_backward({x, code});
     ctx->saved_data["pad"] = pad;
     return y;
   }
 
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
-    const at::Tensor code = ctx->get_saved_variables()[0];
+    const auto saved = ctx->get_saved_variables();
+    const at::Tensor &x = saved[0], &code = saved[1];
     at::Tensor dy = grads[0];
-    const auto sizes = ctx->saved_data["sizes"].toIntVector();
     const int64_t pad = ctx->saved_data["pad"].toInt();
     c10::cuda::CUDAGuard guard(dy.get_device());
-    if (needs_operations(dy)) return {backward_operations(dy, code, sizes, pad), at::Tensor()};
+    if (needs_operations(dy, x)) return {backward_operations(dy, x, code, pad), at::Tensor()};
     dy = dy.contiguous(at::MemoryFormat::ChannelsLast);
     if ((reinterpret_cast<uintptr_t>(dy.data_ptr()) & 15) != 0) dy = dy.clone();   // a view into another gradient
-    auto dx = at::empty(sizes, dy.options(), at::MemoryFormat::ChannelsLast);
+    auto dx = at::empty(x.sizes(), dy.options(), at::MemoryFormat::ChannelsLast);
     const Pool s = shape(dx, pad);
     TORCH_CHECK(plain(dy) && dy.size(2) == s.oh && dy.size(3) == s.ow && code.is_cuda() && code.get_device() == dy.get_device() &&
                     code.is_contiguous() && code.numel() == dy.numel(), "dy must match the output");

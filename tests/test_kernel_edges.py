@@ -702,6 +702,21 @@ def test_max_pool_gradients_that_pytorch_has_to_look_into():
         assert torch.equal(got.primal, ref.primal) and torch.equal(got.tangent, ref.tangent)
 
 
+def test_max_pool_gradient_has_a_derivative_of_zeros_by_the_input():
+    """As nn.MaxPool2d's, also where the gradient that comes in does not require one."""
+    x = torch.randn(2, 8, 9, 9, device=DEV, generator=_gen(37)).to(torch.bfloat16).contiguous(memory_format=torch.channels_last).requires_grad_(True)
+    for y in (FusedMaxPool2d(3, stride=2, padding=1)(x), F.max_pool2d(x, 3, 2, 1)):
+        dx, = torch.autograd.grad(y.sum(), x, create_graph=True)
+        assert dx.requires_grad
+        again, = torch.autograd.grad((dx * dx).sum(), x)
+        assert torch.equal(again, torch.zeros_like(x))
+    y = FusedMaxPool2d(3, stride=2, padding=1)(x)
+    with torch.no_grad():
+        x.mul_(2)
+    with pytest.raises(RuntimeError, match='inplace'):   # the input is saved
+        y.sum().backward()
+
+
 def test_max_pool_leaves_tensors_without_memory_to_pytorch():
     from torch._subclasses.fake_tensor import FakeTensorMode
     with FakeTensorMode():
