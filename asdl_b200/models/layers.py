@@ -131,6 +131,9 @@ class _GroupedCast(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, *weights):
+        ctx.meta = [(w.shape, w.stride()) for w in weights]
+        if not ops.unobserved(*weights):   # writes into views of a buffer are more than a compiler can follow
+            return tuple(w.detach().to(torch.bfloat16) for w in weights)
         total = sum((w.numel() + 7) // 8 * 8 for w in weights)
         flat = torch.empty(total, device=weights[0].device, dtype=torch.bfloat16)
         outs, off = [], 0
@@ -140,7 +143,6 @@ class _GroupedCast(torch.autograd.Function):
             outs.append(chunk.as_strided(w.shape, w.stride()) if w.is_contiguous() or _dense(w)
                         else chunk.view(w.shape))
         _copy_all(outs, [w.detach() for w in weights])
-        ctx.meta = [(w.shape, w.stride()) for w in weights]
         return tuple(outs)
 
     @staticmethod

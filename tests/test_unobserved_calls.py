@@ -36,6 +36,26 @@ def test_casts_of_tensors_without_memory_are_left_to_pytorch(monkeypatch):
         assert all(g.dtype == torch.float32 and g.shape == s for g, s in zip(back, shapes))
 
 
+@pytest.mark.parametrize('device', ['cpu', pytest.param('cuda', marks=pytest.mark.gpu)])
+@pytest.mark.parametrize('backend', ['eager', 'aot_eager'])
+def test_grouped_casts_compile(backend, device):
+    """In a compiled call the casts are operations that the compiler can follow, with the results of the call itself."""
+    torch._dynamo.reset()
+    model = torch.nn.Sequential(torch.nn.Conv2d(8, 16, 3, bias=False), torch.nn.Flatten(), torch.nn.Linear(16 * 9, 10, bias=False))
+    model = model.to(device).to(memory_format=torch.channels_last)
+    x = torch.randn(4, 8, 5, 5, device=device).to(torch.bfloat16)
+
+    def call(inp):
+        with layers.grouped_bf16_weights(model):
+            return model(inp).float()
+
+    want, got = call(x), torch.compile(call, backend=backend)(x)
+    torch.testing.assert_close(got, want, rtol=1e-2, atol=1e-2)
+    grads = [torch.autograd.grad(y.square().sum(), list(model.parameters())) for y in (want, got)]
+    for a, b in zip(*grads):
+        assert a.dtype == b.dtype == torch.float32 and (a - b).norm() <= 2e-2 * a.norm()
+
+
 def test_tensors_without_memory_do_not_reach_a_kernel(monkeypatch):
     monkeypatch.setattr(ops, 'extension', _NoExtension)
     with FakeTensorMode(), torch.device('cuda'):
